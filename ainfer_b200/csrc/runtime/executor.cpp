@@ -714,12 +714,12 @@ int session_sample(Session *s, float temp, int top_k, float top_p, float rep_pen
   }
   if (nseen > 0) S_CHECK(ainfer_memcpy_h2d(s->dev, s->samp_seen, seen, (size_t)nseen * 4));
   S_CHECK(ainfer_memcpy_h2d(s->dev, s->samp_io, rng, 8));
-  auto it = s->kernels.find("SampleToken");
+  auto it = s->kernels.find("SampleTokenCluster");
   ainfer_kernel_t k = nullptr;
   if (it != s->kernels.end()) k = it->second;
   else {
-    if (ainfer_kernel_get(s->dev, "SampleToken", &k) != AINFER_OK) { s->err = "entry SampleToken not found"; return 1; }
-    s->kernels["SampleToken"] = k;
+    if (ainfer_kernel_get(s->dev, "SampleTokenCluster", &k) != AINFER_OK) { s->err = "entry SampleTokenCluster not found"; return 1; }
+    s->kernels["SampleTokenCluster"] = k;
   }
   const float *logits = s->Logits;
   const int32_t *dseen = s->samp_seen;
@@ -734,7 +734,7 @@ int session_sample(Session *s, float temp, int top_k, float top_p, float rep_pen
   S_CHECK(set(sizeof s->samp_mark, &s->samp_mark)); S_CHECK(set(sizeof drng, &drng)); S_CHECK(set(sizeof dtok, &dtok));
   S_CHECK(set(sizeof probs, &probs)); S_CHECK(set(sizeof ctrl, &ctrl)); S_CHECK(set(4, &v)); S_CHECK(set(4, &ns));
   S_CHECK(set(4, &temp)); S_CHECK(set(4, &tk)); S_CHECK(set(4, &top_p)); S_CHECK(set(4, &rep_penalty));
-  S_CHECK(ainfer_kernel_launch(s->dev, k, 1));
+  S_CHECK(ainfer_kernel_launch(s->dev, k, 8));
   uint64_t back[2];
   S_CHECK(ainfer_memcpy_d2h(s->dev, back, s->samp_io, 16));
   *rng = back[0];

@@ -154,3 +154,57 @@ def test_session_sampling(dev):
     assert (t_dev, r_dev) == (t_host, r_host)
     assert sess.sample(0.0)[0] == int(np.argmax(lg))
     sess.close(); model.close()
+
+
+def _kept(lg, temp, top_k, top_p):
+    """The final distribution in 64-bit numpy, and whether the top-p cut lies within rounding of a step."""
+    with np.errstate(over="ignore", invalid="ignore"):
+        p = np.exp((lg.astype(np.float64) - np.float64(lg.max())) / np.float64(np.float32(temp)))
+    p /= p.sum()
+    close = False
+    if 0 < top_k < len(p):
+        keep = np.argsort(-p, kind="stable")[:top_k]
+        q = np.zeros_like(p); q[keep] = p[keep]; p = q / q.sum()
+    if top_p < 1.0:
+        order = np.argsort(-p, kind="stable")
+        cum, want = np.cumsum(p[order]), np.float64(np.float32(top_p))
+        n = int(np.searchsorted(cum, want)) + 1
+        close = bool(np.abs(cum - want).min() < 1e-9)
+        q = np.zeros_like(p); q[order[:n]] = p[order[:n]]; p = q / q.sum()
+    return p, close
+
+
+# vocabularies around the runs of a thread (8192 threads) and what shared memory holds (20 tokens each)
+@pytest.mark.parametrize("V", [1, 7, 1023, 8191, 8192, 8193, 32000, 151936, 163840, 163841])
+@pytest.mark.parametrize("name", ["SampleToken", "SampleTokenCluster"])
+def test_filters_against_plain_numpy(dev, name, V):
+    s = DevSampler(dev, V)
+    s.k = dev.kernel(name)
+    groups = 8 if name.endswith("Cluster") else 1
+    one = s.k
+    s.k = lambda _, *a: one(groups, *a)
+    g = np.random.default_rng(V)
+    normal = (g.standard_normal(V) * 3).astype(np.float32)
+    rows = {"normal": normal, "ties": np.round(normal), "equal": np.zeros(V, np.float32),
+            "masked": np.where(g.random(V) < 0.9, np.float32(-np.inf), normal).astype(np.float32), "wide": normal * 40}
+    rows["masked"][V // 2] = 1.0
+    for kind, lg in rows.items():
+        s.set_logits(lg)
+        for temp, top_k, top_p in ((1.0, 0, 1.0), (0.8, 40, 0.95), (1.0, 1, 1.0), (1.3, V - 1, 0.5), (1e-3, 3, 0.9), (0.9, 0, 0.7), (1.0, 5, 0.0)):
+            tok, _, got = s.draw(17 + V, temp=temp, top_k=top_k, top_p=top_p, probs=True)
+            want, close = _kept(lg, temp, top_k, top_p)
+            if not close:
+                assert np.array_equal(got > 0, want.astype(np.float32) > 0), (kind, temp, top_k, top_p)
+                assert np.allclose(got, want.astype(np.float32), rtol=1e-6, atol=1e-44)   # 64-bit sums, rounded once to 32 bits (subnormal ones too)
+            assert want[tok] > 0 or close
+    if V > 8:   # an undefined logit: no order to filter by, the last token, as in the one-block form before
+        lg = normal.copy(); lg[3] = np.inf
+        s.set_logits(lg)
+        assert s.draw(5, temp=1.0, top_k=4, top_p=0.9)[0] == V - 1
+        s.set_logits(normal)
+        seen = [V - 1, 0, V // 2, 0, V, -1]
+        want = normal.copy()
+        for i in (V - 1, 0, V // 2):
+            want[i] = want[i] / np.float32(1.5) if want[i] > 0 else want[i] * np.float32(1.5)
+        _, _, got = s.draw(5, temp=1.0, rep=1.5, seen=seen, probs=True)
+        assert np.allclose(got, _kept(want, 1.0, 0, 1.0)[0], rtol=1e-6, atol=0)
