@@ -1,37 +1,36 @@
-// Int4GemmA8Tc / Int4GemmA8TcGrouped: W4A8 group-128 GEMM for batches of 1..64 activation rows
-// on the 5th-generation tensor cores (tcgen05.mma kind::i8, accumulators in tensor memory),
-// weights streamed ONCE whatever the batch. This is the batched form of the reference's Int4Gemv
-// (tools/cmdlist/kernels.cpp:148-193; sweep protocol tools/gemv/gemv.cpp:503-601): per output
-// row and batch entry, the exact int32 sum of the 128 nibble x int8 products of a group, then
-// acc = acc + ((float)sum * weight_scale) * activation_scale[g] in ascending group order. The
-// integer sums are exact on any hardware and the fp32 order is the reference's, so every batch
-// entry is bit-identical to the one-row GEMV.
+// Int4GemmA8Tc / Int4GemmA8TcGrouped: W4A8 group-128 GEMM for batches of activation rows on the
+// tensor cores. This is the batched form of the reference's Int4Gemv (tools/cmdlist/kernels.cpp:148-193;
+// sweep protocol tools/gemv/gemv.cpp:503-601): per output row and batch entry, the exact int32 sum of
+// the 128 nibble x int8 products of a group, then acc = acc + ((float)sum * weight_scale) *
+// activation_scale[g] in ascending group order. The integer sums are exact on any hardware and the
+// fp32 order is the reference's, so every batch entry is bit-identical to the one-row GEMV.
 //
 // The grouped form runs a list of problems of the same shape (N, K) in one launch: problem i has
 // its own weight matrix and its own range of activation rows (an expert and the tokens routed to
 // it). The list and its length live in device memory, so routing never goes through the host.
 //
-// One block = 256 threads = 128 weight rows x 2 halves. Thread (r, h) owns row r of the block's
-// row tile: it widens half of the row's packed bytes of a group and, in the epilogue, handles
-// half of the batch columns of accumulator lane r. Per group of 128 weights (one step):
-//   * the row tile's packed bytes arrive by cp.async, four groups (256 contiguous bytes per row)
-//     per stage, two stages; the next stage is in flight while this one is worked on;
-//   * every thread widens its 32 bytes to INT8 in shared memory in the tensor core's K-major
-//     core-matrix layout (8 rows x 16 bytes per core matrix). A nibble moved to the top of its
-//     byte is the signed byte 16 * v, so no sign fix-up is needed; the sum comes out 16 times
-//     too large and is shifted back (exact). Low and high nibbles of a word go to separate
-//     words, which permutes k inside the group; the activations are stored with the same
-//     permutation (the dot product does not care);
-//   * the batch's INT8 activations of that group (fetched into registers one step earlier) are
-//     stored next to it;
-//   * one thread issues four tcgen05.mma (M = 128 rows, N = padded batch, K = 32 each) into one
-//     of two accumulator buffers in tensor memory and commits them to an mbarrier;
-//   * while those run, all threads finish the PREVIOUS step: wait for its mbarrier, read their
-//     lane of the accumulator with tcgen05.ld, rescale and add.
-// The kernel is bound by instruction issue, not by the tensor core or by memory: the loop keeps
-// its bookkeeping in counters and per-tile records in shared memory.
-// Every wait is bounded; a wait that runs out stores a code in the host-visible fault word and
-// the kernel ends (with the tensor memory freed).
+// A block of eight warps walks units of 128 weight rows x up to NT batch entries; a warp owns 16 rows.
+// A stage is two groups of 128 weights: 128 bytes of every row (a whole line), the entries' activations
+// and both scales, copied by cp.async three to five stages deep, two blocks per SM, one block barrier a
+// stage. A lane of mma.sync.m16n8k32 (s8) takes sixteen packed bytes of a row: 32 consecutive weights,
+// widened in registers (a nibble at the top of its byte is the signed byte 16 v: no sign fix-up) and
+// put back into order, are its share of four products; the same 32 activations of an entry are the
+// other operand. The accumulators start at the bits of 1.5 x 2^23, so that a sum IS a float a
+// subtraction away (exact: 16 times a sum is below 2^22).
+//
+// Why not tcgen05 here: the fp32 rescale of every group takes the sums out of the accumulators every four
+// products, and the weights must be widened first. Both are register work: from registers to shared
+// memory, tensor memory and back costs more than the products. A form with tcgen05.mma kind::i8 and
+// warps for copying, widening, issuing and rescaling took 0.7 us a group of a 128 x 16 unit and 2.1 us
+// of 128 x 96 (each hand-over is a fence and a barrier's latency); at 2048 multiply-adds a cycle and SM
+// mma.sync needs 0.07 us per 16 entries, and the weight stream 0.1 us.
+// Bound by the weight stream up to about 24 entries a unit, above by mma.sync.
+// Measured, us (before: tcgen05 with two block barriers a group, 64 entries a launch; the experts' lists up to
+// 8 rows by the dp4a form):
+//   8192 x 2048, 64 / 704 entries      33.8 -> 10.4, 365 -> 68      4096 x 2048, 64   33.2 -> 9.9
+//   2048 x 4096, 64                    61.8 -> 13.3                 151936 x 2048, 64  286 -> 98
+//   experts of 512, gate and up, 1.25 / 3.75 / 13.7 rows on average   136 -> 107, 277 -> 148, 793 -> 174
+//   the same, down                                                     85 -> 72, 173 -> 101, 430 -> 113
 #include "block_dot.cuh"
 
 namespace ainfer {
@@ -50,7 +49,7 @@ struct TcGroup {
   const uint8_t *P;    // packed nibbles [N][K/2]
   const uint16_t *S;   // bf16 scales [N][K/128]
   int32_t x_row0;      // first activation / output row
-  int32_t M;           // rows (1..64)
+  int32_t M;           // rows (1..max_m)
   int32_t y_col;       // first output column
   int32_t pad;
 };
@@ -61,416 +60,316 @@ struct Int4GemmA8TcGroupedArgs {
   const int8_t *XQ;            // [rows][K]
   const float *SQ;             // [rows][K/128]
   float *Y;                    // [rows][ldy]
-  int32_t N, K, max_m, ldy;    // max_m: upper bound of every problem's M (sizes shared memory)
+  int32_t N, K, max_m, ldy;    // max_m: upper bound of every problem's M, at most 64
 };
 
-constexpr int kTcRows = 128;               // weight rows per block tile = accumulator lanes
+constexpr int kTcRows = 128;               // weight rows per unit
 constexpr int kTcThreads = 256;
-constexpr int kTcMaxBatch = 64;
-constexpr int kTcABytes = kTcRows * 128;   // one group of 128 rows as INT8
-constexpr uint32_t kTcSpin = 1u << 22;
+constexpr int kTcSms = 148;
+constexpr uint32_t kTcWBytes = kTcRows * 128;   // a stage's packed weights: two groups
+constexpr uint32_t kTcXPitch = 272;             // bytes between entries of a stage: 256 + 16, so that reads down the entries meet all banks
 
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_byte_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  // shared-memory matrix descriptor, no swizzle, K-major: start address, leading-dimension
-  // byte offset (between the two 16-byte K chunks of one MMA), stride byte offset (between
-  // 8-row core matrices), all in units of 16 bytes; descriptor version 1.
-  return (uint64_t)((smem_byte_addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+__device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
+__device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, int32_t (&v)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-               : "r"(taddr)
-               : "memory");
+__device__ __forceinline__ void cp_async4(uint32_t dst_smem, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst_smem), "l"(src) : "memory");
 }
-
-#ifndef TC_STAMP
-#define TC_STAMP(id)   // stand-alone timing builds record a clock here
-#define TC_STAMP_DECL
-#endif
 
 extern __shared__ __align__(128) unsigned char tc_smem[];
 
-__device__ __forceinline__ void cp_async16(void *dst_smem, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst_smem)), "l"(src) : "memory");
+// Stages that two blocks per SM have room for. A stage: weights | activations | activation scales [2][NT] | weight scales [128][2].
+__host__ __device__ constexpr int tc_stages(int nt) { return nt == 16 ? 5 : nt == 32 ? 4 : 3; }
+__host__ __device__ constexpr uint32_t tc_stage_bytes(int nt) { return kTcWBytes + (uint32_t)nt * kTcXPitch + (uint32_t)nt * 8u + kTcRows * 4u; }
+// Entries per unit of one problem: what finishes first over whole rounds of units on the SMs. A stage costs
+// the products of its entries, and the widening and copying whatever their number.
+__host__ __device__ inline int tc_entries(int N, int M) {
+  const int tiles = (N + kTcRows - 1) / kTcRows;
+  int best = 16;
+  long cost = -1;
+  for (int nt = 16; nt <= 64; nt *= 2) {
+    const long rounds = ((long)tiles * ((M + nt - 1) / nt) + 2 * kTcSms - 1) / (2 * kTcSms), c = rounds * (nt + 12);
+    if (cost < 0 || c < cost) { cost = c; best = nt; }
+    if (nt >= M) break;
+  }
+  return best;
 }
-__device__ __forceinline__ void cp_async4(void *dst_smem, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst_smem)), "l"(src) : "memory");
-}
-
-// A row tile of a problem, as the block's loop needs it (kept in a ring of eight in shared memory).
-struct TcTile {
-  const uint8_t *P;    // first packed row of the tile
-  const uint16_t *S;   // scales of the problem's row 0
-  int32_t x_row0, M, y_col, row0;
-};
-static_assert(sizeof(TcTile) == 32, "ring slot");
+__host__ __device__ inline int tc_entries_grouped(int max_m) { return max_m <= 16 ? 16 : max_m <= 32 ? 32 : 64; }
 
 struct TcShape {
   const TcGroup *groups;   // null: the one problem `single`
+  const int32_t *ngroups;
   TcGroup single;
   const int8_t *XQ;
   const float *SQ;
   float *Y;
-  int32_t N, K, ldy, max_m, ntiles;
+  int32_t N, K, ldy;
+};
+struct TcUnit {
+  const uint8_t *P;        // of the problem's row 0
+  const uint16_t *S;
+  int32_t x0, M, y_col, row0;
 };
 
-__host__ __device__ inline uint32_t tc_npad(uint32_t M) { return M <= 8u ? 8u : ((M + 15u) & ~15u); }
-// Buffers of per-tile scales. A step is finished two steps after it was staged, so a tile's scales
-// are still read during the first two steps that follow it, while the scales of later tiles
-// already arrive (with the first stage of their weights, one stage ahead).
-__host__ __device__ inline uint32_t tc_nsc(uint32_t G) { return G == 1 ? 4u : ((G & 3u) == 0 && G >= 8 ? 2u : 3u); }
-__host__ __device__ inline uint32_t tc_gps(uint32_t G) { return (G & 3u) == 0 ? 4u : ((G & 1u) == 0 ? 2u : 1u); }
-// Shared-memory map: the ring of tile records, two stages of packed weights [128 rows][gps * 64 B] (16-byte pieces of a row
-// swizzled by the row number, so that the row owners' reads spread over the banks), A (INT8
-// weights) [2][8 chunks][16 row blocks][8 rows][16 B], B (INT8 activations) [2][8 chunks]
-// [Npad/8 blocks][8 rows][16 B], per tile the activation scales [max_m][G] fp32 and the row
-// tile's weight scales [128][G] bf16 (two to four buffers of each, see tc_nsc). gps (4, 2 or 1, dividing G) groups travel together: consecutive
-// threads copy consecutive 16-byte pieces of the same row, so a warp's copy instruction reads
-// rows of 256 contiguous bytes (one 64-byte piece from each of 32 rows left HBM at well under
-// half its rate).
-__host__ __device__ inline uint32_t tc_smem_bytes(uint32_t K, uint32_t max_m) {
-  const uint32_t G = K >> 7, gps = tc_gps(G), npad = tc_npad(max_m);
-  const uint32_t nsc = tc_nsc(G);
-  return 2 * kTcRows * gps * 64 + 2 * kTcABytes + 2 * 8 * npad * 16 + nsc * max_m * G * 4 + nsc * kTcRows * G * 2 +
-         8 * (uint32_t)sizeof(TcTile);
+// One block of eight entries: the four products of a group, then rescale and add.
+struct TcScales { float r0, r1; };   // a sixteenth of the weight scales of a lane's rows
+__device__ __forceinline__ void tc_products(int (&d)[4], const uint32_t (&a)[4][4], const uint4 &x0, const uint4 &x1) {
+  d[0] = d[1] = d[2] = d[3] = 0x4B400000;   // 1.5 x 2^23 as a float
+  mma_s8(d, a[0], x0.x, x0.y);
+  mma_s8(d, a[1], x0.z, x0.w);
+  mma_s8(d, a[2], x1.x, x1.y);
+  mma_s8(d, a[3], x1.z, x1.w);
+}
+__device__ __forceinline__ void tc_finish(float (&acc)[4], const int (&d)[4], TcScales c, float2 q) {
+  acc[0] = acc[0] + ((__int_as_float(d[0]) - 12582912.0f) * c.r0) * q.x;
+  acc[1] = acc[1] + ((__int_as_float(d[1]) - 12582912.0f) * c.r0) * q.y;
+  acc[2] = acc[2] + ((__int_as_float(d[2]) - 12582912.0f) * c.r1) * q.x;
+  acc[3] = acc[3] + ((__int_as_float(d[3]) - 12582912.0f) * c.r1) * q.y;
 }
 
+template <int NT>
 __device__ __forceinline__ void tc_body(const TcShape &c) {
-  __shared__ unsigned long long mma_bar[3];
-  __shared__ uint32_t tmem_base_s;
-  __shared__ uint32_t s_fail;
-  const int tid = threadIdx.x, warp = tid >> 5, r = tid & 127, h = tid >> 7;
-  TC_STAMP_DECL;
+  constexpr int ST = tc_stages(NT);
+  constexpr uint32_t SB = tc_stage_bytes(NT), XO = kTcWBytes, QO = XO + NT * kTcXPitch, CO = QO + NT * 8;
+  __shared__ TcUnit ring[8];   // units between the copies and the products (at most ST - 1 apart)
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int K = c.K, G = K >> 7;
-  const int gps = (int)tc_gps((uint32_t)G), QT = G / gps;     // groups per stage, stages per row tile
-  const int ppr = gps * 4, lg_ppr = 31 - __clz(ppr);           // 16-byte pieces per row and stage
-  const int npad_max = (int)tc_npad((uint32_t)c.max_m);
-  const uint32_t w_stage = (uint32_t)kTcRows * (uint32_t)gps * 64u, b_bytes = 8u * (uint32_t)npad_max * 16u;
-  TcTile *ring = reinterpret_cast<TcTile *>(tc_smem);                    // [8]
-  unsigned char *Wst = tc_smem + 8 * sizeof(TcTile);
-  unsigned char *Abuf = Wst + 2 * w_stage;
-  unsigned char *Bbuf = Abuf + 2 * kTcABytes;
-  const int nsc = (int)tc_nsc((uint32_t)G);                              // scale buffers (tile number mod nsc)
-  const int sq_stride = c.max_m * G, sc_stride = kTcRows * G;
-  float *sqs = reinterpret_cast<float *>(Bbuf + 2 * b_bytes);            // [nsc][max_m * G]
-  uint16_t *ssc = reinterpret_cast<uint16_t *>(sqs + nsc * sq_stride);   // [nsc][128][G]
-  uint32_t tmem_cols = 32;
-  while (tmem_cols < 3u * (uint32_t)npad_max) tmem_cols <<= 1;
-  const int tpg = (c.N + kTcRows - 1) / kTcRows;   // row tiles per problem
   const size_t row_bytes = (size_t)(K >> 1);
-  const int ntiles = c.ntiles, stride = (int)gridDim.x;
-
-  // record of the block's n-th tile (global tile blockIdx.x + n * gridDim.x), from a problem record
-  auto make_tile = [&](int t, const TcGroup &g) {
-    const int rt = t % tpg;
-    TcTile ti;
-    ti.P = g.P + (size_t)rt * kTcRows * row_bytes;
-    ti.S = g.S;
-    ti.x_row0 = g.x_row0; ti.M = g.M; ti.y_col = g.y_col; ti.row0 = rt * kTcRows;
-    return ti;
-  };
-  auto load_group = [&](int t) {   // t < ntiles
-    if (!c.groups) return c.single;
-    const uint4 *p = reinterpret_cast<const uint4 *>(c.groups + t / tpg);
-    union { uint4 q[2]; TcGroup g; } u;
-    u.q[0] = __ldg(p); u.q[1] = __ldg(p + 1);
-    return u.g;
-  };
-
-  if (tid == 0) {
-    mbar_init(&mma_bar[0], 1);
-    mbar_init(&mma_bar[1], 1);
-    mbar_init(&mma_bar[2], 1);
-    s_fail = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int n = 0; n < 2; ++n) {
-      const int t = (int)blockIdx.x + n * stride;
-      if (t < ntiles) ring[n] = make_tile(t, load_group(t));
-    }
-  }
-  if (warp == 0) {  // tensor memory: three accumulator buffers of npad_max columns
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_s)), "r"(tmem_cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_base_s;
-  const uint32_t a_addr = smem_addr(Abuf), b_addr = smem_addr(Bbuf);
-  uint32_t phases = 0u;  // bit s: parity of the next completion of accumulator buffer s's barrier
-
-  // thread 0 keeps the problem record of the tile after next in flight
-  TcGroup pend = c.single;
-  if (tid == 0 && (int)blockIdx.x + 2 * stride < ntiles) pend = load_group((int)blockIdx.x + 2 * stride);
-
-  const bool sc_smem = (G & 1) == 0 && G <= 64;   // else the epilogue reads the scales from global memory
-  const int f_pc = tid & (ppr - 1), f_r0 = tid >> lg_ppr, f_rstep = kTcThreads >> lg_ppr;  // this thread's piece and rows in a fetch
-  // stage (n-th tile, quad q) into buffer `stage`; an empty commit when the block has no such tile
-  auto fetch = [&](int n, int sb, int q, int stage) {   // sb: scale buffer of tile n
-    if ((int)blockIdx.x + n * stride < ntiles) {
-      const TcTile &ti = ring[n & 7];
-      unsigned char *wd = Wst + stage * w_stage;
-      const int rlast = c.N - 1 - ti.row0;   // rows past the end repeat the last row (never stored)
-      const uint8_t *src0 = ti.P + (size_t)q * (gps * 64) + f_pc * 16;
-#pragma unroll 4
-      for (int rr = f_r0; rr < kTcRows; rr += f_rstep) {
-        const int rs = rr < rlast ? rr : rlast;
-        cp_async16(wd + rr * (gps * 64) + ((f_pc ^ (rr & (ppr - 1))) << 4), src0 + (size_t)rs * row_bytes);
-      }
-      if (q == 0) {   // the tile's activation scales [M][G] and the rows' weight scales [128][G]
-        float *sd = sqs + sb * sq_stride;
-        const float *ss = c.SQ + (size_t)ti.x_row0 * G;
-        for (int i = tid; i < ti.M * G; i += kTcThreads) cp_async4(sd + i, ss + i);
-        if (sc_smem) {
-          // pairs of bf16 scales; a row's G scales are contiguous, and so are the tile's rows
-          const int nrows = rlast + 1 < kTcRows ? rlast + 1 : kTcRows;
-          const uint32_t *sw = reinterpret_cast<const uint32_t *>(ti.S + (size_t)ti.row0 * G);
-          uint32_t *dw = reinterpret_cast<uint32_t *>(ssc + sb * sc_stride);
-          for (int i = tid; i < nrows * G / 2; i += kTcThreads) cp_async4(dw + i, sw + i);
-        }
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // activations of (n-th tile, group g) as 16-byte pieces [m][8]: a thread's first and second piece
-  const int x_src0 = (tid >> 3) * K + (tid & 7) * 16, x_src1 = x_src0 + (kTcThreads >> 3) * K;   // batch entry tid / 8 (+ 32), piece tid % 8
-  const int x_dst0 = (tid >> 6) * 128 + ((tid >> 3) & 7) * 16, x_dst1 = x_dst0 + (kTcThreads >> 6) * 128;
-  auto load_x = [&](int n, int g, uint4 (&x)[2]) {
-    if ((int)blockIdx.x + n * stride < ntiles) {
-      const TcTile &ti = ring[n & 7];
-      const int8_t *xb = c.XQ + (size_t)ti.x_row0 * K + g * 128;
-      if (tid < ti.M * 8) x[0] = __ldg(reinterpret_cast<const uint4 *>(xb + x_src0));
-      if (tid + kTcThreads < ti.M * 8) x[1] = __ldg(reinterpret_cast<const uint4 *>(xb + x_src1));
+  const int tpg = (c.N + kTcRows - 1) / kTcRows;      // row tiles per problem
+  const int nrb = (c.single.M + NT - 1) / NT;         // blocks of entries of the one problem
+  const int stride = (int)gridDim.x;
+  const uint32_t base = smem_addr(tc_smem);
+  if (c.groups) pdl_wait();
+  const int units = c.groups ? __ldcg(c.ngroups) * tpg : tpg * nrb;
+  // ---- copies: this thread's sources of the next stage; rows and entries that do not exist keep what is there (never stored) ----
+  const bool pair_scales = (G & 1) == 0;
+  const int wr = warp * 16 + (lane >> 3), wpc = lane & 7;   // weights: eight neighbours copy a row's line, four rows apart
+  const int xm = tid >> 4, xpc = tid & 15;                  // activations: sixteen neighbours copy an entry's 256 bytes
+  const uint32_t wdst = (uint32_t)wr * 128u + (uint32_t)((wpc ^ ((wr & 1) << 2)) << 4);   // odd rows' halves change places (bank-conflict free reads)
+  const uint32_t xdst = XO + (uint32_t)xm * kTcXPitch + (uint32_t)xpc * 16u;
+  const uint8_t *wp = nullptr;
+  const int8_t *xp = nullptr;
+  const char *sp_src = nullptr;                             // of a scale (activation: threads below 2 NT, weight pairs: from 128 on)
+  uint32_t wmask = 0, xmask = 0, smask = 0, sdst = 0;
+  int lu = blockIdx.x, lg = 0, ls = 0, lk = 0;              // unit, first group, buffer, units begun
+  uint4 rec[2];
+  auto load_rec = [&](int u) {
+    if (c.groups && u < units) {
+      const uint4 *p = reinterpret_cast<const uint4 *>(c.groups + u / tpg);
+      rec[0] = __ldcg(p); rec[1] = __ldcg(p + 1);
     }
   };
-  float acc[kTcMaxBatch / 2];   // batch entry m = 8 * i + 4 * h + j lives in acc[4 * i + j]
+  auto begin_unit = [&]() {   // lu < units; its record is in rec
+    TcUnit n;
+    if (c.groups) {
+      union { uint4 q[2]; TcGroup g; } r;
+      r.q[0] = rec[0]; r.q[1] = rec[1];
+      n.P = r.g.P; n.S = r.g.S; n.x0 = r.g.x_row0; n.M = min(r.g.M, NT); n.y_col = r.g.y_col; n.row0 = (lu % tpg) * kTcRows;
+    } else {
+      const int rb = lu % nrb;
+      n.P = c.single.P; n.S = c.single.S; n.x0 = rb * NT; n.M = min(NT, c.single.M - n.x0); n.y_col = 0; n.row0 = (lu / nrb) * kTcRows;
+    }
+    if (tid == 0) ring[lk & 7] = n;
+    ++lk;
+    const int rows = c.N - n.row0;
+    wp = n.P + (size_t)(n.row0 + wr) * row_bytes + wpc * 16;
+    xp = c.XQ + (size_t)(n.x0 + xm) * K + xpc * 16;
+    wmask = xmask = 0;
 #pragma unroll
-  for (int m = 0; m < kTcMaxBatch / 2; ++m) acc[m] = 0.0f;
-  uint4 xr[2], xn[2];
-  xr[0] = xr[1] = xn[0] = xn[1] = make_uint4(0, 0, 0, 0);
-  fetch(0, 0, 0, 0);
-  load_x(0, 0, xr);
-
-  int n = 0, q = 0, gl = 0, g = 0;   // tile of the block, stage of the tile, group of the stage / of the tile
-  int stage = 0;                      // buffer of the stage being worked on
-  int buf = 0;                        // accumulator / staging buffer of the step being staged
-  bool live = (int)blockIdx.x < ntiles;
-  // Steps whose products are in flight (at most two): a step is finished two steps after it was
-  // staged, so that neither the issue of its products nor their latency is waited for.
-  int pending = 0, p1_g = 0, p1_n = 0, p1_sb = 0, p2_g = 0, p2_n = 0, p2_sb = 0;   // p1: the last step, p2: the one before
-  int tb = 0, eb = 0;                    // accumulator buffer of the step being staged / of the oldest pending step
-  int sb_cur = 0, sb_next = 1;           // scale buffers of the current / next tile
+    for (int i = 0; i < 4; ++i) wmask |= (wr + 4 * i < rows ? 1u : 0u) << i;
+#pragma unroll
+    for (int i = 0; i < NT / 16; ++i) xmask |= (xm + 16 * i < n.M ? 1u : 0u) << i;
+    smask = 0;
+    if (tid < 2 * NT) {
+      const int m = tid >> 1, k = tid & 1;
+      sp_src = reinterpret_cast<const char *>(c.SQ + (size_t)(n.x0 + m) * G + k);
+      sdst = QO + (uint32_t)(k * NT + m) * 4u;
+      smask = m < n.M ? 1u + (uint32_t)k : 0u;
+    } else if (tid >= 128 && pair_scales) {
+      const int r = tid - 128;
+      sp_src = reinterpret_cast<const char *>(n.S + (size_t)(n.row0 + r) * G);
+      sdst = CO + (uint32_t)r * 4u;
+      smask = r < rows ? 1u : 0u;
+    }
+    load_rec(lu + stride);
+  };
+  auto copy_w = [&]() {
+    if (wpc < 4 * (G - lg)) {
+      const uint32_t dst = base + (uint32_t)ls * SB + wdst;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (wmask >> i & 1u) cp_async16(dst + (uint32_t)i * 512u, wp + (size_t)(4 * i) * row_bytes);
+    }
+  };
+  auto copy_x = [&]() {
+    const uint32_t dst = base + (uint32_t)ls * SB;
+    if (xpc < 8 * (G - lg)) {
+#pragma unroll
+      for (int i = 0; i < NT / 16; ++i)
+        if (xmask >> i & 1u) cp_async16(dst + xdst + (uint32_t)(16 * i) * kTcXPitch, xp + (size_t)(16 * i) * K);
+    }
+    if (smask && (int)smask <= G - lg) cp_async4(dst + sdst, sp_src);
+  };
+  auto advance = [&]() {
+    wp += 128;
+    xp += 256;
+    sp_src += tid < 2 * NT ? 8 : 4;
+    ls = ls == ST - 1 ? 0 : ls + 1;
+    if ((lg += 2) >= G) {
+      lg = 0;
+      lu += stride;
+      if (lu < units) begin_unit();
+    }
+  };
+  auto commit = []() { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  load_rec(lu);
+  if (lu < units) begin_unit();
+  if (c.groups) {
 #pragma unroll 1
-  while (live || pending) {
-    TC_STAMP(1);
-    const bool do_epi = live ? pending == 2 : pending > 0;
-    const int e_g = pending == 2 ? p2_g : p1_g, e_n = pending == 2 ? p2_n : p1_n, e_sb = pending == 2 ? p2_sb : p1_sb;
-    if (do_epi) {
-      // the oldest pending step's products are complete: its accumulators can be read, and the
-      // staging buffer it read (the one this step writes) is free
-      const uint32_t par = (phases >> eb) & 1u;
-      bool ok = mbar_try(&mma_bar[eb], par);
-      for (uint32_t it = 0; !ok && it < kTcSpin && !*reinterpret_cast<volatile uint32_t *>(&s_fail); ++it) ok = mbar_try(&mma_bar[eb], par);
-      if (!ok) {
-        s_fail = 1;
-        if (g_stream_fault_word) *reinterpret_cast<volatile unsigned int *>(g_stream_fault_word) = 1;
-      }
-      phases ^= 1u << eb;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    for (int i = 0; i < ST - 1; ++i) {
+      if (lu < units) { copy_w(); copy_x(); advance(); }
+      commit();
     }
-    if (live) {
-      if (__builtin_expect(gl == 0, 0)) {
-        // stage boundary: start the next stage (the next quad of this tile, or the first of the
-        // block's next tile), then wait for this one
-        const bool last_q = q + 1 == QT;
-        fetch(last_q ? n + 1 : n, last_q ? sb_next : sb_cur, last_q ? 0 : q + 1, stage ^ 1);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();  // every thread's copies of this stage have landed
-        if (g == 0 && tid == 0) {
-          // tile boundary: publish the record of the tile after next, fetch the one after that
-          const int t2 = (int)blockIdx.x + (n + 2) * stride, t3 = t2 + stride;
-          if (t2 < ntiles) ring[(n + 2) & 7] = make_tile(t2, pend);
-          if (t3 < ntiles) pend = load_group(t3);
-        }
-      }
-      TC_STAMP(2);
-      const TcTile &ti = ring[n & 7];
-      const int M = ti.M, npad = (int)tc_npad((uint32_t)M);
-      const uint32_t b_chunk = (uint32_t)npad * 16u;
-      // the next step's activations (same tile, or the first group of the block's next tile)
-      if (g + 1 < G) load_x(n, g + 1, xn); else load_x(n + 1, 0, xn);
-      // ---- stage this step: half of the row's 128 weights as INT8 (16 * v), and the batch's activations ----
-      {
-        const unsigned char *wrow = Wst + stage * w_stage + r * (gps * 64);
-        unsigned char *ab = Abuf + buf * kTcABytes + (r >> 3) * 128 + (r & 7) * 16;
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int jj = 2 * h + u;
-          const uint4 cur = *reinterpret_cast<const uint4 *>(wrow + (((gl * 4 + jj) ^ (r & (ppr - 1))) << 4));
-          // packed words (x, y) -> chunk 2jj, (z, w) -> chunk 2jj + 1: [low nibbles, high nibbles] per word
-          const uint4 c0 = make_uint4((cur.x << 4) & 0xF0F0F0F0u, cur.x & 0xF0F0F0F0u, (cur.y << 4) & 0xF0F0F0F0u, cur.y & 0xF0F0F0F0u);
-          const uint4 c1 = make_uint4((cur.z << 4) & 0xF0F0F0F0u, cur.z & 0xF0F0F0F0u, (cur.w << 4) & 0xF0F0F0F0u, cur.w & 0xF0F0F0F0u);
-          *reinterpret_cast<uint4 *>(ab + (2 * jj) * 2048) = c0;
-          *reinterpret_cast<uint4 *>(ab + (2 * jj + 1) * 2048) = c1;
-        }
-        unsigned char *bb = Bbuf + buf * b_bytes + (tid & 7) * b_chunk;
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (tid + u * kTcThreads < M * 8) {
-            const uint4 v = xr[u];
-            const uint4 pp = make_uint4(__byte_perm(v.x, v.y, 0x6420), __byte_perm(v.x, v.y, 0x7531), __byte_perm(v.z, v.w, 0x6420),
-                                        __byte_perm(v.z, v.w, 0x7531));
-            *reinterpret_cast<uint4 *>(bb + (u ? x_dst1 : x_dst0)) = pp;
-          }
-        }
-      }
+  } else {   // the one problem's weights travel before the predecessor is done
+#pragma unroll 1
+    for (int i = 0; i < ST - 1 && lu < units; ++i) { copy_w(); advance(); }
+    pdl_wait();
+    lu = blockIdx.x; lg = 0; ls = 0; lk = 0;
+    if (lu < units) begin_unit();
+#pragma unroll 1
+    for (int i = 0; i < ST - 1; ++i) {
+      if (lu < units) { copy_x(); advance(); }
+      commit();
     }
-    TC_STAMP(3);
-    // generic-proxy writes -> visible to the tensor core's reads, then everyone has written
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    TC_STAMP(4);
-    if (live && tid == 0) {
-      const int npad = (int)tc_npad((uint32_t)ring[n & 7].M);
-      const uint32_t b_chunk = (uint32_t)npad * 16u;
-      // instruction descriptor: D = S32, A = B = signed 8 bit, both K-major, N = npad, M = 128
-      const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
-      const uint32_t d = tmem_base + (uint32_t)tb * (uint32_t)npad_max;
-      // the four products differ only in the start addresses (low bits of the descriptors, in 16-byte units)
-      const uint64_t da = umma_desc(a_addr + buf * kTcABytes, 2048u, 128u);
-      const uint64_t db = umma_desc(b_addr + buf * b_bytes, b_chunk, 128u);
+  }
+  // ---- products ----
+  float acc[NT / 8][4];
 #pragma unroll
-      for (int qq = 0; qq < 4; ++qq)
-        umma_i8(d, da + (uint64_t)(qq * (4096 >> 4)), db + (uint64_t)(qq * ((2 * b_chunk) >> 4)), idesc, qq > 0 ? 1u : 0u);
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&mma_bar[tb]))
-                   : "memory");
-    }
-    TC_STAMP(5);
-    if (do_epi) {
-      // ---- finish the oldest pending step (group e_g of tile e_n) ----
-      // everything that does not depend on the products first: the row's weight scale of the
-      // group and the first activation scales
-      const TcTile &pt = ring[e_n & 7];
-      const int pM = pt.M;
-      float sc;
-      if (sc_smem) {
-        sc = bf16_to_f32(ssc[e_sb * sc_stride + r * G + e_g]);
+  for (int j = 0; j < NT / 8; ++j)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[j][q] = 0.0f;
+  const int r0 = warp * 16 + g;
+  int cs = 0, ck = 0;
+#pragma unroll 1
+  for (int u = blockIdx.x; u < units; u += stride, ++ck) {
+    int nb = 0;
+#pragma unroll 1
+    for (int g0 = 0; g0 < G; g0 += 2) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+      __syncthreads();   // every thread's copies of this stage have landed; the last stage's readers are done
+      if (lu < units) { copy_w(); copy_x(); advance(); }
+      commit();
+      const TcUnit &n = ring[ck & 7];
+      if (g0 == 0) nb = (n.M + 7) >> 3;
+      const uint32_t sb = base + (uint32_t)cs * SB;
+      const unsigned char *sp = tc_smem + (uint32_t)cs * SB;
+      uint32_t s0, s1;   // scales of rows r0 and r0 + 8 (two groups each)
+      const int ng = min(2, G - g0);
+      if (pair_scales) {
+        s0 = *reinterpret_cast<const uint32_t *>(sp + CO + r0 * 4);
+        s1 = *reinterpret_cast<const uint32_t *>(sp + CO + (r0 + 8) * 4);
       } else {
-        const int prow = pt.row0 + r < c.N ? pt.row0 + r : c.N - 1;
-        sc = bf16_to_f32(__ldg(pt.S + (size_t)prow * G + e_g));
+        const uint16_t *w0 = n.S + (size_t)min(n.row0 + r0, c.N - 1) * G + g0, *w1 = n.S + (size_t)min(n.row0 + r0 + 8, c.N - 1) * G + g0;
+        s0 = __ldg(w0) | (uint32_t)__ldg(w0 + ng - 1) << 16;
+        s1 = __ldg(w1) | (uint32_t)__ldg(w1 + ng - 1) << 16;
       }
-      const float *sqg = sqs + e_sb * sq_stride + (4 * h) * G + e_g;   // this half's first batch entry
-      float sq0[4];
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) sq0[jj] = 4 * h + jj < pM ? sqg[jj * G] : 0.0f;
-      const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)eb * (uint32_t)npad_max + (uint32_t)(4 * h);
-      if (4 * h < pM) {   // uniform across the warp
-        int32_t v[4];
-        TC_STAMP(8);
-        tmem_ld4(taddr, v);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        TC_STAMP(9);
+      for (int gl = 0; gl < 2; ++gl) {
+        if (gl >= ng) break;
+        uint32_t a[4][4];   // of product s: row r0, row r0 + 8, then their next four weights
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) acc[jj] = acc[jj] + ((float)(v[jj] >> 4) * sc) * sq0[jj];   // entries past M: never stored
-      }
-      if (8 + 4 * h < pM) {
+        for (int h = 0; h < 2; ++h) {
+          const uint4 p = lds128(sb + (uint32_t)(r0 + 8 * h) * 128u + (uint32_t)(((gl * 4 + t) ^ ((g & 1) << 2)) << 4));
+          const uint32_t w[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
-        for (int i = 1; i < kTcMaxBatch / 8; ++i) {
-          const int m0 = 8 * i + 4 * h;
-          if (m0 < pM) {
-            float sqv[4];
+          for (int s = 0; s < 4; ++s) {   // low and high nibbles alternate
+            const uint32_t lo = (w[s] << 4) & 0xF0F0F0F0u, hi = w[s] & 0xF0F0F0F0u;
+            a[s][h] = __byte_perm(lo, hi, 0x5140);
+            a[s][2 + h] = __byte_perm(lo, hi, 0x7362);
+          }
+        }
+        TcScales sc;
+        sc.r0 = __uint_as_float(gl ? s0 & 0xFFFF0000u : s0 << 16) * 0.0625f;
+        sc.r1 = __uint_as_float(gl ? s1 & 0xFFFF0000u : s1 << 16) * 0.0625f;
+        const uint32_t xb = sb + XO + (uint32_t)g * kTcXPitch + (uint32_t)(gl * 128 + t * 32);
+        const float *sq = reinterpret_cast<const float *>(sp + QO) + gl * NT + 2 * t;
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) sqv[jj] = m0 + jj < pM ? sqg[(8 * i + jj) * G] : 0.0f;
-            int32_t v[4];
-            tmem_ld4(taddr + (uint32_t)(8 * i), v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) acc[4 * i + jj] = acc[4 * i + jj] + ((float)(v[jj] >> 4) * sc) * sqv[jj];
+        for (int j = 0; j < NT / 8; j += 2) {
+          if (j + 1 < nb) {   // two blocks side by side: their products are chains of four
+            const uint32_t xj = xb + (uint32_t)j * 8u * kTcXPitch;
+            const uint4 x0 = lds128(xj), x1 = lds128(xj + 16u), x2 = lds128(xj + 8u * kTcXPitch), x3 = lds128(xj + 8u * kTcXPitch + 16u);
+            const float2 q0 = *reinterpret_cast<const float2 *>(sq + 8 * j), q1 = *reinterpret_cast<const float2 *>(sq + 8 * j + 8);
+            int d0[4], d1[4];
+            tc_products(d0, a, x0, x1);
+            tc_products(d1, a, x2, x3);
+            tc_finish(acc[j], d0, sc, q0);
+            tc_finish(acc[j + 1], d1, sc, q1);
+          } else if (j < nb) {
+            const uint32_t xj = xb + (uint32_t)j * 8u * kTcXPitch;
+            const uint4 x0 = lds128(xj), x1 = lds128(xj + 16u);
+            const float2 q0 = *reinterpret_cast<const float2 *>(sq + 8 * j);
+            int d0[4];
+            tc_products(d0, a, x0, x1);
+            tc_finish(acc[j], d0, sc, q0);
           }
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      TC_STAMP(7);
-      if (__builtin_expect(e_g == G - 1, 0)) {
-        // the row tile is complete: store it, start the next one from zero, and switch to the
-        // next tile's scales (prefetched when this tile began)
-        const bool in_range = pt.row0 + r < c.N;
-        float *yb = c.Y + (size_t)pt.x_row0 * c.ldy + pt.y_col + pt.row0 + r;
-#pragma unroll
-        for (int i = 0; i < kTcMaxBatch / 8; ++i)
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const int m = 8 * i + 4 * h + jj;
-            if (m < pM && in_range) yb[(size_t)m * c.ldy] = acc[4 * i + jj];
-            acc[4 * i + jj] = 0.0f;
-          }
-      }
+      cs = cs == ST - 1 ? 0 : cs + 1;
     }
-    if (do_epi) {
-      --pending;
-      eb = eb == 2 ? 0 : eb + 1;
-    }
-    if (live) {
-      p2_g = p1_g; p2_n = p1_n; p2_sb = p1_sb;
-      p1_g = g; p1_n = n; p1_sb = sb_cur;
-      ++pending;
-      tb = tb == 2 ? 0 : tb + 1;
-      buf ^= 1;
-      xr[0] = xn[0]; xr[1] = xn[1];
-      ++g; ++gl;
-      if (gl == gps) { gl = 0; ++q; stage ^= 1; }
-      if (g == G) {
-        g = 0; q = 0; ++n;
-        sb_cur = sb_next;
-        sb_next = sb_next + 1 == nsc ? 0 : sb_next + 1;
-        live = (int)blockIdx.x + n * stride < ntiles;
+    const TcUnit &n = ring[ck & 7];
+    float *y = c.Y + (size_t)n.x0 * c.ldy + n.y_col + n.row0 + r0;
+    const bool in0 = n.row0 + r0 < c.N, in1 = n.row0 + r0 + 8 < c.N;
+    const int M = n.M;
+#pragma unroll
+    for (int j = 0; j < NT / 8; ++j) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int m = 8 * j + 2 * t + (q & 1);
+        if (m < M && (q < 2 ? in0 : in1)) y[(size_t)m * c.ldy + (q < 2 ? 0 : 8)] = acc[j][q];
+        acc[j][q] = 0.0f;
       }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
 }
 
+__device__ __forceinline__ void tc_dispatch(const TcShape &c, int nt) {
+  if (nt == 16) tc_body<16>(c);
+  else if (nt == 32) tc_body<32>(c);
+  else tc_body<64>(c);
+}
 __global__ void __launch_bounds__(kTcThreads, 2) Int4GemmA8Tc(const Int4GemmA8TcArgs a) {
   TcShape c;
   c.groups = nullptr;
+  c.ngroups = nullptr;
   c.single.P = a.P; c.single.S = a.S; c.single.x_row0 = 0; c.single.M = a.M; c.single.y_col = 0; c.single.pad = 0;
   c.XQ = a.XQ; c.SQ = a.SQ; c.Y = a.Y;
-  c.N = a.N; c.K = a.K; c.ldy = a.ldy; c.max_m = a.M;
-  c.ntiles = (a.N + kTcRows - 1) / kTcRows;
-  tc_body(c);
+  c.N = a.N; c.K = a.K; c.ldy = a.ldy;
+  tc_dispatch(c, tc_entries(a.N, a.M));
 }
 
 __global__ void __launch_bounds__(kTcThreads, 2) Int4GemmA8TcGrouped(const Int4GemmA8TcGroupedArgs a) {
   TcShape c;
   c.groups = a.Groups;
+  c.ngroups = a.NGroups;
   c.single = TcGroup{nullptr, nullptr, 0, 0, 0, 0};
   c.XQ = a.XQ; c.SQ = a.SQ; c.Y = a.Y;
-  c.N = a.N; c.K = a.K; c.ldy = a.ldy; c.max_m = a.max_m;
-  c.ntiles = __ldg(a.NGroups) * ((a.N + kTcRows - 1) / kTcRows);
-  tc_body(c);
+  c.N = a.N; c.K = a.K; c.ldy = a.ldy;
+  tc_dispatch(c, tc_entries_grouped(a.max_m));
 }
 
+static uint32_t tc_smem_bytes(int nt) { return (uint32_t)tc_stages(nt) * tc_stage_bytes(nt); }
 static uint32_t tc_smem_fn(const void *args) {
   const Int4GemmA8TcArgs *a = (const Int4GemmA8TcArgs *)args;
-  return tc_smem_bytes((uint32_t)a->K, (uint32_t)a->M);
+  return tc_smem_bytes(tc_entries(a->N, a->M));
 }
-static uint32_t tc_grouped_smem_fn(const void *args) {
-  const Int4GemmA8TcGroupedArgs *a = (const Int4GemmA8TcGroupedArgs *)args;
-  return tc_smem_bytes((uint32_t)a->K, (uint32_t)a->max_m);
-}
+static uint32_t tc_grouped_smem_fn(const void *args) { return tc_smem_bytes(tc_entries_grouped(((const Int4GemmA8TcGroupedArgs *)args)->max_m)); }
 
 #define F(f) AINFER_ARG(Int4GemmA8TcArgs, f)
 AINFER_REGISTER(Int4GemmA8Tc, Int4GemmA8TcArgs, kTcThreads, 0, 0, tc_smem_fn, F(P), F(S), F(XQ), F(SQ), F(Y), F(N), F(K), F(M), F(ldy));
@@ -479,5 +378,8 @@ AINFER_REGISTER(Int4GemmA8Tc, Int4GemmA8TcArgs, kTcThreads, 0, 0, tc_smem_fn, F(
 AINFER_REGISTER(Int4GemmA8TcGrouped, Int4GemmA8TcGroupedArgs, kTcThreads, 0, 0, tc_grouped_smem_fn, F(Groups), F(NGroups), F(XQ), F(SQ),
                 F(Y), F(N), F(K), F(max_m), F(ldy));
 #undef F
+
+AINFER_EARLY_LAUNCH(Int4GemmA8Tc);
+AINFER_EARLY_LAUNCH(Int4GemmA8TcGrouped);
 
 }  // namespace ainfer

@@ -25,7 +25,6 @@
 #include "arch.h"
 #include "ep.h"
 #include "executor.h"
-#include "row_slabs.h"
 
 namespace ainfer {
 
@@ -49,7 +48,6 @@ struct Prefill {
   float *Q16 = nullptr, *K16 = nullptr, *V16 = nullptr;
   float *Qn = nullptr, *Pm = nullptr, *Pse = nullptr, *Pacc = nullptr;   // per-row attention scratch
   std::map<std::string, ainfer_kernel_t> kernels;
-  RowSlabCache slabs;   // problem lists of the GEMMs with few output rows (row_slabs.h)
   // architectures with a row engine: the rows' sequence (0), its first row (0), and the rows whose logits are wanted
   int32_t *Seq = nullptr, *First = nullptr, *Want = nullptr;
   int logits_cap = 0;                            // rows Logits holds
@@ -104,18 +102,9 @@ struct Launcher : KernelCalls {   // immediate launches, or appended to recorded
              Y, (int32_t)N, (int32_t)K, (int32_t)rows, (int32_t)N);
       return;
     }
-    if (row_slabs_pay(N, K, rows)) {
-      // few output rows: slabs of eight rows through the dp4a kernel beat the tensor-core kernel's latency (row_slabs.h)
-      RowSlabs sl;
-      if (row_slabs_get(s->dev, p->slabs, p->owned, t, rows, &sl, s->err)) { status = 1; return; }
-      launch("Int4GemvA8MultiGrouped", 2u * (uint32_t)s->sm_count, (const void *)sl.groups, (const int32_t *)sl.count, XQ, SQ, Y, (int32_t)N,
-             (int32_t)K, (int32_t)N);
-      return;
-    }
-    const uint32_t tiles = (uint32_t)((N + 127) / 128);
-    for (int r0 = 0; r0 < rows; r0 += 64)   // the tensor-core kernel takes 64 rows a launch
-      launch("Int4GemmA8Tc", std::min<uint32_t>(tiles, 2u * (uint32_t)s->sm_count), (const uint8_t *)t.data, (const uint16_t *)t.scales,
-             XQ + (size_t)r0 * K, SQ + (size_t)r0 * G, Y + (size_t)r0 * N, (int32_t)N, (int32_t)K, (int32_t)std::min(64, rows - r0), (int32_t)N);
+    const long units = (long)((N + 127) / 128) * ((rows + 15) / 16);
+    launch("Int4GemmA8Tc", (uint32_t)std::min<long>(units, 2L * s->sm_count), (const uint8_t *)t.data, (const uint16_t *)t.scales, XQ, SQ, Y, (int32_t)N,
+           (int32_t)K, (int32_t)rows, (int32_t)N);
   }
 };
 
