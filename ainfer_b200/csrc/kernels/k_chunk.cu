@@ -20,12 +20,25 @@ struct ChunkConvSiluArgs {
   float *Snap;        // optional: the history [C][3] after row m at Snap + m * snap_stride (to roll a speculative chunk back); null: none
   int64_t snap_stride;
 };
+// Launched with ceil(C / 256) x (any number of) blocks: the rows are cut into that many runs, since a row
+// needs the three before it and not their results. (One run for all rows was a chain of loads: 109 us for
+// 192 rows of 8192 channels; runs of 16 rows 12 us.) The first run's threads read the history, and so they
+// are the ones that replace it.
 __global__ void __launch_bounds__(256) ChunkConvSilu(const ChunkConvSiluArgs a) {
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c >= a.C) return;
-  float h0 = a.CS[c * 3 + 0], h1 = a.CS[c * 3 + 1], h2 = a.CS[c * 3 + 2];
+  const int cb = (a.C + 255) / 256, runs = max(1, (int)gridDim.x / cb), run = blockIdx.x / cb;
+  const int c = (blockIdx.x % cb) * 256 + threadIdx.x;
+  const int per = (a.M + runs - 1) / runs, m0 = run * per, m1 = min(m0 + per, a.M);
+  if (c >= a.C || run >= runs || (m0 >= m1 && run > 0)) return;
+  // rows before the first come from the history, oldest first
+  auto row = [&](int m) { return m >= 0 ? a.QKV[(size_t)m * a.C + c] : a.CS[c * 3 + 3 + m]; };
+  float h0 = row(m0 - 3), h1 = row(m0 - 2), h2 = row(m0 - 1);
+  if (run == 0) {
+    const float n0 = row(a.M - 3), n1 = row(a.M - 2), n2 = row(a.M - 1);
+    a.CS[c * 3 + 0] = n0; a.CS[c * 3 + 1] = n1; a.CS[c * 3 + 2] = n2;
+  }
   const float4 w = __ldg(reinterpret_cast<const float4 *>(a.CW) + c);
-  for (int m = 0; m < a.M; ++m) {
+#pragma unroll 4
+  for (int m = m0; m < m1; ++m) {
     const float x = a.QKV[(size_t)m * a.C + c];
     float acc = h0 * w.x;
     acc = acc + h1 * w.y;
@@ -38,7 +51,6 @@ __global__ void __launch_bounds__(256) ChunkConvSilu(const ChunkConvSiluArgs a) 
       sn[0] = h0; sn[1] = h1; sn[2] = h2;
     }
   }
-  a.CS[c * 3 + 0] = h0; a.CS[c * 3 + 1] = h1; a.CS[c * 3 + 2] = h2;
 }
 
 // ---- ChunkBetaDecay: beta = sigmoid(b), g = -exp(A_log) * softplus(a + dt_bias) for M rows ----
@@ -73,99 +85,148 @@ struct ChunkDeltaNetArgs {
   float *Snap;       // optional: the state [nV][128][128] after row m at Snap + m * snap_stride (to roll a speculative chunk back); null: none
   int64_t snap_stride;
 };
-constexpr int kChunkRows = 64;   // rows whose normalised q / k are staged at a time
+constexpr int kChunkRows = 32;      // rows whose normalised q / k are staged at a time (two buffers)
+constexpr int kChunkWarps = 4, kChunkHelpers = 8, kChunkThreads = (kChunkWarps + kChunkHelpers) * 32;
+constexpr int kChunkRow = 4 * 36;   // floats of a staged row: four quarters of 32, apart so that a warp's reads of them meet different banks
+constexpr int kChunkBuffer = kChunkRows * (2 * kChunkRow + 32);   // floats: q, k, the slice's values
 
 extern __shared__ __align__(16) float chunk_smem[];
 
-// One block of 256 threads per (head, 32-column slice); grid = nV * 4. Per row the arithmetic of
-// deltanet_step_body: S *= exp(g); kv = tree8 of 16-row fma chains; d = (v - kv) * beta;
-// S += k d; o = tree8 of fma chains with q.
-__global__ void __launch_bounds__(256) ChunkDeltaNet(const ChunkDeltaNetArgs a) {
+// One block per (head, 32-column slice); grid = nV * 4. Per row the arithmetic of deltanet_step_body:
+// S *= exp(g); kv = tree8 of 16-row fma chains; d = (v - kv) * beta; S += k d; o = tree8 of fma chains
+// with q. A warp holds eight columns, a lane two of a column's eight segments of 16 rows (two chains side by
+// side), so that the tree is one addition and two exchanges inside the warp and the rows of a chunk need no
+// barrier; a row's output is summed beside the next row's kv. Eight more warps normalise the next chunk's
+// q and k meanwhile and fetch its values. Bound by the chain of a row. (Segments in different warps, two
+// block barriers a row: 130 us for 192 rows of 32 heads; this form 58.)
+__global__ void __launch_bounds__(kChunkThreads) ChunkDeltaNet(const ChunkDeltaNetArgs a) {
   constexpr int D = 128, SEG = kDnSeg;
-  float *qs = chunk_smem;                       // [kChunkRows][128] normalised, scaled q
-  float *ks = qs + kChunkRows * D;              // [kChunkRows][128] normalised k
-  __shared__ float part[2][8][32];
-  __shared__ float s_beta[kChunkRows], s_gt[kChunkRows];
+  __shared__ float s_beta[2][kChunkRows], s_gt[2][kChunkRows];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.x / kDnSlices, slice = blockIdx.x % kDnSlices;
   if (h >= a.nV) return;
   const int kh = h / (a.nV / a.nK);
-  const int col = slice * 32 + lane;
   const int C = 2 * a.nK * D + a.nV * D;
-  float *Sh = a.S + (size_t)h * D * D;
-  float s[SEG];
+  const int chunks = (a.M + kChunkRows - 1) / kChunkRows;
+  auto stage = [&](int ch) {   // l2norm of the rows' q and k (a warp per (row, which)), values, beta and decay of the rows
+    float *qs = chunk_smem + (ch & 1) * kChunkBuffer, *ks = qs + kChunkRows * kChunkRow, *vs = ks + kChunkRows * kChunkRow;
+    const int m0 = ch * kChunkRows, rows = min(kChunkRows, a.M - m0), hw = warp - kChunkWarps;
+    const int which = hw & 1;
+    const float *base = a.Mx + (size_t)m0 * C;
+    const float *src = base + (which == 0 ? (size_t)kh * D : (size_t)a.nK * D + (size_t)kh * D) + lane;
+    for (int m = hw >> 1; m < rows; m += 2 * kChunkHelpers) {   // four rows' loads in flight
+      float x[4][4];
 #pragma unroll
-  for (int r = 0; r < SEG; ++r) s[r] = Sh[(size_t)(warp * SEG + r) * D + col];
-  for (int m0 = 0; m0 < a.M; m0 += kChunkRows) {
-    const int rows = a.M - m0 < kChunkRows ? a.M - m0 : kChunkRows;
-    __syncthreads();   // the previous rows' q / k are no longer read
-    // l2norm of the rows' q and k (a warp per (row, which)), beta and decay of the rows
-    for (int t = warp; t < rows * 2; t += 8) {
-      const int m = t >> 1, which = t & 1;
-      const float *src = a.Mx + (size_t)(m0 + m) * C + (which == 0 ? (size_t)kh * D : (size_t)a.nK * D + (size_t)kh * D);
-      float x[4];
-      float ss = 0.0f;
+      for (int u = 0; u < 4; ++u) {
+        const float *r = src + (size_t)min(m + u * (kChunkHelpers / 2), rows - 1) * C;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        x[i] = src[lane + 32 * i];
-        ss = fmaf(x[i], x[i], ss);
+        for (int i = 0; i < 4; ++i) x[u][i] = r[32 * i];
       }
-      ss = warp_tree_sum(ss);
-      const float inv = 1.0f / sqrtf(ss + 1e-6f);
-      const float f = inv * (which == 0 ? 0.0883883476483184405f : 1.0f);  // 128^-1/2 for q
-      float *dst = (which == 0 ? qs : ks) + m * D;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dst[lane + 32 * i] = x[i] * f;
+      for (int u = 0; u < 4; ++u) {
+        const int mm = m + u * (kChunkHelpers / 2);
+        float ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ss = fmaf(x[u][i], x[u][i], ss);
+        ss = warp_tree_sum(ss);
+        const float inv = 1.0f / sqrtf(ss + 1e-6f);
+        const float f = inv * (which == 0 ? 0.0883883476483184405f : 1.0f);  // 128^-1/2 for q
+        float *dst = (which == 0 ? qs : ks) + mm * kChunkRow;
+        if (mm < rows) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) dst[36 * i + lane] = x[u][i] * f;
+        }
+      }
     }
-    for (int m = threadIdx.x; m < rows; m += 256) {
-      s_beta[m] = a.Bt[(size_t)(m0 + m) * a.nV + h];
-      s_gt[m] = det_expf(a.Gt[(size_t)(m0 + m) * a.nV + h]);
+    float v[kChunkRows / kChunkHelpers];
+#pragma unroll
+    for (int u = 0; u < kChunkRows / kChunkHelpers; ++u)
+      v[u] = base[(size_t)min(hw + u * kChunkHelpers, rows - 1) * C + (size_t)2 * a.nK * D + (size_t)h * D + slice * 32 + lane];
+#pragma unroll
+    for (int u = 0; u < kChunkRows / kChunkHelpers; ++u) vs[(hw + u * kChunkHelpers) * 32 + lane] = v[u];
+    const int m = (int)threadIdx.x - kChunkWarps * 32;
+    if (m < rows) {
+      s_beta[ch & 1][m] = a.Bt[(size_t)(m0 + m) * a.nV + h];
+      s_gt[ch & 1][m] = det_expf(a.Gt[(size_t)(m0 + m) * a.nV + h]);
     }
-    __syncthreads();
-    float val = a.Mx[(size_t)m0 * C + (size_t)2 * a.nK * D + (size_t)h * D + col];
-    for (int m = 0; m < rows; ++m) {
-      const float *kr = ks + m * D + warp * SEG, *qr = qs + m * D + warp * SEG;
-      const float gt = s_gt[m], beta = s_beta[m];
-      const float val_next = m + 1 < rows ? a.Mx[(size_t)(m0 + m + 1) * C + (size_t)2 * a.nK * D + (size_t)h * D + col] : 0.0f;
-      float acc = 0.0f;
+  };
+  const bool helper = warp >= kChunkWarps;
+  const int quarter = lane & 3, wcol = warp * 8 + (lane >> 2), col = slice * 32 + wcol;   // a lane's segments: 2 quarter, 2 quarter + 1
+  float *Sh = a.S + (size_t)h * D * D + (size_t)quarter * (2 * SEG) * D + col;
+  float s[2 * SEG], po = 0.0f;
+  float *out = a.Out + (size_t)h * D + col;   // of the last row begun
+  if (helper) {
+    stage(0);
+  } else {
 #pragma unroll
-      for (int r = 0; r < SEG; ++r) {
-        s[r] = s[r] * gt;
-        acc = fmaf(s[r], kr[r], acc);
-      }
-      part[0][warp][lane] = acc;
-      __syncthreads();
-      const float kv = ((part[0][0][lane] + part[0][1][lane]) + (part[0][2][lane] + part[0][3][lane])) +
-                       ((part[0][4][lane] + part[0][5][lane]) + (part[0][6][lane] + part[0][7][lane]));
-      const float dl = (val - kv) * beta;
-      acc = 0.0f;
-#pragma unroll
-      for (int r = 0; r < SEG; ++r) {
-        s[r] = fmaf(kr[r], dl, s[r]);
-        acc = fmaf(s[r], qr[r], acc);
-      }
-      part[1][warp][lane] = acc;
-      __syncthreads();   // also: every thread has read part[0] of this row
-      if (warp == 0) {
-        const float o = ((part[1][0][lane] + part[1][1][lane]) + (part[1][2][lane] + part[1][3][lane])) +
-                        ((part[1][4][lane] + part[1][5][lane]) + (part[1][6][lane] + part[1][7][lane]));
-        a.Out[((size_t)(m0 + m) * a.nV + h) * D + col] = o;
-      }
-      if (a.Snap) {
-        float *sn = a.Snap + (size_t)(m0 + m) * a.snap_stride + (size_t)h * D * D;
-#pragma unroll
-        for (int r = 0; r < SEG; ++r) sn[(size_t)(warp * SEG + r) * D + col] = s[r];
-      }
-      val = val_next;
-      // part[1] of this row is read by warp 0 only, before it writes part[1] of the next row
-      // (it passes the next row's first barrier in between, as every writer of part[1] does)
-    }
+    for (int r = 0; r < 2 * SEG; ++r) s[r] = Sh[(size_t)r * D];
   }
+  __syncthreads();
+  for (int ch = 0; ch < chunks; ++ch) {
+    if (helper) {
+      if (ch + 1 < chunks) stage(ch + 1);
+    } else {
+      const float *qs = chunk_smem + (ch & 1) * kChunkBuffer, *ks = qs + kChunkRows * kChunkRow, *vs = ks + kChunkRows * kChunkRow + wcol;
+      const int m0 = ch * kChunkRows, rows = min(kChunkRows, a.M - m0);
+      qs += quarter * 36;
+      ks += quarter * 36;
+#pragma unroll 1
+      for (int m = 0; m < rows; ++m) {
+        const float gt = s_gt[ch & 1][m], beta = s_beta[ch & 1][m], val = vs[m * 32];
+        float k[2 * SEG], q[2 * SEG];
 #pragma unroll
-  for (int r = 0; r < SEG; ++r) Sh[(size_t)(warp * SEG + r) * D + col] = s[r];
+        for (int i = 0; i < 2 * SEG / 4; ++i) {
+          const float4 k4 = *reinterpret_cast<const float4 *>(ks + m * kChunkRow + 4 * i);
+          k[4 * i] = k4.x; k[4 * i + 1] = k4.y; k[4 * i + 2] = k4.z; k[4 * i + 3] = k4.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 2 * SEG / 4; ++i) {
+          const float4 q4 = *reinterpret_cast<const float4 *>(qs + m * kChunkRow + 4 * i);
+          q[4 * i] = q4.x; q[4 * i + 1] = q4.y; q[4 * i + 2] = q4.z; q[4 * i + 3] = q4.w;
+        }
+        float c0 = 0.0f, c1 = 0.0f;
+#pragma unroll
+        for (int r = 0; r < SEG; ++r) {
+          s[r] = s[r] * gt;
+          s[SEG + r] = s[SEG + r] * gt;
+          c0 = fmaf(s[r], k[r], c0);
+          c1 = fmaf(s[SEG + r], k[SEG + r], c1);
+        }
+        float kv = c0 + c1, o = po;   // the tree's first level; then this row's kv beside the last row's output
+        kv = kv + __shfl_xor_sync(kFull, kv, 1);
+        o = o + __shfl_xor_sync(kFull, o, 1);
+        kv = kv + __shfl_xor_sync(kFull, kv, 2);
+        o = o + __shfl_xor_sync(kFull, o, 2);
+        if (quarter == 0 && m0 + m > 0) out[(size_t)(m0 + m - 1) * a.nV * D] = o;
+        const float dl = (val - kv) * beta;
+        c0 = c1 = 0.0f;
+#pragma unroll
+        for (int r = 0; r < SEG; ++r) {
+          s[r] = fmaf(k[r], dl, s[r]);
+          s[SEG + r] = fmaf(k[SEG + r], dl, s[SEG + r]);
+          c0 = fmaf(s[r], q[r], c0);
+          c1 = fmaf(s[SEG + r], q[SEG + r], c1);
+        }
+        po = c0 + c1;
+        if (a.Snap) {
+          float *sn = a.Snap + (size_t)(m0 + m) * a.snap_stride + (size_t)h * D * D + (size_t)quarter * (2 * SEG) * D + col;
+#pragma unroll
+          for (int r = 0; r < 2 * SEG; ++r) sn[(size_t)r * D] = s[r];
+        }
+      }
+    }
+    __syncthreads();   // the next chunk is staged, this one is read
+  }
+  if (!helper) {
+    float o = po + __shfl_xor_sync(kFull, po, 1);
+    o = o + __shfl_xor_sync(kFull, o, 2);
+    if (quarter == 0 && a.M > 0) out[(size_t)(a.M - 1) * a.nV * D] = o;
+#pragma unroll
+    for (int r = 0; r < 2 * SEG; ++r) Sh[(size_t)r * D] = s[r];
+  }
 }
 
-static uint32_t chunk_dn_smem_fn(const void *) { return 2u * kChunkRows * 128u * 4u; }
+static uint32_t chunk_dn_smem_fn(const void *) { return 2u * kChunkBuffer * 4u; }
 
 #define F(f) AINFER_ARG(ChunkConvSiluArgs, f)
 AINFER_REGISTER(ChunkConvSilu, ChunkConvSiluArgs, 256, 256, 0, nullptr, F(Mx), F(QKV), F(CS), F(CW), F(C), F(M), F(Snap), F(snap_stride));
@@ -174,7 +235,7 @@ AINFER_REGISTER(ChunkConvSilu, ChunkConvSiluArgs, 256, 256, 0, nullptr, F(Mx), F
 AINFER_REGISTER(ChunkBetaDecay, ChunkBetaDecayArgs, 256, 256, 0, nullptr, F(B), F(A), F(ALog), F(DtBias), F(Bt), F(Gt), F(nV), F(count));
 #undef F
 #define F(f) AINFER_ARG(ChunkDeltaNetArgs, f)
-AINFER_REGISTER(ChunkDeltaNet, ChunkDeltaNetArgs, 256, 1, 0, chunk_dn_smem_fn, F(Out), F(Mx), F(S), F(Bt), F(Gt), F(nK), F(nV), F(M), F(Snap), F(snap_stride));
+AINFER_REGISTER(ChunkDeltaNet, ChunkDeltaNetArgs, kChunkThreads, 1, 0, chunk_dn_smem_fn, F(Out), F(Mx), F(S), F(Bt), F(Gt), F(nK), F(nV), F(M), F(Snap), F(snap_stride));
 #undef F
 
 }  // namespace ainfer
