@@ -30,96 +30,92 @@ struct RouterLogitsRowsArgs {
   const float *Bias;     // optional [E]: added to the routed experts' logits (load generators); null: none
   float *Logits;         // [rows][E+1]
   int32_t E, H, rows;
-  int32_t tokens_per_block;   // launched with ceil((E + 1) / 8) x ceil(rows / tokens_per_block) blocks
+  int32_t tokens_per_block;   // 8 or 16; launched with ceil((E + 1) / 32) x ceil(rows / tokens_per_block) blocks
 };
-// One warp per router row and block of tokens; per token the sums of RouterTopK (router_row_fma
-// order, then the lane tree). The row's first chunk of weights is fetched once, and four tokens
-// are summed side by side: a token's sum is one chain of dependent additions per lane, so four
-// chains in flight is what keeps the lanes busy.
-// kSmem: the block's tokens' activations were staged in shared memory (hn points there, token stride H)
-template <bool kSmem>
-__device__ __forceinline__ void router_rows_compute(const RouterLogitsRowsArgs &a, const uint16_t *w, const RouterRowRegs &r0,
-                                                    const float *hn_base, int t_begin, int t_end, int e, bool store, float bias,
-                                                    int lane) {
-  const int n = a.H / 256;
-  for (int t = t_begin; t < t_end; t += 4) {
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    RouterRowRegs r = r0;
-    const float *hn[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) hn[u] = hn_base + (size_t)((t + u < t_end ? t + u : t_end - 1) - (kSmem ? t_begin : 0)) * a.H;   // past the end: the last token again, not stored
-    for (int i0 = 0;;) {
-#pragma unroll
-      for (int c = 0; c < kRouterChunk; ++c) {
-        const int ic = i0 + c < n ? i0 + c : n - 1, k0 = (ic * 32 + lane) * 8;
-        float4 x0[4], x1[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (kSmem) {
-            x0[u] = *reinterpret_cast<const float4 *>(hn[u] + k0);
-            x1[u] = *reinterpret_cast<const float4 *>(hn[u] + k0 + 4);
-          } else {
-            x0[u] = __ldcg(reinterpret_cast<const float4 *>(hn[u] + k0));
-            x1[u] = __ldcg(reinterpret_cast<const float4 *>(hn[u] + k0 + 4));
-          }
-        }
-        if (i0 + c < n) {
-          const uint4 wv = r.w[c];
-          const float w0 = u2f(wv.x << 16), w1 = u2f(wv.x & 0xFFFF0000u), w2 = u2f(wv.y << 16), w3 = u2f(wv.y & 0xFFFF0000u),
-                      w4 = u2f(wv.z << 16), w5 = u2f(wv.z & 0xFFFF0000u), w6 = u2f(wv.w << 16), w7 = u2f(wv.w & 0xFFFF0000u);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {   // router_row_fma's order for each token
-            float s = acc[u];
-            s = fmaf(w0, x0[u].x, s);
-            s = fmaf(w1, x0[u].y, s);
-            s = fmaf(w2, x0[u].z, s);
-            s = fmaf(w3, x0[u].w, s);
-            s = fmaf(w4, x1[u].x, s);
-            s = fmaf(w5, x1[u].y, s);
-            s = fmaf(w6, x1[u].z, s);
-            s = fmaf(w7, x1[u].w, s);
-            acc[u] = s;
-          }
-        }
-      }
-      i0 += kRouterChunk;
-      if (i0 >= n) break;
-      router_row_load(r, w, i0, n, lane);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float sum = warp_tree_sum(acc[u]);
-      if (lane == 0 && store && t + u < t_end) a.Logits[(size_t)(t + u) * (a.E + 1) + e] = a.Bias ? sum + bias : sum;
-    }
-  }
-}
-constexpr int kRouterStageFloats = 8192;   // 32 KB: four tokens of 2048
-__global__ void __launch_bounds__(256, 2) RouterLogitsRows(const RouterLogitsRowsArgs a) {
-  // The block's tokens are read by all eight warps: staged once in shared memory they cross from
-  // L2 once per block instead of once per warp (at 64 tokens and 513 rows the per-warp reads were
-  // 266 MB a launch, and the launch took as long as that takes).
-  __shared__ __align__(16) float hs[kRouterStageFloats];
+// Every sum is RouterTopK's: a lane's chain over its eight values of every 256, then the lane tree. A warp
+// sums four router rows against all of the block's tokens, so that a weight is fetched once per block of
+// tokens and an activation is read from shared memory once per four rows: 512 multiply-adds per lane and
+// chunk for 32 16-byte reads of activations at 16 tokens, which the shared memory serves in the time of the
+// multiply-adds. Activations are staged 1024 columns at a time, a lane's two quarters of its eight values
+// apart (side by side they meet the same banks). (One router row per warp and four tokens: bound by those
+// reads, 74 us for 192 tokens of 513 x 2048; this form 25.)
+constexpr int kRlRows = 32, kRlCols = 1024, kRlChunks = kRlCols / 256;
+template <int TT>
+__device__ __forceinline__ void router_logits_rows_body(const RouterLogitsRowsArgs &a) {
+  extern __shared__ __align__(16) float rl_smem[];   // [TT][kRlChunks][2][32 lanes][4]
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nrows = a.E + (a.Wsg ? 1 : 0), n = a.H / 256;
-  const int nrb = (a.E + 1 + 7) / 8, rb = blockIdx.x % nrb, tb = blockIdx.x / nrb;
-  const int t_begin = tb * a.tokens_per_block;
-  const int t_end = t_begin + a.tokens_per_block < a.rows ? t_begin + a.tokens_per_block : a.rows;
-  const int e_raw = rb * 8 + warp, e = e_raw < nrows ? e_raw : nrows - 1;   // a warp past the last row repeats it and stores nothing
-  const uint16_t *w = e < a.E ? a.Wr + (size_t)e * a.H : a.Wsg;
-  const float bias = a.Bias && e < a.E ? __ldg(a.Bias + e) : 0.0f;
-  RouterRowRegs r0;
-  router_row_load(r0, w, 0, n, lane);
-  const bool staged = (t_end - t_begin) * a.H <= kRouterStageFloats;   // the same for every thread of the block
-  if (staged) {
-    const float4 *src = reinterpret_cast<const float4 *>(a.Hn + (size_t)t_begin * a.H);
-    const int n4 = (t_end - t_begin) * a.H / 4;
-    for (int i = threadIdx.x; i < n4; i += 256) reinterpret_cast<float4 *>(hs)[i] = __ldcg(src + i);
+  const int nrb = (a.E + 1 + kRlRows - 1) / kRlRows, e0 = (blockIdx.x % nrb) * kRlRows + warp * 4, t0 = (blockIdx.x / nrb) * TT;
+  const uint4 *w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {   // past the last row: that row again, not stored
+    const int e = min(e0 + j, nrows - 1);
+    w[j] = reinterpret_cast<const uint4 *>(e < a.E ? a.Wr + (size_t)e * a.H : a.Wsg) + lane;
+  }
+  float acc[TT][4];
+#pragma unroll
+  for (int u = 0; u < TT; ++u)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[u][j] = 0.0f;
+  pdl_wait();
+  for (int i0 = 0; i0 < n; i0 += kRlChunks) {
+    const int nc = min(kRlChunks, n - i0);
+    __syncthreads();   // the last columns' readers are done
+    for (int i = threadIdx.x; i < TT * nc * 64; i += 256) {
+      const int u = i / (nc * 64), f = i % (nc * 64), c = f >> 6, q = f & 63;   // token (past the end: the last one, not stored), chunk, quarter
+      const float4 v = __ldcg(reinterpret_cast<const float4 *>(a.Hn + (size_t)min(t0 + u, a.rows - 1) * a.H + (size_t)(i0 + c) * 256) + q);
+      reinterpret_cast<float4 *>(rl_smem)[((u * kRlChunks + c) * 2 + (q & 1)) * 32 + (q >> 1)] = v;
+    }
     __syncthreads();
-    router_rows_compute<true>(a, w, r0, hs, t_begin, t_end, e, e_raw < nrows, bias, lane);
-  } else {
-    router_rows_compute<false>(a, w, r0, a.Hn, t_begin, t_end, e, e_raw < nrows, bias, lane);
+    uint4 wv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) wv[j] = __ldg(w[j] + (size_t)i0 * 32);
+#pragma unroll 1
+    for (int c = 0; c < nc; ++c) {
+      float f[4][8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        f[j][0] = u2f(wv[j].x << 16); f[j][1] = u2f(wv[j].x & 0xFFFF0000u); f[j][2] = u2f(wv[j].y << 16); f[j][3] = u2f(wv[j].y & 0xFFFF0000u);
+        f[j][4] = u2f(wv[j].z << 16); f[j][5] = u2f(wv[j].z & 0xFFFF0000u); f[j][6] = u2f(wv[j].w << 16); f[j][7] = u2f(wv[j].w & 0xFFFF0000u);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) wv[j] = __ldg(w[j] + (size_t)min(i0 + c + 1, n - 1) * 32);
+      const float4 *x = reinterpret_cast<const float4 *>(rl_smem) + c * 64 + lane;
+#pragma unroll
+      for (int u = 0; u < TT; ++u) {
+        const float4 x0 = x[u * (kRlChunks * 64)], x1 = x[u * (kRlChunks * 64) + 32];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float s = acc[u][j];
+          s = fmaf(f[j][0], x0.x, s);
+          s = fmaf(f[j][1], x0.y, s);
+          s = fmaf(f[j][2], x0.z, s);
+          s = fmaf(f[j][3], x0.w, s);
+          s = fmaf(f[j][4], x1.x, s);
+          s = fmaf(f[j][5], x1.y, s);
+          s = fmaf(f[j][6], x1.z, s);
+          s = fmaf(f[j][7], x1.w, s);
+          acc[u][j] = s;
+        }
+      }
+    }
+  }
+  const int own = warp_tree_owner<8>(lane);   // of eight sums (two tokens x four rows), the one this lane ends with
+#pragma unroll
+  for (int u = 0; u < TT; u += 2) {
+    const float v[8] = {acc[u][0], acc[u][1], acc[u][2], acc[u][3], acc[u + 1][0], acc[u + 1][1], acc[u + 1][2], acc[u + 1][3]};
+    const float sum = warp_tree_sum_multi<8>(v, lane);
+    const int t = t0 + u + (own >> 2), e = e0 + (own & 3);
+    if ((lane & 3) == 0 && t < a.rows && e < nrows)
+      a.Logits[(size_t)t * (a.E + 1) + e] = a.Bias && e < a.E ? sum + __ldg(a.Bias + e) : a.Bias ? sum + 0.0f : sum;
   }
 }
+__global__ void __launch_bounds__(256, 2) RouterLogitsRows(const RouterLogitsRowsArgs a) {
+  if (a.tokens_per_block == 16) router_logits_rows_body<16>(a);
+  else router_logits_rows_body<8>(a);
+}
+static uint32_t router_rows_smem(const void *args) { return (uint32_t)((const RouterLogitsRowsArgs *)args)->tokens_per_block * kRlCols * 4u; }
 struct RouterSelectRowsArgs {
   const float *Logits;   // [rows][E+1]
   int32_t *SelIdx;       // [rows][k+1]
@@ -129,6 +125,8 @@ struct RouterSelectRowsArgs {
 };
 __global__ void __launch_bounds__(256) RouterSelectRows(const RouterSelectRowsArgs a) {
   __shared__ float sp[1024 + 1];
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x;
   router_select(a.Logits + (size_t)t * (a.E + 1), a.E, a.k, a.has_shared != 0, sp, a.SelIdx + (size_t)t * (a.k + 1),
                 a.SelW + (size_t)t * (a.k + 1), a.NearGap + t);
@@ -324,6 +322,105 @@ __global__ void __launch_bounds__(128) EpGather(const EpGatherArgs a) {
   for (int j = threadIdx.x; j < a.H / 128; j += blockDim.x) s[j] = reinterpret_cast<const float *>(src + a.H)[j];
 }
 
+// ---- one rank: its own rows need no dispatch buffers ----
+// Item i = token * k + slot; its place among the rows grouped by expert goes to ItemRow (the order within
+// an expert is free: a row's products do not depend on its place).
+constexpr int kEpLocalItems = 8192;
+struct EpGroupLocalArgs {
+  const int32_t *SelIdx;      // [n][k+1]
+  const ExpertW *Experts;     // the layer's table [E+1]
+  int32_t *Sorted;            // [n*k]: item, grouped by expert
+  int32_t *ItemRow;           // [n*k]: place of an item
+  EpTcGroup *GroupsGateUp;    // gate and up problem of every active expert and cut
+  EpTcGroup *GroupsDown;
+  int32_t *Counts;            // [8] as EpGroup's
+  int32_t n, k, E, I;
+  int32_t shared_row0, shared_rows, max_rows;
+};
+__global__ void __launch_bounds__(1024) EpGroupLocal(const EpGroupLocalArgs a) {
+  __shared__ int hist[1024], start[1024], wsum[2][33];
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, items = a.n * a.k;
+  hist[tid] = 0;
+  pdl_wait();
+  __syncthreads();
+  constexpr int kPer = kEpLocalItems / 1024;
+  int ex[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int i = tid + q * 1024;
+    ex[q] = i < items ? a.SelIdx[(size_t)(i / a.k) * (a.k + 1) + i % a.k] : -1;
+  }
+#pragma unroll
+  for (int q = 0; q < kPer; ++q)
+    if (ex[q] >= 0) atomicAdd(&hist[ex[q]], 1);
+  __syncthreads();
+  const int c = hist[tid], np = (c + a.max_rows - 1) / a.max_rows;   // items and problems of expert tid
+  int sc = c, sp = np;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int vc = __shfl_up_sync(kFull, sc, off), vp = __shfl_up_sync(kFull, sp, off);
+    if (lane >= off) { sc += vc; sp += vp; }
+  }
+  if (lane == 31) { wsum[0][warp] = sc; wsum[1][warp] = sp; }
+  __syncthreads();
+  if (warp < 2) {
+    const int own = wsum[warp][lane];
+    int v = own;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(kFull, v, off);
+      if (lane >= off) v += o;
+    }
+    wsum[warp][lane] = v - own;
+    if (lane == 31) wsum[warp][32] = v;
+  }
+  __syncthreads();
+  const int first = wsum[0][warp] + sc - c, g0 = wsum[1][warp] + sp - np, total = wsum[1][32];
+  start[tid] = first;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kPer; ++q)
+    if (ex[q] >= 0) {
+      const int i = tid + q * 1024, pos = atomicAdd(&start[ex[q]], 1);
+      a.Sorted[pos] = i;
+      a.ItemRow[i] = pos;
+    }
+  auto problems = [&](const ExpertW &w, int row0, int rows, int g) {
+    for (int j = 0; j * a.max_rows < rows; ++j, ++g) {
+      const int r0 = row0 + j * a.max_rows, mr = min(a.max_rows, rows - j * a.max_rows);
+      a.GroupsGateUp[2 * g] = EpTcGroup{w.gP, w.gS, r0, mr, 0, 0};
+      a.GroupsGateUp[2 * g + 1] = EpTcGroup{w.uP, w.uS, r0, mr, a.I, 0};
+      a.GroupsDown[g] = EpTcGroup{w.dP, w.dS, r0, mr, 0, 0};
+    }
+  };
+  if (c > 0) problems(a.Experts[tid], first, c, g0);
+  if (tid == 1023) {
+    if (a.shared_rows > 0) problems(a.Experts[a.E], a.shared_row0, a.shared_rows, total);
+    const int all = total + (a.shared_rows + a.max_rows - 1) / a.max_rows;
+    *reinterpret_cast<int4 *>(a.Counts) = make_int4(items, 0, 0, 2 * all);
+    *reinterpret_cast<int4 *>(a.Counts + 4) = make_int4(all, 0, 0, 0);
+  }
+}
+struct EpGatherLocalArgs {
+  const int8_t *Q8;        // [n][H]
+  const float *SQ;         // [n][H/128]
+  const int32_t *Sorted;   // [items]
+  int8_t *XQ;              // [items][H]
+  float *XS;               // [items][H/128]
+  int32_t H, k;
+};
+__global__ void __launch_bounds__(128) EpGatherLocal(const EpGatherLocalArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int pos = blockIdx.x, t = a.Sorted[pos] / a.k;
+  const uint4 *q = reinterpret_cast<const uint4 *>(a.Q8 + (size_t)t * a.H);
+  uint4 *d = reinterpret_cast<uint4 *>(a.XQ + (size_t)pos * a.H);
+  for (int j = threadIdx.x; j < a.H / 16; j += 128) d[j] = q[j];
+  const float *s = a.SQ + (size_t)t * (a.H / 128);
+  for (int j = threadIdx.x; j < a.H / 128; j += 128) a.XS[(size_t)pos * (a.H / 128) + j] = s[j];
+}
+
 // ---- between the expert GEMMs: act = silu(gate) * up, then the per-128 activation quantiser ----
 // (SiluMul tools/cmdlist/kernels.cpp:29-37, ScalesMax + Quantize :551-579.) One warp per group of
 // 128, a lane holds four consecutive elements.
@@ -334,9 +431,12 @@ struct SiluQuantRowsArgs {
   float *ASQ;              // [rows][I/128]
   int32_t I;
   int32_t always_from;     // rows from this one on are always in use
+  int32_t front;           // blocks below it take their own row, the others the rows from always_from on
 };
 __global__ void __launch_bounds__(128) SiluQuantRows(const SiluQuantRowsArgs a) {
-  const int row = blockIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row = (int)blockIdx.x < a.front ? (int)blockIdx.x : a.always_from + (int)blockIdx.x - a.front;
   if (a.Counts && row < a.always_from && row >= __ldg(a.Counts)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float *g = a.GU + (size_t)row * 2 * a.I, *u = g + a.I;
@@ -387,11 +487,14 @@ struct EpCombineArgs {
   const float *SelW;        // [n][k+1]
   const float *Ysh;         // [n][H] shared expert's output (null: none)
   float *X;                 // [n][H]
+  float *X2;                // a second copy (the next layer's input; may be Res)
   int32_t k, H;
   uint32_t slot_bytes;
 };
 // Launched with tokens x ceil(H / 256) blocks.
 __global__ void __launch_bounds__(256) EpCombine(const EpCombineArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int bpr = (a.H + 255) / 256;
   const int t = blockIdx.x / bpr;
   const int n = (blockIdx.x % bpr) * 256 + threadIdx.x;
@@ -403,11 +506,13 @@ __global__ void __launch_bounds__(256) EpCombine(const EpCombineArgs a) {
     acc = acc + a.SelW[(size_t)t * (a.k + 1) + j] * y;
   }
   if (a.Ysh) acc = acc + a.SelW[(size_t)t * (a.k + 1) + a.k] * a.Ysh[(size_t)t * a.H + n];
-  a.X[(size_t)t * a.H + n] = a.Res[(size_t)t * a.H + n] + acc;
+  const float x = a.Res[(size_t)t * a.H + n] + acc;
+  a.X[(size_t)t * a.H + n] = x;
+  a.X2[(size_t)t * a.H + n] = x;
 }
 
 #define F(f) AINFER_ARG(RouterLogitsRowsArgs, f)
-AINFER_REGISTER(RouterLogitsRows, RouterLogitsRowsArgs, 256, 8, 0, nullptr, F(Wr), F(Wsg), F(Hn), F(Bias), F(Logits), F(E), F(H), F(rows),
+AINFER_REGISTER(RouterLogitsRows, RouterLogitsRowsArgs, 256, 0, 0, router_rows_smem, F(Wr), F(Wsg), F(Hn), F(Bias), F(Logits), F(E), F(H), F(rows),
                 F(tokens_per_block));
 #undef F
 #define F(f) AINFER_ARG(RouterSelectRowsArgs, f)
@@ -427,14 +532,28 @@ AINFER_REGISTER(EpGroup, EpGroupArgs, 1024, 0, 0, nullptr, F(Recv), F(Experts), 
 #define F(f) AINFER_ARG(EpGatherArgs, f)
 AINFER_REGISTER(EpGather, EpGatherArgs, 128, 1, 0, nullptr, F(Recv), F(Sorted), F(Counts), F(XQ), F(SQ), F(H), F(cap), F(slot_bytes));
 #undef F
+#define F(f) AINFER_ARG(EpGroupLocalArgs, f)
+AINFER_REGISTER(EpGroupLocal, EpGroupLocalArgs, 1024, 0, 0, nullptr, F(SelIdx), F(Experts), F(Sorted), F(ItemRow), F(GroupsGateUp), F(GroupsDown),
+                F(Counts), F(n), F(k), F(E), F(I), F(shared_row0), F(shared_rows), F(max_rows));
+#undef F
+#define F(f) AINFER_ARG(EpGatherLocalArgs, f)
+AINFER_REGISTER(EpGatherLocal, EpGatherLocalArgs, 128, 1, 0, nullptr, F(Q8), F(SQ), F(Sorted), F(XQ), F(XS), F(H), F(k));
+#undef F
 #define F(f) AINFER_ARG(SiluQuantRowsArgs, f)
-AINFER_REGISTER(SiluQuantRows, SiluQuantRowsArgs, 128, 1, 0, nullptr, F(GU), F(Counts), F(AQ), F(ASQ), F(I), F(always_from));
+AINFER_REGISTER(SiluQuantRows, SiluQuantRowsArgs, 128, 1, 0, nullptr, F(GU), F(Counts), F(AQ), F(ASQ), F(I), F(always_from), F(front));
 #undef F
 #define F(f) AINFER_ARG(EpScatterArgs, f)
 AINFER_REGISTER(EpScatter, EpScatterArgs, 128, 1, 0, nullptr, F(Y), F(Sorted), F(Counts), F(Ret), F(H), F(slot_bytes));
 #undef F
 #define F(f) AINFER_ARG(EpCombineArgs, f)
-AINFER_REGISTER(EpCombine, EpCombineArgs, 256, 0, 0, nullptr, F(Res), F(Back), F(ItemDest), F(SelW), F(Ysh), F(X), F(k), F(H), F(slot_bytes));
+AINFER_REGISTER(EpCombine, EpCombineArgs, 256, 0, 0, nullptr, F(Res), F(Back), F(ItemDest), F(SelW), F(Ysh), F(X), F(X2), F(k), F(H), F(slot_bytes));
 #undef F
+
+AINFER_EARLY_LAUNCH(RouterLogitsRows);
+AINFER_EARLY_LAUNCH(RouterSelectRows);
+AINFER_EARLY_LAUNCH(EpGroupLocal);
+AINFER_EARLY_LAUNCH(EpGatherLocal);
+AINFER_EARLY_LAUNCH(SiluQuantRows);
+AINFER_EARLY_LAUNCH(EpCombine);
 
 }  // namespace ainfer

@@ -100,7 +100,7 @@ int EpMoe::alloc(T **p, size_t bytes) {
 }
 
 namespace {
-struct Rec {   // appends launches to a list; arguments by index in member order
+struct Rec {   // appends launches to a list (none: launches at once); arguments by index in member order
   EpMoe *e;
   ainfer_list_t list;
   int status = 0;
@@ -130,7 +130,10 @@ struct Rec {   // appends launches to a list; arguments by index in member order
     uint32_t idx = 0;
     (set(k, idx, args), ...);
     if (status) return;
-    if (ainfer_list_append_launch(list, k, groups) != AINFER_OK) { e->err = ainfer_last_error(e->dev); status = 1; }
+    if ((list ? ainfer_list_append_launch(list, k, groups) : ainfer_kernel_launch(e->dev, k, groups)) != AINFER_OK) {
+      e->err = ainfer_last_error(e->dev);
+      status = 1;
+    }
   }
   void copy(void *dst, const void *src, size_t bytes) {
     if (status) return;
@@ -153,7 +156,8 @@ int EpMoe::create(DeviceModel *model, const void *id128, int rank_, int world_, 
   n = batch / world;
   epr = E / world;
   cap = n * k;
-  if (cap > 2048 || batch * k > 2048) { err = "usage: batch x top-k above the planner's limit (2048 items)"; return 2; }
+  const int most = world == 1 && (flags & EP_LARGE) ? 8192 : 2048;
+  if (cap > most || batch * k > most) { err = "usage: batch x top-k above the planner's limit (" + std::to_string(most) + " items)"; return 2; }
   // shapes the dp4a kernel does not take run every expert as one tensor-core problem, which holds at most 64 rows
   if (batch > 64 && !(256 % (H / 128) == 0 && 256 % (I / 128) == 0)) { err = "usage: more than 64 rows need hidden and intermediate sizes whose group counts divide 256"; return 2; }
   slot_d = (uint32_t)((16 + (size_t)cap * 16 + (size_t)cap * item_bytes(H) + 15) & ~(size_t)15);
@@ -169,8 +173,10 @@ int EpMoe::create(DeviceModel *model, const void *id128, int rank_, int world_, 
   r |= alloc(&Logits, (size_t)n * (E + 1) * 4); r |= alloc(&Bias, (size_t)E * 4);
   r |= alloc(&SelIdx, (size_t)n * (k + 1) * 4); r |= alloc(&SelW, (size_t)n * (k + 1) * 4); r |= alloc(&NearGap, (size_t)n * 4);
   r |= alloc(&ItemDest, (size_t)cap * 4);
-  r |= alloc(&Send, (size_t)world * slot_d); r |= alloc(&Recv, (size_t)world * slot_d);
-  r |= alloc(&Ret, (size_t)world * slot_r); r |= alloc(&Back, (size_t)world * slot_r);
+  if (world > 1) {
+    r |= alloc(&Send, (size_t)world * slot_d); r |= alloc(&Recv, (size_t)world * slot_d);
+    r |= alloc(&Ret, (size_t)world * slot_r); r |= alloc(&Back, (size_t)world * slot_r);
+  }
   r |= alloc(&Sorted, (size_t)rows * 4); r |= alloc(&Counts, 32);
   r |= alloc(&GroupsGU, (size_t)2 * (epr + 1) * 32); r |= alloc(&GroupsD, (size_t)(epr + 1) * 32);
   const size_t nlarge = (size_t)epr + 1 + (size_t)rows / 64 + (size_t)n / 64 + 2;   // an expert with more than 64 rows is cut into 64-row problems
@@ -196,16 +202,57 @@ int EpMoe::create(DeviceModel *model, const void *id128, int rank_, int world_, 
   return 0;
 }
 
+namespace {
+// Norm and quantiser of `rows` owned rows, router logits, selection: the part both forms of the block begin with.
+int emit_route(EpMoe *e, Rec &r, int L, int rows) {
+  const ModelConfig &c = e->m->cfg;
+  const std::string p = layer_prefix(L);
+  DeviceTensor router = e->m->tensor(p + "mlp.gate.weight");
+  DeviceTensor sgate = e->m->tensor(p + "mlp.shared_expert_gate.weight");
+  if (!router.entry || (e->shared && !sgate.entry)) { e->err = "missing " + p + "mlp.gate.weight / shared_expert_gate.weight"; return 1; }
+  const bool add = (e->flags & EP_RES_ADD) != 0;
+  r.launch("RmsNormQuant", (uint32_t)rows, (const float *)e->Res, (const float *)(add ? e->Add : nullptr), (float *)(add ? e->ResSum : nullptr),
+           (const float *)(e->m->post_norm + (size_t)L * e->H), e->Hn, e->Q8, e->SQ, (int32_t)e->H, (float)c.rms_eps);
+  const int tpb = rows > 128 ? 16 : 8;   // tokens per block: fewer reads of the weights, or enough blocks
+  r.launch("RouterLogitsRows", (uint32_t)(((e->E + 1 + 31) / 32) * ((rows + tpb - 1) / tpb)), (const uint16_t *)router.data,
+           (const uint16_t *)(e->shared ? sgate.data : nullptr), (const float *)e->Hn,
+           (const float *)((e->flags & EP_ROUTER_BIAS) ? e->Bias : nullptr), e->Logits, (int32_t)e->E, (int32_t)e->H, (int32_t)rows, (int32_t)tpb);
+  r.launch("RouterSelectRows", (uint32_t)rows, (const float *)e->Logits, e->SelIdx, e->SelW, e->NearGap, (int32_t)e->E, (int32_t)e->k,
+           (int32_t)(e->shared ? 1 : 0));
+  return 0;
+}
+// The experts' products over the grouped rows: problems of GroupsGUL / GroupsDL.
+void emit_experts(EpMoe *e, Rec &r, int front, int shared_rows, int max_rows) {   // front: rows the received items may take
+  const uint32_t blocks = (uint32_t)(2 * e->sm_count);
+  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsGUL, (const int32_t *)(e->Counts + 3), (const int8_t *)e->XQs, (const float *)e->SQs,
+           e->GU, (int32_t)e->I, (int32_t)e->H, (int32_t)max_rows, (int32_t)(2 * e->I));
+  r.launch("SiluQuantRows", (uint32_t)(front + shared_rows), (const float *)e->GU, (const int32_t *)e->Counts, e->AQ, e->ASQ, (int32_t)e->I,
+           (int32_t)(e->world * e->cap), (int32_t)front);
+  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsDL, (const int32_t *)(e->Counts + 4), (const int8_t *)e->AQ, (const float *)e->ASQ,
+           e->Y2, (int32_t)e->H, (int32_t)e->I, (int32_t)max_rows, (int32_t)e->H);
+}
+// One rank: `rows` of its rows, no dispatch. (A dispatch buffer, its copy, the un-permute and its copy moved
+// every item's 2 KB four times and its 8 KB output three times; the planner walked all earlier items of each.)
+int emit_local(EpMoe *e, Rec &r, int L, int rows) {
+  if (emit_route(e, r, L, rows)) return 1;
+  const ExpertW *tab = (const ExpertW *)e->m->expert_tables + (size_t)L * (e->E + 1);
+  const int items = rows * e->k, shared_rows = e->shared ? rows : 0, cut = std::min(rows, 64);
+  r.launch("EpGroupLocal", 1u, (const int32_t *)e->SelIdx, tab, e->Sorted, e->ItemDest, e->GroupsGUL, e->GroupsDL, e->Counts, (int32_t)rows,
+           (int32_t)e->k, (int32_t)e->E, (int32_t)e->I, (int32_t)e->cap, (int32_t)shared_rows, (int32_t)cut);
+  r.launch("EpGatherLocal", (uint32_t)items, (const int8_t *)e->Q8, (const float *)e->SQ, (const int32_t *)e->Sorted, e->XQs, e->SQs, (int32_t)e->H,
+           (int32_t)e->k);
+  emit_experts(e, r, items, shared_rows, cut);
+  const float *res_in = (e->flags & EP_RES_ADD) ? e->ResSum : e->Res;   // what the combine adds the experts' outputs to
+  r.launch("EpCombine", (uint32_t)(rows * ((e->H + 255) / 256)), res_in, (const unsigned char *)e->Y2, (const int32_t *)e->ItemDest,
+           (const float *)e->SelW, (const float *)(e->shared ? e->Ysh : nullptr), e->X, e->Res, (int32_t)e->k, (int32_t)e->H, (uint32_t)0);
+  return r.status;
+}
+}  // namespace
+
 // Records the lists of one layer: [A, B, C] for several ranks, [all] for one.
 int EpMoe::record_layer(int L) {
-  const ModelConfig &c = m->cfg;
-  const int G = H / 128, rows = world * cap;
-  const std::string p = layer_prefix(L);
-  DeviceTensor router = m->tensor(p + "mlp.gate.weight");
-  DeviceTensor sgate = m->tensor(p + "mlp.shared_expert_gate.weight");
-  if (!router.entry || (shared && !sgate.entry)) { err = "missing " + p + "mlp.gate.weight / shared_expert_gate.weight"; return 1; }
+  const int rows = world * cap;
   const ExpertW *tab = (const ExpertW *)m->expert_tables + (size_t)L * (E + 1);
-  const float eps = (float)c.rms_eps;
   auto new_list = [&](ainfer_list_t *l) {
     if (ainfer_list_create(dev, l) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }
     impl->lists.push_back(*l);
@@ -216,52 +263,31 @@ int EpMoe::record_layer(int L) {
     if (ainfer_list_close(r.list) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }
     return 0;
   };
-  const uint32_t tc_blocks = (uint32_t)(2 * sm_count);
   ainfer_list_t la = nullptr;
   if (new_list(&la)) return 1;
   Rec r{this, la};
+  if (world == 1) return emit_local(this, r, L, n) ? 1 : close(r);
   // ---- A: route the owned rows and pack their items ----
   const float *res_in = (flags & EP_RES_ADD) ? ResSum : Res;   // what the combine adds the experts' outputs to
-  r.launch("RmsNormQuant", (uint32_t)n, (const float *)Res, (const float *)((flags & EP_RES_ADD) ? Add : nullptr),
-           (float *)((flags & EP_RES_ADD) ? ResSum : nullptr), (const float *)(m->post_norm + (size_t)L * H), Hn, Q8, SQ,
-           (int32_t)H, eps);
-  const int tpb = 4;   // tokens per block of the router: enough blocks to fill the device, weights re-read from L2
-  r.launch("RouterLogitsRows", (uint32_t)(((E + 1 + 7) / 8) * ((n + tpb - 1) / tpb)), (const uint16_t *)router.data,
-           (const uint16_t *)(shared ? sgate.data : nullptr), (const float *)Hn,
-           (const float *)((flags & EP_ROUTER_BIAS) ? Bias : nullptr), Logits, (int32_t)E, (int32_t)H, (int32_t)n, (int32_t)tpb);
-  r.launch("RouterSelectRows", (uint32_t)n, (const float *)Logits, SelIdx, SelW, NearGap, (int32_t)E, (int32_t)k, (int32_t)(shared ? 1 : 0));
+  if (emit_route(this, r, L, n)) return 1;
   r.launch("EpPlan", 1u, (const int32_t *)SelIdx, Send, ItemDest, (int32_t)n, (int32_t)k, (int32_t)epr, (int32_t)world, (int32_t)cap, slot_d);
   r.launch("EpPack", (uint32_t)cap, (const int8_t *)Q8, (const float *)SQ, (const int32_t *)ItemDest, Send, (int32_t)k, (int32_t)H, (int32_t)cap,
            slot_d);
-  if (world > 1) {
-    if (close(r) || new_list(&la)) return 1;
-    r.list = la;
-  } else {
-    r.copy(Recv, Send, slot_d);
-  }
+  if (close(r) || new_list(&la)) return 1;
+  r.list = la;
   // ---- B: the experts of this rank on everything received ----
   r.launch("EpGroup", 1u, (const unsigned char *)Recv, tab, Sorted, GroupsGU, GroupsD, GroupsGUL, GroupsDL, Counts, (int32_t)world, (int32_t)rank, (int32_t)epr,
            (int32_t)cap, (int32_t)I, slot_d, (int32_t)rows, (int32_t)(shared ? n : 0), (int32_t)E,
            (int32_t)0, (int32_t)64);   // every expert in the second pair of lists, in problems of at most 64 rows
   r.launch("EpGather", (uint32_t)rows, (const unsigned char *)Recv, (const int32_t *)Sorted, (const int32_t *)Counts, XQs, SQs, (int32_t)H,
            (int32_t)cap, slot_d);
-  r.launch("Int4GemmA8TcGrouped", tc_blocks, (const void *)GroupsGUL, (const int32_t *)(Counts + 3), (const int8_t *)XQs, (const float *)SQs, GU, (int32_t)I,
-           (int32_t)H, (int32_t)std::min(batch, 64), (int32_t)(2 * I));
-  r.launch("SiluQuantRows", (uint32_t)(rows + (shared ? n : 0)), (const float *)GU, (const int32_t *)Counts, AQ, ASQ, (int32_t)I, (int32_t)rows);
-  r.launch("Int4GemmA8TcGrouped", tc_blocks, (const void *)GroupsDL, (const int32_t *)(Counts + 4), (const int8_t *)AQ, (const float *)ASQ, Y2, (int32_t)H,
-           (int32_t)I, (int32_t)std::min(batch, 64), (int32_t)H);
+  emit_experts(this, r, rows, shared ? n : 0, std::min(batch, 64));
   r.launch("EpScatter", (uint32_t)rows, (const float *)Y2, (const int32_t *)Sorted, (const int32_t *)Counts, Ret, (int32_t)H, slot_r);
-  if (world > 1) {
-    if (close(r) || new_list(&la)) return 1;
-    r.list = la;
-  } else {
-    r.copy(Back, Ret, slot_r);
-  }
+  if (close(r) || new_list(&la)) return 1;
+  r.list = la;
   // ---- C: combine ----
   r.launch("EpCombine", (uint32_t)(n * ((H + 255) / 256)), res_in, (const unsigned char *)Back, (const int32_t *)ItemDest,
-           (const float *)SelW, (const float *)(shared ? Ysh : nullptr), X, (int32_t)k, (int32_t)H, slot_r);
-  r.copy(Res, X, (size_t)n * H * 4);   // the next layer's input: layers chain through "res"
-  (void)G;
+           (const float *)SelW, (const float *)(shared ? Ysh : nullptr), X, Res, (int32_t)k, (int32_t)H, slot_r);
   return close(r);
 }
 
@@ -318,7 +344,7 @@ int EpMoe::run_layer(int L, bool chain, float *seg_ms) {
     if (stamp(4)) return 1;
     EP_CHECK(ainfer_list_execute(impl->lists[i + 2]));
   }
-  (void)chain;   // the layer's last list already copies x to res
+  (void)chain;   // the layer's last kernel already writes x to res as well
   if (stamp(5)) return 1;
   if (seg_ms) {
     EP_CHECK(ainfer_sync(dev, ~0ull));
@@ -329,6 +355,13 @@ int EpMoe::run_layer(int L, bool chain, float *seg_ms) {
     }
   }
   return 0;
+}
+
+int EpMoe::run_rows(int L, int rows) {
+  if (world > 1) return run_layer(L, true, nullptr);
+  if (L < 0 || L >= m->cfg.layers + m->cfg.mtp_layers || rows < 0 || rows > n) { err = "usage: no such layer, or more rows than the block holds"; return 2; }
+  Rec r{this, nullptr};
+  return rows ? emit_local(this, r, L, rows) : 0;
 }
 
 int EpMoe::run_stack(int first, int count, float *seg_ms) {

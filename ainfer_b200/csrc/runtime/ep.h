@@ -11,7 +11,8 @@ namespace ainfer {
 
 enum EpFlags {
   EP_ROUTER_BIAS = 1,  // add the "router_bias" buffer to the routed experts' logits (load generators)
-  EP_RES_ADD = 2       // the block's residual input is "res" + "add" (the mixer's output not yet added)
+  EP_RES_ADD = 2,      // the block's residual input is "res" + "add" (the mixer's output not yet added)
+  EP_LARGE = 64        // one rank: up to 8192 (row, expert) items instead of 2048
 };
 
 // Fills 128 bytes with a fresh NCCL id (rank 0 calls, the caller hands it to every rank).
@@ -50,6 +51,8 @@ struct EpMoe {
   // 5 floats, accumulated): device time of route+pack, dispatch, experts, return, shared+combine;
   // asking for it synchronises after the layer.
   int run_layer(int L, bool chain, float *seg_ms);
+  // run_layer for the first `rows` owned rows (one rank: launched at once; several: all rows).
+  int run_rows(int L, int rows);
   int run_stack(int first, int count, float *seg_ms);
   void destroy();
 

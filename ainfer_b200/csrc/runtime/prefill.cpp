@@ -1,5 +1,5 @@
 // Chunked prefill: advances a session's state (DeltaNet state, conv history, INT8 KV cache) over a
-// run of prompt tokens, up to 64 rows at a time, instead of one decode step per token. The chunk
+// run of prompt tokens, up to 768 rows at a time, instead of one decode step per token. The chunk
 // orchestration of the reference (tools/cmdlist/chunklayer_replay.cpp:366-443: ChunkGemm,
 // ChunkSsmConv, ChunkSsmRecur, ChunkAttn per layer, state persisting across chunk replays) with
 // this library's row-batched kernels:
@@ -33,6 +33,7 @@ struct Prefill {
   EpMoe ep;
   bool ep_ready = false;
   int rows_cap = 64;
+  int att_rows = 64;                             // rows that attend at a time (their partials are the largest buffer)
   std::vector<void *> owned;
   // row buffers
   int32_t *Ctrl = nullptr, *OutT = nullptr;      // [rows][4], [rows]
@@ -125,7 +126,8 @@ int prefill_create(Session *s, int rows_cap, bool verify, Prefill **out, int ep_
     *out = p;
     return 0;
   }
-  const int R = p->rows_cap, H = c.hidden, C = c.conv_dim(), VD = c.value_dim(), nV = c.lin_v_heads;
+  p->att_rows = std::min(p->rows_cap, 192);
+  const int R = p->rows_cap, RA = p->att_rows, H = c.hidden, C = c.conv_dim(), VD = c.value_dim(), nV = c.lin_v_heads;
   const int QN = c.q_heads * 2 * c.head_dim, KN = c.kv_heads * c.head_dim, AK = c.q_heads * c.head_dim;
   const int maxK = std::max(H, std::max(VD, AK));
   int r = 0;
@@ -136,8 +138,8 @@ int prefill_create(Session *s, int rows_cap, bool verify, Prefill **out, int ep_
   r |= palloc(p, (size_t)R * nV, &p->Bt); r |= palloc(p, (size_t)R * nV, &p->Gt);
   r |= palloc(p, (size_t)R * VD, &p->O);
   r |= palloc(p, (size_t)R * QN, &p->Q16); r |= palloc(p, (size_t)R * KN, &p->K16); r |= palloc(p, (size_t)R * KN, &p->V16);
-  r |= palloc(p, (size_t)R * AK, &p->Qn); r |= palloc(p, (size_t)R * c.q_heads * s->max_chunks, &p->Pm);
-  r |= palloc(p, (size_t)R * c.q_heads * s->max_chunks, &p->Pse); r |= palloc(p, (size_t)R * c.q_heads * s->max_chunks * c.head_dim, &p->Pacc);
+  r |= palloc(p, (size_t)R * AK, &p->Qn); r |= palloc(p, (size_t)RA * c.q_heads * s->max_chunks, &p->Pm);
+  r |= palloc(p, (size_t)RA * c.q_heads * s->max_chunks, &p->Pse); r |= palloc(p, (size_t)RA * c.q_heads * s->max_chunks * c.head_dim, &p->Pacc);
   if (verify) {
     p->snap_s_stride = (size_t)c.n_lin() * nV * 128 * 128;
     p->snap_c_stride = (size_t)c.n_lin() * C * 3;
@@ -146,7 +148,7 @@ int prefill_create(Session *s, int rows_cap, bool verify, Prefill **out, int ep_
   }
   if (!r) {
     // the expert-parallel block counts rows over all ranks: every rank brings R of them
-    int e = p->ep.create(s->m, ep_world > 1 ? id128 : nullptr, ep_rank, ep_world, R * ep_world, EP_RES_ADD);
+    int e = p->ep.create(s->m, ep_world > 1 ? id128 : nullptr, ep_rank, ep_world, R * ep_world, EP_RES_ADD | EP_LARGE);
     if (e) { s->err = "prefill: " + p->ep.err; r = e; }
     else p->ep_ready = true;
   }
@@ -248,26 +250,30 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
         const size_t kv_off = (size_t)slot * s->max_ctx * nKV;
         int8_t *Kc = s->Kc + kv_off * D, *Vc = s->Vc + kv_off * D;
         uint16_t *Ks = s->Ks + kv_off, *Vs = s->Vs + kv_off;
-        // all rows at once, three launches: every row appends its K / V (its own cache position), then
-        // every row attends to the cache up to its own position (rows before it included: the appends of
-        // the whole pass are complete), then the merges. Per row the arithmetic is the decode kernels'.
-        auto attn = [&](const char *name, int groups) {
-          l.launch(name, (uint32_t)(rows * groups), (const float *)p->Q16, (const float *)p->K16, (const float *)p->V16,
-                   (const float *)(m->q_norm + (size_t)slot * D), (const float *)(m->k_norm + (size_t)slot * D), (const float *)m->rope_cos,
-                   (const float *)m->rope_sin, (const int32_t *)p->Ctrl, p->Qn, Kc, Vc, Ks, Vs, p->Pm, p->Pse, p->Pacc, p->Q8, p->SQ, (int32_t)nQ,
-                   (int32_t)nKV, (int32_t)c.rotary_dim, (int32_t)s->max_ctx, (int32_t)s->max_chunks, (int32_t)rows, (int32_t)groups, eps,
-                   (int64_t)0);
+        // every row appends its K / V (its own cache position); then, some rows at a time, every row
+        // attends to the cache up to its own position (rows before it included: the appends of the whole
+        // pass are complete), and the merges. Per row the arithmetic is the decode kernels'.
+        auto attn = [&](const char *name, int r0, int n_rows, int groups) {
+          l.launch(name, (uint32_t)(n_rows * groups), (const float *)(p->Q16 + (size_t)r0 * 2 * AK), (const float *)(p->K16 + (size_t)r0 * nKV * D),
+                   (const float *)(p->V16 + (size_t)r0 * nKV * D), (const float *)(m->q_norm + (size_t)slot * D),
+                   (const float *)(m->k_norm + (size_t)slot * D), (const float *)m->rope_cos, (const float *)m->rope_sin,
+                   (const int32_t *)(p->Ctrl + (size_t)r0 * 4), p->Qn + (size_t)r0 * AK, Kc, Vc, Ks, Vs, p->Pm, p->Pse, p->Pacc, p->Q8 + (size_t)r0 * AK,
+                   p->SQ + (size_t)r0 * (AK / 128), (int32_t)nQ, (int32_t)nKV, (int32_t)c.rotary_dim, (int32_t)s->max_ctx, (int32_t)s->max_chunks,
+                   (int32_t)n_rows, (int32_t)groups, eps, (int64_t)0);
         };
-        attn("BatchAttnPrep", (nQ + 2 * nKV + 7) / 8);
-        attn("BatchAttnSplit", std::max(1, std::min(s->max_chunks * nKV, (s->sm_count * 8 + rows - 1) / rows)));
-        attn("BatchAttnCombine", nQ);
+        attn("BatchAttnPrep", 0, rows, (nQ + 2 * nKV + 7) / 8);
+        for (int r0 = 0; r0 < rows; r0 += p->att_rows) {
+          const int some = std::min(p->att_rows, rows - r0);
+          attn("BatchAttnSplit", r0, some, std::max(1, std::min(s->max_chunks * nKV, (s->sm_count * 8 + some - 1) / some)));
+          attn("BatchAttnCombine", r0, some, nQ);
+        }
         l.gemm(m->tensor(pf + "self_attn.o_proj.weight"), p->Q8, p->SQ, ep.Add, AK, rows);
       } else {
         l.gemm(m->tensor(pf + "linear_attn.in_proj_qkv.weight"), p->Q8, p->SQ, p->Pq, H, rows);
         l.gemm(m->tensor(pf + "linear_attn.in_proj_z.weight"), p->Q8, p->SQ, p->Z, H, rows);
         l.gemm(m->tensor(pf + "linear_attn.in_proj_b.weight"), p->Q8, p->SQ, p->Br, H, rows);
         l.gemm(m->tensor(pf + "linear_attn.in_proj_a.weight"), p->Q8, p->SQ, p->Ar, H, rows);
-        l.launch("ChunkConvSilu", (uint32_t)((C + 255) / 256), p->Mx, (const float *)p->Pq, s->conv + (size_t)slot * C * 3,
+        l.launch("ChunkConvSilu", (uint32_t)((C + 255) / 256 * ((rows + 15) / 16)), p->Mx, (const float *)p->Pq, s->conv + (size_t)slot * C * 3,
                  (const float *)(m->conv_w + (size_t)slot * C * 4), (int32_t)C, (int32_t)rows,
                  (float *)(verify ? p->SnapC + (size_t)slot * C * 3 : nullptr), (int64_t)p->snap_c_stride);
         l.launch("ChunkBetaDecay", (uint32_t)((rows * nV + 255) / 256), (const float *)p->Br, (const float *)p->Ar,
@@ -284,8 +290,9 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
       if (l.recording) {
         l.cut(true);
       } else {
-        // x = (x + mixer) + MoE(norm(x + mixer)) for the rows; rows past `rows` hold stale values and are ignored
-        int e = ep.run_layer(L, true, nullptr);
+        // x = (x + mixer) + MoE(norm(x + mixer)) for the rows (several ranks: for all rows of the buffers, those past
+        // `rows` hold stale values and are ignored)
+        int e = ep.run_rows(L, rows);
         if (e) { s->err = "prefill: " + ep.err; return e; }
       }
     }
@@ -313,8 +320,10 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
       return e;
     }
   }
-  for (int t0 = 0; t0 < n; t0 += p->rows_cap) {
-    const int rows = std::min(p->rows_cap, n - t0);
+  // passes of equal size, as few as the buffers allow (several ranks: whole buffers, the ranks' calls must agree)
+  const int passes = std::max(1, (n + p->rows_cap - 1) / p->rows_cap), per = ep.world > 1 ? p->rows_cap : std::max(1, (n + passes - 1) / passes);
+  for (int t0 = 0; t0 < n; t0 += per) {
+    const int rows = std::min(per, n - t0);
     for (int i = 0; i < rows; ++i) {
       ctrl[4 * i] = tokens[t0 + i];
       ctrl[4 * i + 1] = start_pos + t0 + i;

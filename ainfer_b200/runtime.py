@@ -215,7 +215,7 @@ class Session:
         return tok.value, state.value
 
     def prefill(self, tokens, start_pos=0):
-        """Advances the state over the tokens in passes of up to 192 rows (no logits)."""
+        """Advances the state over the tokens in passes of up to 768 rows (no logits)."""
         t = np.ascontiguousarray(tokens, np.int32)
         _check(load().ainfer_session_prefill(self.h, t.ctypes.data_as(C.POINTER(C.c_int)), len(t), int(start_pos)))
 
@@ -227,7 +227,7 @@ class Session:
         return out
 
     def prefill_rows(self, rows):
-        """Rows per pass of the next prefill (rows x world x top-k <= 2048; default the largest multiple of 8 within that, at most 192)."""
+        """Rows per pass of the next prefill (one rank: rows x top-k <= 8192, default at most 768; several: rows x world x top-k <= 2048, default at most 192)."""
         _check(load().ainfer_session_prefill_rows(self.h, int(rows)))
 
     def prefill_ep(self, rank, world, nccl_id=None):

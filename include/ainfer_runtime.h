@@ -103,15 +103,16 @@ int ainfer_session_step(ainfer_session_t s, int token, int pos, int *out_token);
 int ainfer_session_generate(ainfer_session_t s, const int *prompt, int P, int G, int start_pos,
                             int *out_tokens, float *gen_ms);
 /* Chunked prefill: advances the session's state (DeltaNet state, conv history, INT8 KV cache) over
- * n tokens at positions start_pos.. in passes of up to 192 rows, without logits (chunk orchestration
+ * n tokens at positions start_pos.. in passes of up to 768 rows, without logits (chunk orchestration
  * of tools/cmdlist/chunklayer_replay.cpp:366-443). The state afterwards is bit-identical to n calls
  * of ainfer_session_step; follow with ainfer_session_generate(s, &last_prompt_id, 1, G, start_pos + n, ...). */
 int ainfer_session_prefill(ainfer_session_t s, const int *tokens, int n, int start_pos);
 /* The same, returning the logits [n_want][V] (host) of the listed rows: indices into tokens, ascending. */
 int ainfer_session_prefill_logits(ainfer_session_t s, const int *tokens, int n, int start_pos, const int *want, int n_want,
                                   float *out);
-/* Rows per pass of the next prefill object (1 <= rows, rows x world x top-k <= 2048; default: the
- * largest multiple of 8 within that bound, at most 192). Drops the current prefill object. */
+/* Rows per pass of the next prefill object (1 <= rows; at most what rows x world x top-k <= 2048 allows, on one
+ * rank rows x top-k <= 8192; default: the largest multiple of 8 within that bound, at most 192, on one rank
+ * 768). Drops the current prefill object. */
 int ainfer_session_prefill_rows(ainfer_session_t s, int rows);
 /* Expert parallelism for this session's prefill (config "prefill ... at 8 GPUs with expert
  * parallelism"): every rank prefills its OWN sequence, the MoE block of each pass exchanges rows
