@@ -72,6 +72,12 @@ __device__ __forceinline__ void timeline_mark(int id, bool any_block = false) {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
+// Barrier over every thread of the cluster's blocks; orders their shared-memory accesses.
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Control block words, tools/decode/decode_l0.cpp:41-43.
 enum { CTRL_TOKEN = 0, CTRL_POS = 1, CTRL_LEN = 2, CTRL_SELECTED = 3 };
 

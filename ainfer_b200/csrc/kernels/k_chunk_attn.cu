@@ -210,6 +210,144 @@ AINFER_REGISTER(ChunkAttnRowsF32, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_rows_
 AINFER_REGISTER(ChunkAttnRowsB16, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_rows_smem, CAR_FIELDS);
 #undef F
 
+// The same in fp32 for head sizes up to 128, as two small matrix products in registers. A block takes 32 rows of
+// one head against tiles of 64 keys; 16 lanes share four rows: a thread holds 4 x 4 scores (its keys 16 apart)
+// and 4 x DP / 16 sums. Bound by the fused multiply-adds: scores read eight 16-byte pieces of shared memory for
+// 64 of them, sums twelve for 128, where the form above read two words for each (and one key per lane). Rows are
+// padded by four floats, so eight lanes' pieces fall into different banks. Scores add up in the order of the
+// dimensions, sums in the order of the keys, as above. 777 rows, 8 heads of 128, one chunk: 762 us above, 159 here.
+constexpr int kCtRows = 32, kCtKeys = 64, kCtPP = kCtKeys + 4;
+template <int DP>
+__device__ __forceinline__ void chunk_attn_tile_body(const ChunkAttnRowsArgs &a) {
+  extern __shared__ __align__(16) float ca_smem[];   // q [32][DP + 4], k [64][DP + 4], weights [32][68]
+  constexpr int P = DP + 4, NC = DP / 64;
+  const int D = a.D, h = blockIdx.x % a.H, r0 = blockIdx.x / a.H * kCtRows, g = h / (a.H / a.G);
+  float *qs = ca_smem, *ks = qs + kCtRows * P, *ws = ks + kCtKeys * P;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int nr = min(kCtRows, a.rows - r0), KW = a.G * D;
+  const float *Q = reinterpret_cast<const float *>(a.Q) + (size_t)r0 * a.H * D + (size_t)h * D, *K = reinterpret_cast<const float *>(a.Kc) + (size_t)g * D;
+  const bool vec = (D & 3) == 0 && (((uintptr_t)a.Q | (uintptr_t)a.Kc) & 15) == 0;
+  auto load = [&](float *dst, const float *src, int d, bool in) {   // values d .. d + 3 of a row, zeros beyond D
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (in && vec && d < D) v = *reinterpret_cast<const float4 *>(src);
+    else if (in && d < D) v = make_float4(src[0], d + 1 < D ? src[1] : 0.0f, d + 2 < D ? src[2] : 0.0f, d + 3 < D ? src[3] : 0.0f);
+    *reinterpret_cast<float4 *>(dst) = v;
+  };
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int i = tid; i < kCtRows * (DP / 4); i += 128) {
+    const int rr = i / (DP / 4), d = i % (DP / 4) * 4;
+    load(qs + rr * P + d, Q + (size_t)rr * a.H * D + d, d, rr < nr);
+  }
+  const int pos0 = a.Ctrl[4 * r0 + CTRL_POS];
+  const float mul = a.scale, temp = a.Temp[h];
+  const float *lb = a.LB + (size_t)h * a.lb_len;
+  float m[4], l[4], acc[4][4 * NC];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY; l[i] = 0.0f;
+#pragma unroll
+    for (int x = 0; x < 4 * NC; ++x) acc[i][x] = 0.0f;
+  }
+  const int lo = pos0 - pos0 % a.chunk, hi = pos0 + nr - 1;
+  for (int k0 = lo; k0 <= hi; k0 += kCtKeys) {
+    __syncthreads();
+#pragma unroll 4
+    for (int i = tid; i < kCtKeys * (DP / 4); i += 128) {
+      const int kk = i / (DP / 4), d = i % (DP / 4) * 4, p = k0 + kk;
+      load(ks + kk * P + d, K + (size_t)(p % a.cap) * KW + d, d, p <= hi);
+    }
+    __syncthreads();
+    float s[4][4] = {};
+#pragma unroll 4
+    for (int d = 0; d < DP; d += 4) {
+      float4 q[4], k[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4 *>(qs + (ty * 4 + i) * P + d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4 *>(ks + (tx + 16 * j) * P + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          s[i][j] = fmaf(q[i].w, k[j].w, fmaf(q[i].z, k[j].z, fmaf(q[i].y, k[j].y, fmaf(q[i].x, k[j].x, s[i][j]))));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int p = pos0 + ty * 4 + i, first = p - p % a.chunk;
+      bool see[4];
+      float mx = m[i], sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int kp = k0 + tx + 16 * j;
+        see[j] = kp <= p && kp >= first && p <= hi;
+        s[i][j] = see[j] ? s[i][j] * mul * temp - lb[p - kp] : -INFINITY;
+        mx = fmaxf(mx, s[i][j]);
+      }
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, off));
+      const float base = mx == -INFINITY ? 0.0f : mx, corr = expf(m[i] - base);   // nothing visible yet: everything stays zero
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float w = see[j] ? expf(s[i][j] - base) : 0.0f;
+        sum += w;
+        ws[(ty * 4 + i) * kCtPP + tx + 16 * j] = w;
+      }
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
+      m[i] = mx;
+      l[i] = fmaf(l[i], corr, sum);
+#pragma unroll
+      for (int x = 0; x < 4 * NC; ++x) acc[i][x] *= corr;
+    }
+    __syncwarp();   // a row's weights are written and read by 16 lanes of one warp
+#pragma unroll 2
+    for (int j = 0; j < kCtKeys; j += 4) {
+      float4 w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4 *>(ws + (ty * 4 + i) * kCtPP + j);
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const float4 v = *reinterpret_cast<const float4 *>(ks + (j + jj) * P + 64 * c + tx * 4);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float wi = jj == 0 ? w[i].x : jj == 1 ? w[i].y : jj == 2 ? w[i].z : w[i].w;
+            acc[i][4 * c] = fmaf(wi, v.x, acc[i][4 * c]);
+            acc[i][4 * c + 1] = fmaf(wi, v.y, acc[i][4 * c + 1]);
+            acc[i][4 * c + 2] = fmaf(wi, v.z, acc[i][4 * c + 2]);
+            acc[i][4 * c + 3] = fmaf(wi, v.w, acc[i][4 * c + 3]);
+          }
+        }
+    }
+    __syncwarp();
+  }
+  float *O = reinterpret_cast<float *>(a.O) + (size_t)r0 * a.ldo + (size_t)h * D;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int rr = ty * 4 + i;
+    if (rr >= nr) continue;
+#pragma unroll
+    for (int x = 0; x < 4 * NC; ++x) {
+      const int d = x / 4 * 64 + tx * 4 + x % 4;
+      if (d < D) O[(size_t)rr * a.ldo + d] = acc[i][x] / l[i];
+    }
+  }
+}
+__global__ void __launch_bounds__(128) ChunkAttnTile64(const ChunkAttnRowsArgs a) { chunk_attn_tile_body<64>(a); }
+__global__ void __launch_bounds__(128) ChunkAttnTile128(const ChunkAttnRowsArgs a) { chunk_attn_tile_body<128>(a); }
+template <int DP>
+static uint32_t chunk_attn_tile_smem(const void *) {
+  return 4u * (uint32_t)((kCtRows + kCtKeys) * (DP + 4) + kCtRows * kCtPP);
+}
+#define F(f) AINFER_ARG(ChunkAttnRowsArgs, f)
+AINFER_REGISTER(ChunkAttnTile64, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<64>, CAR_FIELDS);
+AINFER_REGISTER(ChunkAttnTile128, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<128>, CAR_FIELDS);
+#undef F
+AINFER_EARLY_LAUNCH(ChunkAttnTile64);
+AINFER_EARLY_LAUNCH(ChunkAttnTile128);
+
 // ------------------------------------------------------- ChunkAttnStep ---
 // One decode step of every sequence: convolution, append, and attention over the sequence's current
 // chunk in one launch. Blocks: sequence x key head x split. A split takes a contiguous share of the

@@ -1,12 +1,13 @@
 // Dense layers with bf16 weights W [N][ldw] (rows padded with zeros to a multiple of 8 values).
 //
-//   LinearRows        fp32 activations, fp32 sums on the CUDA cores (the 32-bit form)
+//   LinearRows*       fp32 activations, fp32 sums on the CUDA cores (the 32-bit form)
 //   StreamGemv        one fp32 row, weights streamed once: y = act(W x + bias)
 //   HyperStreamGemv   the same, x made in the kernel from the residual streams: stream update of the
 //                     previous sublayer, weighted read, RMS norm, optional token shift (every block
 //                     makes the row for itself; block 0 stores the updated streams and the shift row)
 // act: 0 none, 1 relu squared, 2 cap tanh(v / cap).
 #include "hyper_core.cuh"
+#include "linear_rows.cuh"
 #include "stream_gemv.cuh"
 
 namespace ainfer {
@@ -20,49 +21,88 @@ struct LinearRowsArgs {
   int32_t rows, N, K, ldx, ldw, ldy, act;
   float cap;
 };
-constexpr int kLrTile = 64, kLrK = 16;
-__global__ void __launch_bounds__(256) LinearRows(const LinearRowsArgs a) {
+// Tiles of BM rows and BN outputs; the CL blocks of a cluster share a tile, each a part of K (whole steps of 16),
+// and add their sums up in rank order through shared memory, each for its share of the tile's rows.
+// 64 x 64 tiles for rows in plenty, 16 x 128 for up to 16: a tile of 64 would multiply zeros mostly.
+template <int BM, int BN, int CL>
+__device__ __forceinline__ void linear_rows_body(const LinearRowsArgs &a) {
+  using Tile = LinearRowsTile<BM, BN>;
+  __shared__ __align__(16) union { typename Tile::Shared tiles; float sums[BM][BN]; } sh;
+  const int nt = (a.N + BN - 1) / BN, t = blockIdx.x / CL, rank = CL > 1 ? blockIdx.x % CL : 0;
+  const int n0 = t % nt * BN, r0 = t / nt * BM, nr = min(BM, a.rows - r0);
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float xs[kLrK][kLrTile + 4], ws[kLrK][kLrTile + 4];
-  const int nt = (a.N + kLrTile - 1) / kLrTile;
-  const int n0 = (blockIdx.x % nt) * kLrTile, r0 = (blockIdx.x / nt) * kLrTile;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < a.K; k0 += kLrK) {
-    for (int i = tid; i < kLrTile * kLrK; i += 256) {
-      const int rr = i / kLrK, k = i % kLrK;
-      const bool kin = k0 + k < a.K;
-      xs[k][rr] = kin && r0 + rr < a.rows ? a.X[(size_t)(r0 + rr) * a.ldx + k0 + k] : 0.0f;
-      ws[k][rr] = kin && n0 + rr < a.N ? bf16_to_f32(a.W[(size_t)(n0 + rr) * a.ldw + k0 + k]) : 0.0f;
+  const int steps = (a.K + kLrK - 1) / kLrK, per = (steps + CL - 1) / CL;
+  Tile c;
+  if (nr > 0)
+    c.run(sh.tiles, a.X + (size_t)r0 * a.ldx, a.ldx, nr, a.W + (size_t)n0 * a.ldw, a.ldw, a.N - n0, min(a.K, rank * per * kLrK),
+          min(a.K, (rank + 1) * per * kLrK));
+  auto put = [&](int r, int n, const float (&v)[4]) {   // four outputs of a row
+    if (r >= nr) return;
+    float *y = a.Y + (size_t)(r0 + r) * a.ldy;
+    float o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = n + j < a.N ? apply_act(v[j] + (a.Bias ? a.Bias[n + j] : 0.0f), a.act, a.cap) : 0.0f;
+    if (n + 3 < a.N && ((a.ldy & 3) == 0 && ((uintptr_t)a.Y & 15) == 0)) {
+      *reinterpret_cast<float4 *>(y + n) = make_float4(o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (n + j < a.N) y[n + j] = o[j];
     }
-    __syncthreads();
+  };
+  if constexpr (CL == 1) {
 #pragma unroll
-    for (int k = 0; k < kLrK; ++k) {
-      float xv[4], wv[4];
+    for (int i = 0; i < Tile::TM; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) { xv[i] = xs[k][ty * 4 + i]; wv[i] = ws[k][tx * 4 + i]; }
+      for (int j = 0; j < Tile::TN; j += 4) {
+        const float v[4] = {c.acc[i][j], c.acc[i][j + 1], c.acc[i][j + 2], c.acc[i][j + 3]};
+        put(Tile::row(i), n0 + Tile::col(j), v);
+      }
+  } else {
+    __syncthreads();   // the last step's readers are done
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < Tile::TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv[i], wv[j], acc[i][j]);
+      for (int j = 0; j < Tile::TN; j += 4)
+        *reinterpret_cast<float4 *>(&sh.sums[Tile::row(i)][Tile::col(j)]) = make_float4(c.acc[i][j], c.acc[i][j + 1], c.acc[i][j + 2], c.acc[i][j + 3]);
+    cluster_sync_all();
+    for (int i = threadIdx.x; i < BM * BN / CL / 4; i += kLrThreads) {
+      const int r = rank * (BM / CL) + i / (BN / 4), n = i % (BN / 4) * 4;
+      uint32_t at = smem_addr(&sh.sums[r][n]);
+      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int s = 0; s < CL; ++s) {
+        uint32_t peer;
+        float p[4];
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(s));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p[0]), "=f"(p[1]), "=f"(p[2]), "=f"(p[3]) : "r"(peer) : "memory");
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] += p[j];
+      }
+      put(r, n0 + n, v);
     }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r0 + ty * 4 + i;
-    if (r >= a.rows) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < a.N) a.Y[(size_t)r * a.ldy + n] = apply_act(acc[i][j] + (a.Bias ? a.Bias[n] : 0.0f), a.act, a.cap);
-    }
+    cluster_sync_all();   // a block's sums stay until every reader is done
   }
 }
 #define F(f) AINFER_ARG(LinearRowsArgs, f)
-AINFER_REGISTER(LinearRows, LinearRowsArgs, 256, 0, 0, nullptr, F(X), F(W), F(Bias), F(Y), F(rows), F(N), F(K), F(ldx), F(ldw), F(ldy),
-                F(act), F(cap));
+#define LR_FIELDS F(X), F(W), F(Bias), F(Y), F(rows), F(N), F(K), F(ldx), F(ldw), F(ldy), F(act), F(cap)
+#define LR_KERNEL(NAME, BM, BN, CL)                                                                                                        \
+  __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kLrThreads) NAME(const LinearRowsArgs a) { linear_rows_body<BM, BN, CL>(a); } \
+  AINFER_REGISTER(NAME, LinearRowsArgs, kLrThreads, 0, 0, nullptr, LR_FIELDS);                                                             \
+  AINFER_EARLY_LAUNCH(NAME)
+__global__ void __launch_bounds__(kLrThreads) LinearRows(const LinearRowsArgs a) { linear_rows_body<64, 64, 1>(a); }
+AINFER_REGISTER(LinearRows, LinearRowsArgs, kLrThreads, 0, 0, nullptr, LR_FIELDS);
+AINFER_EARLY_LAUNCH(LinearRows);
+__global__ void __launch_bounds__(kLrThreads) LinearRowsFew(const LinearRowsArgs a) { linear_rows_body<16, 128, 1>(a); }
+AINFER_REGISTER(LinearRowsFew, LinearRowsArgs, kLrThreads, 0, 0, nullptr, LR_FIELDS);
+AINFER_EARLY_LAUNCH(LinearRowsFew);
+LR_KERNEL(LinearRowsSplit2, 64, 64, 2);
+LR_KERNEL(LinearRowsSplit4, 64, 64, 4);
+LR_KERNEL(LinearRowsSplit8, 64, 64, 8);
+LR_KERNEL(LinearRowsFewSplit2, 16, 128, 2);
+LR_KERNEL(LinearRowsFewSplit4, 16, 128, 4);
+LR_KERNEL(LinearRowsFewSplit8, 16, 128, 8);
 #undef F
 
 // ---------------------------------------------------------- StreamGemv ---
@@ -184,7 +224,6 @@ __global__ void __launch_bounds__(256) PackRowsBf16(const PackRowsBf16Args a) {
 AINFER_REGISTER(PackRowsBf16, PackRowsBf16Args, 256, 0, 0, nullptr, F(Dst), F(Src), F(N), F(K), F(ld));
 #undef F
 
-AINFER_EARLY_LAUNCH(LinearRows);
 AINFER_EARLY_LAUNCH(StreamGemv);
 AINFER_EARLY_LAUNCH(HyperStreamGemv);
 

@@ -281,10 +281,6 @@ __host__ __device__ inline uint32_t lts_stages(int nt) {
   const uint32_t s = ((uint32_t)kLtBudget / 2 + 8192 - (uint32_t)nt * 512u) / lt_stage_bytes(nt);
   return s > 8 ? 8 : s;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 template <int CL>
 __device__ __forceinline__ void linear_tc_split(const LinearTcArgs &a) {
   extern __shared__ __align__(1024) unsigned char lt_smem_raw[];

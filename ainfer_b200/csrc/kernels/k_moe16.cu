@@ -8,7 +8,7 @@
 // experts' outputs there, and the consumer of the outputs adds each row's up by place and weight.
 // Decode step: ExpertUpStreamGemv chooses for itself in every block and streams the chosen experts'
 // rows only; ExpertDownStreamGemv adds the experts' outputs in rank order.
-#include "row_types.cuh"
+#include "linear_rows.cuh"
 #include "stream_gemv.cuh"
 
 namespace ainfer {
@@ -191,52 +191,32 @@ struct LinearRowsGroupedArgs {
   const int32_t *Count;
   int32_t N, K, ldx, ldw, ldy, act;
 };
-constexpr int kLgTile = 64, kLgK = 16;
-__global__ void __launch_bounds__(256) LinearRowsGrouped(const LinearRowsGroupedArgs a) {
+__global__ void __launch_bounds__(kLrThreads) LinearRowsGrouped(const LinearRowsGroupedArgs a) {
+  using Tile = LinearRowsTile<64, 64>;
+  __shared__ __align__(16) Tile::Shared sh;
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float xs[kLgK][kLgTile + 4], ws[kLgK][kLgTile + 4];
-  const int n_tiles = (a.N + kLgTile - 1) / kLgTile, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int units = a.Count[0] * n_tiles;
+  const int n_tiles = (a.N + 63) / 64, units = a.Count[0] * n_tiles;
   for (int u = blockIdx.x; u < units; u += gridDim.x) {
     const int4 t = a.Tiles[u / n_tiles];
-    const int n0 = (u % n_tiles) * kLgTile;
-    const uint16_t *W = a.W + (size_t)t.x * a.N * a.ldw;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < a.K; k0 += kLgK) {
-      for (int i = tid; i < kLgTile * kLgK; i += 256) {
-        const int rr = i / kLgK, k = i % kLgK;
-        const bool kin = k0 + k < a.K;
-        xs[k][rr] = kin && rr < t.z ? a.X[(size_t)(t.y + rr) * a.ldx + k0 + k] : 0.0f;
-        ws[k][rr] = kin && n0 + rr < a.N ? bf16_to_f32(W[(size_t)(n0 + rr) * a.ldw + k0 + k]) : 0.0f;
-      }
-      __syncthreads();
+    const int n0 = (u % n_tiles) * 64;
+    Tile c;
+    __syncthreads();   // the last unit's readers are done
+    if (t.z > 0) c.run(sh, a.X + (size_t)t.y * a.ldx, a.ldx, t.z, a.W + ((size_t)t.x * a.N + n0) * a.ldw, a.ldw, a.N - n0, 0, a.K);
 #pragma unroll
-      for (int k = 0; k < kLgK; ++k) {
-        float xv[4], wv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { xv[i] = xs[k][ty * 4 + i]; wv[i] = ws[k][tx * 4 + i]; }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv[i], wv[j], acc[i][j]);
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty * 4 + i;
+    for (int i = 0; i < Tile::TM; ++i) {
+      const int r = Tile::row(i);
       if (r >= t.z) continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int n = n0 + tx * 4 + j;
-        if (n < a.N) a.Y[(size_t)(t.y + r) * a.ldy + n] = apply_act(acc[i][j], a.act, 0.0f);
+      for (int j = 0; j < Tile::TN; ++j) {
+        const int n = n0 + Tile::col(j);
+        if (n < a.N) a.Y[(size_t)(t.y + r) * a.ldy + n] = apply_act(c.acc[i][j], a.act, 0.0f);
       }
     }
   }
 }
 #define F(f) AINFER_ARG(LinearRowsGroupedArgs, f)
-AINFER_REGISTER(LinearRowsGrouped, LinearRowsGroupedArgs, 256, 0, 0, nullptr, F(X), F(W), F(Y), F(Tiles), F(Count), F(N), F(K), F(ldx), F(ldw),
+AINFER_REGISTER(LinearRowsGrouped, LinearRowsGroupedArgs, kLrThreads, 0, 0, nullptr, F(X), F(W), F(Y), F(Tiles), F(Count), F(N), F(K), F(ldx), F(ldw),
                 F(ldy), F(act));
 #undef F
 

@@ -148,8 +148,16 @@ int RowEngineBase::alloc_bytes(size_t bytes, void **out) {
 void RowEngineBase::linear(KernelCalls &k, const RowMatrix &mt, const char *Xp, int ldx, int rows, void *Yp, int ldy, int act, bool out16, float cap) {
   if (k.status) return;
   if (f32) {
-    k.launch("LinearRows", (uint32_t)(((mt.N + 63) / 64) * ((rows + 63) / 64)), (const float *)Xp, mt.w, mt.bias, (float *)Yp, (int32_t)rows,
-             (int32_t)mt.N, (int32_t)mt.K, (int32_t)ldx, (int32_t)mt.ldw, (int32_t)ldy, (int32_t)act, cap);
+    // Tiles of 64 x 64, or 16 x 128 for up to 16 rows. A block of 64 threads multiplies alone on a quarter of an SM's
+    // schedulers, so K is split over a cluster until there are four blocks an SM, down to 128 columns a block.
+    const bool few = rows <= 16;
+    const int tiles = few ? (mt.N + 127) / 128 : ((mt.N + 63) / 64) * ((rows + 63) / 64);
+    int cl = 0;
+    while (cl < 3 && (tiles << cl) < 4 * sm_count && mt.K >= (256 << cl)) ++cl;
+    static const char *const names[2][4] = {{"LinearRows", "LinearRowsSplit2", "LinearRowsSplit4", "LinearRowsSplit8"},
+                                            {"LinearRowsFew", "LinearRowsFewSplit2", "LinearRowsFewSplit4", "LinearRowsFewSplit8"}};
+    k.launch(names[few][cl], (uint32_t)(tiles << cl), (const float *)Xp, mt.w, mt.bias, (float *)Yp, (int32_t)rows, (int32_t)mt.N, (int32_t)mt.K,
+             (int32_t)ldx, (int32_t)mt.ldw, (int32_t)ldy, (int32_t)act, cap);
     return;
   }
   const int n_tiles = (mt.N + 127) / 128, kb = (mt.K + 63) / 64;

@@ -345,10 +345,13 @@ struct Engine : RowEngineBase {
           k.launch(sized("ChunkAttnMma", r.dim).c_str(), (uint32_t)(((R + 63) / 64) * r.heads), (const uint16_t *)Q, (const uint16_t *)s.k, lw.lb,
                    lw.temp, sp.ctrl, (uint16_t *)Att, (int32_t)R, (int32_t)r.heads, (int32_t)r.kv_heads, (int32_t)r.dim, (int32_t)s.cap,
                    (int32_t)s.chunk, (int32_t)lw.lb_len, (int32_t)ldo, (float)r.scale);
-        else
-          k.launch(f32 ? "ChunkAttnRowsF32" : "ChunkAttnRowsB16", (uint32_t)(((R + 15) / 16) * r.heads), (const void *)Q, (const void *)s.k, lw.lb,
+        else {
+          const bool tile = f32 && r.dim <= 128;   // the registers of larger heads' sums would spill
+          k.launch(tile ? r.dim <= 64 ? "ChunkAttnTile64" : "ChunkAttnTile128" : f32 ? "ChunkAttnRowsF32" : "ChunkAttnRowsB16",
+                   (uint32_t)(tile ? (R + 31) / 32 * r.heads : (R + 15) / 16 * r.heads), (const void *)Q, (const void *)s.k, lw.lb,
                    lw.temp, sp.ctrl, (void *)Att, (int32_t)R, (int32_t)r.heads, (int32_t)r.kv_heads, (int32_t)r.dim, (int32_t)s.cap,
                    (int32_t)s.chunk, (int32_t)lw.lb_len, (int32_t)ldo, (float)r.scale);
+        }
       } else {
         attn_step(k, r, lw, s, sp.ctrl, R, C, ldo, b16);
       }

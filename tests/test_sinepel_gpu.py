@@ -222,6 +222,29 @@ def test_chunk_attention_over_rows(dev, T, H, G, D, chunk, cap, kind):
         close(got, want[start:], 1e-5 if kind == "f32" else 3e-2)
 
 
+@pytest.mark.parametrize("T,H,G,D,chunk,cap,first", [(1, 2, 1, 128, 10, 64, 9), (32, 4, 2, 64, 100, 128, 0), (33, 3, 3, 5, 1, 64, 7), (65, 4, 1, 128, 64, 130, 63),
+                                                     (150, 8, 2, 96, 61, 212, 400), (129, 2, 2, 65, 1000, 1129, 871), (97, 2, 1, 128, 64, 256, 1000)])
+def test_chunk_attention_in_tiles_32bit(dev, T, H, G, D, chunk, cap, first):
+    """Rows first .. first + T - 1 with the keys of their chunks in a ring that has turned."""
+    lo, n = first - first % chunk, min(chunk, 512)
+    total = first + T - lo
+    assert total <= cap
+    q, k, r1, r2, temp = _attn_case(total, H, G, D, chunk, T)
+    want = P.shared_kv_attention(q.double(), k.double(), 0.25, temp.double(), r1.double(), r2.double(), chunk).reshape(total, H * D)[first - lo:]
+    ring = torch.full((cap, G * D), 7.0)
+    for i in range(total):
+        ring[(lo + i) % cap] = k[i].reshape(G * D)
+    ldo = H * D + 3
+    o = dev.zeros(T * ldo * 4)
+    dev.kernel("ChunkAttnTile64" if D <= 64 else "ChunkAttnTile128")(
+        -(-T // 32) * H, dev.upload(f32(q[first - lo:].reshape(T, H * D))), dev.upload(f32(ring)), _table(dev, r1, r2, max(n, total)), dev.upload(f32(temp)),
+        dev.upload(ctrl(range(first, first + T))), o, T, H, G, D, cap, chunk, max(n, total), ldo, 0.25)
+    dev.sync()
+    got = dev.download(o, (T, ldo), np.float32)
+    close(got[:, :H * D], want, 1e-5)
+    assert not got[:, H * D:].any()
+
+
 @pytest.mark.parametrize("kind", ["f32", "b16", "mma"])
 @pytest.mark.parametrize("H,G,D,chunk,taps,splits", [(16, 1, 96, 190, 3, 4), (4, 2, 192, 130, 4, 3), (4, 2, 256, 64, 2, 2), (4, 2, 16, 24, 3, 1), (6, 2, 20, 100, 1, 5), (8, 1, 64, 150, 4, 2), (3, 3, 33, 1, 2, 3),
                                                      (4, 4, 128, 90, 4, 8), (12, 2, 40, 200, 5, 16)])
@@ -282,6 +305,26 @@ def test_linear_rows_32bit(dev, R, N, K, act):
     dev.kernel("LinearRows")(-(-N // 64) * (-(-R // 64)), dev.upload(f32(x)), dev.upload(bits(wp)), dev.upload(f32(b)), y, R, N, K, K, ldw, N + 2,
                              act, 3.0)
     close(dev.download(y, (R, N + 2), np.float32)[:, :N], ACTS[act](x.double() @ w.double().T + b.double(), 3.0), 1e-5)
+
+
+@pytest.mark.parametrize("few", [False, True])
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("R,N,K,act,pad", [(1, 5, 7, 1, 0), (16, 128, 16, 0, 4), (64, 64, 128, 2, 4), (65, 129, 1000, 0, 0), (15, 260, 530, 1, 2), (130, 200, 4096, 0, 4)])
+def test_linear_rows_32bit_tiles(dev, R, N, K, act, pad, splits, few):
+    """Edges of both tiles, K in parts (empty ones too), rows of 16-byte alignment and others."""
+    g = torch.Generator().manual_seed(R)
+    x, w, b = torch.randn(R, K, generator=g), bf16(torch.randn(N, K, generator=g)), torch.randn(N, generator=g)
+    ldw, ldx, ldy = -(-K // 8) * 8, K + pad, N + pad
+    wp, xp = torch.full((N, ldw), 3.0), torch.full((R, ldx), float("nan"))   # what lies beyond K is not read as a value
+    wp[:, :K], xp[:, :K] = w.float(), x
+    y = dev.zeros(R * ldy * 4)
+    bm, bn = (16, 128) if few else (64, 64)
+    dev.kernel("LinearRows" + ("Few" if few else "") + (f"Split{splits}" if splits > 1 else ""))(
+        -(-N // bn) * -(-R // bm) * splits, dev.upload(f32(xp)), dev.upload(bits(wp)), dev.upload(f32(b)), y, R, N, K, ldx, ldw, ldy, act, 3.0)
+    dev.sync()
+    got = dev.download(y, (R, ldy), np.float32)
+    close(got[:, :N], ACTS[act](x.double() @ w.double().T + b.double(), 3.0), 1e-5)
+    assert not got[:, N:].any()
 
 
 @pytest.mark.parametrize("R,N,K,nt,splits,act,out16", [
