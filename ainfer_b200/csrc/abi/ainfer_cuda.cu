@@ -69,6 +69,7 @@ struct ainfer_device_s {
   cudaStream_t stream = nullptr;
   std::string err;
   uint64_t launches = 0;
+  bool last_early = false;   // the queue's last entry was an immediate launch of a kernel with early_launch
   void *flush_buf = nullptr;
   size_t flush_bytes = 0;
   int sm_count = 0;
@@ -289,24 +290,28 @@ int ainfer_mem_free(ainfer_device_t dev, void *ptr) {
 }
 int ainfer_memcpy_h2d(ainfer_device_t dev, void *dst, const void *src, size_t bytes) {
   if (!dev) return AINFER_ERR_INVALID;
+  dev->last_early = false;
   CU(dev, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, dev->stream));
   CU(dev, cudaStreamSynchronize(dev->stream));
   return AINFER_OK;
 }
 int ainfer_memcpy_d2h(ainfer_device_t dev, void *dst, const void *src, size_t bytes) {
   if (!dev) return AINFER_ERR_INVALID;
+  dev->last_early = false;
   CU(dev, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, dev->stream));
   CU(dev, cudaStreamSynchronize(dev->stream));
   return AINFER_OK;
 }
 int ainfer_memcpy_d2d(ainfer_device_t dev, void *dst, const void *src, size_t bytes) {
   if (!dev) return AINFER_ERR_INVALID;
+  dev->last_early = false;
   CU(dev, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, dev->stream));
   CU(dev, cudaStreamSynchronize(dev->stream));
   return AINFER_OK;
 }
 int ainfer_mem_fill(ainfer_device_t dev, void *dst, int byte_value, size_t bytes) {
   if (!dev) return AINFER_ERR_INVALID;
+  dev->last_early = false;
   CU(dev, cudaMemsetAsync(dst, byte_value, bytes, dev->stream));
   CU(dev, cudaStreamSynchronize(dev->stream));
   return AINFER_OK;
@@ -323,11 +328,13 @@ int ainfer_host_free(ainfer_device_t dev, void *ptr) {
 }
 int ainfer_memcpy_h2d_async(ainfer_device_t dev, void *dst, const void *src, size_t bytes) {
   if (!dev) return AINFER_ERR_INVALID;
+  dev->last_early = false;
   CU(dev, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, dev->stream));
   return AINFER_OK;
 }
 int ainfer_memcpy_d2h_async(ainfer_device_t dev, void *dst, const void *src, size_t bytes) {
   if (!dev) return AINFER_ERR_INVALID;
+  dev->last_early = false;
   CU(dev, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, dev->stream));
   return AINFER_OK;
 }
@@ -480,20 +487,38 @@ int ainfer_kernel_max_groups(ainfer_kernel_t k, uint32_t *groups) {
   return AINFER_OK;
 }
 
-int ainfer_kernel_launch(ainfer_device_t dev, ainfer_kernel_t k, uint32_t groups) {
+static int launch_kernel(ainfer_device_t dev, ainfer_kernel_t k, uint32_t groups, bool next) {
   if (!dev || !k) return AINFER_ERR_INVALID;
   uint32_t smem = 0;
   CU(dev, cudaSetDevice(dev->ordinal));  // function attributes and launches go to the current device
   int r = check_launch(k, groups, &smem);
   if (r) return r;
   void *params[1] = {k->args.data()};
-  if (k->desc->cooperative)
+  if (k->desc->cooperative) {
     CU(dev, cudaLaunchCooperativeKernel(k->desc->fn, dim3(groups), dim3(k->desc->threads), params, smem, dev->stream));
-  else
+  } else if (next && dev->last_early && k->desc->early_launch && dev->early_launch) {
+    // As an edge of a recorded list: the kernel's blocks come up while the predecessor drains and wait there
+    // (griddepcontrol.wait). Both sides must be such kernels: what another kernel wrote may be fetched before the wait.
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cf = {};
+    cf.gridDim = dim3(groups);
+    cf.blockDim = dim3(k->desc->threads);
+    cf.dynamicSmemBytes = smem;
+    cf.stream = dev->stream;
+    cf.attrs = &at;
+    cf.numAttrs = 1;
+    CU(dev, cudaLaunchKernelExC(&cf, k->desc->fn, params));
+  } else {
     CU(dev, cudaLaunchKernel(k->desc->fn, dim3(groups), dim3(k->desc->threads), params, smem, dev->stream));
+  }
+  dev->last_early = k->desc->early_launch != 0;
   dev->launches += 1;
   return AINFER_OK;
 }
+int ainfer_kernel_launch(ainfer_device_t dev, ainfer_kernel_t k, uint32_t groups) { return launch_kernel(dev, k, groups, false); }
+int ainfer_kernel_launch_next(ainfer_device_t dev, ainfer_kernel_t k, uint32_t groups) { return launch_kernel(dev, k, groups, true); }
 
 int ainfer_list_create(ainfer_device_t dev, ainfer_list_t *out) {
   if (!dev || !out) return AINFER_ERR_INVALID;
@@ -611,6 +636,7 @@ int ainfer_list_execute(ainfer_list_t l) {
   if (!l) return AINFER_ERR_INVALID;
   if (!l->closed) return fail(l->dev, AINFER_ERR_INVALID, "execute of a list that is not closed");
   CU(l->dev, cudaSetDevice(l->dev->ordinal));
+  l->dev->last_early = false;
   CU(l->dev, cudaGraphLaunch(l->exec, l->dev->stream));
   l->dev->launches += l->launches;
   return AINFER_OK;
@@ -692,6 +718,7 @@ int ainfer_flush_l2(ainfer_device_t dev) {
     dev->flush_bytes = (size_t)256 << 20;
     CU(dev, cudaMalloc(&dev->flush_buf, dev->flush_bytes));
   }
+  dev->last_early = false;
   CU(dev, cudaMemsetAsync(dev->flush_buf, 0, dev->flush_bytes, dev->stream));
   return AINFER_OK;
 }
@@ -739,6 +766,7 @@ int ainfer_router_topk_static(ainfer_device_t dev, const void *router, const voi
     }
     scratch = g_router_static_ptr[dev->ordinal];
   }
+  dev->last_early = false;
   cudaError_t e = router_static_launch(dev->stream, scratch, router, shared_gate, hn, sel_idx, sel_w, near_gap,
                                        experts, hidden, top_k);
   if (e != cudaSuccess) return fail(dev, AINFER_ERR_DEVICE, std::string("ainfer_router_topk_static: ") + cudaGetErrorString(e));

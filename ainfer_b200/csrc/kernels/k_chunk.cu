@@ -25,6 +25,8 @@ struct ChunkConvSiluArgs {
 // 192 rows of 8192 channels; runs of 16 rows 12 us.) The first run's threads read the history, and so they
 // are the ones that replace it.
 __global__ void __launch_bounds__(256) ChunkConvSilu(const ChunkConvSiluArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int cb = (a.C + 255) / 256, runs = max(1, (int)gridDim.x / cb), run = blockIdx.x / cb;
   const int c = (blockIdx.x % cb) * 256 + threadIdx.x;
   const int per = (a.M + runs - 1) / runs, m0 = run * per, m1 = min(m0 + per, a.M);
@@ -65,6 +67,8 @@ struct ChunkBetaDecayArgs {
   int32_t nV, count;     // count = M * nV
 };
 __global__ void __launch_bounds__(256) ChunkBetaDecay(const ChunkBetaDecayArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= a.count) return;
   const int h = i % a.nV;
@@ -100,6 +104,8 @@ extern __shared__ __align__(16) float chunk_smem[];
 // q and k meanwhile and fetch its values. Bound by the chain of a row. (Segments in different warps, two
 // block barriers a row: 130 us for 192 rows of 32 heads; this form 58.)
 __global__ void __launch_bounds__(kChunkThreads) ChunkDeltaNet(const ChunkDeltaNetArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int D = 128, SEG = kDnSeg;
   __shared__ float s_beta[2][kChunkRows], s_gt[2][kChunkRows];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -237,5 +243,9 @@ AINFER_REGISTER(ChunkBetaDecay, ChunkBetaDecayArgs, 256, 256, 0, nullptr, F(B), 
 #define F(f) AINFER_ARG(ChunkDeltaNetArgs, f)
 AINFER_REGISTER(ChunkDeltaNet, ChunkDeltaNetArgs, kChunkThreads, 1, 0, chunk_dn_smem_fn, F(Out), F(Mx), F(S), F(Bt), F(Gt), F(nK), F(nV), F(M), F(Snap), F(snap_stride));
 #undef F
+
+AINFER_EARLY_LAUNCH(ChunkConvSilu);
+AINFER_EARLY_LAUNCH(ChunkBetaDecay);
+AINFER_EARLY_LAUNCH(ChunkDeltaNet);
 
 }  // namespace ainfer

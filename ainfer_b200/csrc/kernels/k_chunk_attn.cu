@@ -99,8 +99,16 @@ __device__ __forceinline__ void short_conv_body(const ShortConvRowsArgs &a) {
     else st_val(reinterpret_cast<T *>(a.Kc) + (size_t)seq * a.kv_stride + (size_t)(pos % a.cap) * Kn + (c - a.Qc), y);
   }
 }
-__global__ void __launch_bounds__(256) ShortConvRowsF32(const ShortConvRowsArgs a) { short_conv_body<float>(a); }
-__global__ void __launch_bounds__(256) ShortConvRowsB16(const ShortConvRowsArgs a) { short_conv_body<uint16_t>(a); }
+__global__ void __launch_bounds__(256) ShortConvRowsF32(const ShortConvRowsArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  short_conv_body<float>(a);
+}
+__global__ void __launch_bounds__(256) ShortConvRowsB16(const ShortConvRowsArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  short_conv_body<uint16_t>(a);
+}
 #define F(f) AINFER_ARG(ShortConvRowsArgs, f)
 #define CONV_FIELDS                                                                                                                \
   F(U), F(CW), F(State), F(Pend), F(Ctrl), F(Seq), F(First), F(Q), F(Kc), F(kv_stride), F(rows), F(C), F(Qc), F(taps), F(cap), \
@@ -198,8 +206,16 @@ __device__ __forceinline__ void chunk_attn_rows_body(const ChunkAttnRowsArgs &a)
     }
   }
 }
-__global__ void __launch_bounds__(128) ChunkAttnRowsF32(const ChunkAttnRowsArgs a) { chunk_attn_rows_body<float>(a); }
-__global__ void __launch_bounds__(128) ChunkAttnRowsB16(const ChunkAttnRowsArgs a) { chunk_attn_rows_body<uint16_t>(a); }
+__global__ void __launch_bounds__(128) ChunkAttnRowsF32(const ChunkAttnRowsArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  chunk_attn_rows_body<float>(a);
+}
+__global__ void __launch_bounds__(128) ChunkAttnRowsB16(const ChunkAttnRowsArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  chunk_attn_rows_body<uint16_t>(a);
+}
 static uint32_t chunk_attn_rows_smem(const void *args) {
   const int D = ((const ChunkAttnRowsArgs *)args)->D;
   return 4u * (uint32_t)(kCaRows * D + kCaKeys * (D + 1));
@@ -233,8 +249,6 @@ __device__ __forceinline__ void chunk_attn_tile_body(const ChunkAttnRowsArgs &a)
     else if (in && d < D) v = make_float4(src[0], d + 1 < D ? src[1] : 0.0f, d + 2 < D ? src[2] : 0.0f, d + 3 < D ? src[3] : 0.0f);
     *reinterpret_cast<float4 *>(dst) = v;
   };
-  pdl_launch_dependents();
-  pdl_wait();
   for (int i = tid; i < kCtRows * (DP / 4); i += 128) {
     const int rr = i / (DP / 4), d = i % (DP / 4) * 4;
     load(qs + rr * P + d, Q + (size_t)rr * a.H * D + d, d, rr < nr);
@@ -252,7 +266,7 @@ __device__ __forceinline__ void chunk_attn_tile_body(const ChunkAttnRowsArgs &a)
   const int lo = pos0 - pos0 % a.chunk, hi = pos0 + nr - 1;
   for (int k0 = lo; k0 <= hi; k0 += kCtKeys) {
     __syncthreads();
-#pragma unroll 4
+#pragma unroll 8
     for (int i = tid; i < kCtKeys * (DP / 4); i += 128) {
       const int kk = i / (DP / 4), d = i % (DP / 4) * 4, p = k0 + kk;
       load(ks + kk * P + d, K + (size_t)(p % a.cap) * KW + d, d, p <= hi);
@@ -345,8 +359,10 @@ static uint32_t chunk_attn_tile_smem(const void *) {
 AINFER_REGISTER(ChunkAttnTile64, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<64>, CAR_FIELDS);
 AINFER_REGISTER(ChunkAttnTile128, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<128>, CAR_FIELDS);
 #undef F
-AINFER_EARLY_LAUNCH(ChunkAttnTile64);
-AINFER_EARLY_LAUNCH(ChunkAttnTile128);
+AINFER_EARLY_LAUNCH(ShortConvRowsF32);
+AINFER_EARLY_LAUNCH(ShortConvRowsB16);
+AINFER_EARLY_LAUNCH(ChunkAttnRowsF32);
+AINFER_EARLY_LAUNCH(ChunkAttnRowsB16);
 
 // ------------------------------------------------------- ChunkAttnStep ---
 // One decode step of every sequence: convolution, append, and attention over the sequence's current

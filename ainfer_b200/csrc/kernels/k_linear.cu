@@ -89,11 +89,9 @@ __device__ __forceinline__ void linear_rows_body(const LinearRowsArgs &a) {
 #define LR_FIELDS F(X), F(W), F(Bias), F(Y), F(rows), F(N), F(K), F(ldx), F(ldw), F(ldy), F(act), F(cap)
 #define LR_KERNEL(NAME, BM, BN, CL)                                                                                                        \
   __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kLrThreads) NAME(const LinearRowsArgs a) { linear_rows_body<BM, BN, CL>(a); } \
-  AINFER_REGISTER(NAME, LinearRowsArgs, kLrThreads, 0, 0, nullptr, LR_FIELDS);                                                             \
-  AINFER_EARLY_LAUNCH(NAME)
+  AINFER_REGISTER(NAME, LinearRowsArgs, kLrThreads, 0, 0, nullptr, LR_FIELDS)
 __global__ void __launch_bounds__(kLrThreads) LinearRows(const LinearRowsArgs a) { linear_rows_body<64, 64, 1>(a); }
 AINFER_REGISTER(LinearRows, LinearRowsArgs, kLrThreads, 0, 0, nullptr, LR_FIELDS);
-AINFER_EARLY_LAUNCH(LinearRows);
 __global__ void __launch_bounds__(kLrThreads) LinearRowsFew(const LinearRowsArgs a) { linear_rows_body<16, 128, 1>(a); }
 AINFER_REGISTER(LinearRowsFew, LinearRowsArgs, kLrThreads, 0, 0, nullptr, LR_FIELDS);
 AINFER_EARLY_LAUNCH(LinearRowsFew);
@@ -103,6 +101,11 @@ LR_KERNEL(LinearRowsSplit8, 64, 64, 8);
 LR_KERNEL(LinearRowsFewSplit2, 16, 128, 2);
 LR_KERNEL(LinearRowsFewSplit4, 16, 128, 4);
 LR_KERNEL(LinearRowsFewSplit8, 16, 128, 8);
+// The 64 x 64 tiles do not come up early: the blocks would gather on the SMs that the predecessor leaves first, and
+// a launch of a few blocks an SM lasts as long as the fullest one (777-token prompt 1720 us, with early blocks 1860).
+AINFER_EARLY_LAUNCH(LinearRowsFewSplit2);
+AINFER_EARLY_LAUNCH(LinearRowsFewSplit4);
+AINFER_EARLY_LAUNCH(LinearRowsFewSplit8);
 #undef F
 
 // ---------------------------------------------------------- StreamGemv ---

@@ -130,7 +130,9 @@ struct Rec {   // appends launches to a list (none: launches at once); arguments
     uint32_t idx = 0;
     (set(k, idx, args), ...);
     if (status) return;
-    if ((list ? ainfer_list_append_launch(list, k, groups) : ainfer_kernel_launch(e->dev, k, groups)) != AINFER_OK) {
+    // several ranks: exchanges enter the queue between launches
+    if ((list ? ainfer_list_append_launch(list, k, groups)
+              : e->world == 1 ? ainfer_kernel_launch_next(e->dev, k, groups) : ainfer_kernel_launch(e->dev, k, groups)) != AINFER_OK) {
       e->err = ainfer_last_error(e->dev);
       status = 1;
     }

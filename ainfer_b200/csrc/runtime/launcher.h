@@ -17,6 +17,7 @@ struct KernelCalls {
   ainfer_list_t list = nullptr;
   int status = 0;             // first failure; later calls do nothing
   uint64_t launches = 0;
+  bool begun = false;         // a launch went to the queue: later ones continue its chain
 
   KernelCalls(ainfer_device_t d, std::map<std::string, ainfer_kernel_t> *k, std::string *e, ainfer_list_t l = nullptr)
       : dev(d), kernels(k), err(e), list(l) {}
@@ -49,7 +50,10 @@ struct KernelCalls {
     (set(k, idx, args), ...);
     if (status) return;
     if (groups == 0) groups = 1;
-    const int rc = list ? ainfer_list_append_launch(list, k, groups) : ainfer_kernel_launch(dev, k, groups);
+    const int rc = list    ? ainfer_list_append_launch(list, k, groups)
+                   : begun ? ainfer_kernel_launch_next(dev, k, groups)
+                           : ainfer_kernel_launch(dev, k, groups);
+    begun = true;
     if (rc != AINFER_OK) fail(1, std::string(name) + ": " + ainfer_last_error(dev));
     ++launches;
   }

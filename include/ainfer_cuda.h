@@ -121,6 +121,10 @@ int ainfer_list_execute(ainfer_list_t list);
 /* Immediate launch outside any list (the SYCL loop's q.submit,
  * tools/decode/decode.cpp:432-477), asynchronous on the execution queue. */
 int ainfer_kernel_launch(ainfer_device_t dev, ainfer_kernel_t k, uint32_t group_count);
+/* The same for the next kernel of a chain: the caller states that nothing but this library's launches
+ * entered the queue since the chain's first launch, and that the chain writes no weights. A kernel that
+ * waits for its predecessor by itself may then start up while that one drains, as in a recorded list. */
+int ainfer_kernel_launch_next(ainfer_device_t dev, ainfer_kernel_t k, uint32_t group_count);
 /* zeFenceHostSynchronize + zeFenceReset, decode_l0.cpp:717-718. timeout_ns ==
  * UINT64_MAX blocks; otherwise polls and returns AINFER_ERR_TIMEOUT. */
 int ainfer_sync(ainfer_device_t dev, uint64_t timeout_ns);
