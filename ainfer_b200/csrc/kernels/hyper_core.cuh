@@ -24,6 +24,29 @@ __device__ __forceinline__ void load_stream_coef(StreamCoef &c, const float *Mix
   }
 }
 
+// Four consecutive elements whose streams x and sublayer output y are in registers: u, and the updated streams
+// to dst when dst != null. The arithmetic of stream_step.
+template <int ST>
+__device__ __forceinline__ void stream_update(const float4 (&x)[ST], const float4 y, float *dst, const StreamCoef &c, int W, bool update, float (&u)[4]) {
+  float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  auto add = [](float4 &to, float m, const float4 v) {
+    to.x = fmaf(m, v.x, to.x); to.y = fmaf(m, v.y, to.y); to.z = fmaf(m, v.z, to.z); to.w = fmaf(m, v.w, to.w);
+  };
+#pragma unroll
+  for (int t = 0; t < ST; ++t) {
+    float4 a = x[t];
+    if (update) {
+      const float o = c.out[t];
+      a = make_float4(o * y.x, o * y.y, o * y.z, o * y.w);
+#pragma unroll
+      for (int s = 0; s < ST; ++s) add(a, c.mix[s * ST + t], x[s]);
+      if (dst) *reinterpret_cast<float4 *>(dst + (size_t)t * W) = a;
+    }
+    add(r, c.in[t], a);
+  }
+  u[0] = r.x; u[1] = r.y; u[2] = r.z; u[3] = r.w;
+}
+
 // V consecutive elements of a row (V = 4: 16-byte accesses, 1: single elements), ST streams. Returns
 // u; writes the updated streams when dst != null.
 template <int ST, int V>

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kSgThreads, 4) StreamGemv(const StreamGemvArgs
     gemv_produce(c, d, &sh, sg_smem);
   } else {
     pdl_wait();
-    for (int k = threadIdx.x; k < a.ldw; k += kSgWarps * 32) sg_put(lo, hi, k, k < a.K ? a.X[k] : 0.0f);
+    sg_row(lo, hi, a.X, a.K, a.ldw, threadIdx.x, kSgWarps * 32);
     asm volatile("bar.sync 1, 256;" ::: "memory");
     gemv_consume(c, d, &sh, sg_smem, lo, hi, part);
   }
@@ -160,7 +160,62 @@ struct HyperStreamGemvArgs {
   int32_t S, N, K, ldw, rows_pb, act;
   float eps, cap;
 };
-__global__ void __launch_bounds__(kSgThreads, 4) HyperStreamGemv(const HyperStreamGemvArgs a) {
+// The row of up to 2048 elements in whole quads and up to four streams: everything that does not come from the sublayer
+// before (norm weights, shift, the last position's row) is in registers before the dependency wait, the streams
+// and the sublayer's output are one round of loads after it. In loops (as below) every element's norm weight,
+// shift and last row were one more round each.
+constexpr int kHgQuads = 2;
+template <int ST>
+__device__ __forceinline__ void hyper_row_ahead(const HyperStreamGemvArgs &a, const StreamCoef &coef, float *lo, float *hi, float *red) {
+  const int K = a.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = kSgWarps * 32;
+  const int pos = a.Shift ? a.Ctrl[CTRL_POS] : 0;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 nw[kHgQuads], sf[kHgQuads], pv[kHgQuads];
+#pragma unroll
+  for (int q = 0; q < kHgQuads; ++q) {
+    const int k = (q * nth + tid) * 4;
+    nw[q] = k < K ? ld_val4(a.NormW + k) : zero;
+    sf[q] = a.Shift && k < K ? ld_val4(a.Shift + k) : zero;
+    pv[q] = a.Shift && pos > 0 && k < K ? ld_val4(a.State + (size_t)((pos - 1) & 1) * K + k) : zero;   // of the step before
+  }
+  pdl_wait();
+  const bool update = a.Yp != nullptr;
+  float4 x[kHgQuads][ST], y[kHgQuads];
+#pragma unroll
+  for (int q = 0; q < kHgQuads; ++q) {
+    const int k = (q * nth + tid) * 4;
+#pragma unroll
+    for (int s = 0; s < ST; ++s) x[q][s] = k < K ? ld_val4(a.Xin + (size_t)s * K + k) : zero;
+    y[q] = update && k < K ? ld_val4(a.Yp + k) : zero;
+  }
+  float *dst = blockIdx.x == 0 ? a.Xout : nullptr;
+  float u[kHgQuads][4], ss = 0.0f;
+#pragma unroll
+  for (int q = 0; q < kHgQuads; ++q) {
+    const int k = (q * nth + tid) * 4;
+    stream_update<ST>(x[q], y[q], dst && k < K ? dst + k : nullptr, coef, K, update, u[q]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss = fmaf(u[q][i], u[q][i], ss);
+  }
+  ss = warp_tree_sum(ss);
+  if (lane == 0) red[warp] = ss;
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  ss = warp_tree_sum(lane < kSgWarps ? red[lane] : 0.0f);
+  const float inv = 1.0f / sqrtf(ss / (float)K + a.eps);
+  float *next = a.Shift && blockIdx.x == 0 ? a.State + (size_t)(pos & 1) * K : nullptr;
+#pragma unroll
+  for (int q = 0; q < kHgQuads; ++q) {
+    const int k = (q * nth + tid) * 4;
+    float4 v = make_float4(u[q][0] * inv * nw[q].x, u[q][1] * inv * nw[q].y, u[q][2] * inv * nw[q].z, u[q][3] * inv * nw[q].w);
+    if (next && k < K) st_val4(next + k, v);
+    if (a.Shift) {
+      v.x = fmaf(pv[q].x - v.x, sf[q].x, v.x); v.y = fmaf(pv[q].y - v.y, sf[q].y, v.y);
+      v.z = fmaf(pv[q].z - v.z, sf[q].z, v.z); v.w = fmaf(pv[q].w - v.w, sf[q].w, v.w);
+    }
+    if (k < a.ldw) st_val4(((k & 4) ? hi : lo) + (k >> 3) * 4, v);   // zeros between K and ldw
+  }
+}
+__global__ void __launch_bounds__(kSgThreads, 3) HyperStreamGemv(const HyperStreamGemvArgs a) {
   __shared__ GemvShared sh;
   __shared__ StreamCoef coef;
   __shared__ float red[33];
@@ -174,6 +229,13 @@ __global__ void __launch_bounds__(kSgThreads, 4) HyperStreamGemv(const HyperStre
   gemv_init(&sh, d.nst);
   if (tid >= nth) {
     gemv_produce(c, d, &sh, sg_smem);
+  } else if (stream_vec(a.S, K) && K <= kHgQuads * nth * 4) {
+    if (a.S == 4) hyper_row_ahead<4>(a, coef, lo, hi, red);
+    else if (a.S == 3) hyper_row_ahead<3>(a, coef, lo, hi, red);
+    else if (a.S == 2) hyper_row_ahead<2>(a, coef, lo, hi, red);
+    else hyper_row_ahead<1>(a, coef, lo, hi, red);
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    gemv_consume(c, d, &sh, sg_smem, lo, hi, part);
   } else {
     const int lane = tid & 31, warp = tid >> 5;
     pdl_wait();

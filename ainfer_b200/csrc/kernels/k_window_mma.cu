@@ -223,6 +223,8 @@ struct WindowAttnStepMmaArgs {
   float scale, softcap, eps;
 };
 constexpr int kWsStages = 2, kWsMaxSplits = 16;
+// As the chunk form, positions and the first tile (rows of earlier steps) are fetched before the dependency wait. Where
+// another layer of the same step appends the rows (koff < 0), the tile that ends in the step's own row waits.
 template <int DP>
 __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs &a) {
   extern __shared__ __align__(128) unsigned char sm_raw[];
@@ -248,6 +250,7 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
       for (int d = lane; d < E; d += 32) vn[d] = f32_to_bf16(u[a.voff + (size_t)g * E + d]);
   };
   if (split == a.splits) {
+    pdl_wait();
     const bool done = a.own_pool && a.pool > 0 && (pos + 1) % a.pool == 0;
     if (!fresh && !done) return;
     new_key();
@@ -287,9 +290,13 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
     }
     cpa_commit();
   };
-  for (int i = 0; i < kWsStages - 1; ++i) fetch(t0 + i);
-  for (int i = tid; i < 16 * LD; i += 128) Qs[i] = 0;
+  static_assert(kWsStages == 2, "one tile is fetched ahead");
+  const bool ahead = fresh || t0 != nt - 1;
+  if (ahead) fetch(t0);
+  for (int i = tid; i < 16 * LD / 2; i += 128) reinterpret_cast<uint32_t *>(Qs)[i] = 0;
   __syncthreads();
+  pdl_wait();
+  if (!ahead) fetch(t0);
   for (int hh = warp; hh < HG; hh += 4)
     head_norm_turn(u + (size_t)(g * HG + hh) * D, D, a.QN, a.eps, rot, a.rd, [&](int d, float x, float y, bool both) { st_pair(Qs + hh * LD + d, x, y, both); });
   new_key();
@@ -429,7 +436,6 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
 #define WINDOW_STEP(DP)                                                                                              \
   __global__ void __launch_bounds__(128) WindowAttnStepMma##DP(const __grid_constant__ WindowAttnStepMmaArgs a) {    \
     pdl_launch_dependents();                                                                                         \
-    pdl_wait();                                                                                                      \
     window_step_mma_body<DP>(a);                                                                                     \
   }                                                                                                                  \
   static uint32_t window_step_smem##DP(const void *) { return (16 + 2 + 2 * kWsStages * kCmKeys) * (DP + 8) * 2; }   \

@@ -39,6 +39,30 @@ __host__ __device__ inline GemvDims gemv_dims(int ldw) {
 // 16-byte reads: element k of piece k / 8 lies in half (k / 4) % 2 at (k / 8) * 4 + k % 4.
 __device__ __forceinline__ void sg_put(float *lo, float *hi, int k, float v) { ((k & 4) ? hi : lo)[(k >> 3) * 4 + (k & 3)] = v; }
 
+// K values at x as that vector, zeros up to ldw. Rounds of four quads a thread with their loads in flight together
+// (a value a thread and round waited for memory K / 256 times).
+__device__ __forceinline__ void sg_row(float *lo, float *hi, const float *x, int K, int ldw, int tid, int nth) {
+  if ((K & 3) || (reinterpret_cast<unsigned long long>(x) & 15)) {
+    for (int k = tid; k < ldw; k += nth) sg_put(lo, hi, k, k < K ? x[k] : 0.0f);
+    return;
+  }
+  constexpr int Q = 4;
+  for (int k0 = tid * 4; k0 < ldw; k0 += nth * 4 * Q) {
+    float4 v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int k = k0 + q * nth * 4;
+      v[q] = *reinterpret_cast<const float4 *>(x + min(k, K - 4));
+      if (k >= K) v[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int k = k0 + q * nth * 4;
+      if (k < ldw) *reinterpret_cast<float4 *>(((k & 4) ? hi : lo) + (k >> 3) * 4) = v[q];
+    }
+  }
+}
+
 struct GemvShape {
   const uint16_t *W;
   const float *Bias;

@@ -425,7 +425,10 @@ struct Engine : RowEngineBase {
     ldw = round_up((int)W, 8);
     ldq = round_up((int)maxA, 8);
     ldf = round_up((int)maxF, 8);
-    att_splits = step_splits(maxG);
+    int span = 1;
+    for (const RowLayerConfig &r : c.row_layers)
+      if (r.heads) span = std::max(span, std::min(window_of(r), max_ctx) + (r.pool > 0 ? max_ctx / r.pool : 0));
+    att_splits = step_splits(maxG, span);
     for (int i = 0; i < 2; ++i) e |= alloc(R * W, &X[i]);
     e |= alloc(R * ldw * esz(), &H); e |= alloc(R * maxU, &U); e |= alloc(R * maxQ * esz(), &Q);
     e |= alloc(R * ldq * 4, &Att); e |= alloc(y_rows * W, &Y); e |= alloc(R * ldf * 4, &Z);

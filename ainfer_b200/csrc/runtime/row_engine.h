@@ -75,10 +75,17 @@ struct RowEngineBase : RowEngine {
       if (dim <= d) return base + std::to_string(d);
     return base + std::string("256");
   }
-  // blocks of a step's attention over sequences, key heads and splits: few tiles each when there are many sequences
-  int step_splits(int max_kv_heads) const {
-    if (nseq == 1) return std::max(1, std::min(16, 2 * sm_count / max_kv_heads));
-    return std::max(1, std::min(16, 8 * sm_count / (std::min(nseq, 8 * sm_count) * max_kv_heads)));
+  // Blocks of a step's attention per (sequence, key head), at most 16: a launch lasts whole rounds of blocks (three fit
+  // an SM), a block its tiles of 64 keys and about four tiles' time for its start and the merge. `span`: keys a step may see.
+  int step_splits(int max_kv_heads, int span) const {
+    const long pairs = (long)nseq * max_kv_heads, tiles = std::max(1, (span + 63) / 64);
+    int best = 1;
+    long cost = -1;
+    for (int s = 1; s <= 16; ++s) {
+      const long rounds = (pairs * s + 3 * sm_count - 1) / (3 * sm_count), c = rounds * ((tiles + s - 1) / s + 4);
+      if (cost < 0 || c < cost) { cost = c; best = s; }
+    }
+    return best;
   }
 };
 
