@@ -310,8 +310,8 @@ struct Engine : RowEngineBase {
   void hyper(KernelCalls &k, const RowSpan &sp, const float *in, const float *norm, const RowLayerWeights *lw, const LayerState *s, int rows,
              const int32_t *idx, bool store) {
     const ModelConfig &c = m->cfg;
-    // a run of rows per block when rows are plentiful: the token shift re-reads one row per run
-    const int per = lw ? std::max(1, std::min(8, rows / (2 * sm_count))) : 1;
+    // runs of rows, so that two blocks an SM take all: a run loads its weights once and, with token shift, one row again
+    const int per = std::max(1, std::min(8, (rows + 2 * sm_count - 1) / (2 * sm_count)));
     k.launch(f32 ? "HyperNormRowsF32" : "HyperNormRowsB16", (uint32_t)((rows + per - 1) / per), (const float *)X[cur],
              (const float *)(pending ? Y : nullptr), (const float *)(pending ? pending->mix : nullptr),
              (const float *)(pending ? pending->out : nullptr), (float *)(pending && store ? X[cur ^ 1] : nullptr), in, norm,

@@ -385,6 +385,19 @@ def test_decode_gemv_from_streams(dev, S, K, N, pos, shift):
         assert np.array_equal(got[(pos - 1) & 1], f32(st)[(pos - 1) & 1])
 
 
+@pytest.mark.parametrize("S,K,N,pos,shift", [(4, 2048, 40, 5, True), (3, 1028, 15, 2, True), (1, 2044, 8, 0, True), (2, 2040, 9, 3, False), (4, 2052, 10, 4, True)])
+def test_decode_gemv_from_wide_streams(dev, S, K, N, pos, shift):
+    """Around the widest row that is held in registers, and rows that end inside a piece of eight."""
+    test_decode_gemv_from_streams(dev, S, K, N, pos, shift)
+
+
+@pytest.mark.parametrize("out", ["f32", "b16"])
+@pytest.mark.parametrize("W,S,per", [(1024, 4, 8), (1028, 4, 3), (2048, 4, 2), (2052, 4, 3), (2048, 3, 5), (2044, 2, 1), (1020, 1, 3), (4, 4, 2)])
+def test_wide_stream_update_read_norm_and_shift(dev, W, S, per, out):
+    """The same around the widths where a thread holds one quad of a row more, and the widest that is held."""
+    test_stream_update_read_norm_and_shift(dev, W, S, per, out)
+
+
 # -------------------------------------------------------------------- models ---
 L = P.make_layer
 MODELS = {
