@@ -221,6 +221,7 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
   const float *u0 = a.U + (size_t)seq * a.ldu;
   const int slot = pos % a.taps;
   auto channel = [&](int i) { return i >= HG * D ? Qc + g * D + (i - HG * D) : g * HG * D + i; };
+#pragma unroll 1
   for (int i = tid * 4; i < (HG + 1) * D; i += 512) {
     const int c = channel(i);
     float4 y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -255,6 +256,7 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
   penalties(t0);
   __syncthreads();   // Qs is clear
   pdl_wait();
+#pragma unroll 2
   for (int i = tid * 4; i < (HG + 1) * D; i += 512) {
     const bool isk = i >= HG * D;
     const int c = channel(i);
@@ -275,6 +277,7 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
   for (int d = 0; d < DP / 8; ++d)
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[d][i] = 0.0f;
+#pragma unroll 1
   for (int t = t0; t <= t1; ++t) {
     const int k0 = t * kCmKeys + warp * 16;
     cpa_wait<kSmStages - 2>();
@@ -348,6 +351,7 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
   // partials of a (sequence, key head): sums [splits][HG][D], then (maximum, sum) [splits][HG][2]
   float *base_p = a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (D + 4);   // D + 4 keeps 16-byte alignment
   float *base_m = base_p + (size_t)a.splits * HG * D;
+#pragma unroll 1
   for (int i = tid; i < HG * D; i += 128) {
     const int hh = i / D, d = i - hh * D;
     const float M = fmaxf(fmaxf(wm[0][hh], wm[1][hh]), fmaxf(wm[2][hh], wm[3][hh]));
@@ -378,12 +382,14 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
   __threadfence();
   // every split's factor exp2(m_s - M) / L, then the sums with the loads of all splits in flight
   float *fac = os;   // [HG][kSmMaxSplits]
+#pragma unroll 1
   for (int hh = warp; hh < HG; hh += 4) {
     const float2 ml = lane < active ? __ldcg(reinterpret_cast<const float2 *>(base_m) + lane * HG + hh) : make_float2(-INFINITY, 0.0f);
     const float M = warp_max(ml.x), f = fast_exp2(ml.x - M), L = warp_tree_sum(ml.y * f);
     if (lane < kSmMaxSplits) fac[hh * kSmMaxSplits + lane] = lane < active ? f / L : 0.0f;
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = tid * 4; i < HG * D; i += 512) {
     const int hh = i / D;
     const float *p = base_p + i, *f = fac + hh * kSmMaxSplits;

@@ -160,10 +160,10 @@ struct HyperStreamGemvArgs {
   int32_t S, N, K, ldw, rows_pb, act;
   float eps, cap;
 };
-// The row of up to 2048 elements in whole quads and up to four streams: everything that does not come from the sublayer
+// The row of up to 2048 elements in whole quads and four streams: everything that does not come from the sublayer
 // before (norm weights, shift, the last position's row) is in registers before the dependency wait, the streams
 // and the sublayer's output are one round of loads after it. In loops (as below) every element's norm weight,
-// shift and last row were one more round each.
+// shift and last row were one more round each. (One number of streams only: every other one is as much code again.)
 constexpr int kHgQuads = 2;
 template <int ST>
 __device__ __forceinline__ void hyper_row_ahead(const HyperStreamGemvArgs &a, const StreamCoef &coef, float *lo, float *hi, float *red) {
@@ -229,36 +229,33 @@ __global__ void __launch_bounds__(kSgThreads, 3) HyperStreamGemv(const HyperStre
   gemv_init(&sh, d.nst);
   if (tid >= nth) {
     gemv_produce(c, d, &sh, sg_smem);
-  } else if (stream_vec(a.S, K) && K <= kHgQuads * nth * 4) {
-    if (a.S == 4) hyper_row_ahead<4>(a, coef, lo, hi, red);
-    else if (a.S == 3) hyper_row_ahead<3>(a, coef, lo, hi, red);
-    else if (a.S == 2) hyper_row_ahead<2>(a, coef, lo, hi, red);
-    else hyper_row_ahead<1>(a, coef, lo, hi, red);
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    gemv_consume(c, d, &sh, sg_smem, lo, hi, part);
   } else {
-    const int lane = tid & 31, warp = tid >> 5;
-    pdl_wait();
-    float ss = stream_row_any(a.Xin, a.Yp, blockIdx.x == 0 ? a.Xout : nullptr, coef, a.S, K, a.Yp != nullptr, us, tid, nth);
-    ss = warp_tree_sum(ss);
-    if (lane == 0) red[warp] = ss;
-    asm volatile("bar.sync 1, 256;" ::: "memory");   // also: every thread's u is visible
-    ss = warp_tree_sum(lane < kSgWarps ? red[lane] : 0.0f);
-    const float inv = 1.0f / sqrtf(ss / (float)K + a.eps);
-    const int pos = a.Shift ? a.Ctrl[CTRL_POS] : 0;
-    const float *prev = a.Shift ? a.State + (size_t)((pos - 1) & 1) * K : nullptr;
-    float *next = a.Shift && blockIdx.x == 0 ? a.State + (size_t)(pos & 1) * K : nullptr;
-    for (int k = tid; k < a.ldw; k += nth) {
-      float v = 0.0f;
-      if (k < K) {
-        v = us[k] * inv * a.NormW[k];
-        if (a.Shift) {
-          const float pv = pos > 0 ? prev[k] : 0.0f;
-          if (next) next[k] = v;
-          v = fmaf(pv - v, a.Shift[k], v);
+    if (a.S == 4 && stream_vec(a.S, K) && K <= kHgQuads * nth * 4) {
+      hyper_row_ahead<4>(a, coef, lo, hi, red);
+    } else {
+      const int lane = tid & 31, warp = tid >> 5;
+      pdl_wait();
+      float ss = stream_row_any(a.Xin, a.Yp, blockIdx.x == 0 ? a.Xout : nullptr, coef, a.S, K, a.Yp != nullptr, us, tid, nth);
+      ss = warp_tree_sum(ss);
+      if (lane == 0) red[warp] = ss;
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // also: every thread's u is visible
+      ss = warp_tree_sum(lane < kSgWarps ? red[lane] : 0.0f);
+      const float inv = 1.0f / sqrtf(ss / (float)K + a.eps);
+      const int pos = a.Shift ? a.Ctrl[CTRL_POS] : 0;
+      const float *prev = a.Shift ? a.State + (size_t)((pos - 1) & 1) * K : nullptr;
+      float *next = a.Shift && blockIdx.x == 0 ? a.State + (size_t)(pos & 1) * K : nullptr;
+      for (int k = tid; k < a.ldw; k += nth) {
+        float v = 0.0f;
+        if (k < K) {
+          v = us[k] * inv * a.NormW[k];
+          if (a.Shift) {
+            const float pv = pos > 0 ? prev[k] : 0.0f;
+            if (next) next[k] = v;
+            v = fmaf(pv - v, a.Shift[k], v);
+          }
         }
+        sg_put(lo, hi, k, v);
       }
-      sg_put(lo, hi, k, v);
     }
     asm volatile("bar.sync 1, 256;" ::: "memory");
     gemv_consume(c, d, &sh, sg_smem, lo, hi, part);

@@ -225,6 +225,8 @@ struct WindowAttnStepMmaArgs {
 constexpr int kWsStages = 2, kWsMaxSplits = 16;
 // As the chunk form, positions and the first tile (rows of earlier steps) are fetched before the dependency wait. Where
 // another layer of the same step appends the rows (koff < 0), the tile that ends in the step's own row waits.
+// Loops stay rolled: a step runs the kernel once, and a third of its stalls were on code not yet fetched (90 KB of it; with
+// 64 KB the launch costs a decode step of Robopel, width 1024, 10 us and not 16).
 template <int DP>
 __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs &a) {
   extern __shared__ __align__(128) unsigned char sm_raw[];
@@ -245,7 +247,7 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
   const bool fresh = a.koff >= 0;
   auto new_key = [&]() {   // warp 2: the key, warp 3: the value
     if (!fresh) return;
-    if (warp == 2) head_norm_turn(u + a.koff + (size_t)g * D, D, a.KN, a.eps, rot, a.rd, [&](int d, float x, float y, bool both) { st_pair(kn + d, x, y, both); });
+    if (warp == 2) head_norm_turn<(DP + 63) / 64>(u + a.koff + (size_t)g * D, D, a.KN, a.eps, rot, a.rd, [&](int d, float x, float y, bool both) { st_pair(kn + d, x, y, both); });
     if (warp == 3)
       for (int d = lane; d < E; d += 32) vn[d] = f32_to_bf16(u[a.voff + (size_t)g * E + d]);
   };
@@ -255,6 +257,7 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
     if (!fresh && !done) return;
     new_key();
     __syncthreads();
+#pragma unroll 1
     for (int i = tid; i < D + E; i += 128) {
       const bool isv = i >= D;
       const int x = isv ? i - D : i, w = isv ? VW : KW;
@@ -297,8 +300,9 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
   __syncthreads();
   pdl_wait();
   if (!ahead) fetch(t0);
+#pragma unroll 1
   for (int hh = warp; hh < HG; hh += 4)
-    head_norm_turn(u + (size_t)(g * HG + hh) * D, D, a.QN, a.eps, rot, a.rd, [&](int d, float x, float y, bool both) { st_pair(Qs + hh * LD + d, x, y, both); });
+    head_norm_turn<(DP + 63) / 64>(u + (size_t)(g * HG + hh) * D, D, a.QN, a.eps, rot, a.rd, [&](int d, float x, float y, bool both) { st_pair(Qs + hh * LD + d, x, y, both); });
   new_key();
   __syncthreads();
   uint32_t q[DP / 16][4];
@@ -310,6 +314,7 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
   for (int d = 0; d < DP / 8; ++d)
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[d][i] = 0.0f;
+#pragma unroll 1
   for (int t = t0; t < t1; ++t) {
     const bool pooled = t < nbt;
     const int k0 = (pooled ? t : tok0 + t - nbt) * kCmKeys + warp * 16, stage = (t - t0) % kWsStages;
@@ -383,6 +388,7 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
   // partials of a (sequence, key head): sums [splits][HG][E], then (maximum, sum) [splits][HG][2]
   float *base_p = a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (E + 4);   // E + 4 keeps 16-byte alignment
   float *base_m = base_p + (size_t)a.splits * HG * E;
+#pragma unroll 1
   for (int i = tid; i < HG * E; i += 128) {
     const int hh = i / E, d = i - hh * E;
     const float M = fmaxf(fmaxf(wm[0][hh], wm[1][hh]), fmaxf(wm[2][hh], wm[3][hh]));
@@ -413,12 +419,14 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
   __threadfence();
   // every split's factor exp2(m_s - M) / L, then the sums with the loads of all splits in flight
   float *fac = os;   // [HG][kWsMaxSplits]
+#pragma unroll 1
   for (int hh = warp; hh < HG; hh += 4) {
     const float2 ml = lane < active ? __ldcg(reinterpret_cast<const float2 *>(base_m) + lane * HG + hh) : make_float2(-INFINITY, 0.0f);
     const float M = warp_max(ml.x), f = fast_exp2(ml.x - M), L = warp_tree_sum(ml.y * f) + sink(hh, M);
     if (lane < kWsMaxSplits) fac[hh * kWsMaxSplits + lane] = lane < active ? f / L : 0.0f;
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = tid * 4; i < HG * E; i += 512) {
     const int hh = i / E;
     const float *p = base_p + i, *f = fac + hh * kWsMaxSplits;

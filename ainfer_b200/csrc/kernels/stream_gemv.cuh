@@ -43,10 +43,12 @@ __device__ __forceinline__ void sg_put(float *lo, float *hi, int k, float v) { (
 // (a value a thread and round waited for memory K / 256 times).
 __device__ __forceinline__ void sg_row(float *lo, float *hi, const float *x, int K, int ldw, int tid, int nth) {
   if ((K & 3) || (reinterpret_cast<unsigned long long>(x) & 15)) {
+#pragma unroll 1
     for (int k = tid; k < ldw; k += nth) sg_put(lo, hi, k, k < K ? x[k] : 0.0f);
     return;
   }
   constexpr int Q = 4;
+#pragma unroll 1
   for (int k0 = tid * 4; k0 < ldw; k0 += nth * 4 * Q) {
     float4 v[Q];
 #pragma unroll
@@ -107,6 +109,7 @@ __device__ __forceinline__ void gemv_next(GemvCursor &r, const GemvDims &d) {
 // Lane 0 of the producer warp: rows [n0, n1) of W.
 __device__ __forceinline__ void gemv_produce_rows(const uint16_t *W, int n0, int n1, int ldw, const GemvDims &d, GemvShared *sh, unsigned char *ring,
                                                   GemvCursor &r) {
+#pragma unroll 1
   for (int n = n0; n < n1; n += d.tile_rows) {
     if (!sg_wait(sh, &sh->empty[r.st], r.ph)) break;
     const uint32_t bytes = (uint32_t)min(d.tile_rows, n1 - n) * (uint32_t)ldw * 2u;
@@ -142,16 +145,20 @@ __device__ __forceinline__ void gemv_consume_rows(int rows, int ldw, const GemvD
                                                   const float *hi, float *part, GemvCursor &cur, float factor = 1.0f, bool add = false) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pieces = ldw >> 3;
   const int mine = warp % d.wpr, r_step = kSgWarps / d.wpr;
+  // the loops stay rolled: a decode step runs every kernel once, and fetching code is a good part of its time
+#pragma unroll 1
   for (int n = 0; n < rows; n += d.tile_rows) {
     const int nr = min(d.tile_rows, rows - n);
     sg_wait(sh, &sh->full[cur.st], cur.ph);
     __syncwarp();
     const unsigned char *tile = ring + (size_t)cur.st * d.stage_bytes;
+#pragma unroll 1
     for (int r = warp / d.wpr; r < nr; r += r_step) {
       const uint4 *row = reinterpret_cast<const uint4 *>(tile + (size_t)r * ldw * 2);
       float s0 = 0.0f, s1 = 0.0f;
       int i = mine * 32 + lane;
       const int step = 32 * d.wpr;
+#pragma unroll 2
       for (; i + step < pieces; i += 2 * step) {
         s0 = dot8(row[i], *reinterpret_cast<const float4 *>(lo + 4 * i), *reinterpret_cast<const float4 *>(hi + 4 * i), s0);
         const int k = i + step;
@@ -178,8 +185,10 @@ __device__ __forceinline__ void gemv_consume(const GemvShape &c, const GemvDims 
 // After the block's last barrier: one thread per row.
 __device__ __forceinline__ void gemv_store(const GemvShape &c, const GemvDims &d, const float *part) {
   const int n0 = blockIdx.x * c.rows_pb, n1 = min(c.N, n0 + c.rows_pb);
+#pragma unroll 1
   for (int n = n0 + threadIdx.x; n < n1; n += kSgThreads) {
     float v = 0.0f;
+#pragma unroll 1
     for (int i = 0; i < d.wpr; ++i) v += part[(n - n0) * d.wpr + i];
     c.Y[n] = apply_act(v + (c.Bias ? c.Bias[n] : 0.0f), c.act, c.cap);
   }

@@ -33,16 +33,16 @@ __device__ __forceinline__ void st_pair(uint16_t *p, float x, float y, bool both
 
 // One warp: a head's D values at src, divided by their root mean square and times w (w null: as they
 // are), then the first rd of them turned in neighbouring pairs by rot (cosine, sine per pair);
-// put(d, x, y, both): values d and d + 1, the second only if `both`. D <= 512.
+// put(d, x, y, both): values d and d + 1, the second only if `both`. D <= 64 PAIRS.
 constexpr int kHeadPairs = 8;   // pairs of a lane
-template <typename P>
+template <int PAIRS = kHeadPairs, typename P>
 __device__ __forceinline__ void head_norm_turn(const float *src, int D, const float *w, float eps, const float2 *rot, int rd, P put) {
   const int lane = threadIdx.x & 31;
-  float2 v[kHeadPairs];
+  float2 v[PAIRS];
   float ss = 0.0f;
   const bool wide = (reinterpret_cast<unsigned long long>(src) & 7) == 0;
 #pragma unroll
-  for (int i = 0; i < kHeadPairs; ++i) {
+  for (int i = 0; i < PAIRS; ++i) {
     const int d = (i * 32 + lane) * 2;
     v[i] = make_float2(0.0f, 0.0f);
     if (d + 1 < D && wide) v[i] = *reinterpret_cast<const float2 *>(src + d);
@@ -53,13 +53,13 @@ __device__ __forceinline__ void head_norm_turn(const float *src, int D, const fl
     if (i * 64 >= D) break;
   }
 #pragma unroll
-  for (int i = 0; i < kHeadPairs; ++i) {
+  for (int i = 0; i < PAIRS; ++i) {
     if (i * 64 >= D) break;
     ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, ss));
   }
   const float inv = w ? 1.0f / sqrtf(warp_tree_sum(ss) / (float)D + eps) : 1.0f;
 #pragma unroll
-  for (int i = 0; i < kHeadPairs; ++i) {
+  for (int i = 0; i < PAIRS; ++i) {
     if (i * 64 >= D) break;
     const int d = (i * 32 + lane) * 2;
     float x = v[i].x, y = v[i].y;
