@@ -561,6 +561,8 @@ int session_create(DeviceModel *m, int max_ctx, int flags, Session **out, std::s
   void *hp = nullptr;
   if (ainfer_host_alloc(s->dev, (size_t)max_ctx * 4 + 64, &hp) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return fail(1); }
   s->host_tok = (int32_t *)hp;
+  if (ainfer_host_alloc(s->dev, sizeof(Session::HostIo), &hp) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return fail(1); }
+  s->host_io = (Session::HostIo *)hp;
 
   // ---- record ----
   Recorder rec(s);
@@ -635,6 +637,7 @@ void session_destroy(Session *s) {
   for (auto &kv : s->kernels) ainfer_kernel_release(kv.second);
   for (void *p : s->owned) ainfer_mem_free(s->dev, p);
   if (s->host_tok) ainfer_host_free(s->dev, s->host_tok);
+  if (s->host_io) ainfer_host_free(s->dev, s->host_io);
   delete s;
 }
 
@@ -676,11 +679,15 @@ static int run_token(Session *s, bool with_tail) {
 }
 
 // The persistent kernel reports a barrier that ran out of polls through a sticky
-// error word instead of hanging; surface it as a device error.
+// error word instead of hanging; surface it as a device error. Queued before the copy
+// that the caller waits for, looked at after it.
+static int queue_step_error(Session *s) {
+  if (s->persistent) S_CHECK(ainfer_memcpy_d2h_async(s->dev, &s->host_io->error, s->step_error, 4));
+  return 0;
+}
 static int check_step_error(Session *s) {
   if (!s->persistent) return 0;
-  int32_t e = 0;
-  S_CHECK(ainfer_memcpy_d2h(s->dev, &e, s->step_error, 4));
+  const int32_t e = s->host_io->error;
   if (e != 0) {
     s->err = "device error: a bounded wait of the persistent decode kernel ran out (status " +
              std::to_string(e) + ")";
@@ -694,10 +701,11 @@ int session_step(Session *s, int token, int pos, int *out_token) {
     s->err = "context overflow: pos " + std::to_string(pos) + " >= MAXCTX " + std::to_string(s->max_ctx);
     return 3;
   }
-  ainfer_control c{token, pos, pos + 1, -1};
-  S_CHECK(ainfer_control_write(s->dev, s->ctrl, &c));
+  s->host_io->control = ainfer_control{token, pos, pos + 1, -1};
+  S_CHECK(ainfer_control_write_async(s->dev, s->ctrl, &s->host_io->control));
   int r = run_token(s, true);
   if (r) return r;
+  if (queue_step_error(s)) return 1;
   S_CHECK(ainfer_memcpy_d2h(s->dev, s->host_tok, s->out_tok, 4));
   if (out_token) *out_token = s->host_tok[0];
   return check_step_error(s);
@@ -713,7 +721,8 @@ int session_sample(Session *s, float temp, int top_k, float top_p, float rep_pen
       return 1;
   }
   if (nseen > 0) S_CHECK(ainfer_memcpy_h2d(s->dev, s->samp_seen, seen, (size_t)nseen * 4));
-  S_CHECK(ainfer_memcpy_h2d(s->dev, s->samp_io, rng, 8));
+  s->host_io->rng = *rng;
+  S_CHECK(ainfer_memcpy_h2d_async(s->dev, s->samp_io, &s->host_io->rng, 8));
   auto it = s->kernels.find("SampleTokenCluster");
   ainfer_kernel_t k = nullptr;
   if (it != s->kernels.end()) k = it->second;
@@ -735,8 +744,8 @@ int session_sample(Session *s, float temp, int top_k, float top_p, float rep_pen
   S_CHECK(set(sizeof probs, &probs)); S_CHECK(set(sizeof ctrl, &ctrl)); S_CHECK(set(4, &v)); S_CHECK(set(4, &ns));
   S_CHECK(set(4, &temp)); S_CHECK(set(4, &tk)); S_CHECK(set(4, &top_p)); S_CHECK(set(4, &rep_penalty));
   S_CHECK(ainfer_kernel_launch(s->dev, k, 8));
-  uint64_t back[2];
-  S_CHECK(ainfer_memcpy_d2h(s->dev, back, s->samp_io, 16));
+  const uint64_t *back = s->host_io->drawn;
+  S_CHECK(ainfer_memcpy_d2h(s->dev, s->host_io->drawn, s->samp_io, 16));
   *rng = back[0];
   *out_token = (int)(int32_t)(back[1] & 0xFFFFFFFFu);
   return 0;
@@ -749,8 +758,8 @@ int session_mtp_draft(Session *s, int next_token, int pos, int from_trunk, int *
     return 3;
   }
   if (from_trunk) S_CHECK(ainfer_memcpy_d2d(s->dev, s->Hm, s->X, (size_t)s->m->cfg.hidden * 4));
-  ainfer_control c{next_token, pos, pos + 1, -1};
-  S_CHECK(ainfer_control_write(s->dev, s->ctrl_m, &c));
+  s->host_io->control = ainfer_control{next_token, pos, pos + 1, -1};
+  S_CHECK(ainfer_control_write_async(s->dev, s->ctrl_m, &s->host_io->control));
   S_CHECK(ainfer_list_execute(s->mtp_list));
   S_CHECK(ainfer_memcpy_d2h(s->dev, s->host_tok, s->out_tok_m, 4));
   if (draft_token) *draft_token = s->host_tok[0];
@@ -859,10 +868,12 @@ int session_generate(Session *s, const int *prompt, int P, int G, int start_pos,
     ainfer_event_destroy(e1);
   }
   if (G > 0) {
+    if (queue_step_error(s)) return 1;
     // tokens were logged on the device at the position of the input that produced them
     S_CHECK(ainfer_memcpy_d2h(s->dev, s->host_tok, s->history + (start_pos + P - 1), (size_t)G * 4));
     for (int g = 0; g < G; ++g) out_tokens[g] = s->host_tok[g];
   } else {
+    if (queue_step_error(s)) return 1;
     S_CHECK(ainfer_sync(s->dev, UINT64_MAX));
   }
   return check_step_error(s);

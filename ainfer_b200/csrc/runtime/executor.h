@@ -51,6 +51,10 @@ struct Session {
   int32_t *history = nullptr;   // device ring of selected tokens, indexed by position
   int32_t *out_tok = nullptr;   // device [1]
   int32_t *host_tok = nullptr;  // pinned [max_ctx]
+  // pinned: what a step or a draw sends and gets back. Its copies are queued beside the work and waited for once,
+  // by the call's last copy; a pageable one is a wait each (a step and a draw of the smallest preset 196 us, now 172)
+  struct HostIo { ainfer_control control; uint64_t rng, drawn[2]; int32_t error; };
+  HostIo *host_io = nullptr;
   // scratch (singletons)
   float *X = nullptr, *Tmp = nullptr, *Hn = nullptr, *Mix = nullptr;
   int8_t *Q8 = nullptr; float *SQ = nullptr;
