@@ -425,10 +425,7 @@ struct Engine : RowEngineBase {
     ldw = round_up((int)W, 8);
     ldq = round_up((int)maxA, 8);
     ldf = round_up((int)maxF, 8);
-    int span = 1;
-    for (const RowLayerConfig &r : c.row_layers)
-      if (r.heads) span = std::max(span, std::min(window_of(r), max_ctx) + (r.pool > 0 ? max_ctx / r.pool : 0));
-    att_splits = step_splits(maxG, span);
+    att_splits = step_splits(maxG);
     for (int i = 0; i < 2; ++i) e |= alloc(R * W, &X[i]);
     e |= alloc(R * ldw * esz(), &H); e |= alloc(R * maxU, &U); e |= alloc(R * maxQ * esz(), &Q);
     e |= alloc(R * ldq * 4, &Att); e |= alloc(y_rows * W, &Y); e |= alloc(R * ldf * 4, &Z);
@@ -556,13 +553,15 @@ struct Engine : RowEngineBase {
                (const int32_t *)Count, (int32_t)N, (int32_t)mt.K, (int32_t)ldx, (int32_t)mt.ldw, (int32_t)ldy, (int32_t)act);
       return;
     }
+    // tiles of 256 outputs by pairs of blocks where the rows of a tile are many and there are rounds of them (as in linear())
+    const bool pair = nt >= 96 && N % 256 == 0 && units >= 2 * sm_count;
     TensorMap wm, xm;
     if (ainfer_tensor_map_bf16(dev, &wm, mt.w, (uint64_t)mt.N, (uint64_t)mt.K, (uint64_t)mt.ldw, 128) != AINFER_OK ||
-        ainfer_tensor_map_bf16(dev, &xm, Xp, (uint64_t)slots, (uint64_t)mt.K, (uint64_t)ldx, (uint32_t)nt) != AINFER_OK) {
+        ainfer_tensor_map_bf16(dev, &xm, Xp, (uint64_t)slots, (uint64_t)mt.K, (uint64_t)ldx, (uint32_t)(pair ? nt / 2 : nt)) != AINFER_OK) {
       k.fail(1, ainfer_last_error(dev));
       return;
     }
-    k.launch("LinearTcGrouped", (uint32_t)std::min<long>(units, sm_count), wm, xm, Yp, (const void *)Tiles, (const int32_t *)Count, (int32_t)N,
+    k.launch(pair ? "LinearTcGroupedPair" : "LinearTcGrouped", (uint32_t)(pair ? sm_count / 2 * 2 : std::min<long>(units, sm_count)), wm, xm, Yp, (const void *)Tiles, (const int32_t *)Count, (int32_t)N,
              (int32_t)mt.K, (int32_t)nt, (int32_t)ldy, (int32_t)act, (int32_t)(out16 ? 1 : 0));
   }
 

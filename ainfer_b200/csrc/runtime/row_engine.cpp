@@ -163,21 +163,33 @@ void RowEngineBase::linear(KernelCalls &k, const RowMatrix &mt, const char *Xp, 
   const int n_tiles = (mt.N + 127) / 128, kb = (mt.K + 63) / 64;
   int nt = rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128;
   const bool few = 2 * n_tiles * ((rows + 127) / 128) <= sm_count;   // tiles of 128 rows leave most SMs idle: split K instead
+  bool pair = false;   // tiles of 256 outputs by pairs of blocks
   if (rows > 128 && !few) {
-    // rows of a tile: as large as possible (operand traffic), but a launch lasts whole rounds of tiles over the SMs
-    long best = -1;
-    for (int t = 256; t >= 96; t -= 16) {
-      const long rounds = ((long)n_tiles * ((rows + t - 1) / t) + sm_count - 1) / sm_count, cost = rounds * (t + 48);
-      if (best < 0 || cost < best) { best = cost; nt = t; }
-    }
+    // rows of a tile: as large as possible (operand traffic), but a launch lasts whole rounds of tiles over the SMs. A
+    // pair's tile takes 1 / 1.15 of the time and the launch about 3.5 us more (60 rows of a tile at K = 2048). Measured at 2048 rows,
+    // us alone / in pairs: 2048 x 2048 (outputs x K) 22.7 / 24.7, 2560 x 2048 31.3 / 32.3, 8192 x 2048 64.3 / 57.4, 2048 x 8192 60.4 / 53.3.
+    double best = -1;
+    for (int p = 0; p < 2; ++p)
+      for (int t = 256; t >= 96; t -= 16) {
+        const int width = p ? 256 : 128, slots = p ? sm_count / 2 : sm_count;
+        const long tiles = (long)((mt.N + width - 1) / width) * ((rows + t - 1) / t), rounds = (tiles + slots - 1) / slots;
+        const double cost = p ? rounds * (t + 48.0) + 74.0 * 2048 / mt.K : rounds * (1.15 * t + 48.0);
+        if (best < 0 || cost < best) { best = cost; nt = t; pair = p; }
+      }
   }
   const int tiles = n_tiles * ((rows + nt - 1) / nt);
   int splits = 1;   // few tiles: a cluster of blocks per tile, each a part of K
   while ((rows <= 128 || few) && splits < 8 && tiles * splits * 2 <= sm_count && kb >= splits * 4) splits *= 2;
   TensorMap wm, xm;
   if (ainfer_tensor_map_bf16(dev, &wm, mt.w, (uint64_t)mt.N, (uint64_t)mt.K, (uint64_t)mt.ldw, 128) != AINFER_OK ||
-      ainfer_tensor_map_bf16(dev, &xm, Xp, (uint64_t)rows, (uint64_t)mt.K, (uint64_t)ldx, (uint32_t)nt) != AINFER_OK) {
+      ainfer_tensor_map_bf16(dev, &xm, Xp, (uint64_t)rows, (uint64_t)mt.K, (uint64_t)ldx, (uint32_t)(pair ? nt / 2 : nt)) != AINFER_OK) {
     k.fail(1, ainfer_last_error(dev));
+    return;
+  }
+  if (pair) {
+    const int t = (mt.N + 255) / 256 * ((rows + nt - 1) / nt);
+    k.launch("LinearTcPair", (uint32_t)(2 * std::min(t, sm_count / 2)), wm, xm, mt.bias, Yp, (int32_t)rows, (int32_t)mt.N, (int32_t)mt.K, (int32_t)nt,
+             (int32_t)ldy, (int32_t)act, (int32_t)(out16 ? 1 : 0), cap);
     return;
   }
   static const char *const names[] = {"LinearTc", "LinearTcSplit2", "LinearTcSplit4", "LinearTcSplit8"};

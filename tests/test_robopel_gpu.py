@@ -283,6 +283,27 @@ def test_mixture_over_rows(dev, E, I, top, W, F, R, kind, nt):
     close(got[:seen], want[:seen], 1e-5 if kind == "f32" else 2e-2)
 
 
+@pytest.mark.parametrize("E,N,K,nt,rows", [(1, 256, 64, 96, [1]), (3, 512, 200, 96, [95, 0, 100]), (4, 256, 520, 144, [144, 145, 1, 300]), (2, 768, 72, 256, [600, 129])])
+def test_grouped_products_in_pairs(dev, E, N, K, nt, rows):
+    """Tiles of two blocks over the experts' rows: ends of an expert's rows are not the next one's."""
+    g = torch.Generator().manual_seed(N)
+    R, ldw = sum(rows), -(-K // 8) * 8
+    x, w = bf16(torch.randn(R, K, generator=g)), bf16(torch.randn(E, N, K, generator=g))
+    xp, wp = torch.zeros(R, ldw), torch.zeros(E * N, ldw)
+    xp[:, :K], wp[:, :K] = x.float(), w.float().reshape(E * N, K)
+    tiles, want, p = [], np.zeros((R, N)), 0
+    for e, n in enumerate(rows):
+        want[p:p + n] = (x[p:p + n].double() @ w[e].double().T).numpy()
+        tiles += [(e, p + i, min(nt, n - i), 0) for i in range(0, n, nt)]
+        p += n
+    y = dev.zeros(R * N * 4)
+    tm = dev.tensor_map_bf16
+    dev.kernel("LinearTcGroupedPair")(4, tm(dev.upload(bits(wp)), E * N, K, ldw, 128), tm(dev.upload(bits(xp)), R, K, ldw, nt // 2), y,
+                                      dev.upload(np.int32(tiles)), dev.upload(np.int32([len(tiles)])), N, K, nt, N, 0, 0)
+    dev.sync()
+    close(dev.download(y, (R, N), np.float32), want, 1e-5)
+
+
 @pytest.mark.parametrize("E,I,top,W,F,R", CASES)
 def test_mixture_step(dev, E, I, top, W, F, R):
     x, logits, corr, up, dn = _mixture_case(E, I, top, W, F, min(R, 8))

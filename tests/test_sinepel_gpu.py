@@ -347,6 +347,25 @@ def test_linear_tensor_cores(dev, R, N, K, nt, splits, act, out16):
         close(from_bits(raw, (R, N)) if out16 else raw, want, 2e-2 if out16 else 1e-5)
 
 
+@pytest.mark.parametrize("R,N,K,nt,act,out16", [
+    (1, 5, 40, 96, 0, 0), (97, 130, 200, 96, 2, 0), (240, 256, 64, 240, 1, 1), (241, 512, 136, 240, 0, 0), (1000, 1536, 320, 256, 1, 1),
+    (520, 640, 1024, 112, 0, 0), (129, 257, 72, 144, 1, 0), (401, 200, 264, 176, 2, 1), (300, 1300, 4096, 128, 0, 1)])
+def test_linear_tensor_cores_in_pairs(dev, R, N, K, nt, act, out16):
+    """Tiles of 256 outputs by two blocks: one round of them and several, odd numbers of 128, halves of rows beyond the last."""
+    g = torch.Generator().manual_seed(R)
+    x, w, b = bf16(torch.randn(R, K, generator=g)), bf16(torch.randn(N, K, generator=g)), torch.randn(N, generator=g)
+    dx, dw = dev.upload(bits(x)), dev.upload(bits(w))
+    tiles = -(-N // 256) * (-(-R // nt))
+    want = ACTS[act](x.double() @ w.double().T + b.double(), 3.0)
+    for pairs in (tiles, min(tiles, 2)):
+        y = dev.zeros(R * N * 4)
+        dev.kernel("LinearTcPair")(2 * pairs, dev.tensor_map_bf16(dw, N, K, K, 128), dev.tensor_map_bf16(dx, R, K, K, nt // 2), dev.upload(f32(b)), y, R, N, K,
+                                   nt, N, act, out16, 3.0)
+        dev.sync()
+        raw = dev.download(y, (R, N), np.uint16 if out16 else np.float32)
+        close(from_bits(raw, (R, N)) if out16 else raw, want, 2e-2 if out16 else 1e-5)
+
+
 @pytest.mark.parametrize("N,K,rows_pb,act", [(7, 50, 3, 0), (64, 1000, 22, 1), (601, 256, 201, 2), (33, 4096, 11, 0), (9, 20000, 5, 0), (500, 2560, 250, 0),
                                              (3, 8, 1, 0)])
 def test_decode_gemv(dev, N, K, rows_pb, act):
