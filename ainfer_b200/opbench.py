@@ -141,7 +141,7 @@ def gemv_multi_once(dev, N, K, M, reps=20, groups=0):
 
 
 def gemm_tc_once(dev, N, K, M, reps=20, groups=0, kernel="Int4GemmA8Tc"):
-    """Int4GemmA8Tc (W4A8 on tcgen05, 1 <= M <= 64, weights streamed once) on one shape: recorded list
+    """Int4GemmA8Tc (W4A8 on the tensor cores, 1 <= M <= 64, weights streamed once) on one shape: recorded list
     rotating over enough weight buffers to exceed L2, timed as a whole on the device."""
     wbytes = N * K // 2 + N * K // 128 * 2
     nbuf = max(1, min(64, -(-(256 << 20) // wbytes)))
@@ -255,7 +255,7 @@ def main(argv=None):
     g.add_argument("--sweep", action="store_true")
     g.add_argument("--a16", action="store_true", help="bf16 activations (Int4GemmA16, M up to 64) instead of W4A8")
     g.add_argument("--multi", action="store_true", help="W4A8 for M up to 8 with the weights streamed once (Int4GemvA8Multi, dp4a)")
-    g.add_argument("--tc", action="store_true", help="W4A8 on the tcgen05 tensor cores (Int4GemmA8Tc, M up to 64)")
+    g.add_argument("--tc", action="store_true", help="W4A8 on the tensor cores (Int4GemmA8Tc, M up to 64)")
     g.add_argument("--groups", type=int, default=0, help="thread groups per launch (default: by shape)")
     g.add_argument("--flush", action="store_true", help="time single launches after an L2 rewrite")
     ll = sub.add_parser("listlat", help="device time per node of a recorded list of tiny dependent launches")
