@@ -63,6 +63,7 @@ SIGNATURES = {
     "ainfer_list_destroy": (_i, [_vp]),
     "ainfer_list_execute": (_i, [_vp]),
     "ainfer_kernel_launch": (_i, [_vp, _vp, _u32]),
+    "ainfer_kernel_launch_next": (_i, [_vp, _vp, _u32]),
     "ainfer_sync": (_i, [_vp, _u64]),
     "ainfer_control_write": (_i, [_vp, _vp, C.POINTER(Control)]),
     "ainfer_control_write_async": (_i, [_vp, _vp, C.POINTER(Control)]),
