@@ -189,7 +189,7 @@ constexpr int kSmStages = 3, kSmMaxSplits = 16;   // at most 16 splits
 // dependency wait, while the block would only stand by: positions, the first tiles of keys (of earlier steps; the row of
 // this step is put in later), the convolution over the history, and the first tile's penalties. What is left is
 // one load, the second half of the convolution, the tiles and the merge (with the rows of the GEMVs fetched ahead as
-// well: a token of four layers of 2048 at position 1500 279 us, now 243; 16 sequences at 600 308 us, now 271).
+// well: a token of four layers of 2048 at position 1500 279 us, now 243; 16 sequences at 600 308 us, now 280).
 template <int DP>
 __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &a) {
   extern __shared__ __align__(128) unsigned char sm_raw[];

@@ -76,23 +76,12 @@ struct RowEngineBase : RowEngine {
     return base + std::string("256");
   }
   // Blocks of a step's attention per (sequence, key head): few tiles each when there are many sequences. The cut decides
-  // the order of sums, and in a model with mixtures a last bit can choose another expert, so theirs stays with this rule
-  // (the one below: 64 sequences of Robopel 436 -> 424 us, some rows with other experts).
+  // the order of the sums, so it depends on the sequences and heads alone and not on the context that was asked for:
+  // the same tokens give the same logits in a session or batch of any length. (A cut by whole rounds of blocks over the
+  // keys of the longest context took 257 us against 280 for 16 sequences of Sinepel at 600, with other last bits.)
   int step_splits(int max_kv_heads) const {
     if (nseq == 1) return std::max(1, std::min(16, 2 * sm_count / max_kv_heads));
     return std::max(1, std::min(16, 8 * sm_count / (std::min(nseq, 8 * sm_count) * max_kv_heads)));
-  }
-  // The same, at most 16: a launch lasts whole rounds of blocks (three fit
-  // an SM), a block its tiles of 64 keys and about four tiles' time for its start and the merge. `span`: keys a step may see.
-  int step_splits(int max_kv_heads, int span) const {
-    const long pairs = (long)nseq * max_kv_heads, tiles = std::max(1, (span + 63) / 64);
-    int best = 1;
-    long cost = -1;
-    for (int s = 1; s <= 16; ++s) {
-      const long rounds = (pairs * s + 3 * sm_count - 1) / (3 * sm_count), c = rounds * ((tiles + s - 1) / s + 4);
-      if (cost < 0 || c < cost) { cost = c; best = s; }
-    }
-    return best;
   }
 };
 

@@ -277,9 +277,7 @@ struct Engine : RowEngineBase {
       ts.push_back({s.pend_shift, s.shift, nullptr, nullptr, C, 1});   // steps keep their convolution ring themselves
     }
     ldw = round_up((int)W, 8); ldq = round_up(maxQ, 8); ldf = round_up(maxF, 8);
-    int span = 1;
-    for (const LayerState &s : st) span = std::max(span, std::min(s.chunk, max_ctx));
-    att_splits = step_splits(maxG, span);
+    att_splits = step_splits(maxG);
     for (int i = 0; i < 2; ++i) e |= alloc(R * S * W, &X[i]);
     e |= alloc(R * ldw * esz(), &H); e |= alloc(R * maxC, &U); e |= alloc(R * ldq * esz(), &Q);
     e |= alloc(R * ldq * 4, &Att); e |= alloc(R * W, &Y); e |= alloc(R * ldf * 4, &Act);

@@ -635,6 +635,33 @@ def test_long_context_over_ring_ends(dev, rt, tmp_path, kind):
     model.close()
 
 
+@pytest.mark.parametrize("seqs", [1, 3])
+def test_logits_do_not_depend_on_the_context_asked_for(dev, rt, tmp_path, seqs):
+    """Steps at position 1000 of a chunk: bit for bit the same in a session or batch that just holds them and in a longer one."""
+    c = P.make_config(width=64, vocab=64, streams=2, max_positions=4096, layers=[L(heads=4, kv_heads=1, dim=32, conv=4, chunk=3000, ff=64)])
+    P.write_model(str(tmp_path), c, P.make_weights(c, 4))
+    model = rt.Model(dev, str(tmp_path))
+    toks = np.random.default_rng(3).integers(0, 64, (1002, seqs)).astype(np.int32)
+    got = []
+    for ctx in (1010, 2560):
+        if seqs == 1:
+            s = rt.Session(model, ctx)
+            s.prefill(toks[:1000, 0])
+            for i in (1000, 1001):
+                s.step(int(toks[i, 0]), i)
+            got.append(s.logits())
+        else:
+            s = rt.BatchDecode(model, seqs, ctx)
+            for i in range(1002):
+                s.set_inputs(toks[i], np.full(seqs, i, np.int32))
+                s.step()
+            s.dev.sync()
+            got.append(s.read("logits", np.float32))
+        s.close()
+    model.close()
+    assert np.array_equal(got[0], got[1])
+
+
 def test_limits_are_refused(dev, rt, tmp_path):
     c = P.make_config(max_positions=20, layers=[L()])
     P.write_model(str(tmp_path), c, P.make_weights(c, 0))
