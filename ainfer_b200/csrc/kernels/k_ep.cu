@@ -437,7 +437,8 @@ __global__ void __launch_bounds__(128) SiluQuantRows(const SiluQuantRowsArgs a) 
   pdl_launch_dependents();
   pdl_wait();
   const int row = (int)blockIdx.x < a.front ? (int)blockIdx.x : a.always_from + (int)blockIdx.x - a.front;
-  if (a.Counts && row < a.always_from && row >= __ldg(a.Counts)) return;
+  // Counts is written by a kernel that this one may have started beside: not through the read-only path
+  if (a.Counts && row < a.always_from && row >= __ldcg(a.Counts)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float *g = a.GU + (size_t)row * 2 * a.I, *u = g + a.I;
   for (int grp = warp; grp < a.I / 128; grp += 4) {

@@ -301,3 +301,26 @@ def test_oracle_preset_table_equals_runtime_presets():
     from ainfer_b200 import runtime
     for name in ("tiny", "mini", "mini-mtp", "small", "full"):
         assert json.loads(O.preset_json(name)) == json.loads(runtime.preset_config_json(name)), name
+
+
+# what a model holds: written once, before any launch that reads it
+CONSTANT_FIELDS = {"W", "CW", "Wr", "Wsg", "Bias", "Experts", "P", "S", "LB"}
+
+
+@pytest.mark.parametrize("source", ["k_ep.cu"])
+def test_early_kernels_read_results_coherently(source):
+    """A kernel marked for early launch may be resident while the kernels before it write: what they write must not be
+    read through the read-only path (__ldg), which a dependency wait does not order."""
+    text = open(os.path.join(ROOT, "ainfer_b200", "csrc", "kernels", source)).read()
+    marked = re.findall(r"^AINFER_EARLY_LAUNCH\((\w+)\)", text, re.M)
+    assert marked
+    for name in marked:
+        start = text.index("{", re.search(r"__global__[^;{]*\b%s\(" % name, text).start())
+        depth, end = 0, start
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[end], 0)
+            end += 1
+            if depth == 0:
+                break
+        read = set(re.findall(r"__ldg\([^;]*?\ba\.(\w+)", text[start:end]))
+        assert read <= CONSTANT_FIELDS, (name, read - CONSTANT_FIELDS)

@@ -48,6 +48,23 @@ def test_prefill_equals_token_by_token_decode(dev, preset, P, splits, flags):
     a.close(); b.close(); c.close(); model.close()
 
 
+def test_a_long_prompt_after_a_short_one(dev):
+    """Two rows, then three hundred on the same session: nothing of the smaller pass (row counts, problem lists) is met again."""
+    from ainfer_b200 import runtime
+    model = runtime.Model(dev, "synth:mini:seed=4")
+    prompt = np.random.default_rng(7).integers(0, model.config["vocab"], 302).astype(np.int32)
+    a, b = runtime.Session(model, 320), runtime.Session(model, 320)
+    for i, t in enumerate(prompt):
+        a.step(int(t), i)
+    for _ in range(3):
+        b.reset()
+        b.prefill(prompt[:2])
+        b.prefill(prompt[2:], start_pos=2)
+        for name, dt in STATE:
+            assert np.array_equal(a.read(name, dt), b.read(name, dt)), name
+    a.close(); b.close(); model.close()
+
+
 def test_prefill_rejects_context_overflow(dev):
     from ainfer_b200 import runtime
     model = runtime.Model(dev, "synth:tiny:seed=0")
