@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256) Int4GemmA16(const Int4GemmA16Args a) {
     for (int i = tid; i < MT * 8 * 16; i += 256) {  // 16-byte pieces: 16 per row
       const int m = i >> 4, piece = i & 15;
       uint4 v = make_uint4(0, 0, 0, 0);
-      if (m < a.M) v = __ldg(reinterpret_cast<const uint4 *>(a.X + (size_t)m * a.K + (size_t)g * 128) + piece);
+      if (m < a.M) v = __ldcg(reinterpret_cast<const uint4 *>(a.X + (size_t)m * a.K + (size_t)g * 128) + piece);   // the predecessor's output: not read-only
       *reinterpret_cast<uint4 *>(&xs[b][m * kA16RowStride + piece * 8]) = v;
     }
   };
