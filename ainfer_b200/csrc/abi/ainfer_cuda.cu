@@ -38,6 +38,10 @@ void mark_kernel_early_launch(const char *name) {
   for (auto &d : registry())
     if (std::strcmp(d.name, name) == 0) d.early_launch = 1;
 }
+void mark_kernel_ahead(const char *name, int offset) {
+  for (auto &d : registry())
+    if (std::strcmp(d.name, name) == 0) d.ahead_offset = offset;
+}
 static std::vector<FaultHook> &fault_hooks() {
   static std::vector<FaultHook> h;
   return h;
@@ -148,6 +152,7 @@ struct ainfer_list_s {
   bool has_last = false;
   bool last_is_kernel = false;
   bool closed = false;
+  bool one_step = false;     // ainfer_list_one_step
   uint32_t launches = 0;
 };
 struct ainfer_event_s {
@@ -487,12 +492,17 @@ int ainfer_kernel_max_groups(ainfer_kernel_t k, uint32_t *groups) {
   return AINFER_OK;
 }
 
+static void set_ahead(ainfer_kernel_t k, int32_t bits) {
+  if (k->desc->ahead_offset >= 0) std::memcpy(k->args.data() + k->desc->ahead_offset, &bits, sizeof bits);
+}
+
 static int launch_kernel(ainfer_device_t dev, ainfer_kernel_t k, uint32_t groups, bool next) {
   if (!dev || !k) return AINFER_ERR_INVALID;
   uint32_t smem = 0;
   CU(dev, cudaSetDevice(dev->ordinal));  // function attributes and launches go to the current device
   int r = check_launch(k, groups, &smem);
   if (r) return r;
+  set_ahead(k, next ? AHEAD_WEIGHTS : 0);   // a chain writes no weights; its launches may write positions and state
   void *params[1] = {k->args.data()};
   if (k->desc->cooperative) {
     CU(dev, cudaLaunchCooperativeKernel(k->desc->fn, dim3(groups), dim3(k->desc->threads), params, smem, dev->stream));
@@ -541,6 +551,7 @@ int ainfer_list_append_launch(ainfer_list_t l, ainfer_kernel_t k, uint32_t group
   CU(l->dev, cudaSetDevice(l->dev->ordinal));
   int r = check_launch(k, groups, &smem);
   if (r) return r;
+  set_ahead(k, l->one_step ? AHEAD_WEIGHTS | AHEAD_STATE : 0);
   void *params[1] = {k->args.data()};
   cudaKernelNodeParams np;
   std::memset(&np, 0, sizeof np);
@@ -610,6 +621,12 @@ int ainfer_list_append_fill(ainfer_list_t l, void *dst, int byte_value, size_t b
   l->last_is_kernel = false;
   l->last = node;
   l->has_last = true;
+  return AINFER_OK;
+}
+int ainfer_list_one_step(ainfer_list_t l) {
+  if (!l) return AINFER_ERR_INVALID;
+  if (l->closed || l->has_last) return fail(l->dev, AINFER_ERR_INVALID, "one_step of a list that has entries");
+  l->one_step = true;
   return AINFER_OK;
 }
 int ainfer_list_close(ainfer_list_t l) {

@@ -183,10 +183,11 @@ struct ChunkAttnStepMmaArgs {
   void *O;                 // [seq][ldo]
   int32_t nseq, H, G, D, taps, cap, chunk, lb_len, splits, ldu, ldo, out16;   // splits <= 16, ldu a multiple of 4
   float scale;
+  int32_t ahead;           // LaunchAhead
 };
 constexpr int kSmStages = 3, kSmMaxSplits = 16;   // at most 16 splits
-// Bound by a chain of latencies, so all that does not come from the step's own projections is done before the
-// dependency wait, while the block would only stand by: positions, the first tiles of keys (of earlier steps; the row of
+// Bound by a chain of latencies, so in a list of one step all that does not come from the step's own projections is done
+// before the dependency wait, while the block would only stand by: positions, the first tiles of keys (of earlier steps; the row of
 // this step is put in later), the convolution over the history, and the first tile's penalties. What is left is
 // one load, the second half of the convolution, the tiles and the merge (with the rows of the GEMVs fetched ahead as
 // well: a token of four layers of 2048 at position 1500 279 us, now 243; 16 sequences at 600 308 us, now 280).
@@ -203,6 +204,7 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
   float *past = reinterpret_cast<float *>(Ks + kSmStages * kCmKeys * LD);   // [(HG + 1) D]: the convolution over the history
   const int split = blockIdx.x % a.splits, g = blockIdx.x / a.splits % a.G, seq = blockIdx.x / (a.splits * a.G);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (!(a.ahead & AHEAD_STATE)) pdl_wait();
   const int pos = a.Ctrl[4 * seq + CTRL_POS], lo = pos - pos % a.chunk;
   const int t_lo = lo / kCmKeys, t_hi = pos / kCmKeys, nt = t_hi - t_lo + 1;
   const int per = (nt + a.splits - 1) / a.splits, active = (nt + per - 1) / per;
@@ -425,7 +427,8 @@ CHUNK_STEP(256)
   F(U), F(CW), F(State), F(Ctrl), F(Kc), F(kv_stride), F(LB), F(Temp), F(Part), F(Count), F(O), F(nseq), F(H), F(G), F(D), F(taps), \
       F(cap), F(chunk), F(lb_len), F(splits), F(ldu), F(ldo), F(out16), F(scale)
 #define CS_REGISTER(DP) \
-  AINFER_REGISTER(ChunkAttnStepMma##DP, ChunkAttnStepMmaArgs, 128, 0, 0, chunk_step_smem##DP, CS_FIELDS); AINFER_EARLY_LAUNCH(ChunkAttnStepMma##DP)
+  AINFER_REGISTER(ChunkAttnStepMma##DP, ChunkAttnStepMmaArgs, 128, 0, 0, chunk_step_smem##DP, CS_FIELDS); \
+  AINFER_EARLY_LAUNCH_AHEAD(ChunkAttnStepMma##DP, ChunkAttnStepMmaArgs)
 CS_REGISTER(32);
 CS_REGISTER(64);
 CS_REGISTER(96);

@@ -42,6 +42,7 @@ struct Int4GemmA8TcArgs {
   const float *SQ;     // [M][K/128] activation group scales
   float *Y;            // [M][ldy]
   int32_t N, K, M, ldy;
+  int32_t ahead;       // LaunchAhead
 };
 
 // One problem of a grouped launch: Y[x_row0 + m][y_col + n] = sum_k W[n][k] * X[x_row0 + m][k].
@@ -109,6 +110,7 @@ struct TcShape {
   const float *SQ;
   float *Y;
   int32_t N, K, ldy;
+  bool ahead;              // the one problem's weights may travel before the dependency wait
 };
 struct TcUnit {
   const uint8_t *P;        // of the problem's row 0
@@ -145,7 +147,7 @@ __device__ __forceinline__ void tc_body(const TcShape &c) {
   const int nrb = (c.single.M + NT - 1) / NT;         // blocks of entries of the one problem
   const int stride = (int)gridDim.x;
   const uint32_t base = smem_addr(tc_smem);
-  if (c.groups) pdl_wait();
+  if (!c.ahead) pdl_wait();
   const int units = c.groups ? __ldcg(c.ngroups) * tpg : tpg * nrb;
   // ---- copies: this thread's sources of the next stage; rows and entries that do not exist keep what is there (never stored) ----
   const bool pair_scales = (G & 1) == 0;
@@ -236,7 +238,7 @@ __device__ __forceinline__ void tc_body(const TcShape &c) {
       if (lu < units) { copy_w(); copy_x(); advance(); }
       commit();
     }
-  } else {   // the one problem's weights travel before the predecessor is done
+  } else {   // the one problem's weights travel before the predecessor is done, where none writes weights
 #pragma unroll 1
     for (int i = 0; i < ST - 1 && lu < units; ++i) { copy_w(); advance(); }
     pdl_wait();
@@ -351,6 +353,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) Int4GemmA8Tc(const Int4GemmA8Tc
   c.single.P = a.P; c.single.S = a.S; c.single.x_row0 = 0; c.single.M = a.M; c.single.y_col = 0; c.single.pad = 0;
   c.XQ = a.XQ; c.SQ = a.SQ; c.Y = a.Y;
   c.N = a.N; c.K = a.K; c.ldy = a.ldy;
+  c.ahead = (a.ahead & AHEAD_WEIGHTS) != 0;
   tc_dispatch(c, tc_entries(a.N, a.M));
 }
 
@@ -361,6 +364,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) Int4GemmA8TcGrouped(const Int4G
   c.single = TcGroup{nullptr, nullptr, 0, 0, 0, 0};
   c.XQ = a.XQ; c.SQ = a.SQ; c.Y = a.Y;
   c.N = a.N; c.K = a.K; c.ldy = a.ldy;
+  c.ahead = false;
   tc_dispatch(c, tc_entries_grouped(a.max_m));
 }
 
@@ -379,7 +383,7 @@ AINFER_REGISTER(Int4GemmA8TcGrouped, Int4GemmA8TcGroupedArgs, kTcThreads, 0, 0, 
                 F(Y), F(N), F(K), F(max_m), F(ldy));
 #undef F
 
-AINFER_EARLY_LAUNCH(Int4GemmA8Tc);
+AINFER_EARLY_LAUNCH_AHEAD(Int4GemmA8Tc, Int4GemmA8TcArgs);
 AINFER_EARLY_LAUNCH(Int4GemmA8TcGrouped);
 
 }  // namespace ainfer

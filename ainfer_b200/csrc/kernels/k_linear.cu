@@ -159,15 +159,17 @@ struct HyperStreamGemvArgs {
   float *Y;
   int32_t S, N, K, ldw, rows_pb, act;
   float eps, cap;
+  int32_t ahead;           // LaunchAhead
 };
 // The row of up to 2048 elements in whole quads and four streams: everything that does not come from the sublayer
-// before (norm weights, shift, the last position's row) is in registers before the dependency wait, the streams
+// before (norm weights, shift, the last position's row in a list of one step) is in registers before the dependency wait, the streams
 // and the sublayer's output are one round of loads after it. In loops (as below) every element's norm weight,
 // shift and last row were one more round each. (One number of streams only: every other one is as much code again.)
 constexpr int kHgQuads = 2;
 template <int ST>
 __device__ __forceinline__ void hyper_row_ahead(const HyperStreamGemvArgs &a, const StreamCoef &coef, float *lo, float *hi, float *red) {
   const int K = a.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = kSgWarps * 32;
+  if (!(a.ahead & AHEAD_STATE)) pdl_wait();
   const int pos = a.Shift ? a.Ctrl[CTRL_POS] : 0;
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float4 nw[kHgQuads], sf[kHgQuads], pv[kHgQuads];
@@ -287,6 +289,6 @@ AINFER_REGISTER(PackRowsBf16, PackRowsBf16Args, 256, 0, 0, nullptr, F(Dst), F(Sr
 #undef F
 
 AINFER_EARLY_LAUNCH(StreamGemv);
-AINFER_EARLY_LAUNCH(HyperStreamGemv);
+AINFER_EARLY_LAUNCH_AHEAD(HyperStreamGemv, HyperStreamGemvArgs);
 
 }  // namespace ainfer

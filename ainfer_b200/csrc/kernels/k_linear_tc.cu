@@ -41,6 +41,7 @@ struct LinearTcArgs {
   void *Y;               // [rows][ldy]
   int32_t rows, N, K, nt, ldy, act, out16;
   float cap;
+  int32_t ahead;         // LaunchAhead
 };
 
 struct LinearTcGroupedArgs {
@@ -223,9 +224,9 @@ __device__ __forceinline__ void linear_tc_body(const Args &a) {
   if constexpr (PAIR) cluster_sync_all();   // both blocks' barriers are there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sh.tmem;
-  int pre = 0;   // stages of the first tile whose weights travel before the dependency wait (they do not depend on it)
+  int pre = 0;   // stages of the first tile whose weights travel before the dependency wait, where no launch before writes weights
   if constexpr (std::is_same<Args, LinearTcArgs>::value) {
-    if (warp == 0 && lane == 0 && first < lt_tiles(a, n_tiles)) {
+    if ((a.ahead & AHEAD_WEIGHTS) && warp == 0 && lane == 0 && first < lt_tiles(a, n_tiles)) {
       const LtTile t = lt_tile<TILE_N>(a, first, n_tiles);
       for (; pre < nst && pre < kb; ++pre) lt_fetch_w<PAIR>(a, &sh, base, stage_bytes, pre, rank, pre * 64, t.w0);
     }
@@ -515,8 +516,8 @@ AINFER_REGISTER(LinearTcGroupedPair, LinearTcGroupedArgs, kLtWide, 2, 0, linear_
 #undef F
 
 AINFER_EARLY_LAUNCH(LinearTcGrouped);
-AINFER_EARLY_LAUNCH(LinearTc);
-AINFER_EARLY_LAUNCH(LinearTcPair);
+AINFER_EARLY_LAUNCH_AHEAD(LinearTc, LinearTcArgs);
+AINFER_EARLY_LAUNCH_AHEAD(LinearTcPair, LinearTcArgs);
 AINFER_EARLY_LAUNCH(LinearTcGroupedPair);
 AINFER_EARLY_LAUNCH(LinearTcSplit2);
 AINFER_EARLY_LAUNCH(LinearTcSplit4);

@@ -221,9 +221,10 @@ struct WindowAttnStepMmaArgs {
   int32_t nseq, H, G, D, E, rd, cap, window, pool, koff, voff, goff;
   int32_t own_pool, splits, ldu, ldo, out16;   // splits <= 16
   float scale, softcap, eps;
+  int32_t ahead;           // LaunchAhead
 };
 constexpr int kWsStages = 2, kWsMaxSplits = 16;
-// As the chunk form, positions and the first tile (rows of earlier steps) are fetched before the dependency wait. Where
+// As the chunk form, a list of one step fetches positions and the first tile (rows of earlier steps) before the dependency wait. Where
 // another layer of the same step appends the rows (koff < 0), the tile that ends in the step's own row waits.
 // Loops stay rolled: a step runs the kernel once, and a third of its stalls were on code not yet fetched (90 KB of it; with
 // 64 KB the launch costs a decode step of Robopel, width 1024, 10 us and not 16).
@@ -239,6 +240,7 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
   const int D = a.D, E = a.E, HG = a.H / a.G, KW = a.G * D, VW = a.G * E;
   const int per_seq = a.splits + 1, split = blockIdx.x % per_seq, g = blockIdx.x / per_seq % a.G, seq = blockIdx.x / (per_seq * a.G);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (!(a.ahead & AHEAD_STATE)) pdl_wait();
   const int pos = a.Ctrl[4 * seq + CTRL_POS];
   const float *u = a.U + (size_t)seq * a.ldu;
   const float2 *rot = a.Rot + (size_t)pos * (a.rd >> 1);
@@ -460,7 +462,8 @@ WINDOW_STEP(256)
       F(Count), F(O), F(nseq), F(H), F(G), F(D), F(E), F(rd), F(cap), F(window), F(pool), F(koff), F(voff), F(goff), F(own_pool), F(splits), \
       F(ldu), F(ldo), F(out16), F(scale), F(softcap), F(eps)
 #define WS_REGISTER(DP) \
-  AINFER_REGISTER(WindowAttnStepMma##DP, WindowAttnStepMmaArgs, 128, 0, 0, window_step_smem##DP, WS_FIELDS); AINFER_EARLY_LAUNCH(WindowAttnStepMma##DP)
+  AINFER_REGISTER(WindowAttnStepMma##DP, WindowAttnStepMmaArgs, 128, 0, 0, window_step_smem##DP, WS_FIELDS); \
+  AINFER_EARLY_LAUNCH_AHEAD(WindowAttnStepMma##DP, WindowAttnStepMmaArgs)
 WS_REGISTER(32);
 WS_REGISTER(64);
 WS_REGISTER(96);

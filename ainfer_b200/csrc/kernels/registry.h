@@ -30,6 +30,17 @@ struct KernelDesc {
   // 1: the kernel orders itself after its predecessor with griddepcontrol.wait, so a
   // command list may launch it early (programmatic dependency) to overlap its start-up
   int early_launch = 0;
+  // Where the argument struct keeps the bits of LaunchAhead, -1: nowhere. Not an argument: every launch sets it
+  // from what its list or chain was promised.
+  int ahead_offset = -1;
+};
+
+// What an early launch may read before its dependency wait, since no launch it can overtake writes it. A kernel triggers
+// its successor in its first instruction, so one that does not wait can be ahead of every launch back to the last
+// ordinary one, not only of its predecessor.
+enum LaunchAhead {
+  AHEAD_WEIGHTS = 1,   // weights
+  AHEAD_STATE = 2      // position, state and caches as earlier steps left them
 };
 
 void register_kernel(const KernelDesc &d);
@@ -62,6 +73,11 @@ struct EarlyLaunchMark {
   explicit EarlyLaunchMark(const char *name) { mark_kernel_early_launch(name); }
 };
 
+void mark_kernel_ahead(const char *name, int offset);
+struct AheadMark {
+  AheadMark(const char *name, int offset) { mark_kernel_ahead(name, offset); }
+};
+
 struct Registrar {
   explicit Registrar(const KernelDesc &d) { register_kernel(d); }
 };
@@ -87,3 +103,7 @@ struct Registrar {
 // After AINFER_REGISTER(NAME, ...): the kernel calls pdl_wait() before it touches anything a
 // predecessor writes (or that a predecessor still reads and it overwrites).
 #define AINFER_EARLY_LAUNCH(NAME) static ::ainfer::EarlyLaunchMark NAME##_early(#NAME)
+// The same for a kernel with a member int32_t ahead in its argument struct T: it reads what those bits allow before it waits.
+#define AINFER_EARLY_LAUNCH_AHEAD(NAME, T) \
+  AINFER_EARLY_LAUNCH(NAME);               \
+  static ::ainfer::AheadMark NAME##_ahead(#NAME, (int)offsetof(T, ahead))

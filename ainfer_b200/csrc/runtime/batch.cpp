@@ -114,7 +114,7 @@ int BatchDecode::create_rows(int owned, bool f32) {
   for (int i = 0; i < n; ++i) id[(size_t)i] = i;
   if (ainfer_memcpy_h2d(dev, seq, id.data(), id.size() * 4) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }
   ainfer_list_t l = nullptr;
-  if (ainfer_list_create(dev, &l) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }
+  if (ainfer_list_create(dev, &l) != AINFER_OK || ainfer_list_one_step(l) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }
   lists.push_back(l);
   tail_list = l;
   Rec rec(this, l);
@@ -138,7 +138,7 @@ int BatchDecode::record() {
   DeviceTensor emb = m->tensor("model.language_model.embed_tokens.weight");
   if (!emb.entry) { err = "missing model.language_model.embed_tokens.weight"; return 1; }
   auto new_list = [&](ainfer_list_t *l) {
-    if (ainfer_list_create(dev, l) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }
+    if (ainfer_list_create(dev, l) != AINFER_OK || ainfer_list_one_step(*l) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }
     lists.push_back(*l);
     return 0;
   };

@@ -567,7 +567,7 @@ int session_create(DeviceModel *m, int max_ctx, int flags, Session **out, std::s
   // ---- record ----
   Recorder rec(s);
   auto new_list = [&](ainfer_list_t *l) {
-    if (ainfer_list_create(s->dev, l) != AINFER_OK) { s->err = "list create failed"; rec.status = 1; }
+    if (ainfer_list_create(s->dev, l) != AINFER_OK || ainfer_list_one_step(*l) != AINFER_OK) { s->err = "list create failed"; rec.status = 1; }
     rec.list = *l;
   };
   if ((flags & (SESSION_PERSISTENT | SESSION_STAGE_CLOCK)) && !(flags & SESSION_PER_LAYER_LISTS)) {

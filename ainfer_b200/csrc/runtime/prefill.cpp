@@ -83,7 +83,7 @@ struct Launcher : KernelCalls {   // immediate launches, or appended to recorded
       p->vlists.push_back(list);
       list = nullptr;
     }
-    if (open_next && ainfer_list_create(s->dev, &list) != AINFER_OK) { s->err = ainfer_last_error(s->dev); status = 1; }
+    if (open_next && (ainfer_list_create(s->dev, &list) != AINFER_OK || ainfer_list_one_step(list) != AINFER_OK)) { s->err = ainfer_last_error(s->dev); status = 1; }
   }
   // Y[rows][N] = X[rows][K] . W^T on the tensor cores
   void gemm(const DeviceTensor &t, const int8_t *XQ, const float *SQ, float *Y, int K, int rows) {

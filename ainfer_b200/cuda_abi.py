@@ -60,6 +60,7 @@ SIGNATURES = {
     "ainfer_list_append_fill": (_i, [_vp, _vp, _i, _sz]),
     "ainfer_list_close": (_i, [_vp]),
     "ainfer_list_launch_count": (_i, [_vp, C.POINTER(_u32)]),
+    "ainfer_list_one_step": (_i, [_vp]),
     "ainfer_list_destroy": (_i, [_vp]),
     "ainfer_list_execute": (_i, [_vp]),
     "ainfer_kernel_launch": (_i, [_vp, _vp, _u32]),
@@ -266,6 +267,10 @@ class CommandList:
         h = C.c_void_p()
         dev.check(dev.L.ainfer_list_create(dev.h, C.byref(h)))
         self.h = h
+
+    def one_step(self):
+        """Before the first append: the list holds one decode step (ainfer_list_one_step)."""
+        self.dev.check(self.dev.L.ainfer_list_one_step(self.h))
 
     def append(self, kernel, groups):
         self.dev.check(self.dev.L.ainfer_list_append_launch(self.h, kernel.h, groups))

@@ -113,6 +113,11 @@ int ainfer_list_create(ainfer_device_t dev, ainfer_list_t *out);
 int ainfer_list_append_launch(ainfer_list_t list, ainfer_kernel_t k, uint32_t group_count);
 int ainfer_list_append_memcpy(ainfer_list_t list, void *dst, const void *src, size_t bytes);
 int ainfer_list_append_fill(ainfer_list_t list, void *dst, int byte_value, size_t bytes);
+/* States, before the first append, that the list holds one decode step: none of its launches writes weights,
+ * or a position, state or cache row that a later launch of the list reads as an earlier step's. Kernels that wait
+ * for their predecessor by themselves may then read those before they wait; in any other list every launch
+ * finds what the launches before it wrote. No counterpart in the reference: its barriers are full ones. */
+int ainfer_list_one_step(ainfer_list_t list);
 int ainfer_list_close(ainfer_list_t list);
 int ainfer_list_launch_count(ainfer_list_t list, uint32_t *launches);
 int ainfer_list_destroy(ainfer_list_t list);

@@ -417,6 +417,87 @@ def test_wide_stream_update_read_norm_and_shift(dev, W, S, per, out):
     test_stream_update_read_norm_and_shift(dev, W, S, per, out)
 
 
+@pytest.mark.parametrize("what", ["chunk", "streams"])
+def test_a_list_of_several_steps_is_ordered(dev, what):
+    """Six positions in one list: every step finds the position that ControlAdvance set and the state the steps before it left,
+    although the kernels may start before those are done. The same launches one by one give the same bits."""
+    g = torch.Generator().manual_seed(3)
+    rn = lambda *s: torch.randn(*s, generator=g)   # noqa: E731
+    up = lambda t: dev.upload(f32(t))   # noqa: E731
+    steps, pos0 = 6, 63
+    if what == "chunk":      # convolution ring, keys over the end of a tile, position
+        H, G, D, taps, cap, chunk, splits = 8, 2, 64, 4, 128, 500, 3
+        C, Q, K = (H + G) * D, H * D, G * D
+        st0, kc0 = f32(rn(1, taps, C)), bits(rn(1, cap, K))
+        du, dcw, dtemp = up(rn(1, C)), up(rn(taps, C)), up(torch.rand(H, generator=g))
+        lb = _table(dev, torch.rand(H, generator=g), torch.rand(H, generator=g), 500)
+        outs = [dev.zeros(Q * 4) for _ in range(steps)]
+        k = dev.kernel("ChunkAttnStepMma64")
+
+        def run(st, state, launch):
+            kc, cnt, part = dev.upload(kc0), dev.zeros(G * 4), dev.zeros(splits * H * (D + 4) * 4)
+            for o in outs:
+                k.set_args(du, dcw, state, st, kc, cap * K, lb, dtemp, part, cnt, o, 1, H, G, D, taps, cap, chunk, 500, splits, C, Q, 0, 0.3)
+                launch(k, G * splits)
+                launch(adv, 1)
+            return kc, (cap, K), np.int16
+    else:                    # token shift by position parity, eight outputs a block
+        S, K, N = 4, 1024, 2000
+        st0 = f32(rn(2, K))
+        x, mix, o, i, nw, sh = up(rn(S, K)), up(rn(S, S)), up(rn(S)), up(rn(S)), up(rn(K)), up(torch.rand(K, generator=g))
+        w, y = dev.upload(bits(rn(N, K))), up(rn(K))
+        outs = [dev.zeros(N * 4) for _ in range(steps)]
+        k = dev.kernel("HyperStreamGemv")
+
+        def run(st, state, launch):
+            xs = [x] + [dev.zeros(S * K * 4) for _ in range(steps)]
+            for n, out in enumerate(outs):
+                k.set_args(xs[n], y, mix, o, xs[n + 1], i, nw, sh, state, st, w, 0, out, S, N, K, K, 8, 0, 1e-3, 0.0)
+                launch(k, N // 8)
+                launch(adv, 1)
+            return xs[-1], (S, K), np.float32
+    adv = dev.kernel("ControlAdvance")
+    got = []
+    for one_by_one in (True, False):
+        st, state = dev.upload(ctrl([pos0])), dev.upload(st0)
+        adv.set_args(st, st, 0)
+        if one_by_one:
+            last = run(st, state, lambda kern, n: kern.launch(n))
+        else:
+            lst = dev.new_list()
+            last = run(st, state, lambda kern, n: lst.append(kern, n))
+            lst.close()
+            lst.execute()
+        dev.sync()
+        got.append([dev.download(o, 500, np.float32) for o in outs] + [dev.download(state, st0.shape, np.float32), dev.download(last[0], *last[1:])])
+        assert dev.download(st, 4, np.int32)[1] == pos0 + steps
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
+def test_weights_made_inside_a_list(dev):
+    """A list may make the weights of its next product; a list of one step states that it does not."""
+    from ainfer_b200 import cuda_abi
+    g = torch.Generator().manual_seed(1)
+    R, K, N = 300, 256, 384
+    x, w = bf16(torch.randn(R, K, generator=g)), bf16(torch.randn(N, K, generator=g))
+    a, b = dev.zeros(R * N * 2), dev.zeros(R * R * 4)
+    dx, dw, tm = dev.upload(bits(x)), dev.upload(bits(w)), dev.tensor_map_bf16
+    k, lst = dev.kernel("LinearTc"), dev.new_list()
+    k.set_args(tm(dw, N, K, K, 128), tm(dx, R, K, K, 128), 0, a, R, N, K, 128, N, 0, 1, 0.0)
+    lst.append(k, 9)
+    k.set_args(tm(a, R, N, N, 128), tm(a, R, N, N, 128), 0, b, R, R, N, 128, R, 0, 0, 0.0)     # its rows against themselves
+    lst.append(k, 9)
+    with pytest.raises(cuda_abi.AinferError):
+        lst.one_step()
+    lst.close()
+    lst.execute()
+    dev.sync()
+    h = torch.from_numpy(from_bits(dev.download(a, (R, N), np.uint16), (R, N))).double()
+    close(h.numpy(), x.double() @ w.double().T, 1e-2)
+    close(dev.download(b, (R, R), np.float32), h @ h.T, 1e-5)
+
+
 # -------------------------------------------------------------------- models ---
 L = P.make_layer
 MODELS = {
