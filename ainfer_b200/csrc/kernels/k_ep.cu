@@ -30,7 +30,7 @@ struct RouterLogitsRowsArgs {
   const float *Bias;     // optional [E]: added to the routed experts' logits (load generators); null: none
   float *Logits;         // [rows][E+1]
   int32_t E, H, rows;
-  int32_t tokens_per_block;   // 8 or 16; launched with ceil((E + 1) / 32) x ceil(rows / tokens_per_block) blocks
+  int32_t tokens_per_block;   // a unit takes 16 tokens where this is 16 or more, else 8; blocks walk the units, any number of them
 };
 // Every sum is RouterTopK's: a lane's chain over its eight values of every 256, then the lane tree. A warp
 // sums four router rows against all of the block's tokens, so that a weight is fetched once per block of
@@ -40,13 +40,13 @@ struct RouterLogitsRowsArgs {
 // apart (side by side they meet the same banks). (One router row per warp and four tokens: bound by those
 // reads, 74 us for 192 tokens of 513 x 2048; this form 25.)
 constexpr int kRlRows = 32, kRlCols = 1024, kRlChunks = kRlCols / 256;
+__host__ __device__ inline int rl_tokens(int tokens_per_block) { return tokens_per_block >= 16 ? 16 : 8; }
 template <int TT>
-__device__ __forceinline__ void router_logits_rows_body(const RouterLogitsRowsArgs &a) {
+__device__ __forceinline__ void router_logits_rows_unit(const RouterLogitsRowsArgs &a, int unit) {
   extern __shared__ __align__(16) float rl_smem[];   // [TT][kRlChunks][2][32 lanes][4]
-  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nrows = a.E + (a.Wsg ? 1 : 0), n = a.H / 256;
-  const int nrb = (a.E + 1 + kRlRows - 1) / kRlRows, e0 = (blockIdx.x % nrb) * kRlRows + warp * 4, t0 = (blockIdx.x / nrb) * TT;
+  const int nrb = (a.E + 1 + kRlRows - 1) / kRlRows, e0 = (unit % nrb) * kRlRows + warp * 4, t0 = (unit / nrb) * TT;
   const uint4 *w[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {   // past the last row: that row again, not stored
@@ -58,7 +58,6 @@ __device__ __forceinline__ void router_logits_rows_body(const RouterLogitsRowsAr
   for (int u = 0; u < TT; ++u)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[u][j] = 0.0f;
-  pdl_wait();
   for (int i0 = 0; i0 < n; i0 += kRlChunks) {
     const int nc = min(kRlChunks, n - i0);
     __syncthreads();   // the last columns' readers are done
@@ -112,10 +111,16 @@ __device__ __forceinline__ void router_logits_rows_body(const RouterLogitsRowsAr
   }
 }
 __global__ void __launch_bounds__(256, 2) RouterLogitsRows(const RouterLogitsRowsArgs a) {
-  if (a.tokens_per_block == 16) router_logits_rows_body<16>(a);
-  else router_logits_rows_body<8>(a);
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tt = rl_tokens(a.tokens_per_block), units = (a.E + 1 + kRlRows - 1) / kRlRows * ((a.rows + tt - 1) / tt);
+#pragma unroll 1
+  for (int u = blockIdx.x; u < units; u += gridDim.x) {
+    if (tt == 16) router_logits_rows_unit<16>(a, u);
+    else router_logits_rows_unit<8>(a, u);
+  }
 }
-static uint32_t router_rows_smem(const void *args) { return (uint32_t)((const RouterLogitsRowsArgs *)args)->tokens_per_block * kRlCols * 4u; }
+static uint32_t router_rows_smem(const void *args) { return (uint32_t)rl_tokens(((const RouterLogitsRowsArgs *)args)->tokens_per_block) * kRlCols * 4u; }
 struct RouterSelectRowsArgs {
   const float *Logits;   // [rows][E+1]
   int32_t *SelIdx;       // [rows][k+1]

@@ -396,6 +396,28 @@ def test_moe_block(dev, E, k, H, I):
     assert np.array_equal(dev.download(dX, H, np.float32), res + acc)
 
 
+@pytest.mark.parametrize("E,H,rows,shared", [(64, 1024, 3, True), (31, 256, 17, True), (40, 1280, 33, False)])
+def test_router_logits_of_rows(dev, E, H, rows, shared):
+    """Every logit bit for bit, whatever the tokens per block and the number of blocks; nothing past the logits is written."""
+    L = O.lib()
+    rng = np.random.default_rng(E)
+    hn = rng.standard_normal((rows, H)).astype(np.float32)
+    W = O.bf16_bits((rng.standard_normal((E + 1, H)) * 0.05).astype(np.float32))
+    n = E + 1 if shared else E
+    want = np.full((rows, E + 1), 7.0, np.float32)
+    for t in range(rows):
+        want[t, :n] = [L.orc_dot_bf16(np.ascontiguousarray(W[e]), hn[t], H) for e in range(n)]
+    dW, dHn, size = dev.upload(W), dev.upload(hn), rows * (E + 1)
+    k = dev.kernel("RouterLogitsRows")
+    for tokens, groups in ((4, -(-(E + 1) // 8) * -(-rows // 4)), (8, 3), (16, 1), (16, 40), (1, 2), (7, 5), (64, 2), (1000, 1)):
+        out = dev.upload(np.full(size + 64, 7.0, np.float32))
+        k(groups, dW, dW + E * H * 2 if shared else 0, dHn, 0, out, E, H, rows, tokens)
+        dev.sync()
+        got = dev.download(out, size + 64, np.float32)
+        assert np.array_equal(got[:size].reshape(rows, E + 1), want), (tokens, groups)
+        assert np.all(got[size:] == 7.0)
+
+
 def test_argmax_first_max_wins_and_advance(dev):
     rng = np.random.default_rng(5)
     V = 151936
