@@ -20,16 +20,17 @@ struct ChunkConvSiluArgs {
   float *Snap;        // optional: the history [C][3] after row m at Snap + m * snap_stride (to roll a speculative chunk back); null: none
   int64_t snap_stride;
 };
-// Launched with ceil(C / 256) x (any number of) blocks: the rows are cut into that many runs, since a row
-// needs the three before it and not their results. (One run for all rows was a chain of loads: 109 us for
-// 192 rows of 8192 channels; runs of 16 rows 12 us.) The first run's threads read the history, and so they
-// are the ones that replace it.
+// Launched with ceil(C / 256) x (any number of) blocks: the rows are cut into at most that many runs, since a
+// row needs the three before it and not their results. (One run for all rows was a chain of loads: 109 us for
+// 192 rows of 8192 channels; runs of 16 rows 12 us.) No run but the last is shorter than the history's three
+// rows, so that only the first one's threads read the history, and they are the ones that replace it.
+// With more than one run Mx and QKV are different buffers.
 __global__ void __launch_bounds__(256) ChunkConvSilu(const ChunkConvSiluArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   const int cb = (a.C + 255) / 256, runs = max(1, (int)gridDim.x / cb), run = blockIdx.x / cb;
   const int c = (blockIdx.x % cb) * 256 + threadIdx.x;
-  const int per = (a.M + runs - 1) / runs, m0 = run * per, m1 = min(m0 + per, a.M);
+  const int per = max(3, (a.M + runs - 1) / runs), m0 = run * per, m1 = min(m0 + per, a.M);
   if (c >= a.C || run >= runs || (m0 >= m1 && run > 0)) return;
   // rows before the first come from the history, oldest first
   auto row = [&](int m) { return m >= 0 ? a.QKV[(size_t)m * a.C + c] : a.CS[c * 3 + 3 + m]; };

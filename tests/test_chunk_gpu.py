@@ -104,6 +104,29 @@ def test_chunk_conv_silu_equals_sequential(dev, C, chunks):
     assert np.array_equal(dev.download(dCS, C * 3, np.float32), cs)
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 17, 33])
+def test_chunk_conv_silu_in_runs(dev, M):
+    """Any number of runs of rows, more than there are rows too: outputs, history and snapshots of one row after the other."""
+    L = O.lib()
+    rng = np.random.default_rng(M)
+    C = 520
+    x = rng.standard_normal((M, C)).astype(np.float32)
+    cw = (rng.standard_normal((C, 4)) * 0.5).astype(np.float32)
+    cs0 = rng.standard_normal((C, 3)).astype(np.float32)
+    cs, want, hist = cs0.copy().reshape(-1), np.zeros((M, C), np.float32), []
+    for m in range(M):
+        L.orc_conv_silu(np.ascontiguousarray(x[m]), cs, cw.reshape(-1), C, want[m])
+        hist.append(cs.copy())
+    k, dX, dCW = dev.kernel("ChunkConvSilu"), dev.upload(x), dev.upload(cw)
+    for runs in (1, 2, 3, M, 2 * M, 40):
+        dMx, dCS, dSn = dev.zeros(M * C * 4), dev.upload(cs0), dev.zeros(M * C * 12)
+        k(-(-C // 256) * runs, dMx, dX, dCS, dCW, C, M, dSn, C * 3)
+        dev.sync()
+        assert np.array_equal(dev.download(dMx, (M, C), np.float32), want), runs
+        assert np.array_equal(dev.download(dCS, C * 3, np.float32), cs), runs
+        assert np.array_equal(dev.download(dSn, (M, C * 3), np.float32), np.stack(hist)), runs
+
+
 def test_chunk_snapshots_hold_the_state_after_every_row(dev):
     """Speculative rows: with a snapshot buffer the kernels also keep the state after each row, so a
     caller can roll back to any of them."""
