@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kChunkThreads) ChunkDeltaNet(const ChunkDeltaN
   float s[2 * SEG], po = 0.0f;
   float *out = a.Out + (size_t)h * D + col;   // of the last row begun
   if (helper) {
-    stage(0);
+    if (chunks > 0) stage(0);
   } else {
 #pragma unroll
     for (int r = 0; r < 2 * SEG; ++r) s[r] = Sh[(size_t)r * D];

@@ -127,6 +127,16 @@ def test_chunk_conv_silu_in_runs(dev, M):
         assert np.array_equal(dev.download(dSn, (M, C * 3), np.float32), np.stack(hist)), runs
 
 
+def test_chunk_delta_net_of_no_rows(dev):
+    """Leaves the state and the outputs as they are, and reads no row (the pointer to them may be null)."""
+    S0 = np.random.default_rng(2).standard_normal((4, D * D)).astype(np.float32)
+    dS, dOut = dev.upload(S0), dev.upload(np.full(4 * D, 3.0, np.float32))
+    dev.kernel("ChunkDeltaNet")(16, dOut, 0, dS, 0, 0, 2, 4, 0, 0, 0)
+    dev.sync()
+    assert np.array_equal(dev.download(dS, (4, D * D), np.float32), S0)
+    assert np.all(dev.download(dOut, 4 * D, np.float32) == 3.0)
+
+
 def test_chunk_snapshots_hold_the_state_after_every_row(dev):
     """Speculative rows: with a snapshot buffer the kernels also keep the state after each row, so a
     caller can roll back to any of them."""
