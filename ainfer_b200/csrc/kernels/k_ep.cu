@@ -196,24 +196,35 @@ struct EpTcGroup {           // = TcGroup of the grouped tensor-core GEMM
   int32_t x_row0, M, y_col, pad;
 };
 static_assert(sizeof(EpTcGroup) == 32, "layout of the grouped GEMM's problem record");
+// Counts of a grouping: items in total; gate/up and down problems of experts with at most eight rows; the same of experts
+// with more; gate/up and down problems in the lists.
+constexpr int kEpFewRows = 8, kEpCountGateUp = 5, kEpCountDown = 6;
+__device__ __forceinline__ void ep_store_counts(int32_t *c, int items, int few, int all) {
+  reinterpret_cast<int4 *>(c)[0] = make_int4(items, 2 * few, few, 2 * (all - few));
+  reinterpret_cast<int4 *>(c)[1] = make_int4(all - few, 2 * all, all, 0);
+}
+// The problems of one expert's rows, at most max_rows each, from index g of the lists on.
+__device__ __forceinline__ void ep_problems(EpTcGroup *gate_up, EpTcGroup *down, const ExpertW &w, int row0, int rows, int max_rows, int I, int g) {
+  for (int j = 0; j * max_rows < rows; ++j, ++g) {
+    const int r0 = row0 + j * max_rows, mr = min(max_rows, rows - j * max_rows);
+    gate_up[2 * g] = EpTcGroup{w.gP, w.gS, r0, mr, 0, 0};
+    gate_up[2 * g + 1] = EpTcGroup{w.uP, w.uS, r0, mr, I, 0};
+    down[g] = EpTcGroup{w.dP, w.dS, r0, mr, 0, 0};
+  }
+}
 struct EpGroupArgs {
   const unsigned char *Recv;  // dispatch buffer received (R slots)
   const ExpertW *Experts;     // the layer's table [E+1]
   int32_t *Sorted;            // [R*cap]: src << 16 | index in the source's slot, grouped by expert
-  // Problems are listed by size: up to small_rows rows for the dp4a kernel that streams weights
-  // once (Int4GemvA8MultiGrouped), more for the tensor-core kernel (Int4GemmA8TcGrouped).
-  EpTcGroup *GroupsGateUp;    // [2 * (experts_per_rank + 1)]: gate and up problem of every active expert with few rows
-  EpTcGroup *GroupsDown;      // [experts_per_rank + 1]
-  EpTcGroup *GroupsGateUpL;   // the same for experts with many rows
-  EpTcGroup *GroupsDownL;
-  int32_t *Counts;            // [8]: items in total, gate/up and down problems (few rows), gate/up and down problems (many rows)
+  EpTcGroup *GroupsGateUp;    // gate and up problem of every active expert and cut
+  EpTcGroup *GroupsDown;
+  int32_t *Counts;            // [8], see ep_store_counts
   int32_t world, rank, experts_per_rank, cap, I;
   uint32_t slot_bytes;
   // The shared expert of this rank's own rows rides in the same launches as one more problem:
   // its activations are rows [shared_row0, shared_row0 + shared_rows) of the grouped layout
   // (the owner's quantiser writes them there). shared_rows == 0: none.
   int32_t shared_row0, shared_rows, shared_expert;
-  int32_t small_rows;   // problems up to this many rows go to the first pair of lists (a large value: all of them)
   int32_t max_rows;     // an expert with more rows is cut into problems of at most this many (same weights, consecutive rows)
 };
 // One block. Items are numbered (source rank, index) in ascending order; an item's row in the
@@ -222,7 +233,7 @@ struct EpGroupArgs {
 __global__ void __launch_bounds__(1024) EpGroup(const EpGroupArgs a) {
   __shared__ short le[kEpMaxItems];          // local expert of every received item
   __shared__ int base[65];                   // first item number of every source
-  __shared__ int hist[1024], start[1024], active[1024];   // active: index in its list, many-row experts offset by 1 << 20
+  __shared__ int hist[1024], start[1024], active[1024];   // active: index of the expert's first problem
   const int tid = threadIdx.x;
   if (tid == 0) {
     int s = 0;
@@ -245,57 +256,30 @@ __global__ void __launch_bounds__(1024) EpGroup(const EpGroupArgs a) {
   }
   __syncthreads();
   if (tid < 32) {   // exclusive scans over the experts (counts, and "has items" flags): one warp, chunks of 32
-    int run = 0, nact = 0, nactl = 0;
+    int run = 0, all = 0, few = 0;
     for (int e0 = 0; e0 < a.experts_per_rank; e0 += 32) {
       const int e = e0 + tid;
-      const int c = e < a.experts_per_rank ? hist[e] : 0, f = c > 0 && c <= a.small_rows;
-      const int fl = c > a.small_rows ? (c + a.max_rows - 1) / a.max_rows : 0;   // problems in the many-row lists
-      int sc = c, sf = f, sl = fl;
+      const int c = e < a.experts_per_rank ? hist[e] : 0, np = (c + a.max_rows - 1) / a.max_rows;
+      int sc = c, sp = np;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
-        const int vc = __shfl_up_sync(kFull, sc, off), vf = __shfl_up_sync(kFull, sf, off), vl = __shfl_up_sync(kFull, sl, off);
-        if (tid >= off) { sc += vc; sf += vf; sl += vl; }
+        const int vc = __shfl_up_sync(kFull, sc, off), vp = __shfl_up_sync(kFull, sp, off);
+        if (tid >= off) { sc += vc; sp += vp; }
       }
-      if (e < a.experts_per_rank) { start[e] = run + sc - c; active[e] = fl ? (1 << 20) + nactl + sl - fl : nact + sf - f; }
+      if (e < a.experts_per_rank) { start[e] = run + sc - c; active[e] = all + sp - np; }
       run += __shfl_sync(kFull, sc, 31);
-      nact += __shfl_sync(kFull, sf, 31);
-      nactl += __shfl_sync(kFull, sl, 31);
+      all += __shfl_sync(kFull, sp, 31);
+      few += __popc(__ballot_sync(kFull, c > 0 && c <= kEpFewRows));
     }
     if (tid == 0) {
-      const int sh = a.shared_rows > 0 && a.shared_rows <= a.small_rows ? 1 : 0;
-      const int shl = a.shared_rows > a.small_rows ? (a.shared_rows + a.max_rows - 1) / a.max_rows : 0;
-      if (sh || shl) {
-        const ExpertW w = a.Experts[a.shared_expert];
-        const int cut = sh ? a.shared_rows : a.max_rows;
-        for (int j = 0; j < sh + shl; ++j) {
-          const int r0 = a.shared_row0 + j * cut, mr = min(cut, a.shared_rows - j * cut);
-          EpTcGroup *gu = sh ? a.GroupsGateUp + 2 * nact : a.GroupsGateUpL + 2 * (nactl + j), *gd = sh ? a.GroupsDown + nact : a.GroupsDownL + nactl + j;
-          gu[0] = EpTcGroup{w.gP, w.gS, r0, mr, 0, 0};
-          gu[1] = EpTcGroup{w.uP, w.uS, r0, mr, a.I, 0};
-          gd[0] = EpTcGroup{w.dP, w.dS, r0, mr, 0, 0};
-        }
-      }
-      *reinterpret_cast<int4 *>(a.Counts) = make_int4(total, 2 * (nact + sh), nact + sh, 2 * (nactl + shl));
-      *reinterpret_cast<int4 *>(a.Counts + 4) = make_int4(nactl + shl, 0, 0, 0);
+      const int sh = (a.shared_rows + a.max_rows - 1) / a.max_rows;
+      if (sh > 0) ep_problems(a.GroupsGateUp, a.GroupsDown, a.Experts[a.shared_expert], a.shared_row0, a.shared_rows, a.max_rows, a.I, all);
+      ep_store_counts(a.Counts, total, few + (a.shared_rows > 0 && a.shared_rows <= kEpFewRows), all + sh);
     }
   }
   __syncthreads();
-  for (int e = tid; e < a.experts_per_rank; e += blockDim.x) {
-    const int c = hist[e];
-    if (c > 0) {
-      const ExpertW w = a.Experts[a.rank * a.experts_per_rank + e];
-      const bool large = active[e] >= (1 << 20);
-      const int g = active[e] & ((1 << 20) - 1);
-      const int cut = large ? a.max_rows : c, np = (c + cut - 1) / cut;
-      for (int j = 0; j < np; ++j) {
-        const int r0 = start[e] + j * cut, mr = min(cut, c - j * cut);
-        EpTcGroup *gu = (large ? a.GroupsGateUpL : a.GroupsGateUp) + 2 * (g + j), *gd = (large ? a.GroupsDownL : a.GroupsDown) + g + j;
-        gu[0] = EpTcGroup{w.gP, w.gS, r0, mr, 0, 0};
-        gu[1] = EpTcGroup{w.uP, w.uS, r0, mr, a.I, 0};
-        gd[0] = EpTcGroup{w.dP, w.dS, r0, mr, 0, 0};
-      }
-    }
-  }
+  for (int e = tid; e < a.experts_per_rank; e += blockDim.x)
+    if (hist[e] > 0) ep_problems(a.GroupsGateUp, a.GroupsDown, a.Experts[a.rank * a.experts_per_rank + e], start[e], hist[e], a.max_rows, a.I, active[e]);
   for (int it = tid; it < total; it += blockDim.x) {
     const int l = le[it];
     int pos = start[l];
@@ -338,7 +322,7 @@ struct EpGroupLocalArgs {
   int32_t *ItemRow;           // [n*k]: place of an item
   EpTcGroup *GroupsGateUp;    // gate and up problem of every active expert and cut
   EpTcGroup *GroupsDown;
-  int32_t *Counts;            // [8] as EpGroup's
+  int32_t *Counts;            // [8], see ep_store_counts
   int32_t n, k, E, I;
   int32_t shared_row0, shared_rows, max_rows;
 };
@@ -391,20 +375,11 @@ __global__ void __launch_bounds__(1024) EpGroupLocal(const EpGroupLocalArgs a) {
       a.Sorted[pos] = i;
       a.ItemRow[i] = pos;
     }
-  auto problems = [&](const ExpertW &w, int row0, int rows, int g) {
-    for (int j = 0; j * a.max_rows < rows; ++j, ++g) {
-      const int r0 = row0 + j * a.max_rows, mr = min(a.max_rows, rows - j * a.max_rows);
-      a.GroupsGateUp[2 * g] = EpTcGroup{w.gP, w.gS, r0, mr, 0, 0};
-      a.GroupsGateUp[2 * g + 1] = EpTcGroup{w.uP, w.uS, r0, mr, a.I, 0};
-      a.GroupsDown[g] = EpTcGroup{w.dP, w.dS, r0, mr, 0, 0};
-    }
-  };
-  if (c > 0) problems(a.Experts[tid], first, c, g0);
+  if (c > 0) ep_problems(a.GroupsGateUp, a.GroupsDown, a.Experts[tid], first, c, a.max_rows, a.I, g0);
+  const int few = __syncthreads_count(c > 0 && c <= kEpFewRows);
   if (tid == 1023) {
-    if (a.shared_rows > 0) problems(a.Experts[a.E], a.shared_row0, a.shared_rows, total);
-    const int all = total + (a.shared_rows + a.max_rows - 1) / a.max_rows;
-    *reinterpret_cast<int4 *>(a.Counts) = make_int4(items, 0, 0, 2 * all);
-    *reinterpret_cast<int4 *>(a.Counts + 4) = make_int4(all, 0, 0, 0);
+    if (a.shared_rows > 0) ep_problems(a.GroupsGateUp, a.GroupsDown, a.Experts[a.E], a.shared_row0, a.shared_rows, a.max_rows, a.I, total);
+    ep_store_counts(a.Counts, items, few + (a.shared_rows > 0 && a.shared_rows <= kEpFewRows), total + (a.shared_rows + a.max_rows - 1) / a.max_rows);
   }
 }
 struct EpGatherLocalArgs {
@@ -532,8 +507,8 @@ AINFER_REGISTER(EpPlan, EpPlanArgs, 1024, 0, 0, nullptr, F(SelIdx), F(Send), F(I
 AINFER_REGISTER(EpPack, EpPackArgs, 128, 1, 0, nullptr, F(Q8), F(SQ), F(ItemDest), F(Send), F(k), F(H), F(cap), F(slot_bytes));
 #undef F
 #define F(f) AINFER_ARG(EpGroupArgs, f)
-AINFER_REGISTER(EpGroup, EpGroupArgs, 1024, 0, 0, nullptr, F(Recv), F(Experts), F(Sorted), F(GroupsGateUp), F(GroupsDown), F(GroupsGateUpL), F(GroupsDownL), F(Counts), F(world),
-                F(rank), F(experts_per_rank), F(cap), F(I), F(slot_bytes), F(shared_row0), F(shared_rows), F(shared_expert), F(small_rows), F(max_rows));
+AINFER_REGISTER(EpGroup, EpGroupArgs, 1024, 0, 0, nullptr, F(Recv), F(Experts), F(Sorted), F(GroupsGateUp), F(GroupsDown), F(Counts), F(world),
+                F(rank), F(experts_per_rank), F(cap), F(I), F(slot_bytes), F(shared_row0), F(shared_rows), F(shared_expert), F(max_rows));
 #undef F
 #define F(f) AINFER_ARG(EpGatherArgs, f)
 AINFER_REGISTER(EpGather, EpGatherArgs, 128, 1, 0, nullptr, F(Recv), F(Sorted), F(Counts), F(XQ), F(SQ), F(H), F(cap), F(slot_bytes));

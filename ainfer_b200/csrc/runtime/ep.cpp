@@ -160,7 +160,7 @@ int EpMoe::create(DeviceModel *model, const void *id128, int rank_, int world_, 
   cap = n * k;
   const int most = world == 1 && (flags & EP_LARGE) ? 8192 : 2048;
   if (cap > most || batch * k > most) { err = "usage: batch x top-k above the planner's limit (" + std::to_string(most) + " items)"; return 2; }
-  // shapes the dp4a kernel does not take run every expert as one tensor-core problem, which holds at most 64 rows
+  // a limit of the forms this block was first built from; problems of at most 64 rows would take these shapes too
   if (batch > 64 && !(256 % (H / 128) == 0 && 256 % (I / 128) == 0)) { err = "usage: more than 64 rows need hidden and intermediate sizes whose group counts divide 256"; return 2; }
   slot_d = (uint32_t)((16 + (size_t)cap * 16 + (size_t)cap * item_bytes(H) + 15) & ~(size_t)15);
   slot_r = (uint32_t)((size_t)cap * H * 4);
@@ -180,9 +180,8 @@ int EpMoe::create(DeviceModel *model, const void *id128, int rank_, int world_, 
     r |= alloc(&Ret, (size_t)world * slot_r); r |= alloc(&Back, (size_t)world * slot_r);
   }
   r |= alloc(&Sorted, (size_t)rows * 4); r |= alloc(&Counts, 32);
-  r |= alloc(&GroupsGU, (size_t)2 * (epr + 1) * 32); r |= alloc(&GroupsD, (size_t)(epr + 1) * 32);
-  const size_t nlarge = (size_t)epr + 1 + (size_t)rows / 64 + (size_t)n / 64 + 2;   // an expert with more than 64 rows is cut into 64-row problems
-  r |= alloc(&GroupsGUL, 2 * nlarge * 32); r |= alloc(&GroupsDL, nlarge * 32);
+  const size_t most_problems = (size_t)epr + 1 + (size_t)rows / 64 + (size_t)n / 64 + 2;   // an expert with more than 64 rows is cut into 64-row problems
+  r |= alloc(&GroupsGU, 2 * most_problems * 32); r |= alloc(&GroupsD, most_problems * 32);
   r |= alloc(&XQs, (size_t)(rows + n) * H); r |= alloc(&SQs, (size_t)(rows + n) * G * 4);
   r |= alloc(&GU, (size_t)(rows + shn) * 2 * I * 4); r |= alloc(&AQ, (size_t)(rows + shn) * I);
   r |= alloc(&ASQ, (size_t)(rows + shn) * (I / 128) * 4);
@@ -223,14 +222,14 @@ int emit_route(EpMoe *e, Rec &r, int L, int rows) {
            (int32_t)(e->shared ? 1 : 0));
   return 0;
 }
-// The experts' products over the grouped rows: problems of GroupsGUL / GroupsDL.
+// The experts' products over the grouped rows: problems of GroupsGU / GroupsD.
 void emit_experts(EpMoe *e, Rec &r, int front, int shared_rows, int max_rows) {   // front: rows the received items may take
   const uint32_t blocks = (uint32_t)(2 * e->sm_count);
-  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsGUL, (const int32_t *)(e->Counts + 3), (const int8_t *)e->XQs, (const float *)e->SQs,
+  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsGU, (const int32_t *)(e->Counts + 5), (const int8_t *)e->XQs, (const float *)e->SQs,
            e->GU, (int32_t)e->I, (int32_t)e->H, (int32_t)max_rows, (int32_t)(2 * e->I));
   r.launch("SiluQuantRows", (uint32_t)(front + shared_rows), (const float *)e->GU, (const int32_t *)e->Counts, e->AQ, e->ASQ, (int32_t)e->I,
            (int32_t)(e->world * e->cap), (int32_t)front);
-  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsDL, (const int32_t *)(e->Counts + 4), (const int8_t *)e->AQ, (const float *)e->ASQ,
+  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsD, (const int32_t *)(e->Counts + 6), (const int8_t *)e->AQ, (const float *)e->ASQ,
            e->Y2, (int32_t)e->H, (int32_t)e->I, (int32_t)max_rows, (int32_t)e->H);
 }
 // One rank: `rows` of its rows, no dispatch. (A dispatch buffer, its copy, the un-permute and its copy moved
@@ -239,7 +238,7 @@ int emit_local(EpMoe *e, Rec &r, int L, int rows) {
   if (emit_route(e, r, L, rows)) return 1;
   const ExpertW *tab = (const ExpertW *)e->m->expert_tables + (size_t)L * (e->E + 1);
   const int items = rows * e->k, shared_rows = e->shared ? rows : 0, cut = std::min(rows, 64);
-  r.launch("EpGroupLocal", 1u, (const int32_t *)e->SelIdx, tab, e->Sorted, e->ItemDest, e->GroupsGUL, e->GroupsDL, e->Counts, (int32_t)rows,
+  r.launch("EpGroupLocal", 1u, (const int32_t *)e->SelIdx, tab, e->Sorted, e->ItemDest, e->GroupsGU, e->GroupsD, e->Counts, (int32_t)rows,
            (int32_t)e->k, (int32_t)e->E, (int32_t)e->I, (int32_t)e->cap, (int32_t)shared_rows, (int32_t)cut);
   r.launch("EpGatherLocal", (uint32_t)items, (const int8_t *)e->Q8, (const float *)e->SQ, (const int32_t *)e->Sorted, e->XQs, e->SQs, (int32_t)e->H,
            (int32_t)e->k);
@@ -278,9 +277,9 @@ int EpMoe::record_layer(int L) {
   if (close(r) || new_list(&la)) return 1;
   r.list = la;
   // ---- B: the experts of this rank on everything received ----
-  r.launch("EpGroup", 1u, (const unsigned char *)Recv, tab, Sorted, GroupsGU, GroupsD, GroupsGUL, GroupsDL, Counts, (int32_t)world, (int32_t)rank, (int32_t)epr,
+  r.launch("EpGroup", 1u, (const unsigned char *)Recv, tab, Sorted, GroupsGU, GroupsD, Counts, (int32_t)world, (int32_t)rank, (int32_t)epr,
            (int32_t)cap, (int32_t)I, slot_d, (int32_t)rows, (int32_t)(shared ? n : 0), (int32_t)E,
-           (int32_t)0, (int32_t)64);   // every expert in the second pair of lists, in problems of at most 64 rows
+           (int32_t)64);
   r.launch("EpGather", (uint32_t)rows, (const unsigned char *)Recv, (const int32_t *)Sorted, (const int32_t *)Counts, XQs, SQs, (int32_t)H,
            (int32_t)cap, slot_d);
   emit_experts(this, r, rows, shared ? n : 0, std::min(batch, 64));

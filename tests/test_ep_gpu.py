@@ -62,6 +62,93 @@ def test_one_rank_equals_oracle(preset, batch, layer):
     ep.close(); model.close(); dev.close()
 
 
+@pytest.mark.parametrize("batch", [3, 8, 9, 100])
+def test_counts_by_rows_of_an_expert(batch):
+    """The "counts" buffer: items, problems of experts with at most eight rows, of experts with more (cut at 64), and of both."""
+    from ainfer_b200 import cuda_abi, runtime
+    dev = cuda_abi.Device(0)
+    model = runtime.Model(dev, "synth:tiny:seed=2")
+    k = model.config["top_k"]
+    ep = runtime.EpMoe(model, batch)
+    ep.layer(0, _batch(model.config["hidden"], batch))
+    routed = ep.read("sel_idx", np.int32).reshape(batch, k + 1)[:, :k]
+    rows = np.append(np.bincount(routed.ravel(), minlength=model.config["experts"]), batch)     # the shared expert has them all
+    few, every = int(((rows > 0) & (rows <= 8)).sum()), sum(-(-int(c) // 64) for c in rows)
+    assert ep.read("counts", np.int32).tolist()[:7] == [batch * k, 2 * few, few, 2 * (every - few), every - few, 2 * every, every]
+    ep.close(); model.close(); dev.close()
+
+
+@pytest.mark.parametrize("world,n,cut", [(2, 20, 16), (4, 3, 64), (2, 40, 64), (1, 9, 5)])
+def test_kernels_of_several_ranks_one_after_the_other(world, n, cut):
+    """Plan, pack, group, gather, both grouped products, scatter and combine of every rank, one rank after the other on one
+    GPU with copies in the exchanges' place, against the oracle's products and sums: every row bit for bit."""
+    from ainfer_b200 import cuda_abi
+    L = O.lib()
+    dev = cuda_abi.Device(0)
+    rng = np.random.default_rng(world * 100 + n)
+    E, k, H, I = 16, 3, 256, 128
+    epr, cap = E // world, n * k
+    item, rows = H + ((H // 128 * 4 + 15) & ~15), world * n * k
+    slot_d, slot_r = (16 + cap * 16 + cap * item + 15) & ~15, cap * H * 4
+    W = [[O.quantize_int4((rng.standard_normal(sh) * 0.05).astype(np.float32)) for sh in ((I, H), (I, H), (H, I))] for _ in range(E + 1)]
+    tab = np.zeros((E + 1, 6), np.uint64)
+    for e in range(E + 1):
+        tab[e] = [dev.upload(a) for w in W[e] for a in w]
+    d_tab = dev.upload(tab.view(np.uint8))
+
+    def expert(e, q, s):
+        g, u = O.gemv_a8(*W[e][0], q, s), O.gemv_a8(*W[e][1], q, s)
+        act = np.array([(a / (np.float32(1.0) + np.float32(L.orc_expf(float(-a))))) * b for a, b in zip(g, u)], np.float32)
+        return O.gemv_a8(*W[e][2], *O.aquant(act))
+    p = np.exp(-0.3 * np.arange(E)); p /= p.sum()          # a few experts get most rows
+    ranks = []
+    for r in range(world):
+        x, res = rng.standard_normal((n, H)).astype(np.float32), rng.standard_normal((n, H)).astype(np.float32)
+        q = [O.aquant(v) for v in x]
+        sel = np.array([np.append(rng.choice(E, k, replace=False, p=p), E) for _ in range(n)], np.int32)
+        sw = rng.random((n, k + 1)).astype(np.float32)
+        want = np.zeros((n, H), np.float32)
+        for t in range(n):
+            acc = np.zeros(H, np.float32)
+            for j in range(k + 1):
+                acc = acc + sw[t, j] * expert(int(sel[t, j]), *q[t])
+            want[t] = res[t] + acc
+        d = dict(want=want, sel=dev.upload(sel), sw=dev.upload(sw), res=dev.upload(res), dest=dev.zeros(cap * 4), send=dev.zeros(world * slot_d),
+                 recv=dev.zeros(world * slot_d), ret=dev.zeros(world * slot_r), back=dev.zeros(world * slot_r), sorted=dev.zeros(rows * 4),
+                 counts=dev.zeros(32), gu=dev.zeros(64 * (2 * rows + 64)), gd=dev.zeros(64 * (rows + 64)), xq=dev.zeros((rows + n) * H),
+                 xs=dev.zeros((rows + n) * (H // 128) * 4), h=dev.zeros((rows + n) * 2 * I * 4), aq=dev.zeros((rows + n) * I),
+                 as_=dev.zeros((rows + n) * (I // 128) * 4), y=dev.zeros((rows + n) * H * 4), x=dev.zeros(n * H * 4))
+        d["q8"], d["sq"] = d["xq"] + rows * H, d["xs"] + rows * (H // 128) * 4
+        dev.write(d["q8"], np.stack([a for a, _ in q])); dev.write(d["sq"], np.stack([b for _, b in q]))
+        dev.kernel("EpPlan")(1, d["sel"], d["send"], d["dest"], n, k, epr, world, cap, slot_d)
+        dev.kernel("EpPack")(cap, d["q8"], d["sq"], d["dest"], d["send"], k, H, cap, slot_d)
+        ranks.append(d)
+
+    def exchange(src, dst, slot):
+        for a in range(world):
+            for b in range(world):
+                dev.copy_d2d(ranks[b][dst] + a * slot, ranks[a][src] + b * slot, slot)
+    exchange("send", "recv", slot_d)
+    for r, d in enumerate(ranks):
+        dev.kernel("EpGroup")(1, d["recv"], d_tab, d["sorted"], d["gu"], d["gd"], d["counts"], world, r, epr, cap, I, slot_d, rows, n, E, cut)
+        dev.kernel("EpGather")(rows, d["recv"], d["sorted"], d["counts"], d["xq"], d["xs"], H, cap, slot_d)
+        grouped = dev.kernel("Int4GemmA8TcGrouped")
+        grouped(37, d["gu"], d["counts"] + 20, d["xq"], d["xs"], d["h"], I, H, cut, 2 * I)
+        dev.kernel("SiluQuantRows")(rows + n, d["h"], d["counts"], d["aq"], d["as_"], I, rows, rows)
+        grouped(37, d["gd"], d["counts"] + 24, d["aq"], d["as_"], d["y"], H, I, cut, H)
+        dev.kernel("EpScatter")(rows, d["y"], d["sorted"], d["counts"], d["ret"], H, slot_r)
+    exchange("ret", "back", slot_r)
+    received = 0
+    for d in ranks:
+        dev.kernel("EpCombine")(n * -(-H // 256), d["res"], d["back"], d["dest"], d["sw"], d["y"] + rows * H * 4, d["x"], d["res"], k, H, slot_r)
+        dev.sync()
+        assert np.array_equal(dev.download(d["x"], (n, H), np.float32), d["want"])
+        assert np.array_equal(dev.download(d["res"], (n, H), np.float32), d["want"])
+        received += int(dev.download(d["counts"], 8, np.int32)[0])
+    assert received == world * cap
+    dev.close()
+
+
 def test_usage_errors():
     from ainfer_b200 import cuda_abi, runtime
     dev = cuda_abi.Device(0)
