@@ -272,7 +272,7 @@ int ainfer_ep_create(ainfer_model_t m, const void *id128, int rank, int world, i
   if (m->m->rows) return set_err(2, "usage: the expert-parallel block is the INT4 hybrid's");
   *out = nullptr;
   ainfer_ep_s *h = new ainfer_ep_s;
-  int r = h->e.create(m->m, id128, rank, world, batch, flags);
+  int r = h->e.create(m->m, id128, rank, world, batch, flags & (EP_ROUTER_BIAS | EP_RES_ADD));   // the larger planner is the prompt passes' own
   if (r) {
     set_err(r, h->e.err);
     h->e.destroy();

@@ -160,6 +160,19 @@ def test_usage_errors():
     model.close(); dev.close()
 
 
+def test_the_planner_of_prompt_passes_is_not_asked_for_by_a_flag():
+    """The documented limit of batch x top-k holds whatever other bits a caller sets."""
+    from ainfer_b200 import cuda_abi, runtime
+    dev = cuda_abi.Device(0)
+    model = runtime.Model(dev, "synth:tiny:seed=0")
+    for bit in range(2, 12):
+        with pytest.raises(Exception) as e:
+            runtime.EpMoe(model, 1025, flags=1 << bit)
+        assert "usage" in str(e.value)
+    runtime.EpMoe(model, 1024, flags=4).close()
+    model.close(); dev.close()
+
+
 def _rank_main(rank, world, conn, q, preset, batch, layer):
     os.environ["NCCL_NVLS_ENABLE"] = "0"
     from ainfer_b200 import cuda_abi, runtime
