@@ -170,10 +170,13 @@ static int ensure_prefill(Session *s) {
   if (!s->prefill) {
     // rows per pass: the planner of the expert-parallel block takes 2048 (row, expert) items over all ranks, and
     // 8192 on one rank, where a pass of many rows crosses the experts' weights once (a prompt of 701 tokens
-    // through the full preset: 99 ms in four passes, 63 ms in one)
+    // through the full preset: 99 ms in four passes, 63 ms in one). 768 = four blocks of the 192 rows that attend at a
+    // time, the largest such number within 8192 items at top-k 10. On one rank no more rows than the context holds: the
+    // buffers are the session's own, 374 MiB at 768 rows of the full preset.
     const int topk = s->m->cfg.top_k > 0 ? s->m->cfg.top_k : 1;
     const int most = std::max(1, (s->pf_world == 1 ? 8192 : 2048) / (topk * s->pf_world));   // rows a rank may bring to a pass
     int rows = s->pf_rows > 0 ? s->pf_rows : std::min(s->pf_world == 1 ? 768 : 192, most >= 8 ? most / 8 * 8 : most);
+    if (s->pf_world == 1) rows = std::min(rows, std::max(8, s->max_ctx));
     rows = std::max(1, std::min(rows, most));
     int r = prefill_create(s, rows, false, &s->prefill, s->pf_rank, s->pf_world, s->pf_id);
     if (r) return set_err(r, s->err);

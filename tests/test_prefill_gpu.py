@@ -65,6 +65,22 @@ def test_a_long_prompt_after_a_short_one(dev):
     a.close(); b.close(); model.close()
 
 
+def test_pass_buffers_follow_the_context(dev):
+    """A session of a short context allocates for the rows it can meet, and reads its whole context."""
+    from ainfer_b200 import runtime
+    model = runtime.Model(dev, "synth:small:seed=4")
+    ids = np.random.default_rng(1).integers(0, model.config["vocab"], 1024).astype(np.int32)
+    used = []
+    for ctx in (32, 1024):
+        s = runtime.Session(model, ctx)
+        free = dev.info().free_mem
+        s.prefill(ids[:ctx])
+        used.append(free - dev.info().free_mem)
+        s.close()
+    model.close()
+    assert used[0] < used[1] / 4, used
+
+
 def test_prefill_rejects_context_overflow(dev):
     from ainfer_b200 import runtime
     model = runtime.Model(dev, "synth:tiny:seed=0")
