@@ -1,7 +1,6 @@
-"""Int4GemmA8Tc (W4A8 group-128 GEMM on tcgen05 tensor cores, accumulators in tensor memory,
-weights streamed once for the whole batch) against the CPU oracle's one-row GEMV: every batch
-entry bit for bit, for the batch widths and shapes of the operator sweep, ragged row counts and
-several row tiles per block."""
+"""Int4GemmA8Tc (W4A8 group-128 GEMM on the tensor cores by mma.sync, weights widened in registers) against
+the CPU oracle's one-row GEMV: every batch entry bit for bit, for the batch widths and shapes of the
+operator sweep, ragged row counts, several row tiles per block, and units of 16, 32 and 64 entries."""
 import numpy as np
 import pytest
 
@@ -28,7 +27,9 @@ def run_tc(dev, P, S, xq, sq, N, K, M, groups=None):
 
 
 @pytest.mark.parametrize("N,K,M", [(136, 2048, 1), (136, 2048, 8), (512, 2048, 2), (512, 2048, 4), (2048, 512, 8),
-                                   (300, 128, 3), (1000, 1024, 16), (4096, 2048, 64), (2048, 512, 64), (640, 4096, 37)])
+                                   (300, 128, 3), (1000, 1024, 16), (4096, 2048, 64), (2048, 512, 64), (640, 4096, 37),
+                                   # more than 64 entries, an odd number of groups: units of 16, 32 and 64 entries
+                                   (1000, 384, 65), (4096, 384, 701), (8192, 384, 150)])
 def test_gemm_a8_tc_bit_exact(dev, N, K, M):
     rng = np.random.default_rng(N * 7 + K + M)
     w = (rng.standard_normal((N, K)) * 0.02).astype(np.float32)

@@ -1,5 +1,5 @@
-"""Chunked prefill (ainfer_session_prefill: up to 192 prompt rows per pass through row-batched
-kernels: tensor-core GEMMs, DeltaNet chunk kernels, per-row attention, the batched MoE block)
+"""Chunked prefill (ainfer_session_prefill: up to 768 prompt rows per pass, 192 with several ranks, through
+row-batched kernels: tensor-core GEMMs, DeltaNet chunk kernels, per-row attention, the batched MoE block)
 against token-by-token decoding of the same prompt: the tokens generated afterwards and the whole
 session state (DeltaNet state, conv history, INT8 KV cache and its scales) must be bit-identical."""
 import numpy as np
@@ -20,7 +20,7 @@ def dev():
 
 @pytest.mark.parametrize("preset,P,splits,flags", [("tiny", 150, [149], 0), ("mini", 131, [64, 1, 65], 0),
                                                    ("mini", 70, [69], 16), ("small", 100, [99], 16),
-                                                   ("mini", 461, [460], 0), ("small", 300, [299], 16)])   # passes of 192 rows and a ragged last one
+                                                   ("mini", 461, [460], 0), ("small", 300, [299], 16)])   # several blocks of rows that attend at a time
 def test_prefill_equals_token_by_token_decode(dev, preset, P, splits, flags):
     from ainfer_b200 import runtime
     model = runtime.Model(dev, f"synth:{preset}:seed=4")
@@ -31,7 +31,7 @@ def test_prefill_equals_token_by_token_decode(dev, preset, P, splits, flags):
     want = a.generate(prompt, G)
     b = runtime.Session(model, P + G + 8, flags)
     pos = 0
-    for n in splits:                      # several calls: the state carries over, chunks of 64 inside a call
+    for n in splits:                      # several calls: the state carries over
         b.prefill(prompt[pos:pos + n], start_pos=pos)
         pos += n
     assert pos == P - 1
@@ -46,6 +46,26 @@ def test_prefill_equals_token_by_token_decode(dev, preset, P, splits, flags):
     for name, dt in STATE:
         assert np.array_equal(a.read(name, dt), b.read(name, dt)), name
     a.close(); b.close(); c.close(); model.close()
+
+
+# rows: of a pass (None: as many as the library takes), 461 / 192: three passes of 154, 153 and 154; 2100: three of 700 in four blocks
+# that attend; 2048 x top-4 and 819 x top-10: the planner's 8192 items
+@pytest.mark.parametrize("preset,n,rows", [("mini", 461, 192), ("mini", 461, 7), ("tiny", 461, 100), ("mini", 2100, None), ("mini", 2048, 2048),
+                                           ("small", 819, 819), ("small", 900, None)])
+def test_passes_inside_a_call_hand_the_state_on(dev, preset, n, rows):
+    from ainfer_b200 import runtime
+    model = runtime.Model(dev, f"synth:{preset}:seed=4")
+    ids = np.random.default_rng(n).integers(0, model.config["vocab"], n + 1).astype(np.int32)
+    a, b = runtime.Session(model, n + 8), runtime.Session(model, n + 8)
+    for i in range(n):
+        a.step(int(ids[i]), i)
+    if rows:
+        b.prefill_rows(rows)
+    b.prefill(ids[:n])
+    for name, dt in STATE:
+        assert np.array_equal(a.read(name, dt), b.read(name, dt)), name
+    assert a.generate(ids[n:], 4, start_pos=n).tolist() == b.generate(ids[n:], 4, start_pos=n).tolist()
+    a.close(); b.close(); model.close()
 
 
 def test_a_long_prompt_after_a_short_one(dev):
@@ -110,7 +130,7 @@ def _ep_rank_main(rank, world, conn, q, preset, P):
     alone.prefill(prompt[:P - 1])
     ep = runtime.Session(model, P + G + 8)
     ep.prefill_ep(rank, world, nid)
-    ep.prefill(prompt[:P - 1])              # passes of 64 / world rows, the MoE block exchanged between the ranks
+    ep.prefill(prompt[:P - 1])              # the MoE block exchanged between the ranks
     same = all(np.array_equal(alone.read(name, dt), ep.read(name, dt)) for name, dt in STATE)
     t_alone = alone.generate(prompt[P - 1:], G, start_pos=P - 1)
     t_ep = ep.generate(prompt[P - 1:], G, start_pos=P - 1)
