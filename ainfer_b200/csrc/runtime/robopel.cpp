@@ -553,8 +553,9 @@ struct Engine : RowEngineBase {
                (const int32_t *)Count, (int32_t)N, (int32_t)mt.K, (int32_t)ldx, (int32_t)mt.ldw, (int32_t)ldy, (int32_t)act);
       return;
     }
-    // tiles of 256 outputs by pairs of blocks where the rows of a tile are many and there are rounds of them (as in linear())
-    const bool pair = nt >= 96 && N % 256 == 0 && units >= 2 * sm_count;
+    // tiles of 256 outputs by pairs of blocks: an expert's own outputs only, and rounds by the experts' mean rows
+    const long tiles = (long)r.experts * ((slots / (r.experts + r.identity) + nt - 1) / nt);
+    const bool pair = N % 256 == 0 && pairs_pay(nt, (tiles * (N / 128) + sm_count - 1) / sm_count, mt.K);
     TensorMap wm, xm;
     if (ainfer_tensor_map_bf16(dev, &wm, mt.w, (uint64_t)mt.N, (uint64_t)mt.K, (uint64_t)mt.ldw, 128) != AINFER_OK ||
         ainfer_tensor_map_bf16(dev, &xm, Xp, (uint64_t)slots, (uint64_t)mt.K, (uint64_t)ldx, (uint32_t)(pair ? nt / 2 : nt)) != AINFER_OK) {

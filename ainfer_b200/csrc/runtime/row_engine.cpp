@@ -165,17 +165,14 @@ void RowEngineBase::linear(KernelCalls &k, const RowMatrix &mt, const char *Xp, 
   const bool few = 2 * n_tiles * ((rows + 127) / 128) <= sm_count;   // tiles of 128 rows leave most SMs idle: split K instead
   bool pair = false;   // tiles of 256 outputs by pairs of blocks
   if (rows > 128 && !few) {
-    // rows of a tile: as large as possible (operand traffic), but a launch lasts whole rounds of tiles over the SMs. A
-    // pair's tile takes 1 / 1.15 of the time and the launch about 3.5 us more (60 rows of a tile at K = 2048). Measured at 2048 rows,
-    // us alone / in pairs: 2048 x 2048 (outputs x K) 22.7 / 24.7, 2560 x 2048 31.3 / 32.3, 8192 x 2048 64.3 / 57.4, 2048 x 8192 60.4 / 53.3.
-    double best = -1;
-    for (int p = 0; p < 2; ++p)
-      for (int t = 256; t >= 96; t -= 16) {
-        const int width = p ? 256 : 128, slots = p ? sm_count / 2 : sm_count;
-        const long tiles = (long)((mt.N + width - 1) / width) * ((rows + t - 1) / t), rounds = (tiles + slots - 1) / slots;
-        const double cost = p ? rounds * (t + 48.0) + 74.0 * 2048 / mt.K : rounds * (1.15 * t + 48.0);
-        if (best < 0 || cost < best) { best = cost; nt = t; pair = p; }
-      }
+    // rows of a tile: as large as possible (operand traffic), but a launch lasts whole rounds of tiles over the SMs
+    long best = -1, rounds = 0;
+    for (int t = 256; t >= 96; t -= 16) {
+      const long r = ((long)n_tiles * ((rows + t - 1) / t) + sm_count - 1) / sm_count, cost = r * (t + 48);
+      if (best < 0 || cost < best) { best = cost; nt = t; rounds = r; }
+    }
+    const long pairs = sm_count / 2, pair_rounds = ((long)((mt.N + 255) / 256) * ((rows + nt - 1) / nt) + pairs - 1) / pairs;
+    pair = pair_rounds <= rounds && pairs_pay(nt, rounds, mt.K);
   }
   const int tiles = n_tiles * ((rows + nt - 1) / nt);
   int splits = 1;   // few tiles: a cluster of blocks per tile, each a part of K

@@ -75,6 +75,14 @@ struct RowEngineBase : RowEngine {
       if (dim <= d) return base + std::to_string(d);
     return base + std::string("256");
   }
+  // Whether products of many rows go by pairs of blocks (LinearTcPair, LinearTcGroupedPair). A pair starts about a
+  // microsecond later and reads a third less from L2, which shows in wide tiles over a long launch only. us alone / in
+  // pairs, outputs x K: 2048 rows (tiles of 240) 8192 x 2048 59.0 / 55.2, 2048 x 8192 52.3 / 48.9, 4096 x 4096
+  // 53.1 / 50.0, 8192 x 1536 46.3 / 43.6, but 6144 x 1536 (three rounds) 32.5 / 33.3, 4096 x 2048 (two) 29.0 / 30.0, 8192 x
+  // 1024 (four) 34.1 / 36.2; 1800 rows (tiles of 208) 8192 x 2048 54.4 / 53.2, 2048 x 8192 49.0 / 47.6; tiles of 176 always
+  // lose (1500 rows, 8192 x 2048 48.1 / 49.4; 2048 x 8192 44.3 / 46.2). 32 experts of 375 rows 1024 x 2048 61.4 / 56.9,
+  // 2048 x 1024 60.5 / 61.5; of 100 rows 33.8 / 34.9.
+  static bool pairs_pay(int nt, long rounds, int K) { return nt >= 208 && K >= 1536 && rounds * K >= 6144; }
   // Blocks of a step's attention per (sequence, key head): few tiles each when there are many sequences. The cut decides
   // the order of the sums, so it depends on the sequences and heads alone and not on the context that was asked for:
   // the same tokens give the same logits in a session or batch of any length. (A cut by whole rounds of blocks over the
