@@ -115,6 +115,10 @@ __device__ __forceinline__ float stream_step_n(const float *src, const float *y,
 // How a row's elements are dealt to threads: four consecutive ones each, or one.
 __host__ __device__ __forceinline__ bool stream_vec(int S, int W) { return (W & 3) == 0 && S >= 1 && S <= 4; }
 
+// Whether all of the pointers (null ones too) lie on 16 bytes.
+template <typename... P>
+__host__ __device__ __forceinline__ bool on_quads(const P *...p) { return ((reinterpret_cast<unsigned long long>(p) | ...) & 15) == 0; }
+
 template <int ST>
 __device__ __forceinline__ float stream_row(const float *src, const float *y, float *dst, const StreamCoef &c, int W, bool update, float *hs,
                                             int tid, int nth) {

@@ -55,6 +55,10 @@ struct HyperNormRowsArgs {
   float eps;
 };
 
+// Whether the rows go through registers, below: whole quads, up to 2048 elements, small operands on 16 bytes.
+__host__ __device__ __forceinline__ bool hyper_norm_held(const HyperNormRowsArgs &a) {
+  return stream_vec(a.S, a.W) && a.W <= 2048 && on_quads(a.NormW, a.Shift, a.State, a.Pend);
+}
 // Rows of up to 2048 elements in whole quads and up to four streams: a thread owns QN quads of every row and walks
 // the block's rows with them in registers, weights and shift loaded once, the next row's loads in flight while this one is
 // summed and stored. Bound by memory: streams in and out, sublayer output, row (160 MB for 2048 rows of 4 x 2048).
@@ -76,7 +80,7 @@ __device__ __forceinline__ void hyper_norm_run(const HyperNormRowsArgs &a, const
     sf[q] = a.Shift ? ld_val4(a.Shift + at[q]) : zero;
     prev[q] = zero;
   }
-  const bool update = a.Y != nullptr, whole = (a.ldh & 3) == 0;
+  const bool update = a.Y != nullptr, whole = (a.ldh & 3) == 0 && (reinterpret_cast<unsigned long long>(a.H) & (4 * sizeof(T) - 1)) == 0;
   pdl_wait();
   const int r0 = blockIdx.x * a.per, r1 = min(a.rows, r0 + a.per);
   if (r0 >= r1) return;
@@ -157,7 +161,7 @@ __device__ __forceinline__ void hyper_norm_body(const HyperNormRowsArgs &a) {
   const int W = a.W, Wp = (W + 3) & ~3, tid = threadIdx.x;
   load_stream_coef(coef, a.Mix, a.Out, a.In, a.S);   // weights: they do not depend on the predecessor
   __syncthreads();
-  if (stream_vec(a.S, W) && W <= 2048) {
+  if (hyper_norm_held(a)) {
     float(*rd)[8] = reinterpret_cast<float(*)[8]>(red);
     if (a.S == 4) W <= 1024 ? hyper_norm_run<T, 4, 1>(a, coef, rd) : hyper_norm_run<T, 4, 2>(a, coef, rd);
     else if (a.S == 3) hyper_norm_run<T, 3, 2>(a, coef, rd);
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(256, 2) HyperNormRowsB16(const HyperNormRowsAr
 }
 static uint32_t hyper_norm_smem_fn(const void *args) {   // of the form that holds rows in shared memory
   const HyperNormRowsArgs *a = (const HyperNormRowsArgs *)args;
-  return stream_vec(a->S, a->W) && a->W <= 2048 ? 0u : 2u * 4u * (uint32_t)((a->W + 3) & ~3);
+  return hyper_norm_held(*a) ? 0u : 2u * 4u * (uint32_t)((a->W + 3) & ~3);
 }
 #define F(f) AINFER_ARG(HyperNormRowsArgs, f)
 #define HYPER_FIELDS                                                                                                            \

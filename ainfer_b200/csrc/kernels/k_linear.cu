@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kSgThreads, 3) HyperStreamGemv(const HyperStre
   if (tid >= nth) {
     gemv_produce(c, d, &sh, sg_smem);
   } else {
-    if (a.S == 4 && stream_vec(a.S, K) && K <= kHgQuads * nth * 4) {
+    if (a.S == 4 && stream_vec(a.S, K) && K <= kHgQuads * nth * 4 && on_quads(a.NormW, a.Shift, a.State)) {
       hyper_row_ahead<4>(a, coef, lo, hi, red);
     } else {
       const int lane = tid & 31, warp = tid >> 5;

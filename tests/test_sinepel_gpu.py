@@ -498,6 +498,35 @@ def test_weights_made_inside_a_list(dev):
     close(dev.download(b, (R, R), np.float32), h @ h.T, 1e-5)
 
 
+@pytest.mark.parametrize("what", ["HyperNormRowsF32", "HyperNormRowsB16", "HyperStreamGemv"])
+def test_small_operands_off_16_bytes(dev, what):
+    """Norm weights, shift, state and pending rows (and the output) at any multiple of their element, as in every other width."""
+    g = torch.Generator().manual_seed(2)
+    S, W, R, N = 4, 64, 5, 24
+    rn = lambda *s: torch.randn(*s, generator=g)   # noqa: E731
+    up = lambda t: dev.upload(f32(t))              # noqa: E731
+    x, y, mix, o, i, w = up(rn(R, S, W)), up(rn(R, W)), up(rn(S, S)), up(rn(S)), up(rn(S)), dev.upload(bits(rn(N, W)))
+    nw, sh, st = f32(rn(W)), f32(torch.rand(W, generator=g)), f32(rn(2, W))
+    es = 2 if what.endswith("B16") else 4
+    got = []
+    for off in (0, 1):
+        at = lambda a: dev.upload(np.concatenate([np.zeros(off, np.float32), a.ravel()])) + 4 * off   # noqa: E731
+        k = dev.kernel(what)
+        if what == "HyperStreamGemv":
+            state, out = at(st), dev.zeros(N * 4)
+            k(3, x, y, mix, o, 0, i, at(nw), at(sh), state, dev.upload(ctrl([5])), w, 0, out, S, N, W, W, 8, 0, 1e-3, 0.0)
+            got.append([dev.download(out, N, np.float32), dev.download(state, 2 * W, np.float32)])
+        else:
+            pend, h = dev.zeros(W * 4 + 16) + 4 * off, dev.zeros((R * W + 8) * es) + es * off
+            k(2, x, y, mix, o, 0, i, at(nw), at(sh), at(st), pend, dev.upload(ctrl(range(3, 3 + R))), dev.upload(np.int32([0] * R)),
+              dev.upload(np.int32([0] * R)), 0, h, W, S, R, 3, W, 1e-3)
+            raw = dev.download(h, R * W, np.float32 if es == 4 else np.uint16)
+            got.append([raw if es == 4 else from_bits(raw, R * W), dev.download(pend, W, np.float32)])
+    for a, b in zip(*got):
+        assert np.abs(a).max() > 0.1
+        close(b, a, 1e-5 if es == 4 else 1e-2)
+
+
 # -------------------------------------------------------------------- models ---
 L = P.make_layer
 MODELS = {
