@@ -36,7 +36,8 @@ struct LinearRowsTile {
   __device__ static int row(int i) { return (i >> 2) * (BM / (TM / 4)) + (int)threadIdx.x / TX * 4 + (i & 3); }
   __device__ static int col(int j) { return (j >> 2) * (BN / 2) + (int)threadIdx.x % TX * 4 + (j & 3); }
 
-  // Columns [k0, k0 + 16) of `rows` rows of X and `cols` rows of W, zeros beyond K, rows and cols.
+  // Columns [k0, k0 + 16) of `rows` rows of X and `cols` rows of W: zeros beyond K; rows and columns past the last repeat
+  // it (their sums are not stored).
   __device__ __forceinline__ void fetch(const float *X, int ldx, int rows, const uint16_t *W, int ldw, int cols, int k0, int K, bool vec) {
     const int tid = threadIdx.x, r = tid % BM, kx = tid / BM * XP;
     const bool whole = vec && k0 + kLrK <= K;

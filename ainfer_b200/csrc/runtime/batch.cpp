@@ -220,7 +220,7 @@ int BatchDecode::step() {
   for (int L = 0; L < m->cfg.layers; ++L) {
     if (ainfer_list_execute(layer_lists[L]) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }
     // x = (x + mixer) + MoE(norm(x + mixer)) for the rows, experts wherever they live
-    int e = ep.run_layer(L, true, nullptr);
+    int e = ep.run_layer(L, nullptr);
     if (e) { err = ep.err; return e; }
   }
   if (ainfer_list_execute(tail_list) != AINFER_OK) { err = ainfer_last_error(dev); return 1; }

@@ -15,7 +15,7 @@
 // no counterpart for the exchange.
 //
 // NCCL is bound at run time (dlopen of libnccl.so.2, the library the process already uses if any);
-// a world of one rank needs none and replaces the exchanges by device copies inside the list.
+// a world of one rank needs none and groups its own rows in place, without dispatch and return buffers.
 #include "ep.h"
 
 #include <dlfcn.h>
@@ -316,7 +316,7 @@ int EpMoe::exchange(void *send, void *recv, uint32_t slot) {
   return 0;
 }
 
-int EpMoe::run_layer(int L, bool chain, float *seg_ms) {
+int EpMoe::run_layer(int L, float *seg_ms) {
   int r = ensure_layer(L);
   if (r) return r;
   const int i = layer_lists[L];
@@ -345,7 +345,6 @@ int EpMoe::run_layer(int L, bool chain, float *seg_ms) {
     if (stamp(4)) return 1;
     EP_CHECK(ainfer_list_execute(impl->lists[i + 2]));
   }
-  (void)chain;   // the layer's last kernel already writes x to res as well
   if (stamp(5)) return 1;
   if (seg_ms) {
     EP_CHECK(ainfer_sync(dev, ~0ull));
@@ -359,7 +358,7 @@ int EpMoe::run_layer(int L, bool chain, float *seg_ms) {
 }
 
 int EpMoe::run_rows(int L, int rows) {
-  if (world > 1) return run_layer(L, true, nullptr);
+  if (world > 1) return run_layer(L, nullptr);
   if (L < 0 || L >= m->cfg.layers + m->cfg.mtp_layers || rows < 0 || rows > n) { err = "usage: no such layer, or more rows than the block holds"; return 2; }
   Rec r{this, nullptr};
   return rows ? emit_local(this, r, L, rows) : 0;
@@ -367,7 +366,7 @@ int EpMoe::run_rows(int L, int rows) {
 
 int EpMoe::run_stack(int first, int count, float *seg_ms) {
   for (int L = first; L < first + count; ++L) {
-    int r = run_layer(L, true, seg_ms);
+    int r = run_layer(L, seg_ms);
     if (r) return r;
   }
   return 0;

@@ -50,7 +50,7 @@ struct EpMoe {
   // X = Res + MoE(norm_L(Res)) for the owned rows, and Res <- X afterwards (layers chain). seg_ms (optional,
   // 5 floats, accumulated): device time of route+pack, dispatch, experts, return, shared+combine;
   // asking for it synchronises after the layer.
-  int run_layer(int L, bool chain, float *seg_ms);
+  int run_layer(int L, float *seg_ms);
   // run_layer for the first `rows` owned rows (one rank: launched at once; several: all rows).
   int run_rows(int L, int rows);
   int run_stack(int first, int count, float *seg_ms);

@@ -111,7 +111,7 @@ int session_create(DeviceModel *m, int max_ctx, int flags, Session **out, std::s
 // Chunked prefill (prefill.cpp): advances the session's state over n tokens at positions start_pos..
 // without producing logits; bit-identical to n decode steps. The object holds the row buffers.
 struct Prefill;
-// rows_cap: rows per pass (1..64); verify: also allocate what per-row predictions and rollback need.
+// rows_cap: rows per pass; verify: also allocate what per-row predictions and rollback need.
 // ep_world > 1: the MoE block of every pass runs expert-parallel over that many ranks (id128: the NCCL
 // id shared by the ranks); every rank then has to run the same passes (prompts of one length).
 int prefill_create(Session *s, int rows_cap, bool verify, Prefill **out, int ep_rank = 0, int ep_world = 1,

@@ -334,7 +334,7 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
     if (use_lists) {
       for (int L = 0; L < c.layers; ++L) {
         if (ainfer_list_execute(p->vlists[L]) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
-        int e = ep.run_layer(L, true, nullptr);
+        int e = ep.run_layer(L, nullptr);
         if (e) { s->err = "prefill: " + ep.err; return e; }
       }
       if (ainfer_list_execute(p->vlists[c.layers]) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }

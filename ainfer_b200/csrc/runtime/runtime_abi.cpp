@@ -169,10 +169,10 @@ static int ensure_prefill(Session *s) {
   }
   if (!s->prefill) {
     // rows per pass: the planner of the expert-parallel block takes 2048 (row, expert) items over all ranks, and
-    // 8192 on one rank, where a pass of many rows crosses the experts' weights once (a prompt of 701 tokens
-    // through the full preset: 99 ms in four passes, 63 ms in one). 768 = four blocks of the 192 rows that attend at a
-    // time, the largest such number within 8192 items at top-k 10. On one rank no more rows than the context holds: the
-    // buffers are the session's own, 374 MiB at 768 rows of the full preset.
+    // 8192 on one rank, where a pass of many rows crosses the experts' weights once (full preset, 701 tokens in passes
+    // of 192 / 384 / 768 rows 92 / 61 / 43 ms, 4095 tokens 563 / 399 / 312). 768 is four blocks of the 192 rows that
+    // attend at a time, the largest such number within 8192 items at top-k 10. On one rank no more rows than the
+    // context holds: the buffers are the session's own, 374 MiB at 768 rows of the full preset.
     const int topk = s->m->cfg.top_k > 0 ? s->m->cfg.top_k : 1;
     const int most = std::max(1, (s->pf_world == 1 ? 8192 : 2048) / (topk * s->pf_world));   // rows a rank may bring to a pass
     int rows = s->pf_rows > 0 ? s->pf_rows : std::min(s->pf_world == 1 ? 768 : 192, most >= 8 ? most / 8 * 8 : most);
@@ -308,7 +308,7 @@ int ainfer_ep_buffer(ainfer_ep_t ep, const char *which, void **dptr, uint64_t *b
 }
 int ainfer_ep_moe_layer(ainfer_ep_t ep, int layer) {
   if (!ep) return 2;
-  int r = ep->e.run_layer(layer, false, nullptr);
+  int r = ep->e.run_layer(layer, nullptr);
   return set_err(r, ep->e.err);
 }
 int ainfer_ep_moe_stack(ainfer_ep_t ep, int first, int count, float *seg_ms) {

@@ -453,7 +453,7 @@ def run_prefill_ep(args, dev, model, rank, world, dist):
     sec = float(tt[0])
     sess.close()
     most = max(1, 2048 // (model.config["top_k"] * world))
-    rows_pp = min(192, most // 8 * 8 if most >= 8 else most)     # the runtime's default
+    rows_pp = min(192, most // 8 * 8 if most >= 8 else most)     # the runtime's default with several ranks
     return {"workload": f"prefill of {n_tok} seeded tokens on each of {world} ranks (one sequence per rank), passes of {rows_pp} rows, experts split over the ranks",
             "tokens_per_s": world * n_tok / sec, "seconds": sec, "prompt_tokens_per_rank": n_tok, "world": world,
             "rows_per_pass": rows_pp, "scaling": "weak"}
@@ -648,8 +648,8 @@ def run_ours(args):
         "cpu_baseline": cpu, "parity": parity, "ep": ep_line, "batch_decode": batch_line, "mtp": mtp_line,
         "prefill_ep": prefill_ep_line,
         "prefill": None if args.loop_prompt else {"prompt_tokens": P - 1, "seconds": t_prompt_only, "tokens_per_s": (P - 1) / max(t_prompt_only, 1e-9),
-                                                  "how": "chunked prefill, up to 192 rows per pass, one sequence (wall clock around the call, this rank)"},
-        "timing": {"model_fill_s": t_load, "prompt_s": t_prompt, "prompt_by": "token-by-token decode" if args.loop_prompt else "chunked prefill (up to 192 rows per pass)", "timed_wall_s": t_wall, "first_tokens": [int(t) for t in toks0[:8]]},
+                                                  "how": "chunked prefill, up to 768 rows per pass, one sequence (wall clock around the call, this rank)"},
+        "timing": {"model_fill_s": t_load, "prompt_s": t_prompt, "prompt_by": "token-by-token decode" if args.loop_prompt else "chunked prefill (up to 768 rows per pass)", "timed_wall_s": t_wall, "first_tokens": [int(t) for t in toks0[:8]]},
     }
     print(json.dumps(line))
     sess.close(); model.close(); dev.close()
