@@ -160,7 +160,7 @@ def gemm_tc_once(dev, N, K, M, reps=20, groups=0, kernel="Int4GemmA8Tc"):
         kernels.append(g); bufs.append((dP, dS, dY))
     if kernel == "Int4GemvA8Multi":
         groups = groups or min(-(-N // (256 // (K // 128))), dev.info().sm_count * 2)
-    groups = groups or min((N + 127) // 128, dev.info().sm_count * 2)
+    groups = groups or min((N + 127) // 128 * ((M + 15) // 16), dev.info().sm_count * 2)   # as the runtime: a block for every unit of 16 rows
     for i in range(3):
         kernels[i % nbuf].launch(groups)
     cl = dev.new_list()
