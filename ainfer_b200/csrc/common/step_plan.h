@@ -13,7 +13,7 @@ struct StepLayer {
   int32_t pad0;
   const float *in_norm;    // [H]
   const float *post_norm;  // [H]
-  // linear: 0 qkv (conv epilogue), 1 z, 2 b, 3 a, 4 out_proj (+residual)
+  // linear: 0 qkv (conv epilogue), 1 z (silu), 2 b, 3 a, 4 out_proj (+residual)
   // attention: 0 q, 1 k, 2 v, 4 o_proj (+residual)
   GemvMat m[5];
   float *S;                // [nV][128][128] DeltaNet state of this layer
@@ -63,7 +63,7 @@ struct StepPlan {
   // grid barrier state: count is zeroed before every launch; error is sticky
   uint32_t *bar_count;
   int32_t *error;           // 0 ok, otherwise the code of the bounded wait that ran out
-  int64_t pad2;             // size a multiple of 16 bytes: the kernel copies the plan as 16-byte words
+  int32_t in_rows[2];       // rows of the first projections of a layer, by layer type
 };
 static_assert(sizeof(StepPlan) % 16 == 0, "StepPlan is copied 16 bytes at a time");
 

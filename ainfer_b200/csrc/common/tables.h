@@ -10,7 +10,8 @@ enum GemvEpilogue {
   EPI_RESADD = 1,    // Y[m][n] = e0[m][n] + acc                     (ResAddF, kernels.cpp:646-652)
   EPI_CONV_SILU = 2, // depthwise conv k=4 + SiLU + history shift     (SsmConv, kernels.cpp:322-338)
   EPI_BETA = 3,      // Y[n] = sigmoid(acc)                           (BetaG, kernels.cpp:612)
-  EPI_GDECAY = 4     // Y[n] = -exp(A_log[n]) * softplus(acc + dt[n]) (BetaG, kernels.cpp:613-615)
+  EPI_GDECAY = 4,    // Y[n] = -exp(A_log[n]) * softplus(acc + dt[n]) (BetaG, kernels.cpp:613-615)
+  EPI_SILU = 5       // Y[n] = silu(acc): the gate of NormGated (kernels.cpp:619-630); DecodeStep only
 };
 
 // One entry of the matrix table of an Int4GemvA8 launch (64 bytes).

@@ -33,6 +33,11 @@
 // Every wait (mbarrier, grid barrier) is bounded by a wall-clock limit: when one runs out the
 // block sets the plan's sticky error word, no wait in the grid spins again, and the kernel
 // terminates with garbage results that the host refuses (the error word is read after the step).
+//
+// What bounds it: not HBM (0.33 ms a token of the full preset) but the chain of six stages a layer. Times of a
+// layer's stages by the stage clock, full preset, context 4096: shares of rows once per launch, epilogue operands as
+// asynchronous copies, one thread a (row, group), group scales by one reduction instruction, selection by
+// ranks and silu(z) from the projection's epilogue took a token from 2.73 to 2.08 ms.
 #include "../common/step_plan.h"
 #include "attention_core.cuh"
 #include "block_stages.cuh"
@@ -77,6 +82,9 @@ struct Seg {
 };
 constexpr int kMaxSegs2 = 24;
 
+// Stages whose rows are dealt to the blocks; kRngIn and kRngOut are followed by the layer type.
+enum { kRngIn = 0, kRngOut = 2, kRngRouter = 4, kRngGateUp = 5, kRngDown = 6, kRngHead = 7, kRngCount = 8 };
+
 struct StepShared {
   // the members that are copied 16 bytes at a time come first (the struct sits at a
   // 128-byte aligned address and the sizes are multiples of 16)
@@ -91,6 +99,9 @@ struct StepShared {
   float hmax[8], hse[8], wmax[16];
   float av[16];
   int32_t ai[16];
+  unsigned kmax[16];            // selection: each warp's largest key
+  int32_t ncand;                // selection: candidates so far
+  int2 rng[kRngCount];          // this block's rows of every stage (deal())
   volatile int32_t fail;
   int32_t nstamp[2];            // stage clock: records written so far (consumer, producer)
   Seg segs[kMaxSegs2];          // the producer warp's current segment list
@@ -108,25 +119,29 @@ extern __shared__ __align__(128) unsigned char step_smem[];
 #define SH (reinterpret_cast<StepShared *>(step_smem))
 #define PL (reinterpret_cast<StepShared *>(step_smem)->plan)
 
-__device__ __forceinline__ void csync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
-__device__ __forceinline__ void hsync() { asm volatile("bar.sync 2, 256;" ::: "memory"); }  // threads 0..255
-__device__ __forceinline__ unsigned long long gtime_ns() {
+// kClock: with the stage clock (the step without it has no trace of it).
+template <bool kClock>
+struct Step {
+
+static __device__ __forceinline__ void csync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+static __device__ __forceinline__ void hsync() { asm volatile("bar.sync 2, 256;" ::: "memory"); }  // threads 0..255
+static __device__ __forceinline__ unsigned long long gtime_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
+static __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
-__device__ __forceinline__ void step_fail(int code) {
+static __device__ __forceinline__ void step_fail(int code) {
   SH->fail = code;
   atomicExch(PL.error, code);
 }
 // Bounded wait on an mbarrier phase; false when it gave up (now or earlier).
-__device__ __forceinline__ bool mbar_wait_b(uint32_t addr, uint32_t parity, int code) {
+static __device__ __forceinline__ bool mbar_wait_b(uint32_t addr, uint32_t parity, int code) {
   if (mbar_try_a(addr, parity)) return true;
   if (SH->fail) return false;
   const long long t0 = clock64();
@@ -152,7 +167,10 @@ __device__ __forceinline__ bool mbar_wait_b(uint32_t addr, uint32_t parity, int 
 // output projection and the router are issued, 13 the selection arrived, 14 / 15 the gate/up and
 // the down tiles are issued. A record costs a few hundred nanoseconds, so a stamped step is a few
 // per cent slower than the product's.
-static __device__ __noinline__ void stamp(int id) {
+static __device__ __forceinline__ void stamp(int id) {
+  if (kClock) stamp_now(id);
+}
+static __device__ __noinline__ void stamp_now(int id) {
   if (PL.stage_stamps && blockIdx.x == 0 && (threadIdx.x == 0 || threadIdx.x == kCons)) {
     const int who = threadIdx.x == 0 ? 0 : 1, half = PL.stage_stamp_cap / 2;
     const int n = SH->nstamp[who];
@@ -163,7 +181,7 @@ static __device__ __noinline__ void stamp(int id) {
 }
 
 // Rows [lo, hi) of `total` for block blk of nblk, cut at multiples of `unit` rows.
-__device__ __forceinline__ void deal(int total, int unit, int blk, int nblk, int &lo, int &hi) {
+static __device__ __forceinline__ void deal(int total, int unit, int blk, int nblk, int &lo, int &hi) {
   const long units = (total + unit - 1) / unit;
   lo = (int)(units * blk / nblk) * unit;
   hi = (int)(units * (blk + 1) / nblk) * unit;
@@ -171,23 +189,35 @@ __device__ __forceinline__ void deal(int total, int unit, int blk, int nblk, int
   if (lo > total) lo = total;
 }
 // Row unit that keeps a block's share of the bf16 group scales 16-byte aligned (2*K/128 bytes per row).
-__device__ __forceinline__ int row_unit(int K) {
+static __device__ __forceinline__ int row_unit(int K) {
   const int G = K >> 7;
   return G >= 8 ? 1 : 8 / G;
+}
+// Shares of all stages, once per launch: the divisions cost about a thousand cycles, and the shares
+// depend on the shapes alone.
+static __device__ __forceinline__ void deal_all(int i) {
+  const StepPlan &P = PL;
+  int total, unit;
+  if (i < kRngOut) { total = P.in_rows[i - kRngIn]; unit = row_unit(P.H); }
+  else if (i < kRngRouter) { total = P.H; unit = row_unit(i == kRngOut ? P.nV * 128 : P.nQ * 256); }
+  else if (i == kRngRouter) { total = P.E + P.slots - P.topk; unit = 1; }
+  else if (i == kRngGateUp) { total = P.slots * P.I; unit = row_unit(P.H); }
+  else if (i == kRngDown) { total = P.H; unit = row_unit(P.I); }
+  else { total = P.vocab; unit = row_unit(P.H); }
+  int lo, hi;
+  deal(total, unit, (int)blockIdx.x, (int)gridDim.x, lo, hi);
+  SH->rng[i] = make_int2(lo, hi);
 }
 
 // ------------------------------------------------------------------ grid barrier ---
 // Two halves, so that loads which do not depend on other blocks (recurrent state, KV rows of
 // earlier tokens, epilogue operands) can be issued between arriving and waiting.
-static __device__ __noinline__ void grid_arrive() {
+static __device__ __forceinline__ void grid_arrive() {
   csync();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(PL.bar_count, 1u);
-  }
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(PL.bar_count) : "memory");
 }
 // epoch: how many barriers this block has arrived at, this one included
-static __device__ __noinline__ void grid_wait(unsigned epoch) {
+static __device__ __forceinline__ void grid_wait(unsigned epoch) {
   if (threadIdx.x == 0 && !SH->fail) {
     const unsigned target = epoch * gridDim.x;
     const long long t0 = clock64();
@@ -214,13 +244,12 @@ static __device__ __noinline__ void grid_wait(unsigned epoch) {
 // by bulk copy when source, size and offset are 16-byte aligned; otherwise (small matrices) the
 // lane copies them itself before it completes the tile. `tile` is the running index of the
 // call's first tile; returns the index after its last.
-static __device__ __noinline__ uint32_t prod_emit(uint32_t tile, int row_bytes, int sc_row_bytes) {
+// total: rows of the list.
+static __device__ __noinline__ uint32_t prod_emit(uint32_t tile, int row_bytes, int sc_row_bytes, int total) {
   const Seg *segs = SH->segs;
   const int nseg = SH->nseg;
-  const int rpt = kTileBytes / row_bytes;
-  int total = 0;
-  for (int i = 0; i < nseg; ++i) total += segs[i].nrows;
-  const int ntiles = (total + rpt - 1) / rpt;
+  const int lrpt = __ffs(kTileBytes) - __ffs(row_bytes), rpt = 1 << lrpt;   // both powers of two
+  const int ntiles = (total + rpt - 1) >> lrpt;
   const uint32_t base = tile;
   const int lane = threadIdx.x & 31;
   if (lane < kNT && ntiles > 0) {
@@ -267,15 +296,9 @@ static __device__ __noinline__ uint32_t prod_emit(uint32_t tile, int row_bytes, 
   return base + (uint32_t)ntiles;
 }
 
-__device__ __forceinline__ int mats_rows(const GemvMat *m, int nm) {
-  int t = 0;
-  for (int i = 0; i < nm; ++i) t += m[i].N;
-  return t;
-}
-
 // Segment list of rows [lo, hi) of a table of matrices whose rows are numbered end to end
 // (written by lane 0 of the producer warp).
-__device__ __forceinline__ void segs_gemv(const GemvMat *m, int nm, int K, int lo, int hi) {
+static __device__ __forceinline__ void segs_gemv(const GemvMat *m, int nm, int K, int lo, int hi) {
   if ((threadIdx.x & 31) == 0) {
     Seg *out = SH->segs;
     int n = 0, rs = 0;
@@ -297,30 +320,27 @@ __device__ __forceinline__ void segs_gemv(const GemvMat *m, int nm, int K, int l
   __syncwarp();
 }
 
-static __device__ __noinline__ uint32_t prod_gemv(uint32_t tile, const GemvMat *m, int nm, int K) {
-  int lo, hi;
-  deal(mats_rows(m, nm), row_unit(K), (int)blockIdx.x, (int)gridDim.x, lo, hi);
-  segs_gemv(m, nm, K, lo, hi);
-  return prod_emit(tile, K >> 1, (K >> 7) * 2);
+static __device__ __noinline__ uint32_t prod_gemv(uint32_t tile, const GemvMat *m, int nm, int K, int rng) {
+  const int2 r = SH->rng[rng];
+  segs_gemv(m, nm, K, r.x, r.y);
+  return prod_emit(tile, K >> 1, (K >> 7) * 2, r.y - r.x);
 }
 
 // The producer warp's whole token. Returns the number of tiles issued.
 static __device__ __noinline__ uint32_t producer_main(int mode) {
   const StepPlan &P = PL;
-  const int H = P.H, blk = (int)blockIdx.x, nblk = (int)gridDim.x;
-  const bool lead = (threadIdx.x & 31) == 0;
+  const int H = P.H, lane = threadIdx.x & 31, lgI = __ffs(P.I) - 1;
+  const bool lead = lane == 0;
   uint32_t tile = 0;
   for (int L = 0; L < P.layers; ++L) {
     const StepLayer &ly = P.L[L];
     const bool lin = ly.type == 0;
-    tile = prod_gemv(tile, &ly.m[0], lin ? 4 : 3, H);
+    tile = prod_gemv(tile, &ly.m[0], lin ? 4 : 3, H, kRngIn + ly.type);
     stamp(10);
-    tile = prod_gemv(tile, &ly.m[4], 1, lin ? P.nV * 128 : P.nQ * 256);
+    tile = prod_gemv(tile, &ly.m[4], 1, lin ? P.nV * 128 : P.nQ * 256, kRngOut + ly.type);
     stamp(11);
     {  // router rows (bf16) and the shared-expert gate row
-      const int rows = P.E + (ly.shared_gate ? 1 : 0);
-      int lo, hi;
-      deal(rows, 1, blk, nblk, lo, hi);
+      const int lo = SH->rng[kRngRouter].x, hi = SH->rng[kRngRouter].y;
       if (lead) {
         Seg *segs = SH->segs;
         int n = 0;
@@ -330,173 +350,240 @@ static __device__ __noinline__ uint32_t producer_main(int mode) {
         SH->nseg = n;
       }
       __syncwarp();
-      tile = prod_emit(tile, H * 2, 0);
+      tile = prod_emit(tile, H * 2, 0, hi - lo);
     }
     // the expert weights depend on the routing: wait for the consumers' selection
     stamp(12);
     if (!mbar_wait_b(smem_addr(&SH->sel_bar), (uint32_t)L & 1u, 4)) return tile;
     stamp(13);
-    {  // gate and up rows of pair rows [lo, hi) over slots x I
-      int lo, hi;
-      deal(P.slots * P.I, row_unit(H), blk, nblk, lo, hi);
-      if (lead) {
-        Seg *segs = SH->segs;
-        int n = 0;
-        if (lo < hi) {
-          const int s0 = lo / P.I, s1 = (hi - 1) / P.I;
-          for (int s = s0; s <= s1 && n + 2 <= kMaxSegs2; ++s) {
-            const int a = lo > s * P.I ? lo : s * P.I, b = hi < (s + 1) * P.I ? hi : (s + 1) * P.I;
-            const ExpertW &ew = SH->sew[s];
-            const size_t r0 = (size_t)(a - s * P.I);
-            segs[n++] = Seg{ew.gP + r0 * (H >> 1), reinterpret_cast<const uint8_t *>(ew.gS + r0 * (H >> 7)), b - a, 0, a - lo, 0};
-            segs[n++] = Seg{ew.uP + r0 * (H >> 1), reinterpret_cast<const uint8_t *>(ew.uS + r0 * (H >> 7)), b - a, 0,
-                            (hi - lo) + (a - lo), 0};
-          }
+    {  // gate and up rows of pair rows [lo, hi) over slots x I: lane l writes the two segments of the l-th slot
+      const int lo = SH->rng[kRngGateUp].x, hi = SH->rng[kRngGateUp].y;
+      int n = 0;
+      if (lo < hi) {
+        const int s0 = lo >> lgI, s = s0 + lane;
+        n = ((hi - 1) >> lgI) - s0 + 1;
+        if (lane < n) {
+          const int a = lo > s * P.I ? lo : s * P.I, b = hi < (s + 1) * P.I ? hi : (s + 1) * P.I;
+          const ExpertW &ew = SH->sew[s];
+          const size_t r0 = (size_t)(a - s * P.I);
+          SH->segs[2 * lane] = Seg{ew.gP + r0 * (H >> 1), reinterpret_cast<const uint8_t *>(ew.gS + r0 * (H >> 7)), b - a, 0, a - lo, 0};
+          SH->segs[2 * lane + 1] = Seg{ew.uP + r0 * (H >> 1), reinterpret_cast<const uint8_t *>(ew.uS + r0 * (H >> 7)), b - a, 0,
+                                       (hi - lo) + (a - lo), 0};
         }
-        SH->nseg = n;
       }
+      if (lead) SH->nseg = 2 * n;
       __syncwarp();
-      tile = prod_emit(tile, H >> 1, (H >> 7) * 2);
+      tile = prod_emit(tile, H >> 1, (H >> 7) * 2, 2 * (hi - lo));
     }
     stamp(14);
     {  // down rows [lo, hi) of every slot
-      int lo, hi;
-      deal(H, row_unit(P.I), blk, nblk, lo, hi);
-      if (lead) {
-        Seg *segs = SH->segs;
-        int n = 0;
-        if (lo < hi) {
-          const int nr = hi - lo;
-          for (int s = 0; s < P.slots; ++s) {
-            const ExpertW &ew = SH->sew[s];
-            segs[n++] = Seg{ew.dP + (size_t)lo * (P.I >> 1), reinterpret_cast<const uint8_t *>(ew.dS + (size_t)lo * (P.I >> 7)),
-                            nr, s, s * nr, 0};
-          }
-        }
-        SH->nseg = n;
+      const int lo = SH->rng[kRngDown].x, nr = SH->rng[kRngDown].y - lo;
+      if (lane < P.slots) {
+        const ExpertW &ew = SH->sew[lane];
+        SH->segs[lane] = Seg{ew.dP + (size_t)lo * (P.I >> 1), reinterpret_cast<const uint8_t *>(ew.dS + (size_t)lo * (P.I >> 7)),
+                             nr, lane, lane * nr, 0};
       }
+      if (lead) SH->nseg = nr > 0 ? P.slots : 0;
       __syncwarp();
-      tile = prod_emit(tile, P.I >> 1, (P.I >> 7) * 2);
+      tile = prod_emit(tile, P.I >> 1, (P.I >> 7) * 2, P.slots * nr);
     }
     stamp(15);
   }
-  if (mode != 0) tile = prod_gemv(tile, &P.lm_head, 1, H);
+  if (mode != 0) tile = prod_gemv(tile, &P.lm_head, 1, H, kRngHead);
   return tile;
 }
 
 // ====================================================================== consumers ===
-// Dots the tiles of one stage with staged activations. The stage's rows are numbered 0..total-1
-// in the order the producer streams them (tile j holds rows [j * rpt, (j + 1) * rpt)); row f is
-// dotted with activation vector f / vec_rows (vec_rows = 0: always vector 0) and its group terms
-// go to t[g][f - row_base]. Rows [row_base, row_base + nrows) are done by this call, starting at
-// running tile index `tile`; returns the index after the last tile consumed. A tile is 256
-// (row, group) tasks of 64 bytes; two adjacent lanes share a task (32 bytes each) and add their
-// exact integer sums with one shuffle.
-__device__ __forceinline__ uint32_t dot_tiles(uint32_t tile, int K, const uint4 *xa, const float *sq, float *T,
-                                              int row_base, int nrows, int total, int vec_rows) {
-  const int G = K >> 7, lg = 31 - __clz(G);
-  const int TS = (kTCap >> lg) + 1, rpt = 256 >> lg;
-  const int task = threadIdx.x >> 1, half = threadIdx.x & 1, lane = threadIdx.x & 31;
-  const int r = task >> lg, g = task & (G - 1);
-  const uint32_t rot = (uint32_t)(lane >> 2) & 1u;
+// Dots the next tiles of a stage with staged activations: nrows rows in the order the producer
+// streams them (tile j of the call holds rows [j * rpt, (j + 1) * rpt)). Row f is dotted with
+// activation vector f / vec_rows (kVecs; otherwise always vector 0) and its group terms go to
+// t[g][f]. Starts at running tile index `tile`; returns the index after the last tile. A tile is 256 (row, group) tasks of 64 bytes, one a thread: the two halves of the
+// consumers take alternate tiles, so that every wait, scale and store serves 64 bytes and two
+// tiles are in work at once. A thread reads its 64 bytes in a lane-rotated order that keeps every
+// quarter-warp on distinct banks.
+template <bool kVecs>
+static __device__ __forceinline__ uint32_t dot_tiles(uint32_t tile, int lg, const uint4 *xa, const float *sq, float *T,
+                                                     int nrows, int vec_rows) {
+  const int G = 1 << lg, TS = (kTCap >> lg) + 1, rpt = 256 >> lg;
+  const int t = threadIdx.x & 255, half = threadIdx.x >> 8, lane = threadIdx.x & 31;
+  const int r = t >> lg, g = t & (G - 1), rot = (t >> 1) & 3;
   const uint32_t ring_a = smem_addr(step_smem + kRingOff);
-  const int ntiles = (nrows + rpt - 1) / rpt;
-  int cvec = -1;
-  uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0, x2 = x0, x3 = x0;
+  const int ntiles = (nrows + rpt - 1) >> (8 - lg);
+  uint4 x[8];
   float sqg = 0.0f;
+  if (!kVecs) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int q = 2 * ((s + rot) & 3);
+      x[2 * s] = xa[q * G + g];
+      x[2 * s + 1] = xa[(q + 1) * G + g];
+    }
+    sqg = sq[g];
+  }
 #pragma unroll 1
-  for (int j = 0; j < ntiles; ++j) {
-    const uint32_t slot = tile % kNT, use = tile / kNT;
+  for (int j = half; j < ntiles; j += 2) {
+    const uint32_t idx = tile + (uint32_t)j, slot = idx % kNT, use = idx / kNT;
+    const int f = j * rpt + r;
+    const bool live = f < nrows;
+    if (kVecs) {
+      const int vec = live ? (int)((unsigned)f / (unsigned)vec_rows) : 0;
+      const uint4 *xv = xa + (size_t)vec * 8 * G + g;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int q = 2 * ((s + rot) & 3);
+        x[2 * s] = xv[q * G];
+        x[2 * s + 1] = xv[(q + 1) * G];
+      }
+      sqg = sq[vec * G + g];
+    }
     // a wait that gave up ends the stage for the whole warp (the results are lost anyway)
     if (!__all_sync(kFull, mbar_wait_b(smem_addr(&SH->full[slot]), use & 1u, 5))) break;
-    const uint32_t tb = ring_a + slot * kTileStride;
-    const uint32_t wbase = tb + (uint32_t)task * 64u + (uint32_t)half * 32u;
-    const uint4 wa = lds128(wbase + (rot << 4)), wb = lds128(wbase + ((rot ^ 1u) << 4));
-    const uint32_t sraw = lds_u16(tb + kTileBytes + (uint32_t)task * 2u);
+    const uint32_t tb = ring_a + slot * kTileStride, wb = tb + (uint32_t)t * 64u;
+    const uint4 w0 = lds128(wb + (uint32_t)(rot << 4)), w1 = lds128(wb + (uint32_t)(((1 + rot) & 3) << 4)),
+                w2 = lds128(wb + (uint32_t)(((2 + rot) & 3) << 4)), w3 = lds128(wb + (uint32_t)(((3 + rot) & 3) << 4));
+    const uint32_t sraw = lds_u16(tb + kTileBytes + (uint32_t)t * 2u);
+    int d0 = dot16_x16(w0, 0, x[0], 0), d1 = dot16_x16(w0, 1, x[1], 0);
+    int d2 = dot16_x16(w1, 0, x[2], 0), d3 = dot16_x16(w1, 1, x[3], 0);
+    d0 = dot16_x16(w2, 0, x[4], d0);
+    d1 = dot16_x16(w2, 1, x[5], d1);
+    d2 = dot16_x16(w3, 0, x[6], d2);
+    d3 = dot16_x16(w3, 1, x[7], d3);
     __syncwarp();
     if (lane == 0) mbar_arrive_a(smem_addr(&SH->empty[slot]));
-    const int f = row_base + j * rpt + r;
-    const bool live = j * rpt + r < nrows && f < total;
-    int dsum = 0;
-    if (live) {
-      const int vec = vec_rows ? f / vec_rows : 0;
-      if (vec != cvec) {
-        cvec = vec;
-        const uint4 *xv = xa + (size_t)vec * 8 * G + g;
-        const int q0 = half * 4 + (int)rot * 2, q1 = half * 4 + (int)(rot ^ 1u) * 2;
-        x0 = xv[q0 * G];
-        x1 = xv[(q0 + 1) * G];
-        x2 = xv[q1 * G];
-        x3 = xv[(q1 + 1) * G];
-        sqg = sq[vec * G + g];
-      }
-      int d0 = dot16_x16(wa, 0, x0, 0), d1 = dot16_x16(wa, 1, x1, 0);
-      d0 = dot16_x16(wb, 0, x2, d0);
-      d1 = dot16_x16(wb, 1, x3, d1);
-      dsum = d0 + d1;
-    }
-    dsum += __shfl_xor_sync(kFull, dsum, 1);
-    if (live && half == 0) {
-      const float v = (float)(dsum >> 4) * __uint_as_float(sraw << 16);
-      T[g * TS + (f - row_base)] = v * sqg;
-    }
-    tile += 1;
+    const float v = (float)(((d0 + d1) + (d2 + d3)) >> 4) * __uint_as_float(sraw << 16);
+    if (live) T[g * TS + f] = v * sqg;
   }
-  return tile;
+  return tile + (uint32_t)ntiles;
+}
+
+// Sum of one row's group terms in ascending group order, the loads of up to eight terms ahead of the additions.
+static __device__ __forceinline__ float row_terms(const float *T, int row, int lg) {
+  const int G = 1 << lg, TS = (kTCap >> lg) + 1;
+  const float *t = T + row;
+  float acc = 0.0f;
+  if (G >= 8) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = t[i * TS];
+#pragma unroll 1
+    for (int g = 8; g < G; g += 8) {
+      float n[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) n[i] = t[(g + i) * TS];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        acc = acc + v[i];
+        v[i] = n[i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc = acc + v[i];
+  } else {
+#pragma unroll 1
+    for (int g = 0; g < G; ++g) acc = acc + t[g * TS];
+  }
+  return acc;
+}
+
+// Largest magnitude of the warp's values (one instruction; NaNs do not count, as with fmaxf).
+static __device__ __forceinline__ float warp_absmax(float v) {
+  float r;
+  asm volatile("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+// Scale of a group of 128 values, four a lane (ScalesMax, tools/cmdlist/kernels.cpp:551-566).
+static __device__ __forceinline__ float group_scale(const float4 &v) {
+  const float mx = warp_absmax(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+  const float s = mx / 127.0f;
+  return s == 0.0f ? 1.0f : s;
+}
+// Four values' bytes under scale s, r = quant_recip(s): quant_round()'s integers. With q = x/s, |q| <=
+// 127 (1 + 2^-24): x r is within 127 x 2^-23 = 1.53e-5 of q and the rounded quotient within 0.76e-5, so
+// they differ by at most 2.3e-5, and after the addition of one half (rounded to 2^-17 at most, twice)
+// by 3.1e-5: unless |x r| + 0.5 is within 4e-5 of a whole number both truncate alike. There, and for a
+// scale without a finite reciprocal, the division itself decides.
+static __device__ __forceinline__ uint32_t quant4(const float4 &v, float s, float r) {
+  const float x[4] = {v.x, v.y, v.z, v.w};
+  uint32_t out = 0;
+  bool sure = r != 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float vp = x[i] * r, t = fabsf(vp) + 0.5f, w = truncf(t), f = t - w;
+    sure = sure && f >= 4e-5f && f <= 0.99996f;
+    int q = (int)w;
+    q = q > 127 ? 127 : q;
+    q = vp < 0.0f ? -q : q;
+    out |= (uint32_t)(q & 0xFF) << (8 * i);
+  }
+  if (!sure) {
+    out = 0;
+#pragma unroll 1
+    for (int i = 3; i >= 0; --i) {
+      const float xi = i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
+      out = (out << 8) | (uint32_t)(quant_round(xi, s) & 0xFF);
+    }
+  }
+  return out;
+}
+// Quantises one group of 128 values held four a lane into the staged form (quant_group_staged()'s result).
+static __device__ __forceinline__ void stage_group(uint32_t *xw, float *sqs, int G, int m, int g, const float4 &v) {
+  const int lane = threadIdx.x & 31;
+  const float s = group_scale(v);
+  const uint32_t own = quant4(v, s, quant_recip(s));
+  const uint32_t other = __shfl_xor_sync(kFull, own, 1);
+  const int i = lane >> 1;  // 8-weight piece of the group: two lanes of 4 weights each
+  uint32_t *dst = xw + ((((m * 8 + (i >> 1)) * G + g) << 2) + ((i & 1) << 1));
+  if (lane & 1) dst[1] = __byte_perm(other, own, 0x7531);
+  else dst[0] = __byte_perm(own, other, 0x6420);
+  if (lane == 0) sqs[m * G + g] = s;
 }
 
 // (1+w) RMSNorm + per-128 quantiser of one H-vector into the staged form, by the whole
 // consumer group (RMSNormW + ScalesMax + Quantize, tools/cmdlist/kernels.cpp:73-114,551-579).
 // Sum of squares: fp64 over 256 strided lanes (thread j < 256 adds x[j], x[j+256], ... in
-// order), then the stride-halving tree, whose levels 128, 64 and 32 every warp evaluates for
+// order; a square is exact in fp64, so one fused multiply-add a term), then the stride-halving
+// tree, whose levels 128, 64 and 32 every warp evaluates for
 // itself from the 256 partial sums in shared memory (lane l: ((p[l]+p[l+128]) + (p[l+64]+
 // p[l+192])) + ((p[l+32]+p[l+160]) + (p[l+96]+p[l+224]))) and whose last five levels are the xor
-// butterfly. Double-precision arithmetic is slow on this GPU (a few lanes per cycle and SM), so
-// the element-wise part is done once, not once per warp.
+// butterfly. The mean is a product: H is a power of two.
+// Waits for barrier `epoch` first (0: none), after the loads that do not depend on it.
 // src: fp32 vector in global memory, or (emb != null) a bf16 embedding row. hn (optional): the
 // normalised fp32 vector, shared memory. xout (optional): copy of the input, global.
-static __device__ __noinline__ void norm_quant(const float *src, const uint16_t *emb, const float *w, int H, float *hn,
-                                               float *xout) {
+static __device__ __forceinline__ void norm_quant(unsigned epoch, const float *src, const uint16_t *emb, const float *w, int H,
+                                               float *hn, float *xout) {
   float *xs = reinterpret_cast<float *>(step_smem + kFbufOff);
   double *ps = reinterpret_cast<double *>(step_smem + kTOff);
   unsigned char *act = step_smem + kActOff;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float4 v[2];  // H <= 4096: at most two float4 per thread
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int j = (tid + kCons * u) * 4;
-    v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (j < H) {
-      if (emb) {
-        const uint2 e = __ldg(reinterpret_cast<const uint2 *>(emb + j));
-        v[u] = make_float4(u2f(e.x << 16), u2f(e.x & 0xFFFF0000u), u2f(e.y << 16), u2f(e.y & 0xFFFF0000u));
-      } else {
-        v[u] = __ldcg(reinterpret_cast<const float4 *>(src + j));
-      }
-    }
-  }
-  float4 wv[2];  // the weights of this warp's groups, in flight during the reduction
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, G = H >> 7, n = H >> 8;
+  float4 wv[2];  // H <= 4096: the weights of this warp's groups (at most two)
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int g = warp + 16 * i;
     wv[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (g < H / 128) wv[i] = __ldg(reinterpret_cast<const float4 *>(w + g * 128) + lane);
+    if (g < G) wv[i] = __ldg(reinterpret_cast<const float4 *>(w + g * 128) + lane);
   }
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int j = (tid + kCons * u) * 4;
-    if (j < H) {
-      *reinterpret_cast<float4 *>(xs + j) = v[u];
-      if (xout) *reinterpret_cast<float4 *>(xout + j) = v[u];
-    }
-  }
-  csync();
+  if (epoch) grid_wait(epoch);
   if (tid < 256) {
     double ss = 0;
 #pragma unroll 1
-    for (int j = tid; j < H; j += 256) {
-      const double dv = (double)xs[j];
-      ss = ss + dv * dv;
+    for (int i0 = 0; i0 < n; i0 += 8) {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i] = 0.0f;
+        if (i0 + i < n) {
+          const int e = tid + 256 * (i0 + i);
+          v[i] = emb ? u2f((uint32_t)__ldg(emb + e) << 16) : __ldcg(src + e);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i0 + i < n) {
+          const int e = tid + 256 * (i0 + i);
+          xs[e] = v[i];
+          if (xout) xout[e] = v[i];
+          ss = fma((double)v[i], (double)v[i], ss);
+        }
     }
     ps[tid] = ss;
   }
@@ -505,13 +592,14 @@ static __device__ __noinline__ void norm_quant(const float *src, const uint16_t 
              ((ps[lane + 32] + ps[lane + 160]) + (ps[lane + 96] + ps[lane + 224]));
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) t = t + __shfl_xor_sync(kFull, t, off);
-  const float inv = 1.0f / sqrtf((float)(t / (double)H) + PL.eps);
+  const double rH = __hiloint2double((1023 - (__ffs(H) - 1)) << 20, 0);
+  const float inv = 1.0f / sqrtf((float)(t * rH) + PL.eps);
   uint32_t *xw = reinterpret_cast<uint32_t *>(act);
   float *sqs = reinterpret_cast<float *>(act + H);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int g = warp + 16 * i;
-    if (g < H / 128) {
+    if (g < G) {
       const int j = g * 128 + lane * 4;
       const float4 x = *reinterpret_cast<const float4 *>(xs + j);
       float4 y;
@@ -520,109 +608,108 @@ static __device__ __noinline__ void norm_quant(const float *src, const uint16_t 
       y.z = (x.z * inv) * (1.0f + wv[i].z);
       y.w = (x.w * inv) * (1.0f + wv[i].w);
       if (hn) *reinterpret_cast<float4 *>(hn + j) = y;
-      quant_group_staged(xw, sqs, H, 0, g, y);
+      stage_group(xw, sqs, G, 0, g, y);
     }
   }
   csync();
 }
 
 // Stages an already quantised vector (INT8 + group scales in global memory).
-static __device__ __noinline__ void stage_q8(const int8_t *xq, const float *sqg, int K) {
+static __device__ __forceinline__ void stage_q8(const int8_t *xq, const float *sqg, int K) {
   unsigned char *act = step_smem + kActOff;
   uint32_t *xw = reinterpret_cast<uint32_t *>(act);
   float *sqs = reinterpret_cast<float *>(act + K);
+  const int G = K >> 7;
   for (int pc = threadIdx.x; pc < K / 8; pc += kCons) {
     const uint2 v = __ldcg(reinterpret_cast<const uint2 *>(xq + (size_t)pc * 8));
-    xw[staged4_word(K, 0, pc, 0)] = __byte_perm(v.x, v.y, 0x6420);
-    xw[staged4_word(K, 0, pc, 1)] = __byte_perm(v.x, v.y, 0x7531);
+    const int g = pc >> 4, i = pc & 15;
+    uint32_t *dst = xw + ((((i >> 1) * G + g) << 2) + ((i & 1) << 1));
+    dst[0] = __byte_perm(v.x, v.y, 0x6420);
+    dst[1] = __byte_perm(v.x, v.y, 0x7531);
   }
-  for (int g = threadIdx.x; g < K / 128; g += kCons) sqs[g] = __ldcg(sqg + g);
+  for (int g = threadIdx.x; g < G; g += kCons) sqs[g] = __ldcg(sqg + g);
   csync();
 }
 
-// Quantises M contiguous fp32 vectors of K (global memory, M * K <= 8192) into the staged form.
-static __device__ __noinline__ void quant_rows(const float *x, int K, int M) {
-  float *raw = reinterpret_cast<float *>(step_smem + kFbufOff);
+// Quantises M contiguous fp32 vectors of K (global memory, M * K <= 8192) into the staged form: a
+// warp takes whole groups, and the loads of its (at most four) groups are in flight together.
+static __device__ __forceinline__ void quant_rows(const float *x, int lgG, int M) {
   unsigned char *act = step_smem + kActOff;
-  const int n4 = M * K / 4;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = 1 << lgG, n = M << lgG;
+  uint32_t *xw = reinterpret_cast<uint32_t *>(act);
+  float *sqs = reinterpret_cast<float *>(act + (size_t)n * 128);
   float4 v[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const int i = threadIdx.x + kCons * u;
+    const int gi = warp + 16 * u;
     v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (i < n4) v[u] = __ldcg(reinterpret_cast<const float4 *>(x) + i);
+    if (gi < n) v[u] = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)gi * 128) + lane);
   }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const int i = threadIdx.x + kCons * u;
-    if (i < n4) reinterpret_cast<float4 *>(raw)[i] = v[u];
-  }
-  csync();
-  uint32_t *xw = reinterpret_cast<uint32_t *>(act);
-  float *sqs = reinterpret_cast<float *>(act + (size_t)M * K);
-  const int G = K >> 7, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll 1
-  for (int gi = warp; gi < M * G; gi += 16) {
-    const float4 q = reinterpret_cast<const float4 *>(raw + (size_t)gi * 128)[lane];
-    quant_group_staged(xw, sqs, K, gi / G, gi % G, q);
+    const int gi = warp + 16 * u;
+    if (gi < n) stage_group(xw, sqs, G, gi >> lgG, gi & (G - 1), v[u]);
   }
   csync();
 }
 
 // Gated per-head norm + quantiser (RmsInv + NormGated + ScalesMax + Quantize,
-// kernels.cpp:619-644,551-579), one warp per head, into the staged form (K = nV * 128).
-static __device__ __noinline__ void gated_norm_quant(const float *O, const float *Z, const float *W, int nV) {
-  float *os = reinterpret_cast<float *>(step_smem + kFbufOff), *zs = os + 4096;
+// kernels.cpp:619-644,551-579) into the staged form (K = nV * 128 <= 4096): a warp takes whole heads,
+// at most two, side by side. Zs holds silu(z): the projection's epilogue has it from one thread a row,
+// where every block would evaluate nV * 128 exponentials here. Lane l holds values l, l + 32, l + 64 and
+// l + 96 of a head, the terms of its sum of squares.
+static __device__ __forceinline__ void gated_norm_quant(unsigned epoch, const float *O, const float *Zs, const float *W, int nV) {
   unsigned char *act = step_smem + kActOff;
-  const int n4 = nV * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float4 wn = __ldg(reinterpret_cast<const float4 *>(W) + lane);
-  float4 vo[2], vz[2];  // nV * 128 <= 4096 values: at most two float4 of each per thread
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float wn[4];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int i = threadIdx.x + kCons * u;
-    vo[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    vz[u] = vo[u];
-    if (i < n4) {
-      vo[u] = __ldcg(reinterpret_cast<const float4 *>(O) + i);
-      vz[u] = __ldcg(reinterpret_cast<const float4 *>(Z) + i);
-    }
-  }
+  for (int i = 0; i < 4; ++i) wn[i] = __ldg(W + lane + 32 * i);
+  grid_wait(epoch);
+  float o[2][4], z[2][4];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int i = threadIdx.x + kCons * u;
-    if (i < n4) {
-      reinterpret_cast<float4 *>(os)[i] = vo[u];
-      reinterpret_cast<float4 *>(zs)[i] = vz[u];
-    }
-  }
-  csync();
-  const int K = nV * 128;
-  uint32_t *xw = reinterpret_cast<uint32_t *>(act);
-  float *sqs = reinterpret_cast<float *>(act + K);
-#pragma unroll 1
-  for (int h = warp; h < nV; h += 16) {
-    const float *o = os + h * 128, *z = zs + h * 128;
-    float ss = 0.0f;
+  for (int u = 0; u < 2; ++u)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float ov = o[lane + 32 * i];
-      ss = fmaf(ov, ov, ss);
+      const int h = warp + 16 * u, e = h * 128 + lane + 32 * i;
+      o[u][i] = 0.0f;
+      z[u][i] = 0.0f;
+      if (h < nV) {
+        o[u][i] = __ldcg(O + e);
+        z[u][i] = __ldcg(Zs + e);
+      }
     }
-    ss = warp_tree_sum(ss);
-    const float inv = 1.0f / sqrtf(ss / 128.0f + PL.eps);
-    const float4 ov = reinterpret_cast<const float4 *>(o)[lane], zv = reinterpret_cast<const float4 *>(z)[lane];
-    float4 y;
-    y.x = ((wn.x * ov.x) * inv) * (zv.x / (1.0f + det_expf(-zv.x)));
-    y.y = ((wn.y * ov.y) * inv) * (zv.y / (1.0f + det_expf(-zv.y)));
-    y.z = ((wn.z * ov.z) * inv) * (zv.z / (1.0f + det_expf(-zv.z)));
-    y.w = ((wn.w * ov.w) * inv) * (zv.w / (1.0f + det_expf(-zv.w)));
-    quant_group_staged(xw, sqs, K, 0, h, y);
+  int8_t *xb = reinterpret_cast<int8_t *>(act);
+  float *sqs = reinterpret_cast<float *>(act + nV * 128);
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int h = warp + 16 * u;
+    if (h < nV) {
+      float ss = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ss = fmaf(o[u][i], o[u][i], ss);
+      ss = warp_tree_sum(ss);
+      const float inv = 1.0f / sqrtf(ss / 128.0f + PL.eps);
+      float4 y;
+      y.x = ((wn[0] * o[u][0]) * inv) * z[u][0];
+      y.y = ((wn[1] * o[u][1]) * inv) * z[u][1];
+      y.z = ((wn[2] * o[u][2]) * inv) * z[u][2];
+      y.w = ((wn[3] * o[u][3]) * inv) * z[u][3];
+      const float s = group_scale(y);
+      const uint32_t q = quant4(y, s, quant_recip(s));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        // value k of the group: piece k / 8 (two words: even and odd values), byte (k % 8) / 2 of its word
+        const int k = lane + 32 * i, pc = k >> 3;
+        xb[((((pc >> 1) * nV + h) << 2) + ((pc & 1) << 1) + (k & 1)) * 4 + ((k & 7) >> 1)] = (int8_t)(q >> (8 * i));
+      }
+      if (lane == 0) sqs[h] = s;
+    }
   }
   csync();
 }
 
 // Matrix and local row of flat row `flat` of a table of matrices.
-__device__ __forceinline__ int mat_of_row(const GemvMat *m, int nm, int flat, int &n) {
+static __device__ __forceinline__ int mat_of_row(const GemvMat *m, int nm, int flat, int &n) {
   int rs = 0, i = 0;
   while (i < nm - 1 && flat >= rs + m[i].N) {
     rs += m[i].N;
@@ -632,51 +719,104 @@ __device__ __forceinline__ int mat_of_row(const GemvMat *m, int nm, int flat, in
   return i;
 }
 
-// One GEMV stage: this block's rows of the matrices, activations already staged. The operands
-// of the rows' epilogues (residual, conv state, decay constants) are fetched before the dot and
-// stay in flight during it: dot_tiles is inlined here, because across a real call the compiler
-// would have to spill the registers the loads land in, and the spill would wait for the loads.
-static __device__ __noinline__ uint32_t gemv_stage_run(uint32_t tile, const GemvMat *m, int nm, int K) {
-  int lo, hi;
-  deal(mats_rows(m, nm), row_unit(K), (int)blockIdx.x, (int)gridDim.x, lo, hi);
-  if (lo >= hi) return tile;
-  float *T = reinterpret_cast<float *>(step_smem + kTOff);
+// Operands of a row's epilogue that do not depend on its dot product: 32 bytes of shared memory a row,
+// under way during the dot as asynchronous copies (registers that wait for them would be spilled, and the
+// spill would wait): convolution taps [0..3] and history [4..6], or decay constants [4], [5]. All of
+// them are read once a launch, so that no cached line is older than they are; the residual, which
+// other blocks write during the launch, is a plain load past the cache into `res`.
+static __device__ __forceinline__ void cp_async4(float *dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+static __device__ __forceinline__ void row_operands(const GemvMat &mt, int n, float *op, float &res) {
+  const int epi = mt.epi;
+  if (epi == EPI_CONV_SILU) {
+    const float *cs = mt.e1 + (size_t)n * 3;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(op)), "l"(mt.e0 + (size_t)n * 4) : "memory");
+    cp_async4(op + 4, cs);
+    cp_async4(op + 5, cs + 1);
+    cp_async4(op + 6, cs + 2);
+  }
+  if (epi == EPI_GDECAY) {
+    cp_async4(op + 4, mt.e0 + n);
+    cp_async4(op + 5, mt.e2 + n);
+  }
+  res = 0.0f;
+  if (epi == EPI_RESADD) res = __ldcg(mt.e0 + n);
+}
+// gemv_epilogue()'s arithmetic; every kind of row that needs an exponential of its sum shares one.
+static __device__ __forceinline__ void row_epilogue(const GemvMat &mt, int n, float acc, const float *op, float res) {
+  const int epi = mt.epi;
+  float *y = mt.Y + n;
+  if (epi == EPI_STORE) { *y = acc; return; }
+  if (epi == EPI_RESADD) { *y = res + acc; return; }
+  float num = epi == EPI_BETA ? 1.0f : acc, arg = -acc;
+  if (epi == EPI_CONV_SILU) {
+    const float4 cw = *reinterpret_cast<const float4 *>(op);
+    const float c1 = op[5], c2 = op[6];
+    float a = op[4] * cw.x;
+    a = a + c1 * cw.y;
+    a = a + c2 * cw.z;
+    a = a + acc * cw.w;
+    num = a;
+    arg = -a;
+    float *cs = mt.e1 + (size_t)n * 3;
+    cs[0] = c1;
+    cs[1] = c2;
+    cs[2] = acc;
+  }
+  if (epi == EPI_GDECAY) arg = acc + op[5];
+  const float e = det_expf(arg);
+  if (epi != EPI_GDECAY) { *y = num / (1.0f + e); return; }
+  const float soft = arg > 20.0f ? arg : det_logf(1.0f + e);
+  *y = (-det_expf(op[4])) * soft;
+}
+
+// One GEMV stage: this block's rows of the matrices, activations already staged.
+static __device__ __forceinline__ uint32_t gemv_stage_run(uint32_t tile, const GemvMat *m, int nm, int K, int rng) {
+  const int lo = SH->rng[rng].x, nr = SH->rng[rng].y - lo;
+  if (nr <= 0) return tile;
+  float *T = reinterpret_cast<float *>(step_smem + kTOff), *op = reinterpret_cast<float *>(step_smem + kFbufOff) + 4096 + threadIdx.x * 8;
   unsigned char *act = step_smem + kActOff;
-  const int G = K >> 7, nr = hi - lo;
-  EpiOperands eo;
+  const int lg = 31 - __clz(K >> 7);
   int mi = 0, n = 0;
+  float res = 0.0f;
   if ((int)threadIdx.x < nr) {
     mi = mat_of_row(m, nm, lo + threadIdx.x, n);
-    gemv_epilogue_fetch(&m[mi], n, 0, eo);
+    row_operands(m[mi], n, op, res);
   }
-  tile = dot_tiles(tile, K, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + K), T, 0, nr, nr, 0);
+  tile = dot_tiles<false>(tile, lg, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + K), T, nr, 0);
   csync();
-  if ((int)threadIdx.x < nr) gemv_epilogue_with(&m[mi], n, 0, row_sum_rt(T, threadIdx.x, G), eo);
-  for (int r = threadIdx.x + kCons; r < nr; r += kCons) {
-    mi = mat_of_row(m, nm, lo + r, n);
-    gemv_epilogue(&m[mi], n, 0, row_sum_rt(T, r, G));
+#pragma unroll 1
+  for (int r = threadIdx.x; r < nr; r += kCons) {
+    if (r >= kCons) {
+      mi = mat_of_row(m, nm, lo + r, n);
+      row_operands(m[mi], n, op, res);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");   // the thread's own copies
+    row_epilogue(m[mi], n, row_terms(T, r, lg), op, res);
   }
   return tile;
 }
 
 // Router logits of this block's rows from the ring (bf16 rows), activations hn in shared memory.
 // logits[e] = sum_k bf16(W[e][k]) * hn[k]: lane l takes k = (i*32+l)*8+j, fma chain in (i, j)
-// order, then the lane tree (as RouterTopK).
-static __device__ __noinline__ uint32_t router_stage(uint32_t tile, const float *hn, int H, int rows_total) {
-  int lo, hi;
-  deal(rows_total, 1, (int)blockIdx.x, (int)gridDim.x, lo, hi);
-  if (lo >= hi) return tile;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = H / 256;
-  const int rpt = kTileBytes / (H * 2), total = hi - lo, ntiles = (total + rpt - 1) / rpt;
+// order, then the lane tree (as RouterTopK). Tiles go to alternate halves of the consumers, as in dot_tiles.
+static __device__ __forceinline__ uint32_t router_stage(uint32_t tile, const float *hn, int H) {
+  const int lo = SH->rng[kRngRouter].x, total = SH->rng[kRngRouter].y - lo;
+  if (total <= 0) return tile;
+  const int warp = (threadIdx.x >> 5) & 7, half = threadIdx.x >> 8, lane = threadIdx.x & 31, n = H >> 8;
+  const int lrpt = __ffs(kTileBytes) - __ffs(H * 2), rpt = 1 << lrpt, ntiles = (total + rpt - 1) >> lrpt;
   const uint32_t ring_a = smem_addr(step_smem + kRingOff);
 #pragma unroll 1
-  for (int j = 0; j < ntiles; ++j) {
-    const uint32_t slot = tile % kNT, use = tile / kNT;
+  for (int j = half; j < ntiles; j += 2) {
+    const uint32_t idx = tile + (uint32_t)j, slot = idx % kNT, use = idx / kNT;
     if (!__all_sync(kFull, mbar_wait_b(smem_addr(&SH->full[slot]), use & 1u, 5))) break;
     const uint32_t tb = ring_a + slot * kTileStride;
     const int nr = total - j * rpt < rpt ? total - j * rpt : rpt;
-    for (int r = warp; r < nr; r += 16) {
+#pragma unroll 1
+    for (int r = warp; r < nr; r += 8) {
       float acc = 0.0f;
+#pragma unroll 4
       for (int i = 0; i < n; ++i) {
         const int k0 = (i * 32 + lane) * 8;
         const uint4 wv = lds128(tb + (uint32_t)r * (uint32_t)(H * 2) + (uint32_t)k0 * 2u);
@@ -695,71 +835,118 @@ static __device__ __noinline__ uint32_t router_stage(uint32_t tile, const float 
     }
     __syncwarp();
     if (lane == 0) mbar_arrive_a(smem_addr(&SH->empty[slot]));
-    tile += 1;
   }
-  return tile;
+  return tile + (uint32_t)ntiles;
 }
 
-// Softmax over the E router logits, top-k by (probability desc, index asc), renormalised
-// weights, shared-expert gate: the selection of RouterTopK, run by every block for itself.
-static __device__ __noinline__ void router_select_cons(int E, int k, bool has_shared) {
-  float *lg = reinterpret_cast<float *>(step_smem + kFbufOff), *sp = lg + 2048;  // logits, probabilities (E <= 1024)
-  unsigned *ck = reinterpret_cast<unsigned *>(step_smem + kTOff), *ci = ck + kTopkWarps * kTopkMaxSel;
+// Softmax over the E <= 1024 router logits, top-k by (probability desc, index asc), renormalised
+// weights, shared-expert gate: the selection of RouterTopK, run by every block for itself, with the
+// selected experts' pointer records fetched on the way. Order of experts: key = bits of the
+// probability + 1 (it is >= 0, so the bits order like integers), then the lower index. The
+// nsel-th largest of the sixteen warps' largest keys bounds the nsel-th largest of all from below,
+// so the entries at or above it (about 17 of 512 for a top 10) hold the whole selection: they are
+// gathered, and each one's rank is the number of candidates ahead of it (k + 1 rounds of extraction in
+// two levels, and the records fetched after them: 4.5 + 0.8 us a layer; so 2.9). slots <= 12, so nsel <=
+// 13 of the sixteen maxima.
+static __device__ __forceinline__ void router_select_cons(unsigned epoch, const ExpertW *experts, int E, int k, bool has_shared) {
+  float *lg = reinterpret_cast<float *>(step_smem + kFbufOff), *sp = lg + 2048, *pr = lg + 4096;
+  unsigned long long *cand = reinterpret_cast<unsigned long long *>(step_smem + kTOff);   // up to E candidates
   StepShared *sh = SH;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e <= E; e += kCons)
-    if (e < E || has_shared) lg[e] = __ldcg(PL.RLogits + e);
+  grid_wait(epoch);
+#pragma unroll
+  for (int u = 0; u < 3; ++u) {
+    const int e = tid + kCons * u;
+    if (e < E || (has_shared && e == E)) lg[e] = __ldcg(PL.RLogits + e);
+  }
+  if (tid == 0) sh->ncand = 0;
   csync();
   // maximum and sum keep the one-warp partition (lane l takes entries l, l+32, ... in ascending
   // order, then the xor butterfly); every warp evaluates them for itself, which gives every warp
   // the same bits and saves two block barriers and two one-warp sections
   float m = -INFINITY;
+#pragma unroll 8
   for (int e = lane; e < E; e += 32) m = fmaxf(m, lg[e]);
-  m = warp_max(m);
-  for (int e = tid; e < E; e += kCons) sp[e] = det_expf(lg[e] - m);
-  if (tid == 0 && has_shared) sp[E] = lg[E];
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(m));
+  float ex[2] = {0.0f, 0.0f};
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int e = tid + kCons * u;
+    if (e < E) {
+      ex[u] = det_expf(lg[e] - m);
+      sp[e] = ex[u];
+    }
+  }
   csync();
   float sum = 0.0f;
+#pragma unroll 8
   for (int e = lane; e < E; e += 32) sum = sum + sp[e];
   sum = warp_tree_sum(sum);
-  csync();  // every warp has read the exponentials
-  for (int e = tid; e < E; e += kCons) sp[e] = sp[e] / sum;
-  csync();
-  const int nsel = k + 1 < kTopkMaxSel ? k + 1 : kTopkMaxSel;
-  if (warp < kTopkWarps) {
-    const int per = (E + kTopkWarps - 1) / kTopkWarps;
-    unsigned key[4], idx[4];
+  unsigned key[2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int o = lane + 32 * i, e = warp * per + o;
-      const bool ok = o < per && e < E;
-      key[i] = ok ? __float_as_uint(sp[e]) + 1u : 0u;
-      idx[i] = ok ? (unsigned)e : 0x7FFFFFFFu;
+  for (int u = 0; u < 2; ++u) key[u] = tid + kCons * u < E ? __float_as_uint(ex[u] / sum) + 1u : 0u;
+  const unsigned wk = __reduce_max_sync(kFull, key[0] > key[1] ? key[0] : key[1]);
+  if (lane == 0) sh->kmax[warp] = wk;
+  csync();
+  const int nsel = k < E ? k + 1 : k;
+  unsigned bound;
+  {
+    const unsigned mine = lane < 16 ? sh->kmax[lane] : 0u;
+    int ahead = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const unsigned o = sh->kmax[i];
+      ahead += o > mine || (o == mine && i < lane);
     }
-#pragma unroll 1
-    for (int j = 0; j < nsel; ++j) {
-      unsigned wv, wi;
-      topk_extract<4>(key, idx, wv, wi);
-      if (lane == 0) {
-        ck[warp * nsel + j] = wv;
-        ci[warp * nsel + j] = wi;
-      }
+    bound = __reduce_min_sync(kFull, lane < 16 && ahead < nsel ? mine : 0xFFFFFFFFu);
+    if (bound == 0u) bound = 1u;   // fewer warps than nsel hold entries: all of them are candidates
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (key[u] >= bound)
+      cand[atomicAdd(&sh->ncand, 1)] = ((unsigned long long)key[u] << 32) | (0xFFFFFFFFu - (unsigned)(tid + kCons * u));
+  csync();
+  const int nc = sh->ncand;
+  for (int i = warp; i < nc; i += 16) {
+    const unsigned long long c = cand[i];
+    int rank = 0;
+    for (int j0 = 0; j0 < nc; j0 += 32) rank += __popc(__ballot_sync(kFull, j0 + lane < nc && cand[j0 + lane] > c));
+    if (rank > k || rank >= E) continue;
+    const int e = (int)(0xFFFFFFFFu - (unsigned)c);
+    if (rank < k && lane < 3)
+      reinterpret_cast<uint4 *>(sh->sew + rank)[lane] = __ldg(reinterpret_cast<const uint4 *>(experts + e) + lane);
+    if (lane == 0) {
+      pr[rank] = __uint_as_float((unsigned)(c >> 32) - 1u);
+      if (rank < k) sh->sel_idx[rank] = e;
+    }
+  }
+  if (warp == 15) {
+    if (has_shared && lane < 3)
+      reinterpret_cast<uint4 *>(sh->sew + k)[lane] = __ldg(reinterpret_cast<const uint4 *>(experts + E) + lane);
+    if (lane == 0) {
+      sh->sel_idx[k] = E;
+      sh->sel_w[k] = has_shared ? 1.0f / (1.0f + det_expf(-lg[E])) : 0.0f;
     }
   }
   csync();
-  if (warp == 0) {
-    const int ncand = kTopkWarps * nsel;
-    if (ncand <= 128) topk_level2<4>(ck, ci, ncand, sp, E, k, has_shared, sh->sel_idx, sh->sel_w, &sh->gap);
-    else topk_level2<9>(ck, ci, ncand, sp, E, k, has_shared, sh->sel_idx, sh->sel_w, &sh->gap);
+  if (tid == 0) mbar_arrive(&sh->sel_bar);  // the producer may now stream the experts
+  // the weights are needed by the down projection only
+  if (warp == 1) {
+    float s = 0.0f;
+    for (int j = 0; j < k && j < E; ++j) s = s + pr[j];
+    if (lane < k) sh->sel_w[lane] = (lane < E ? pr[lane] : 0.0f) / s;
+    if (lane == 0) {
+      const float lastp = pr[k - 1];
+      sh->gap = k >= E ? 1.0f : (lastp > 0.0f ? (lastp - pr[k]) / lastp : 0.0f);
+    }
   }
-  csync();
 }
 
 // ------------------------------------------------------------ gated delta rule ---
 // One (head, column slice) item per block, 256 threads, state in registers; the arithmetic is
 // DeltaNetStep's (deltanet_core.cuh). The state of the block's first item is loaded before the
 // grid barrier is waited for: it was last written one token ago by this same block.
-static __device__ __noinline__ void deltanet_stage(unsigned epoch, const StepLayer &ly) {
+static __device__ __forceinline__ void deltanet_stage(unsigned epoch, const StepLayer &ly) {
   const StepPlan &P = PL;
   constexpr int D = 128, SEG = kDnSeg;
   DeltaNetStepArgs a{P.O, P.Mx, ly.S, P.Bt, P.Gt, P.nK, P.nV};
@@ -1086,52 +1273,57 @@ static __device__ __noinline__ void attn_combine_stage(int T) {
 }
 
 // ------------------------------------------------------------------- MoE stages ---
-static __device__ __noinline__ uint32_t gateup_stage(uint32_t tile) {
+static __device__ __forceinline__ uint32_t gateup_stage(uint32_t tile) {
   const StepPlan &P = PL;
-  const int H = P.H, I = P.I;
-  int lo, hi;
-  deal(P.slots * I, row_unit(H), (int)blockIdx.x, (int)gridDim.x, lo, hi);
-  if (lo >= hi) return tile;
+  const int H = P.H, lgI = __ffs(P.I) - 1, lg = 31 - __clz(H >> 7);
+  const int lo = SH->rng[kRngGateUp].x, hi = SH->rng[kRngGateUp].y, np = hi - lo;
+  if (np <= 0) return tile;
   float *T = reinterpret_cast<float *>(step_smem + kTOff);
   unsigned char *act = step_smem + kActOff;
-  const int np = hi - lo, G = H >> 7;
-  tile = dot_tiles(tile, H, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + H), T, 0, 2 * np,
-                   2 * np, 0);
+  tile = dot_tiles<false>(tile, lg, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + H), T, 2 * np, 0);
   csync();
   // the producer streams, slot by slot, the slot's gate rows and then its up rows: the pair row
   // lo + r of slot s (rows a .. a + n - 1 of the share belong to it) has its gate term at
   // 2 (a - lo) + i and its up term n rows later
+#pragma unroll 1
   for (int r = threadIdx.x; r < np; r += kCons) {
-    const int s = (lo + r) / I;
-    const int a = lo > s * I ? lo : s * I, b = hi < (s + 1) * I ? hi : (s + 1) * I;
+    const int s = (lo + r) >> lgI;
+    const int a = lo > s * P.I ? lo : s * P.I, b = hi < (s + 1) * P.I ? hi : (s + 1) * P.I;
     const int n = b - a, i = lo + r - a, fg = 2 * (a - lo) + i;
-    const float g = row_sum_rt(T, fg, G), u = row_sum_rt(T, fg + n, G);
-    P.Act[lo + r] = silu_mul(g, u);
+    const float g = row_terms(T, fg, lg), u = row_terms(T, fg + n, lg);
+    P.Act[lo + r] = (g / (1.0f + det_expf(-g))) * u;
   }
   return tile;
 }
 
-static __device__ __noinline__ uint32_t down_stage(uint32_t tile, int L) {
+// Output row n: residual + sum over the slots in rank order of weight x product. One thread a (slot,
+// row) adds the row's group terms, then one a row adds the slots.
+static __device__ __forceinline__ uint32_t down_stage(unsigned epoch, uint32_t tile, int L) {
   const StepPlan &P = PL;
-  const int H = P.H, I = P.I;
-  int lo, hi;
-  deal(H, row_unit(I), (int)blockIdx.x, (int)gridDim.x, lo, hi);
-  quant_rows(P.Act, I, P.slots);
-  stamp(2);
-  if (lo >= hi) return tile;
-  // residual input of this block's rows: in flight while the tiles are dotted (dot_tiles is inlined)
+  const int H = P.H, I = P.I, lg = 31 - __clz(I >> 7);
+  const int lo = SH->rng[kRngDown].x, nr = SH->rng[kRngDown].y - lo;
+  // residual input of this block's rows: complete since the router's barrier
   float res0 = 0.0f;
-  if (lo + (int)threadIdx.x < hi) res0 = __ldcg(P.Tmp + lo + threadIdx.x);
-  float *T = reinterpret_cast<float *>(step_smem + kTOff);
+  if ((int)threadIdx.x < nr) res0 = __ldcg(P.Tmp + lo + threadIdx.x);
+  grid_wait(epoch);
+  quant_rows(P.Act, lg, P.slots);
+  stamp(2);
+  if (nr <= 0) return tile;
+  float *T = reinterpret_cast<float *>(step_smem + kTOff), *ts = reinterpret_cast<float *>(step_smem + kFbufOff);
   unsigned char *act = step_smem + kActOff;
-  tile = dot_tiles(tile, I, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + (size_t)P.slots * I), T,
-                   0, P.slots * (hi - lo), P.slots * (hi - lo), hi - lo);
+  const int n = P.slots * nr;
+  tile = dot_tiles<true>(tile, lg, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + (size_t)P.slots * I), T,
+                         n, nr);
   csync();
-  const int nr = hi - lo, G = I >> 7;
+#pragma unroll 1
+  for (int f = threadIdx.x; f < n; f += kCons) ts[f] = SH->sel_w[f / nr] * row_terms(T, f, lg);
+  csync();
+#pragma unroll 1
   for (int r = threadIdx.x; r < nr; r += kCons) {
     const float res = r < kCons ? res0 : __ldcg(P.Tmp + lo + r);
     float acc = 0.0f;
-    for (int s = 0; s < P.slots; ++s) acc = acc + SH->sel_w[s] * row_sum_rt(T, s * nr + r, G);
+#pragma unroll 4
+    for (int s = 0; s < P.slots; ++s) acc = acc + ts[s * nr + r];
     const float x = res + acc;
     P.X[lo + r] = x;
     if (P.layer_out) P.layer_out[(size_t)L * H + lo + r] = x;
@@ -1140,22 +1332,21 @@ static __device__ __noinline__ uint32_t down_stage(uint32_t tile, int L) {
 }
 
 // LM head in sub-blocks of 16 tiles (t[][] holds 256 rows of K = 2048), running argmax per thread.
-static __device__ __noinline__ uint32_t lm_head_stage(uint32_t tile, float &bv, int &bi) {
+static __device__ __forceinline__ uint32_t lm_head_stage(uint32_t tile, float &bv, int &bi) {
   const StepPlan &P = PL;
-  const int K = P.H, G = K >> 7;
-  int lo, hi;
-  deal(P.vocab, row_unit(K), (int)blockIdx.x, (int)gridDim.x, lo, hi);
+  const int K = P.H, lg = 31 - __clz(K >> 7);
+  const int lo = SH->rng[kRngHead].x, hi = SH->rng[kRngHead].y;
   float *T = reinterpret_cast<float *>(step_smem + kTOff);
   unsigned char *act = step_smem + kActOff;
-  const int sub = kTCap / G;  // rows whose terms fit t[][]: a whole number of tiles
+  const int sub = kTCap >> lg;  // rows whose terms fit t[][]: a whole, even number of tiles
 #pragma unroll 1
   for (int base = 0; base < hi - lo; base += sub) {
     const int nrows = (hi - lo) - base < sub ? (hi - lo) - base : sub;
-    tile = dot_tiles(tile, K, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + K), T, base, nrows,
-                     hi - lo, 0);
+    tile = dot_tiles<false>(tile, lg, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + K), T, nrows, 0);
     csync();
+#pragma unroll 1
     for (int r = threadIdx.x; r < nrows; r += kCons) {
-      const float v = row_sum_rt(T, r, G);
+      const float v = row_terms(T, r, lg);
       const int n = lo + base + r;
       P.Logits[n] = v;
       argmax_merge(bv, bi, v, n);
@@ -1185,7 +1376,7 @@ static __device__ __noinline__ void cons_argmax(float &bv, int &bi) {
   }
 }
 
-static __device__ __noinline__ void consumer_main(int mode) {
+static __device__ __forceinline__ void consumer_main(int mode) {
   const StepPlan &P = PL;
   StepShared *sh = SH;
   const int H = P.H, tid = threadIdx.x;
@@ -1199,7 +1390,7 @@ static __device__ __noinline__ void consumer_main(int mode) {
 
   for (int L = 0; L < P.layers; ++L) {
     // the layer's record into shared memory (the previous layer's is no longer read: every
-    // consumer has passed the grid barrier that ended it)
+    // consumer has passed a block barrier behind its last use)
     {
       const uint4 *src = reinterpret_cast<const uint4 *>(P.L + L);
       if (tid < (int)(sizeof(StepLayer) / 16)) reinterpret_cast<uint4 *>(&sh->ly)[tid] = __ldg(src + tid);
@@ -1207,11 +1398,17 @@ static __device__ __noinline__ void consumer_main(int mode) {
     }
     const StepLayer &ly = sh->ly;
     const bool lin = ly.type == 0;
+    // the layer's table of experts into L2, a line a thread over the grid's first blocks
+    {
+      const int line = (int)blockIdx.x * 2 + tid;
+      if (tid < 2 && line * 128 < (P.E + 1) * (int)sizeof(ExpertW))
+        prefetch_l2(reinterpret_cast<const unsigned char *>(ly.experts) + line * 128);
+    }
     // ---- stage 1: input norm + quantiser, first projections ----
-    norm_quant(P.X, L == 0 ? P.emb + (size_t)tok * H : nullptr, ly.in_norm, H, nullptr,
+    norm_quant(epoch, P.X, L == 0 ? P.emb + (size_t)tok * H : nullptr, ly.in_norm, H, nullptr,
                (L == 0 && (int)blockIdx.x == 0) ? P.X : nullptr);
     stamp(2);
-    tile = gemv_stage_run(tile, &ly.m[0], lin ? 4 : 3, H);
+    tile = gemv_stage_run(tile, &ly.m[0], lin ? 4 : 3, H, kRngIn + ly.type);
     stamp(3);
     grid_arrive();
     ++epoch;
@@ -1219,47 +1416,39 @@ static __device__ __noinline__ void consumer_main(int mode) {
       // ---- stage 2: gated delta rule ----
       deltanet_stage(epoch, ly);  // waits for the barrier inside, after its state loads
       grid_arrive();
-    ++epoch;
-      grid_wait(epoch);
+      ++epoch;
       // ---- stage 3: gated norm, out_proj + residual ----
-      stamp(4);
-      gated_norm_quant(P.O, P.Z, ly.lin_norm, P.nV);
-      stamp(2);
-      tile = gemv_stage_run(tile, &ly.m[4], 1, P.nV * 128);
-      stamp(3);
+      gated_norm_quant(epoch, P.O, P.Z, ly.lin_norm, P.nV);
     } else {
       attn_stage(epoch, ly, pos, T);  // waits for the barrier inside, after its KV loads
       grid_arrive();
-    ++epoch;
+      ++epoch;
       grid_wait(epoch);
       attn_combine_stage(T);
       grid_arrive();
-    ++epoch;
+      ++epoch;
       grid_wait(epoch);
       stage_q8(P.Q8, P.SQ, P.nQ * 256);
-      tile = gemv_stage_run(tile, &ly.m[4], 1, P.nQ * 256);
     }
-    grid_arrive();
-    ++epoch;
-    grid_wait(epoch);
-    // ---- stage 4: post norm + quantiser (kept staged for the experts), router logits ----
-    norm_quant(P.Tmp, nullptr, ly.post_norm, H, hn, nullptr);
     stamp(2);
-    tile = router_stage(tile, hn, H, P.E + (ly.shared_gate ? 1 : 0));
+    tile = gemv_stage_run(tile, &ly.m[4], 1, lin ? P.nV * 128 : P.nQ * 256, kRngOut + ly.type);
     stamp(3);
     grid_arrive();
     ++epoch;
-    grid_wait(epoch);
+    // ---- stage 4: post norm + quantiser (kept staged for the experts), router logits ----
+    norm_quant(epoch, P.Tmp, nullptr, ly.post_norm, H, hn, nullptr);
+    stamp(2);
+    tile = router_stage(tile, hn, H);
+    stamp(3);
+    grid_arrive();
+    ++epoch;
     // ---- stage 5: selection, expert gate/up ----
-    router_select_cons(P.E, P.topk, ly.shared_gate != nullptr);
+    router_select_cons(epoch, ly.experts, P.E, P.topk, ly.shared_gate != nullptr);
     stamp(5);
-    if (tid < P.slots * 3) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(ly.experts + sh->sel_idx[tid / 3]) + tid % 3;
-      reinterpret_cast<uint4 *>(sh->sew + tid / 3)[tid % 3] = __ldg(src);
-    }
-    csync();
-    if (tid == 0) mbar_arrive(&sh->sel_bar);  // the producer may now stream the experts
-    stamp(6);
+    tile = gateup_stage(tile);
+    stamp(3);
+    grid_arrive();
+    ++epoch;
     if ((int)blockIdx.x == 0 && tid <= P.topk) {
       P.SelIdx[tid] = sh->sel_idx[tid];
       P.SelW[tid] = sh->sel_w[tid];
@@ -1269,17 +1458,11 @@ static __device__ __noinline__ void consumer_main(int mode) {
         if (tid == 0) P.near_gap[L] = sh->gap;
       }
     }
-    tile = gateup_stage(tile);
-    stamp(3);
-    grid_arrive();
-    ++epoch;
-    grid_wait(epoch);
     // ---- stage 6: expert down, combine, residual ----
-    tile = down_stage(tile, L);
+    tile = down_stage(epoch, tile, L);
     stamp(3);
     grid_arrive();
     ++epoch;
-    grid_wait(epoch);
   }
 
   if (mode == 0) {
@@ -1294,7 +1477,7 @@ static __device__ __noinline__ void consumer_main(int mode) {
     return;
   }
   // ---- tail: final norm, LM head, first-max-wins argmax, control update ----
-  norm_quant(P.X, nullptr, P.final_norm, H, nullptr, nullptr);
+  norm_quant(epoch, P.X, nullptr, P.final_norm, H, nullptr, nullptr);
   float bv = -INFINITY;
   int bi = 0x7FFFFFFF;
   tile = lm_head_stage(tile, bv, bi);
@@ -1304,9 +1487,9 @@ static __device__ __noinline__ void consumer_main(int mode) {
     P.PI[(int)blockIdx.x] = bi;
   }
   grid_arrive();
-    ++epoch;
-  grid_wait(epoch);
+  ++epoch;
   if ((int)blockIdx.x == 0) {
+    grid_wait(epoch);
     bv = -INFINITY;
     bi = 0x7FFFFFFF;
     for (int i = tid; i < (int)gridDim.x; i += kCons) argmax_merge(bv, bi, __ldcg(P.PV + i), __ldcg(P.PI + i));
@@ -1323,12 +1506,16 @@ static __device__ __noinline__ void consumer_main(int mode) {
   }
 }
 
-__global__ void __launch_bounds__(kStepThreads, 1) DecodeStep(const DecodeStepArgs args) {
+};
+
+template <bool kClock>
+__device__ __forceinline__ void decode_step(const DecodeStepArgs &args) {
+  using B = Step<kClock>;
   StepShared *sh = SH;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kNT; ++i) {
       mbar_init(&sh->full[i], 1);
-      mbar_init(&sh->empty[i], kCons / 32);  // one arrival per consumer warp
+      mbar_init(&sh->empty[i], kCons / 64);  // one arrival per warp of the half that consumes the tile
     }
     mbar_init(&sh->sel_bar, 1);
     sh->fail = 0;
@@ -1340,9 +1527,11 @@ __global__ void __launch_bounds__(kStepThreads, 1) DecodeStep(const DecodeStepAr
   if (threadIdx.x < sizeof(StepPlan) / 16)
     reinterpret_cast<uint4 *>(&sh->plan)[threadIdx.x] = __ldg(reinterpret_cast<const uint4 *>(args.plan) + threadIdx.x);
   __syncthreads();
+  if (threadIdx.x < kRngCount) B::deal_all((int)threadIdx.x);
+  __syncthreads();
   if (*(volatile int *)PL.error != 0) return;  // a previous launch failed: stay out
   if (threadIdx.x >= kCons) {
-    const uint32_t issued = producer_main(args.mode);
+    const uint32_t issued = B::producer_main(args.mode);
     // Nothing may still be landing in this block's shared memory when it retires: every slot
     // owner waits (bounded) for the last tile it issued. In a run without faults the consumers
     // have waited for all of them already.
@@ -1355,13 +1544,16 @@ __global__ void __launch_bounds__(kStepThreads, 1) DecodeStep(const DecodeStepAr
     }
     return;
   }
-  consumer_main(args.mode);
+  B::consumer_main(args.mode);
 }
+__global__ void __launch_bounds__(kStepThreads, 1) DecodeStep(const DecodeStepArgs args) { decode_step<false>(args); }
+__global__ void __launch_bounds__(kStepThreads, 1) DecodeStepClock(const DecodeStepArgs args) { decode_step<true>(args); }
 
 static uint32_t step_smem_fn(const void *) { return (uint32_t)kStepSmemBytes; }
 
 #define F(f) AINFER_ARG(DecodeStepArgs, f)
 AINFER_REGISTER_COOP(DecodeStep, DecodeStepArgs, kStepThreads, 0, 0, step_smem_fn, F(plan), F(mode));
+AINFER_REGISTER_COOP(DecodeStepClock, DecodeStepArgs, kStepThreads, 0, 0, step_smem_fn, F(plan), F(mode));
 #undef F
 
 }  // namespace ainfer

@@ -334,7 +334,7 @@ int build_step(Session *s) {
       ly.type = 0;
       ly.m[0] = make_mat(s, status, p + "linear_attn.in_proj_qkv.weight", H, s->Mx, EPI_CONV_SILU,
                          m->conv_w + (size_t)slot * C * 4, s->conv + (size_t)slot * C * 3, nullptr);
-      ly.m[1] = make_mat(s, status, p + "linear_attn.in_proj_z.weight", H, s->Z, EPI_STORE, nullptr, nullptr, nullptr);
+      ly.m[1] = make_mat(s, status, p + "linear_attn.in_proj_z.weight", H, s->Z, EPI_SILU, nullptr, nullptr, nullptr);
       ly.m[2] = make_mat(s, status, p + "linear_attn.in_proj_b.weight", H, s->Bt, EPI_BETA, nullptr, nullptr, nullptr);
       ly.m[3] = make_mat(s, status, p + "linear_attn.in_proj_a.weight", H, s->Gt, EPI_GDECAY,
                          m->a_log + (size_t)slot * nV, nullptr, m->dt_bias + (size_t)slot * nV);
@@ -378,6 +378,8 @@ int build_step(Session *s) {
     P.stage_stamp_cap = s->stage_stamp_cap;
   }
   P.bar_count = s->bar_count; P.error = s->step_error;
+  P.in_rows[0] = C + VD + 2 * nV;
+  P.in_rows[1] = nQ * 2 * D + 2 * nKV * D;
   StepLayer *dl = nullptr;
   if (salloc(s, layers.size(), &dl, false)) return 1;
   s->step_layers = dl;
@@ -391,8 +393,9 @@ int build_step(Session *s) {
     return 1;
   }
   ainfer_kernel_t k = nullptr;
-  if (ainfer_kernel_get(s->dev, "DecodeStep", &k) != AINFER_OK) { s->err = "entry DecodeStep not found"; return 1; }
-  s->kernels["DecodeStep"] = k;
+  const char *entry = (s->flags & SESSION_STAGE_CLOCK) ? "DecodeStepClock" : "DecodeStep";
+  if (ainfer_kernel_get(s->dev, entry, &k) != AINFER_OK) { s->err = std::string("entry ") + entry + " not found"; return 1; }
+  s->kernels[entry] = k;
   const StepPlan *cdp = dp;
   int32_t mode = 1;
   ainfer_kernel_set_arg(k, 0, sizeof cdp, &cdp);
