@@ -325,6 +325,7 @@ struct EpGroupLocalArgs {
   int32_t *Counts;            // [8], see ep_store_counts
   int32_t n, k, E, I;
   int32_t shared_row0, shared_rows, max_rows;
+  int32_t *Lists;             // optional (null: Counts counts by max_rows): [2] lengths of the lists, and Counts counts by 64 rows
 };
 __global__ void __launch_bounds__(1024) EpGroupLocal(const EpGroupLocalArgs a) {
   __shared__ int hist[1024], start[1024], wsum[2][33];
@@ -377,9 +378,21 @@ __global__ void __launch_bounds__(1024) EpGroupLocal(const EpGroupLocalArgs a) {
     }
   if (c > 0) ep_problems(a.GroupsGateUp, a.GroupsDown, a.Experts[tid], first, c, a.max_rows, a.I, g0);
   const int few = __syncthreads_count(c > 0 && c <= kEpFewRows);
+  int counted = total, by = a.max_rows;
+  if (a.Lists) {   // the documented counts are by 64 rows, whatever the lists' cut
+    by = 64;
+    counted = 0;
+#pragma unroll 1
+    for (int j = 0; j * 64 < a.n; ++j) counted += __syncthreads_count(c > j * 64);   // an expert has an item of a row at most once
+    if (tid == 0) {
+      const int lists = total + (a.shared_rows + a.max_rows - 1) / a.max_rows;
+      a.Lists[0] = 2 * lists;
+      a.Lists[1] = lists;
+    }
+  }
   if (tid == 1023) {
     if (a.shared_rows > 0) ep_problems(a.GroupsGateUp, a.GroupsDown, a.Experts[a.E], a.shared_row0, a.shared_rows, a.max_rows, a.I, total);
-    ep_store_counts(a.Counts, items, few + (a.shared_rows > 0 && a.shared_rows <= kEpFewRows), total + (a.shared_rows + a.max_rows - 1) / a.max_rows);
+    ep_store_counts(a.Counts, items, few + (a.shared_rows > 0 && a.shared_rows <= kEpFewRows), counted + (a.shared_rows + by - 1) / by);
   }
 }
 struct EpGatherLocalArgs {
@@ -515,7 +528,7 @@ AINFER_REGISTER(EpGather, EpGatherArgs, 128, 1, 0, nullptr, F(Recv), F(Sorted), 
 #undef F
 #define F(f) AINFER_ARG(EpGroupLocalArgs, f)
 AINFER_REGISTER(EpGroupLocal, EpGroupLocalArgs, 1024, 0, 0, nullptr, F(SelIdx), F(Experts), F(Sorted), F(ItemRow), F(GroupsGateUp), F(GroupsDown),
-                F(Counts), F(n), F(k), F(E), F(I), F(shared_row0), F(shared_rows), F(max_rows));
+                F(Counts), F(n), F(k), F(E), F(I), F(shared_row0), F(shared_rows), F(max_rows), F(Lists));
 #undef F
 #define F(f) AINFER_ARG(EpGatherLocalArgs, f)
 AINFER_REGISTER(EpGatherLocal, EpGatherLocalArgs, 128, 1, 0, nullptr, F(Q8), F(SQ), F(Sorted), F(XQ), F(XS), F(H), F(k));

@@ -142,6 +142,11 @@ struct Rec {   // appends launches to a list (none: launches at once); arguments
     if (ainfer_list_append_memcpy(list, dst, src, bytes) != AINFER_OK) { e->err = ainfer_last_error(e->dev); status = 1; }
   }
 };
+// Rows of a problem of the experts' products when `items` (row, expert) pairs go to E experts: a unit of 16, 32 or 64
+// rows has five, four or three stages of weights in flight, and most experts should be one unit. Full preset, us of a
+// whole batch step of 64 rows (1.25 rows an expert) in problems of 64 / 32 / 16: 17430 / 16610 / 15270; of a prompt of 701
+// (13.7): 45230 / 44680 / 44890.
+int problem_rows(int items, int E) { return items <= 8 * E ? 16 : items <= 20 * E ? 32 : 64; }
 }  // namespace
 
 int EpMoe::create(DeviceModel *model, const void *id128, int rank_, int world_, int batch_, int flags_) {
@@ -179,8 +184,9 @@ int EpMoe::create(DeviceModel *model, const void *id128, int rank_, int world_, 
     r |= alloc(&Send, (size_t)world * slot_d); r |= alloc(&Recv, (size_t)world * slot_d);
     r |= alloc(&Ret, (size_t)world * slot_r); r |= alloc(&Back, (size_t)world * slot_r);
   }
-  r |= alloc(&Sorted, (size_t)rows * 4); r |= alloc(&Counts, 32);
-  const size_t most_problems = (size_t)epr + 1 + (size_t)rows / 64 + (size_t)n / 64 + 2;   // an expert with more than 64 rows is cut into 64-row problems
+  r |= alloc(&Sorted, (size_t)rows * 4); r |= alloc(&Counts, 32); r |= alloc(&Lists, 16);
+  const int least = world == 1 ? 16 : 64;   // an expert with more rows than problem_rows() is cut into problems of that many
+  const size_t most_problems = (size_t)epr + 1 + (size_t)rows / least + (size_t)n / least + 2;
   r |= alloc(&GroupsGU, 2 * most_problems * 32); r |= alloc(&GroupsD, most_problems * 32);
   r |= alloc(&XQs, (size_t)(rows + n) * H); r |= alloc(&SQs, (size_t)(rows + n) * G * 4);
   r |= alloc(&GU, (size_t)(rows + shn) * 2 * I * 4); r |= alloc(&AQ, (size_t)(rows + shn) * I);
@@ -223,13 +229,13 @@ int emit_route(EpMoe *e, Rec &r, int L, int rows) {
   return 0;
 }
 // The experts' products over the grouped rows: problems of GroupsGU / GroupsD.
-void emit_experts(EpMoe *e, Rec &r, int front, int shared_rows, int max_rows) {   // front: rows the received items may take
+void emit_experts(EpMoe *e, Rec &r, int front, int shared_rows, int max_rows, const int32_t *lists) {   // front: rows the received items may take
   const uint32_t blocks = (uint32_t)(2 * e->sm_count);
-  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsGU, (const int32_t *)(e->Counts + 5), (const int8_t *)e->XQs, (const float *)e->SQs,
+  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsGU, lists, (const int8_t *)e->XQs, (const float *)e->SQs,
            e->GU, (int32_t)e->I, (int32_t)e->H, (int32_t)max_rows, (int32_t)(2 * e->I));
   r.launch("SiluQuantRows", (uint32_t)(front + shared_rows), (const float *)e->GU, (const int32_t *)e->Counts, e->AQ, e->ASQ, (int32_t)e->I,
            (int32_t)(e->world * e->cap), (int32_t)front);
-  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsD, (const int32_t *)(e->Counts + 6), (const int8_t *)e->AQ, (const float *)e->ASQ,
+  r.launch("Int4GemmA8TcGrouped", blocks, (const void *)e->GroupsD, lists + 1, (const int8_t *)e->AQ, (const float *)e->ASQ,
            e->Y2, (int32_t)e->H, (int32_t)e->I, (int32_t)max_rows, (int32_t)e->H);
 }
 // One rank: `rows` of its rows, no dispatch. (A dispatch buffer, its copy, the un-permute and its copy moved
@@ -237,12 +243,12 @@ void emit_experts(EpMoe *e, Rec &r, int front, int shared_rows, int max_rows) { 
 int emit_local(EpMoe *e, Rec &r, int L, int rows) {
   if (emit_route(e, r, L, rows)) return 1;
   const ExpertW *tab = (const ExpertW *)e->m->expert_tables + (size_t)L * (e->E + 1);
-  const int items = rows * e->k, shared_rows = e->shared ? rows : 0, cut = std::min(rows, 64);
+  const int items = rows * e->k, shared_rows = e->shared ? rows : 0, cut = std::min(rows, problem_rows(items, e->E));
   r.launch("EpGroupLocal", 1u, (const int32_t *)e->SelIdx, tab, e->Sorted, e->ItemDest, e->GroupsGU, e->GroupsD, e->Counts, (int32_t)rows,
-           (int32_t)e->k, (int32_t)e->E, (int32_t)e->I, (int32_t)e->cap, (int32_t)shared_rows, (int32_t)cut);
+           (int32_t)e->k, (int32_t)e->E, (int32_t)e->I, (int32_t)e->cap, (int32_t)shared_rows, (int32_t)cut, e->Lists);
   r.launch("EpGatherLocal", (uint32_t)items, (const int8_t *)e->Q8, (const float *)e->SQ, (const int32_t *)e->Sorted, e->XQs, e->SQs, (int32_t)e->H,
            (int32_t)e->k);
-  emit_experts(e, r, items, shared_rows, cut);
+  emit_experts(e, r, items, shared_rows, cut, e->Lists);
   const float *res_in = (e->flags & EP_RES_ADD) ? e->ResSum : e->Res;   // what the combine adds the experts' outputs to
   r.launch("EpCombine", (uint32_t)(rows * ((e->H + 255) / 256)), res_in, (const unsigned char *)e->Y2, (const int32_t *)e->ItemDest,
            (const float *)e->SelW, (const float *)(e->shared ? e->Ysh : nullptr), e->X, e->Res, (int32_t)e->k, (int32_t)e->H, (uint32_t)0);
@@ -282,7 +288,7 @@ int EpMoe::record_layer(int L) {
            (int32_t)64);
   r.launch("EpGather", (uint32_t)rows, (const unsigned char *)Recv, (const int32_t *)Sorted, (const int32_t *)Counts, XQs, SQs, (int32_t)H,
            (int32_t)cap, slot_d);
-  emit_experts(this, r, rows, shared ? n : 0, std::min(batch, 64));
+  emit_experts(this, r, rows, shared ? n : 0, std::min(batch, 64), Counts + 5);
   r.launch("EpScatter", (uint32_t)rows, (const float *)Y2, (const int32_t *)Sorted, (const int32_t *)Counts, Ret, (int32_t)H, slot_r);
   if (close(r) || new_list(&la)) return 1;
   r.list = la;

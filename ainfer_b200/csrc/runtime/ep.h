@@ -38,7 +38,7 @@ struct EpMoe {
   float *SelW = nullptr, *NearGap = nullptr;
   unsigned char *Send = nullptr, *Recv = nullptr, *Ret = nullptr, *Back = nullptr;
   // expert side
-  int32_t *Sorted = nullptr, *Counts = nullptr;
+  int32_t *Sorted = nullptr, *Counts = nullptr, *Lists = nullptr;
   void *GroupsGU = nullptr, *GroupsD = nullptr;   // problem lists
   int8_t *XQs = nullptr, *AQ = nullptr;
   float *SQs = nullptr, *GU = nullptr, *ASQ = nullptr, *Y2 = nullptr;
