@@ -9,15 +9,15 @@
 //     consumers across stage and layer boundaries, limited only by ring space, and stops only
 //     where the addresses depend on data (the routed experts), until the consumers have
 //     selected them;
-//   * sixteen CONSUMER warps run the stages of a layer, separated by grid-wide barriers:
+//   * sixteen CONSUMER warps run the stages of a layer, separated by grid-wide hand-overs:
 //     each stage takes its activations from global memory (L2), its weights from the ring,
-//     and writes its outputs back to global memory for the next stage.
-// So HBM traffic is decoupled from the dependency chain: while the consumers wait at a
-// barrier, the next stages' weights are already landing in shared memory.
+//     and writes its outputs back to global memory for the next stage (words, see below).
+// So HBM traffic is decoupled from the dependency chain: while the consumers wait for one
+// another, the next stages' weights are already landing in shared memory.
 //
 // Stages of a Gated DeltaNet layer (tools/decode/decode_l0.cpp:610-674 in the reference):
 //   1 norm + quantiser, in_proj qkv/z/b/a GEMV with conv / sigmoid / decay epilogues
-//   2 gated delta rule step (state in registers, read once and written once)
+//   2 gated delta rule step (state read once and written once)
 //   3 gated per-head norm + quantiser, out_proj GEMV + residual
 //   4 post norm + quantiser, router logits
 //   5 softmax top-k (every block selects for itself), expert gate/up GEMV + SiLU-mul
@@ -30,14 +30,18 @@
 // The arithmetic of every stage (operation order, reduction shapes) is that of the stand-alone
 // kernels in this directory, so the two paths give bit-identical results.
 //
-// Every wait (mbarrier, grid barrier) is bounded by a wall-clock limit: when one runs out the
+// Every wait (mbarrier, arrivals, words) is bounded by a wall-clock limit: when one runs out the
 // block sets the plan's sticky error word, no wait in the grid spins again, and the kernel
 // terminates with garbage results that the host refuses (the error word is read after the step).
 //
-// What bounds it: not HBM (0.33 ms a token of the full preset) but the chain of six stages a layer. Times of a
-// layer's stages by the stage clock, full preset, context 4096: shares of rows once per launch, epilogue operands as
-// asynchronous copies, one thread a (row, group), group scales by one reduction instruction, selection by
-// ranks and silu(z) from the projection's epilogue took a token from 2.73 to 2.08 ms.
+// What bounds it: not HBM (0.33 ms a token of the full preset) but the chain of six stages a layer, each a
+// hand-over between all blocks (await, gather: about 1500 cycles), a prologue that every block repeats and rows of
+// short loops. Per token, full preset, context 4096: 2.73 ms; 2.08 with shares of rows dealt once a
+// launch, epilogue operands as asynchronous copies, one thread a (row, group), group scales by one
+// reduction instruction, selection by ranks, silu(z) from the projection's epilogue; 1.96 with words instead of
+// barriers and fences, rolled code (instruction-cache misses 0.85 -> 0.32 M a launch of the small preset) and
+// attention with queries in registers. What was slower: the state of the delta rule in registers (unrolled: 2.03),
+// one loop over the stages with the products inlined (2.11: its registers spill), more groups quantised side by side.
 #include "../common/step_plan.h"
 #include "attention_core.cuh"
 #include "block_stages.cuh"
@@ -105,7 +109,7 @@ struct StepShared {
   volatile int32_t fail;
   int32_t nstamp[2];            // stage clock: records written so far (consumer, producer)
   Seg segs[kMaxSegs2];          // the producer warp's current segment list
-  int32_t nseg;
+  float down_recip;             // 1 / rows of the down share
 };
 static_assert(sizeof(StepShared) <= kHdrBytes, "header area");
 static_assert(sizeof(StepPlan) % 16 == 0 && sizeof(StepLayer) % 16 == 0 && sizeof(ExpertW) % 16 == 0 &&
@@ -120,6 +124,11 @@ extern __shared__ __align__(128) unsigned char step_smem[];
 #define PL (reinterpret_cast<StepShared *>(step_smem)->plan)
 
 // kClock: with the stage clock (the step without it has no trace of it).
+//
+// A layer runs every piece of code once, so code is fetched, not reused: straight code takes 1 cycle an
+// instruction from the SM's first-level cache up to about 28 KB, 3 to 4 from the next level (to 128 KB), 64 beyond
+// it, and more where it jumps. Loops are therefore rolled wherever their latency allows, and
+// what two stages share (dot_tiles, norm_quant, gather, divisions) is one function that is called.
 template <bool kClock>
 struct Step {
 
@@ -140,9 +149,8 @@ static __device__ __forceinline__ void step_fail(int code) {
   SH->fail = code;
   atomicExch(PL.error, code);
 }
-// Bounded wait on an mbarrier phase; false when it gave up (now or earlier).
-static __device__ __forceinline__ bool mbar_wait_b(uint32_t addr, uint32_t parity, int code) {
-  if (mbar_try_a(addr, parity)) return true;
+// Bounded wait on an mbarrier phase; false when it gave up (now or earlier). The loop is out of line.
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t addr, uint32_t parity, int code) {
   if (SH->fail) return false;
   const long long t0 = clock64();
 #pragma unroll 1
@@ -157,16 +165,17 @@ static __device__ __forceinline__ bool mbar_wait_b(uint32_t addr, uint32_t parit
     }
   }
 }
+static __device__ __forceinline__ bool mbar_wait_b(uint32_t addr, uint32_t parity, int code) {
+  return mbar_try_a(addr, parity) || mbar_wait_slow(addr, parity, code);
+}
 
 // Optional stage clock (plan->stage_stamps non-null): block 0 appends (id << 48 | %globaltimer)
 // records, consumer thread 0 to the first half of the buffer, the producer thread to the second.
-// Consumer ids: 1 a grid barrier was passed, 2 a stage's prologue (norm / quantiser) is done, 3 its
-// GEMV and epilogues are done, 4 the recurrence's barrier was passed, 5 the experts are selected,
-// 6 their pointer records are fetched, 20-24 inside the attention stage (chunk staged, heads
-// prepared, scores, softmax, values). Producer ids: 10-12 the tiles of the first projections, the
-// output projection and the router are issued, 13 the selection arrived, 14 / 15 the gate/up and
-// the down tiles are issued. A record costs a few hundred nanoseconds, so a stamped step is a few
-// per cent slower than the product's.
+// Consumer ids: 1 a stage's input has arrived (a gather, or the barrier of the attention), 2 its prologue (norm /
+// quantiser) is done, 3 its rows are done, 5 the experts are selected and their pointer records fetched, 20-24 inside
+// the attention stage (heads prepared, scores, softmax, values). Producer ids: 10-11 the tiles of the first projections
+// and the output projection are issued, 12 those of the router, 13 the selection arrived, 14 / 15 the gate/up and the
+// down tiles are issued. A record costs about a hundred nanoseconds.
 static __device__ __forceinline__ void stamp(int id) {
   if (kClock) stamp_now(id);
 }
@@ -207,31 +216,41 @@ static __device__ __forceinline__ void deal_all(int i) {
   int lo, hi;
   deal(total, unit, (int)blockIdx.x, (int)gridDim.x, lo, hi);
   SH->rng[i] = make_int2(lo, hi);
+  if (i == kRngDown) SH->down_recip = hi > lo ? 1.0f / (float)(hi - lo) : 0.0f;
 }
 
-// ------------------------------------------------------------------ grid barrier ---
-// Two halves, so that loads which do not depend on other blocks (recurrent state, KV rows of
-// earlier tokens, epilogue operands) can be issued between arriving and waiting.
-static __device__ __forceinline__ void grid_arrive() {
+// ---------------------------------------------------------------- arrivals ---
+// Every block counts itself once at the end of every stage. The count runs on from launch to launch.
+// Ordered: a grid barrier; not ordered: only a sign that the other blocks' words are (about to be) there.
+template <bool kOrdered>
+static __device__ __forceinline__ void arrive() {
   csync();
-  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(PL.bar_count) : "memory");
+  if (threadIdx.x == 0) {
+    if (kOrdered) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(PL.sync + STEP_BAR) : "memory");
+    else asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(PL.sync + STEP_BAR) : "memory");
+  }
 }
-// epoch: how many barriers this block has arrived at, this one included
-static __device__ __forceinline__ void grid_wait(unsigned epoch) {
-  if (threadIdx.x == 0 && !SH->fail) {
-    const unsigned target = epoch * gridDim.x;
-    const long long t0 = clock64();
+// After 64 polls in vain, and every 64th from then on. t0: clock at the 64th; returns it, or -1 when the wait
+// is over (error word set). By value: a variable whose address is taken lives in memory.
+static __device__ __noinline__ long long poll_late(unsigned n, long long t0) {
+  const long long now = clock64();
+  if (n == 64u) t0 = now;
+  if (!SH->fail) {
+    if (*(volatile int *)PL.error != 0) SH->fail = 1;
+    else if (now - t0 > kWaitCycles) step_fail(1);
+  }
+  return SH->fail ? -1 : t0;
+}
+// Until the count has reached `target`. One thread polls: the words themselves, polled by every thread
+// of every block, keep their own writers out (a router's 513 words took 5.5 us to arrive, against 1.1).
+static __device__ __noinline__ void await(unsigned target) {
+  if (threadIdx.x == 0) {
+    long long t0 = 0;
 #pragma unroll 1
-    for (unsigned i = 0;; ++i) {
-      if (ld_acquire_u32(PL.bar_count) >= target) break;
-      if ((i & 63u) == 63u) {
-        if (*(volatile int *)PL.error != 0) { SH->fail = 1; break; }
-        if (clock64() - t0 > kWaitCycles) { step_fail(1); break; }
-      }
-    }
+    for (unsigned i = 1; (int)(ld_acquire_u32(PL.sync + STEP_BAR) - target) < 0; ++i)
+      if ((i & 63u) == 0u && (t0 = poll_late(i, t0)) < 0) break;
   }
   csync();
-  stamp(1);
 }
 
 // ====================================================================== producer ===
@@ -245,9 +264,8 @@ static __device__ __forceinline__ void grid_wait(unsigned epoch) {
 // lane copies them itself before it completes the tile. `tile` is the running index of the
 // call's first tile; returns the index after its last.
 // total: rows of the list.
-static __device__ __noinline__ uint32_t prod_emit(uint32_t tile, int row_bytes, int sc_row_bytes, int total) {
+static __device__ __forceinline__ uint32_t prod_emit(uint32_t tile, int nseg, int row_bytes, int sc_row_bytes, int total) {
   const Seg *segs = SH->segs;
-  const int nseg = SH->nseg;
   const int lrpt = __ffs(kTileBytes) - __ffs(row_bytes), rpt = 1 << lrpt;   // both powers of two
   const int ntiles = (total + rpt - 1) >> lrpt;
   const uint32_t base = tile;
@@ -277,6 +295,7 @@ static __device__ __noinline__ uint32_t prod_emit(uint32_t tile, int row_bytes, 
           if (ssrc != nullptr && !sc_bulk) {
             const uint16_t *s16 = reinterpret_cast<const uint16_t *>(ssrc);
             uint16_t *d16 = reinterpret_cast<uint16_t *>(dst + kTileBytes + (size_t)rows * sc_row_bytes);
+#pragma unroll 1
             for (uint32_t i = 0; i < sb / 2; ++i) d16[i] = __ldg(s16 + i);
           }
           if (reinterpret_cast<uintptr_t>(src) & 15u) {  // cannot be copied in bulk: report, skip
@@ -296,137 +315,210 @@ static __device__ __noinline__ uint32_t prod_emit(uint32_t tile, int row_bytes, 
   return base + (uint32_t)ntiles;
 }
 
-// Segment list of rows [lo, hi) of a table of matrices whose rows are numbered end to end
-// (written by lane 0 of the producer warp).
-static __device__ __forceinline__ void segs_gemv(const GemvMat *m, int nm, int K, int lo, int hi) {
-  if ((threadIdx.x & 31) == 0) {
-    Seg *out = SH->segs;
-    int n = 0, rs = 0;
-    for (int i = 0; i < nm; ++i) {
-      const int N = m[i].N;
-      const int a = lo > rs ? lo : rs, b = hi < rs + N ? hi : rs + N;
-      if (a < b) {
-        out[n].P = m[i].P + (size_t)(a - rs) * (K >> 1);
-        out[n].S = reinterpret_cast<const uint8_t *>(m[i].S + (size_t)(a - rs) * (K >> 7));
-        out[n].nrows = b - a;
-        out[n].vec = 0;
-        out[n].trow = a - lo;
-        ++n;
-      }
-      rs += N;
-    }
-    SH->nseg = n;
-  }
-  __syncwarp();
-}
-
-static __device__ __noinline__ uint32_t prod_gemv(uint32_t tile, const GemvMat *m, int nm, int K, int rng) {
-  const int2 r = SH->rng[rng];
-  segs_gemv(m, nm, K, r.x, r.y);
-  return prod_emit(tile, K >> 1, (K >> 7) * 2, r.y - r.x);
-}
-
-// The producer warp's whole token. Returns the number of tiles issued.
+// The producer warp's whole token: the lists of a layer's five streams one after the other, a lane a
+// segment. Returns the number of tiles issued.
 static __device__ __noinline__ uint32_t producer_main(int mode) {
   const StepPlan &P = PL;
-  const int H = P.H, lane = threadIdx.x & 31, lgI = __ffs(P.I) - 1;
-  const bool lead = lane == 0;
+  const int H = P.H, I = P.I, lane = threadIdx.x & 31, lgI = __ffs(I) - 1;
   uint32_t tile = 0;
-  for (int L = 0; L < P.layers; ++L) {
+#pragma unroll 1
+  for (int L = 0; L < P.layers + (mode != 0 ? 1 : 0); ++L) {
     const StepLayer &ly = P.L[L];
-    const bool lin = ly.type == 0;
-    tile = prod_gemv(tile, &ly.m[0], lin ? 4 : 3, H, kRngIn + ly.type);
-    stamp(10);
-    tile = prod_gemv(tile, &ly.m[4], 1, lin ? P.nV * 128 : P.nQ * 256, kRngOut + ly.type);
-    stamp(11);
-    {  // router rows (bf16) and the shared-expert gate row
-      const int lo = SH->rng[kRngRouter].x, hi = SH->rng[kRngRouter].y;
-      if (lead) {
-        Seg *segs = SH->segs;
-        int n = 0;
+#pragma unroll 1
+    for (int job = 0; job < 5; ++job) {
+      const bool head = L == P.layers;
+      // first projections (or LM head) | output projection | router and shared-expert gate | gate and up | down
+      const int type = head ? 0 : ly.type;
+      const int2 rows = SH->rng[head ? kRngHead : job == 0 ? kRngIn + type : job == 1 ? kRngOut + type : kRngRouter + job - 2];
+      const int lo = rows.x, hi = rows.y;
+      int K = H, nseg = 0, total = hi - lo;
+      Seg sg = Seg{nullptr, nullptr, 0, 0, 0, 0};
+      if (job < 2) {
+        const GemvMat *m = head ? &P.lm_head : &ly.m[job * 4];
+        nseg = job == 1 || head ? 1 : type == 0 ? 4 : 3;
+        if (job == 1) K = type == 0 ? P.nV * 128 : P.nQ * 256;
+        if (lane < nseg) {
+          int rs = 0;
+          for (int i = 0; i < lane; ++i) rs += m[i].N;
+          const int N = m[lane].N, a = lo > rs ? lo : rs, b = hi < rs + N ? hi : rs + N;
+          if (a < b) sg = Seg{m[lane].P + (size_t)(a - rs) * (K >> 1), reinterpret_cast<const uint8_t *>(m[lane].S + (size_t)(a - rs) * (K >> 7)), b - a, 0, 0, 0};
+        }
+      } else if (job == 2) {   // bf16 rows
+        nseg = 2;
         const int b = hi < P.E ? hi : P.E;
-        if (lo < b) segs[n++] = Seg{reinterpret_cast<const uint8_t *>(ly.router + (size_t)lo * H), nullptr, b - lo, 0, 0, 0};
-        if (hi > P.E) segs[n++] = Seg{reinterpret_cast<const uint8_t *>(ly.shared_gate), nullptr, 1, 0, P.E - lo, 0};
-        SH->nseg = n;
-      }
-      __syncwarp();
-      tile = prod_emit(tile, H * 2, 0, hi - lo);
-    }
-    // the expert weights depend on the routing: wait for the consumers' selection
-    stamp(12);
-    if (!mbar_wait_b(smem_addr(&SH->sel_bar), (uint32_t)L & 1u, 4)) return tile;
-    stamp(13);
-    {  // gate and up rows of pair rows [lo, hi) over slots x I: lane l writes the two segments of the l-th slot
-      const int lo = SH->rng[kRngGateUp].x, hi = SH->rng[kRngGateUp].y;
-      int n = 0;
-      if (lo < hi) {
-        const int s0 = lo >> lgI, s = s0 + lane;
-        n = ((hi - 1) >> lgI) - s0 + 1;
-        if (lane < n) {
-          const int a = lo > s * P.I ? lo : s * P.I, b = hi < (s + 1) * P.I ? hi : (s + 1) * P.I;
-          const ExpertW &ew = SH->sew[s];
-          const size_t r0 = (size_t)(a - s * P.I);
-          SH->segs[2 * lane] = Seg{ew.gP + r0 * (H >> 1), reinterpret_cast<const uint8_t *>(ew.gS + r0 * (H >> 7)), b - a, 0, a - lo, 0};
-          SH->segs[2 * lane + 1] = Seg{ew.uP + r0 * (H >> 1), reinterpret_cast<const uint8_t *>(ew.uS + r0 * (H >> 7)), b - a, 0,
-                                       (hi - lo) + (a - lo), 0};
+        if (lane == 0 && lo < b) sg = Seg{reinterpret_cast<const uint8_t *>(ly.router + (size_t)lo * H), nullptr, b - lo, 0, 0, 0};
+        if (lane == 1 && hi > P.E) sg = Seg{reinterpret_cast<const uint8_t *>(ly.shared_gate), nullptr, 1, 0, 0, 0};
+      } else if (job == 3) {   // pair rows [lo, hi) over slots x I: a slot's gate rows, then its up rows
+        stamp(12);
+        // the expert weights depend on the routing: wait for the consumers' selection
+        if (!mbar_wait_b(smem_addr(&SH->sel_bar), (uint32_t)L & 1u, 4)) return tile;
+        stamp(13);
+        total = 2 * (hi - lo);
+        if (lo < hi) {
+          const int s0 = lo >> lgI, s = s0 + (lane >> 1);
+          nseg = 2 * (((hi - 1) >> lgI) - s0 + 1);
+          if (lane < nseg) {
+            const int a = lo > s * I ? lo : s * I, b = hi < (s + 1) * I ? hi : (s + 1) * I;
+            const ExpertW &ew = SH->sew[s];
+            const size_t r0 = (size_t)(a - s * I);
+            sg = Seg{((lane & 1) ? ew.uP : ew.gP) + r0 * (H >> 1), reinterpret_cast<const uint8_t *>(((lane & 1) ? ew.uS : ew.gS) + r0 * (H >> 7)), b - a, 0, 0, 0};
+          }
+        }
+      } else {   // down rows [lo, hi) of every slot
+        K = I;
+        nseg = P.slots;
+        total = P.slots * (hi - lo);
+        if (lane < nseg) {
+          const ExpertW &ew = SH->sew[lane];
+          sg = Seg{ew.dP + (size_t)lo * (I >> 1), reinterpret_cast<const uint8_t *>(ew.dS + (size_t)lo * (I >> 7)), hi - lo, 0, 0, 0};
         }
       }
-      if (lead) SH->nseg = 2 * n;
+      if (lane < nseg) SH->segs[lane] = sg;
       __syncwarp();
-      tile = prod_emit(tile, H >> 1, (H >> 7) * 2, 2 * (hi - lo));
+      tile = prod_emit(tile, nseg, job == 2 ? H * 2 : K >> 1, job == 2 ? 0 : (K >> 7) * 2, total);
+      stamp(job < 2 ? 10 + job : 11 + job);
+      if (head) break;
     }
-    stamp(14);
-    {  // down rows [lo, hi) of every slot
-      const int lo = SH->rng[kRngDown].x, nr = SH->rng[kRngDown].y - lo;
-      if (lane < P.slots) {
-        const ExpertW &ew = SH->sew[lane];
-        SH->segs[lane] = Seg{ew.dP + (size_t)lo * (P.I >> 1), reinterpret_cast<const uint8_t *>(ew.dS + (size_t)lo * (P.I >> 7)),
-                             nr, lane, lane * nr, 0};
-      }
-      if (lead) SH->nseg = nr > 0 ? P.slots : 0;
-      __syncwarp();
-      tile = prod_emit(tile, P.I >> 1, (P.I >> 7) * 2, P.slots * nr);
-    }
-    stamp(15);
   }
-  if (mode != 0) tile = prod_gemv(tile, &P.lm_head, 1, H, kRngHead);
   return tile;
 }
 
+// ======================================================== words between blocks ===
+// What one stage hands to the next crosses the grid as 64-bit words of a value and a flag (the
+// launch's and layer's number). A word is one access, so the value is there when the flag is, and the
+// writer needs no fence in front of its arrival. Nothing else is ordered, and no
+// stage reads anything of another block in any other way (the chunk partials of the attention, too many
+// for words of twice their size, keep a barrier). Words alternate between two sets by layer: a
+// block writes layer L + 2's only after it has read words that depend on every block's rows of layer L + 1's first
+// stage (the host deals at least one to each), which a block computes after its last read of layer L.
+static __device__ __forceinline__ void put(unsigned long long *p, float v, unsigned flag) {
+  asm volatile("{\n\t.reg .b64 w;\n\tmov.b64 w, {%1, %2};\n\tst.relaxed.gpu.global.b64 [%0], w;\n\t}" ::"l"(p),
+               "r"(__float_as_uint(v)), "r"(flag)
+               : "memory");
+}
+// One word.
+static __device__ __forceinline__ float take(const unsigned long long *p, unsigned flag) {
+  unsigned v, f, n = 0;
+  long long t0 = 0;
+#pragma unroll 1
+  while (true) {
+    asm volatile("{\n\t.reg .b64 w;\n\tld.relaxed.gpu.global.b64 w, [%2];\n\tmov.b64 {%0, %1}, w;\n\t}" : "=r"(v), "=r"(f) : "l"(p) : "memory");
+    if (f == flag) break;
+    if ((++n & 63u) == 0u && (t0 = poll_late(n, t0)) < 0) break;
+  }
+  return __uint_as_float(v);
+}
+// Eight words 32 apart, all in flight together.
+static __device__ __forceinline__ void take8(float (&x)[8], const unsigned long long *p, unsigned flag) {
+  unsigned n = 0;
+  long long t0 = 0;
+#pragma unroll 1
+  while (true) {
+    unsigned f[8];
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      asm volatile("{\n\t.reg .b64 w;\n\tld.relaxed.gpu.global.b64 w, [%2];\n\tmov.b64 {%0, %1}, w;\n\t}"
+                   : "=f"(x[i]), "=r"(f[i])
+                   : "l"(p + 32 * i)
+                   : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ok = ok && f[i] == flag;
+    if (ok || ((++n & 63u) == 0u && (t0 = poll_late(n, t0)) < 0)) break;
+  }
+}
+// n consecutive words (16-byte aligned) into shared memory, by the whole consumer group: up to four
+// pairs a thread in flight. The caller synchronises.
+static __device__ __noinline__ void gather(float *dst, const unsigned long long *src, int n, unsigned flag) {
+  unsigned tries = 0;
+  long long t0 = 0;
+#pragma unroll 1
+  for (int w = 2 * (int)threadIdx.x; w < n; w += 4 * kCons) {
+    unsigned v0[2], f0[2], v1[2], f1[2];
+#pragma unroll 1
+    while (true) {
+      bool ok = true;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        f0[u] = f1[u] = flag;
+        if (w + 2 * kCons * u < n)
+          asm volatile("{\n\t.reg .b64 a, b;\n\tld.relaxed.gpu.global.v2.b64 {a, b}, [%4];\n\tmov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, b;\n\t}"
+                       : "=r"(v0[u]), "=r"(f0[u]), "=r"(v1[u]), "=r"(f1[u])
+                       : "l"(src + w + 2 * kCons * u)
+                       : "memory");
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) ok = ok && f0[u] == flag && (f1[u] == flag || w + 2 * kCons * u + 1 >= n);
+      if (ok) break;
+      if ((++tries & 63u) == 0u && (t0 = poll_late(tries, t0)) < 0) break;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (w + 2 * kCons * u < n) *reinterpret_cast<uint2 *>(dst + w + 2 * kCons * u) = make_uint2(v0[u], v1[u]);
+  }
+}
+
+// num / (1 + exp(arg)) and 1 / sqrt(x): one copy each, see Step.
+static __device__ __noinline__ float over_exp(float num, float arg) { return num / (1.0f + det_expf(arg)); }
+static __device__ __noinline__ float inv_sqrt(float x) { return 1.0f / sqrtf(x); }
+
 // ====================================================================== consumers ===
+// Group terms of a stage's rows: t[row][g], 4-term pieces in an order that turns with the row, so that
+// the thread that adds a row's terms reads them four at a time.
+static __device__ __forceinline__ int term_index(int row, int g, int lg) {
+  return lg >= 2 ? (row << lg) + ((((g >> 2) ^ row) & ((1 << (lg - 2)) - 1)) << 2) + (g & 3) : (row << lg) + g;
+}
+// Sum of one row's group terms in ascending group order.
+static __device__ __forceinline__ float row_terms(const float *T, int row, int lg) {
+  float acc = 0.0f;
+  if (lg >= 2) {
+    const float4 *t = reinterpret_cast<const float4 *>(T + (row << lg));
+    const int n = 1 << (lg - 2);
+    float4 v = t[row & (n - 1)];
+#pragma unroll 1
+    for (int i = 1; i <= n; ++i) {
+      const float4 c = v;
+      if (i < n) v = t[(i ^ row) & (n - 1)];
+      acc = acc + c.x;
+      acc = acc + c.y;
+      acc = acc + c.z;
+      acc = acc + c.w;
+    }
+  } else {
+#pragma unroll 1
+    for (int g = 0; g < 1 << lg; ++g) acc = acc + T[(row << lg) + g];
+  }
+  return acc;
+}
+
 // Dots the next tiles of a stage with staged activations: nrows rows in the order the producer
 // streams them (tile j of the call holds rows [j * rpt, (j + 1) * rpt)). Row f is dotted with
-// activation vector f / vec_rows (kVecs; otherwise always vector 0) and its group terms go to
-// t[g][f]. Starts at running tile index `tile`; returns the index after the last tile. A tile is 256 (row, group) tasks of 64 bytes, one a thread: the two halves of the
-// consumers take alternate tiles, so that every wait, scale and store serves 64 bytes and two
-// tiles are in work at once. A thread reads its 64 bytes in a lane-rotated order that keeps every
-// quarter-warp on distinct banks.
-template <bool kVecs>
-static __device__ __forceinline__ uint32_t dot_tiles(uint32_t tile, int lg, const uint4 *xa, const float *sq, float *T,
-                                                     int nrows, int vec_rows) {
-  const int G = 1 << lg, TS = (kTCap >> lg) + 1, rpt = 256 >> lg;
+// activation vector floor((f + 1/2) vec_recip), vec_recip = 1 / rows of a vector (f < 4096: the error, 2^-22 of the quotient,
+// is far below the half row), and its group terms go to t[f][]. Starts at
+// running tile index `tile`; returns the index after the last tile. A tile is 256 (row, group) tasks of
+// 64 bytes, one a thread: the two halves of the consumers take alternate tiles, so that every
+// wait, scale and store serves 64 bytes and two tiles are in work at once. A thread reads its 64
+// bytes in a lane-rotated order that keeps every quarter-warp on distinct banks. Not inlined: see Step.
+static __device__ __noinline__ uint32_t dot_tiles(uint32_t tile, int lg, int sq_off, int nrows, float vec_recip) {
+  const uint4 *xa = reinterpret_cast<const uint4 *>(step_smem + kActOff);
+  const float *sq = reinterpret_cast<const float *>(step_smem + kActOff + sq_off);
+  float *T = reinterpret_cast<float *>(step_smem + kTOff);
+  const int G = 1 << lg, rpt = 256 >> lg;
   const int t = threadIdx.x & 255, half = threadIdx.x >> 8, lane = threadIdx.x & 31;
   const int r = t >> lg, g = t & (G - 1), rot = (t >> 1) & 3;
   const uint32_t ring_a = smem_addr(step_smem + kRingOff);
   const int ntiles = (nrows + rpt - 1) >> (8 - lg);
   uint4 x[8];
   float sqg = 0.0f;
-  if (!kVecs) {
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int q = 2 * ((s + rot) & 3);
-      x[2 * s] = xa[q * G + g];
-      x[2 * s + 1] = xa[(q + 1) * G + g];
-    }
-    sqg = sq[g];
-  }
+  int cvec = -1;
 #pragma unroll 1
   for (int j = half; j < ntiles; j += 2) {
     const uint32_t idx = tile + (uint32_t)j, slot = idx % kNT, use = idx / kNT;
     const int f = j * rpt + r;
     const bool live = f < nrows;
-    if (kVecs) {
-      const int vec = live ? (int)((unsigned)f / (unsigned)vec_rows) : 0;
+    const int vec = live ? (int)(((float)f + 0.5f) * vec_recip) : 0;
+    if (vec != cvec) {
+      cvec = vec;
       const uint4 *xv = xa + (size_t)vec * 8 * G + g;
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
@@ -451,38 +543,10 @@ static __device__ __forceinline__ uint32_t dot_tiles(uint32_t tile, int lg, cons
     __syncwarp();
     if (lane == 0) mbar_arrive_a(smem_addr(&SH->empty[slot]));
     const float v = (float)(((d0 + d1) + (d2 + d3)) >> 4) * __uint_as_float(sraw << 16);
-    if (live) T[g * TS + f] = v * sqg;
+    if (live) T[term_index(f, g, lg)] = v * sqg;
   }
+  csync();
   return tile + (uint32_t)ntiles;
-}
-
-// Sum of one row's group terms in ascending group order, the loads of up to eight terms ahead of the additions.
-static __device__ __forceinline__ float row_terms(const float *T, int row, int lg) {
-  const int G = 1 << lg, TS = (kTCap >> lg) + 1;
-  const float *t = T + row;
-  float acc = 0.0f;
-  if (G >= 8) {
-    float v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = t[i * TS];
-#pragma unroll 1
-    for (int g = 8; g < G; g += 8) {
-      float n[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) n[i] = t[(g + i) * TS];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        acc = acc + v[i];
-        v[i] = n[i];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc = acc + v[i];
-  } else {
-#pragma unroll 1
-    for (int g = 0; g < G; ++g) acc = acc + t[g * TS];
-  }
-  return acc;
 }
 
 // Largest magnitude of the warp's values (one instruction; NaNs do not count, as with fmaxf).
@@ -491,25 +555,32 @@ static __device__ __forceinline__ float warp_absmax(float v) {
   asm volatile("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
-// Scale of a group of 128 values, four a lane (ScalesMax, tools/cmdlist/kernels.cpp:551-566).
-static __device__ __forceinline__ float group_scale(const float4 &v) {
-  const float mx = warp_absmax(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-  const float s = mx / 127.0f;
-  return s == 0.0f ? 1.0f : s;
+static __device__ __forceinline__ float warp_largest(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
 }
-// Four values' bytes under scale s, r = quant_recip(s): quant_round()'s integers. With q = x/s, |q| <=
-// 127 (1 + 2^-24): x r is within 127 x 2^-23 = 1.53e-5 of q and the rounded quotient within 0.76e-5, so
-// they differ by at most 2.3e-5, and after the addition of one half (rounded to 2^-17 at most, twice)
-// by 3.1e-5: unless |x r| + 0.5 is within 4e-5 of a whole number both truncate alike. There, and for a
-// scale without a finite reciprocal, the division itself decides.
-static __device__ __forceinline__ uint32_t quant4(const float4 &v, float s, float r) {
+// Quantises one group of 128 values held four a lane: (bytes, scale bits); scale s = largest / 127 (ScalesMax +
+// Quantize, tools/cmdlist/kernels.cpp:551-579), the bytes quant_round()'s integers, from the
+// approximate reciprocal r of s, 127 x rcp(largest), which is there before s is. With q = x/s, |q| <= 127 (1 + 2^-24):
+// r is within 2^-22 of 1/s (one ulp of rcp, the product, the rounding of s), so x r within 3.8e-5 of q, rounded
+// to 0.76e-5; the rounded quotient is within 0.76e-5 of q; and the addition of one half rounds to 2^-17 at
+// most, twice: in all 6.1e-5. Unless |x r| + 0.5 is within 8e-5 of a whole number both truncate alike; there, and for an r that
+// is not well inside the range, the division itself decides.
+static __device__ __noinline__ uint2 quant_group(float4 v) {
+  const float mx = warp_absmax(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(mx));
+  r = r * 127.0f;
+  float s = mx / 127.0f;
+  if (s == 0.0f) s = 1.0f;
   const float x[4] = {v.x, v.y, v.z, v.w};
   uint32_t out = 0;
-  bool sure = r != 0.0f;
+  bool sure = r > 1e-30f && r < 1e30f;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float vp = x[i] * r, t = fabsf(vp) + 0.5f, w = truncf(t), f = t - w;
-    sure = sure && f >= 4e-5f && f <= 0.99996f;
+    sure = sure && f >= 8e-5f && f <= 0.99992f;
     int q = (int)w;
     q = q > 127 ? 127 : q;
     q = vp < 0.0f ? -q : q;
@@ -523,19 +594,17 @@ static __device__ __forceinline__ uint32_t quant4(const float4 &v, float s, floa
       out = (out << 8) | (uint32_t)(quant_round(xi, s) & 0xFF);
     }
   }
-  return out;
+  return make_uint2(out, __float_as_uint(s));
 }
-// Quantises one group of 128 values held four a lane into the staged form (quant_group_staged()'s result).
-static __device__ __forceinline__ void stage_group(uint32_t *xw, float *sqs, int G, int m, int g, const float4 &v) {
+// A group's bytes into the staged form (quant_group_staged()'s result).
+static __device__ __forceinline__ void stage_group(uint32_t *xw, float *sqs, int G, int m, int g, const uint2 &qs) {
   const int lane = threadIdx.x & 31;
-  const float s = group_scale(v);
-  const uint32_t own = quant4(v, s, quant_recip(s));
-  const uint32_t other = __shfl_xor_sync(kFull, own, 1);
+  const uint32_t own = qs.x, other = __shfl_xor_sync(kFull, own, 1);
   const int i = lane >> 1;  // 8-weight piece of the group: two lanes of 4 weights each
   uint32_t *dst = xw + ((((m * 8 + (i >> 1)) * G + g) << 2) + ((i & 1) << 1));
   if (lane & 1) dst[1] = __byte_perm(other, own, 0x7531);
   else dst[0] = __byte_perm(own, other, 0x6420);
-  if (lane == 0) sqs[m * G + g] = s;
+  if (lane == 0) sqs[m * G + g] = __uint_as_float(qs.y);
 }
 
 // (1+w) RMSNorm + per-128 quantiser of one H-vector into the staged form, by the whole
@@ -546,44 +615,35 @@ static __device__ __forceinline__ void stage_group(uint32_t *xw, float *sqs, int
 // itself from the 256 partial sums in shared memory (lane l: ((p[l]+p[l+128]) + (p[l+64]+
 // p[l+192])) + ((p[l+32]+p[l+160]) + (p[l+96]+p[l+224]))) and whose last five levels are the xor
 // butterfly. The mean is a product: H is a power of two.
-// Waits for barrier `epoch` first (0: none), after the loads that do not depend on it.
-// src: fp32 vector in global memory, or (emb != null) a bf16 embedding row. hn (optional): the
-// normalised fp32 vector, shared memory. xout (optional): copy of the input, global.
-static __device__ __forceinline__ void norm_quant(unsigned epoch, const float *src, const uint16_t *emb, const float *w, int H,
-                                               float *hn, float *xout) {
-  float *xs = reinterpret_cast<float *>(step_smem + kFbufOff);
+// src: the vector's words, or (emb != null) a bf16 embedding row. hn: the normalised fp32 vector,
+// shared memory. Returns the input at row rows.x + thread, for the threads below rows.y - rows.x: the
+// residual of a later stage.
+static __device__ __noinline__ float norm_quant(unsigned target, const unsigned long long *src, unsigned flag, const uint16_t *emb,
+                                                const float *w, int H, int2 rows) {
+  float *xs = reinterpret_cast<float *>(step_smem + kFbufOff), *hn = xs + 4096;
   double *ps = reinterpret_cast<double *>(step_smem + kTOff);
   unsigned char *act = step_smem + kActOff;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, G = H >> 7, n = H >> 8;
-  float4 wv[2];  // H <= 4096: the weights of this warp's groups (at most two)
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int g = warp + 16 * i;
-    wv[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (g < G) wv[i] = __ldg(reinterpret_cast<const float4 *>(w + g * 128) + lane);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, G = H >> 7;
+  float4 wv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (warp < G) wv = __ldg(reinterpret_cast<const float4 *>(w + warp * 128) + lane);
+  if (emb) {
+#pragma unroll 1
+    for (int j = tid; j < H; j += kCons) xs[j] = u2f((uint32_t)__ldg(emb + j) << 16);
+  } else {
+    await(target);
+    gather(xs, src, H, flag);
   }
-  if (epoch) grid_wait(epoch);
+  csync();
+  stamp(1);
   if (tid < 256) {
     double ss = 0;
 #pragma unroll 1
-    for (int i0 = 0; i0 < n; i0 += 8) {
-      float v[8];
+    for (int j = tid; j < H; j += 1024) {   // four loads ahead of the chain (H >= 1024: all of them in range)
+      float v[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        v[i] = 0.0f;
-        if (i0 + i < n) {
-          const int e = tid + 256 * (i0 + i);
-          v[i] = emb ? u2f((uint32_t)__ldg(emb + e) << 16) : __ldcg(src + e);
-        }
-      }
+      for (int i = 0; i < 4; ++i) v[i] = j + 256 * i < H ? xs[j + 256 * i] : 0.0f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (i0 + i < n) {
-          const int e = tid + 256 * (i0 + i);
-          xs[e] = v[i];
-          if (xout) xout[e] = v[i];
-          ss = fma((double)v[i], (double)v[i], ss);
-        }
+      for (int i = 0; i < 4; ++i) ss = fma((double)v[i], (double)v[i], ss);
     }
     ps[tid] = ss;
   }
@@ -593,117 +653,71 @@ static __device__ __forceinline__ void norm_quant(unsigned epoch, const float *s
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) t = t + __shfl_xor_sync(kFull, t, off);
   const double rH = __hiloint2double((1023 - (__ffs(H) - 1)) << 20, 0);
-  const float inv = 1.0f / sqrtf((float)(t * rH) + PL.eps);
-  uint32_t *xw = reinterpret_cast<uint32_t *>(act);
-  float *sqs = reinterpret_cast<float *>(act + H);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int g = warp + 16 * i;
-    if (g < G) {
-      const int j = g * 128 + lane * 4;
-      const float4 x = *reinterpret_cast<const float4 *>(xs + j);
-      float4 y;
-      y.x = (x.x * inv) * (1.0f + wv[i].x);
-      y.y = (x.y * inv) * (1.0f + wv[i].y);
-      y.z = (x.z * inv) * (1.0f + wv[i].z);
-      y.w = (x.w * inv) * (1.0f + wv[i].w);
-      if (hn) *reinterpret_cast<float4 *>(hn + j) = y;
-      stage_group(xw, sqs, G, 0, g, y);
-    }
+  const float inv = inv_sqrt((float)(t * rH) + PL.eps);
+#pragma unroll 1
+  for (int g = warp; g < G; g += 16) {
+    const int j = g * 128 + lane * 4;
+    const float4 x = *reinterpret_cast<const float4 *>(xs + j);
+    float4 y;
+    y.x = (x.x * inv) * (1.0f + wv.x);
+    y.y = (x.y * inv) * (1.0f + wv.y);
+    y.z = (x.z * inv) * (1.0f + wv.z);
+    y.w = (x.w * inv) * (1.0f + wv.w);
+    if (g + 16 < G) wv = __ldg(reinterpret_cast<const float4 *>(w + (g + 16) * 128) + lane);
+    *reinterpret_cast<float4 *>(hn + j) = y;
+    stage_group(reinterpret_cast<uint32_t *>(act), reinterpret_cast<float *>(act + H), G, 0, g, quant_group(y));
   }
+  const float res = tid < rows.y - rows.x ? xs[rows.x + tid] : 0.0f;
   csync();
-}
-
-// Stages an already quantised vector (INT8 + group scales in global memory).
-static __device__ __forceinline__ void stage_q8(const int8_t *xq, const float *sqg, int K) {
-  unsigned char *act = step_smem + kActOff;
-  uint32_t *xw = reinterpret_cast<uint32_t *>(act);
-  float *sqs = reinterpret_cast<float *>(act + K);
-  const int G = K >> 7;
-  for (int pc = threadIdx.x; pc < K / 8; pc += kCons) {
-    const uint2 v = __ldcg(reinterpret_cast<const uint2 *>(xq + (size_t)pc * 8));
-    const int g = pc >> 4, i = pc & 15;
-    uint32_t *dst = xw + ((((i >> 1) * G + g) << 2) + ((i & 1) << 1));
-    dst[0] = __byte_perm(v.x, v.y, 0x6420);
-    dst[1] = __byte_perm(v.x, v.y, 0x7531);
-  }
-  for (int g = threadIdx.x; g < G; g += kCons) sqs[g] = __ldcg(sqg + g);
-  csync();
-}
-
-// Quantises M contiguous fp32 vectors of K (global memory, M * K <= 8192) into the staged form: a
-// warp takes whole groups, and the loads of its (at most four) groups are in flight together.
-static __device__ __forceinline__ void quant_rows(const float *x, int lgG, int M) {
-  unsigned char *act = step_smem + kActOff;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = 1 << lgG, n = M << lgG;
-  uint32_t *xw = reinterpret_cast<uint32_t *>(act);
-  float *sqs = reinterpret_cast<float *>(act + (size_t)n * 128);
-  float4 v[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int gi = warp + 16 * u;
-    v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (gi < n) v[u] = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)gi * 128) + lane);
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int gi = warp + 16 * u;
-    if (gi < n) stage_group(xw, sqs, G, gi >> lgG, gi & (G - 1), v[u]);
-  }
-  csync();
+  stamp(2);
+  return res;
 }
 
 // Gated per-head norm + quantiser (RmsInv + NormGated + ScalesMax + Quantize,
-// kernels.cpp:619-644,551-579) into the staged form (K = nV * 128 <= 4096): a warp takes whole heads,
-// at most two, side by side. Zs holds silu(z): the projection's epilogue has it from one thread a row,
-// where every block would evaluate nV * 128 exponentials here. Lane l holds values l, l + 32, l + 64 and
+// kernels.cpp:619-644,551-579) into the staged form (K = nV * 128 <= 4096), a warp a head. The
+// words of z hold silu(z): the projection's epilogue has it from one thread a row,
+// where every block would evaluate nV * 128 exponentials here. Lane l takes values l, l + 32, l + 64 and
 // l + 96 of a head, the terms of its sum of squares.
-static __device__ __forceinline__ void gated_norm_quant(unsigned epoch, const float *O, const float *Zs, const float *W, int nV) {
+static __device__ __forceinline__ void gated_norm_quant(unsigned target, const unsigned long long *O, const unsigned long long *Zs,
+                                                        unsigned flag, const float *W, int nV) {
+  float *os = reinterpret_cast<float *>(step_smem + kFbufOff), *zs = os + 4096;
   unsigned char *act = step_smem + kActOff;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float wn[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) wn[i] = __ldg(W + lane + 32 * i);
-  grid_wait(epoch);
-  float o[2][4], z[2][4];
-#pragma unroll
-  for (int u = 0; u < 2; ++u)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int h = warp + 16 * u, e = h * 128 + lane + 32 * i;
-      o[u][i] = 0.0f;
-      z[u][i] = 0.0f;
-      if (h < nV) {
-        o[u][i] = __ldcg(O + e);
-        z[u][i] = __ldcg(Zs + e);
-      }
-    }
+  gather(zs, Zs, nV * 128, flag);   // complete since the recurrence's inputs were
+  await(target);
+  gather(os, O, nV * 128, flag);
+  csync();
+  stamp(1);
   int8_t *xb = reinterpret_cast<int8_t *>(act);
   float *sqs = reinterpret_cast<float *>(act + nV * 128);
+#pragma unroll 1
+  for (int h = warp; h < nV; h += 16) {
+    float o[4], z[4], ss = 0.0f;
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int h = warp + 16 * u;
-    if (h < nV) {
-      float ss = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ss = fmaf(o[u][i], o[u][i], ss);
-      ss = warp_tree_sum(ss);
-      const float inv = 1.0f / sqrtf(ss / 128.0f + PL.eps);
-      float4 y;
-      y.x = ((wn[0] * o[u][0]) * inv) * z[u][0];
-      y.y = ((wn[1] * o[u][1]) * inv) * z[u][1];
-      y.z = ((wn[2] * o[u][2]) * inv) * z[u][2];
-      y.w = ((wn[3] * o[u][3]) * inv) * z[u][3];
-      const float s = group_scale(y);
-      const uint32_t q = quant4(y, s, quant_recip(s));
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // value k of the group: piece k / 8 (two words: even and odd values), byte (k % 8) / 2 of its word
-        const int k = lane + 32 * i, pc = k >> 3;
-        xb[((((pc >> 1) * nV + h) << 2) + ((pc & 1) << 1) + (k & 1)) * 4 + ((k & 7) >> 1)] = (int8_t)(q >> (8 * i));
-      }
-      if (lane == 0) sqs[h] = s;
+    for (int i = 0; i < 4; ++i) {
+      o[i] = os[h * 128 + lane + 32 * i];
+      z[i] = zs[h * 128 + lane + 32 * i];
+      ss = fmaf(o[i], o[i], ss);
     }
+    ss = warp_tree_sum(ss);
+    const float inv = inv_sqrt(ss * 0.0078125f + PL.eps);
+    float4 y;
+    y.x = ((wn[0] * o[0]) * inv) * z[0];
+    y.y = ((wn[1] * o[1]) * inv) * z[1];
+    y.z = ((wn[2] * o[2]) * inv) * z[2];
+    y.w = ((wn[3] * o[3]) * inv) * z[3];
+    const uint2 qs = quant_group(y);
+    const uint32_t q = qs.x;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      // value k of the group: piece k / 8 (two words: even and odd values), byte (k % 8) / 2 of its word
+      const int k = lane + 32 * i, pc = k >> 3;
+      xb[((((pc >> 1) * nV + h) << 2) + ((pc & 1) << 1) + (k & 1)) * 4 + ((k & 7) >> 1)] = (int8_t)(q >> (8 * i));
+    }
+    if (lane == 0) sqs[h] = __uint_as_float(qs.y);
   }
   csync();
 }
@@ -711,6 +725,7 @@ static __device__ __forceinline__ void gated_norm_quant(unsigned epoch, const fl
 // Matrix and local row of flat row `flat` of a table of matrices.
 static __device__ __forceinline__ int mat_of_row(const GemvMat *m, int nm, int flat, int &n) {
   int rs = 0, i = 0;
+#pragma unroll 1
   while (i < nm - 1 && flat >= rs + m[i].N) {
     rs += m[i].N;
     ++i;
@@ -722,16 +737,19 @@ static __device__ __forceinline__ int mat_of_row(const GemvMat *m, int nm, int f
 // Operands of a row's epilogue that do not depend on its dot product: 32 bytes of shared memory a row,
 // under way during the dot as asynchronous copies (registers that wait for them would be spilled, and the
 // spill would wait): convolution taps [0..3] and history [4..6], or decay constants [4], [5]. All of
-// them are read once a launch, so that no cached line is older than they are; the residual, which
-// other blocks write during the launch, is a plain load past the cache into `res`.
+// them are read once a launch, so that no cached line is older than they are.
 static __device__ __forceinline__ void cp_async4(float *dst, const float *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
-static __device__ __forceinline__ void row_operands(const GemvMat &mt, int n, float *op, float &res) {
+static __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+static __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+static __device__ __forceinline__ void row_operands(const GemvMat &mt, int n, float *op) {
   const int epi = mt.epi;
   if (epi == EPI_CONV_SILU) {
     const float *cs = mt.e1 + (size_t)n * 3;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(op)), "l"(mt.e0 + (size_t)n * 4) : "memory");
+    cp_async16(op, mt.e0 + (size_t)n * 4);
     cp_async4(op + 4, cs);
     cp_async4(op + 5, cs + 1);
     cp_async4(op + 6, cs + 2);
@@ -740,15 +758,12 @@ static __device__ __forceinline__ void row_operands(const GemvMat &mt, int n, fl
     cp_async4(op + 4, mt.e0 + n);
     cp_async4(op + 5, mt.e2 + n);
   }
-  res = 0.0f;
-  if (epi == EPI_RESADD) res = __ldcg(mt.e0 + n);
 }
 // gemv_epilogue()'s arithmetic; every kind of row that needs an exponential of its sum shares one.
-static __device__ __forceinline__ void row_epilogue(const GemvMat &mt, int n, float acc, const float *op, float res) {
+static __device__ __forceinline__ float row_epilogue(const GemvMat &mt, int n, float acc, const float *op, float res) {
   const int epi = mt.epi;
-  float *y = mt.Y + n;
-  if (epi == EPI_STORE) { *y = acc; return; }
-  if (epi == EPI_RESADD) { *y = res + acc; return; }
+  if (epi == EPI_STORE) return acc;
+  if (epi == EPI_RESADD) return res + acc;
   float num = epi == EPI_BETA ? 1.0f : acc, arg = -acc;
   if (epi == EPI_CONV_SILU) {
     const float4 cw = *reinterpret_cast<const float4 *>(op);
@@ -765,45 +780,38 @@ static __device__ __forceinline__ void row_epilogue(const GemvMat &mt, int n, fl
     cs[2] = acc;
   }
   if (epi == EPI_GDECAY) arg = acc + op[5];
-  const float e = det_expf(arg);
-  if (epi != EPI_GDECAY) { *y = num / (1.0f + e); return; }
-  const float soft = arg > 20.0f ? arg : det_logf(1.0f + e);
-  *y = (-det_expf(op[4])) * soft;
+  if (epi != EPI_GDECAY) return over_exp(num, arg);
+  const float soft = arg > 20.0f ? arg : det_logf(1.0f + det_expf(arg));
+  return (-det_expf(op[4])) * soft;
 }
 
-// One GEMV stage: this block's rows of the matrices, activations already staged.
-static __device__ __forceinline__ uint32_t gemv_stage_run(uint32_t tile, const GemvMat *m, int nm, int K, int rng) {
-  const int lo = SH->rng[rng].x, nr = SH->rng[rng].y - lo;
-  if (nr <= 0) return tile;
-  float *T = reinterpret_cast<float *>(step_smem + kTOff), *op = reinterpret_cast<float *>(step_smem + kFbufOff) + 4096 + threadIdx.x * 8;
-  unsigned char *act = step_smem + kActOff;
+// One GEMV stage: this block's rows of the matrices, activations already staged; a matrix's Y is its
+// rows' words. res: the residual of row `thread` of the share.
+static __device__ __noinline__ uint32_t gemv_stage_run(uint32_t tile, const GemvMat *m, int nm, int K, int2 rows, unsigned flag, float res) {
+  const int lo = rows.x, nr = rows.y - lo;
+  const float *T = reinterpret_cast<const float *>(step_smem + kTOff);
+  float *op = reinterpret_cast<float *>(step_smem + kFbufOff) + 4096 + threadIdx.x * 8;
   const int lg = 31 - __clz(K >> 7);
   int mi = 0, n = 0;
-  float res = 0.0f;
   if ((int)threadIdx.x < nr) {
     mi = mat_of_row(m, nm, lo + threadIdx.x, n);
-    row_operands(m[mi], n, op, res);
+    row_operands(m[mi], n, op);
   }
-  tile = dot_tiles<false>(tile, lg, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + K), T, nr, 0);
-  csync();
-#pragma unroll 1
-  for (int r = threadIdx.x; r < nr; r += kCons) {
-    if (r >= kCons) {
-      mi = mat_of_row(m, nm, lo + r, n);
-      row_operands(m[mi], n, op, res);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");   // the thread's own copies
-    row_epilogue(m[mi], n, row_terms(T, r, lg), op, res);
+  tile = dot_tiles(tile, lg, K, nr, 0.0f);
+  if ((int)threadIdx.x < nr) {   // nr <= 512
+    cp_async_wait();   // the thread's own copies
+    put(reinterpret_cast<unsigned long long *>(m[mi].Y) + n, row_epilogue(m[mi], n, row_terms(T, threadIdx.x, lg), op, res), flag);
   }
+  stamp(3);
   return tile;
 }
 
 // Router logits of this block's rows from the ring (bf16 rows), activations hn in shared memory.
 // logits[e] = sum_k bf16(W[e][k]) * hn[k]: lane l takes k = (i*32+l)*8+j, fma chain in (i, j)
 // order, then the lane tree (as RouterTopK). Tiles go to alternate halves of the consumers, as in dot_tiles.
-static __device__ __forceinline__ uint32_t router_stage(uint32_t tile, const float *hn, int H) {
+static __device__ __forceinline__ uint32_t router_stage(uint32_t tile, unsigned long long *out, unsigned flag, int H) {
   const int lo = SH->rng[kRngRouter].x, total = SH->rng[kRngRouter].y - lo;
-  if (total <= 0) return tile;
+  const float *hn = reinterpret_cast<const float *>(step_smem + kFbufOff) + 4096;
   const int warp = (threadIdx.x >> 5) & 7, half = threadIdx.x >> 8, lane = threadIdx.x & 31, n = H >> 8;
   const int lrpt = __ffs(kTileBytes) - __ffs(H * 2), rpt = 1 << lrpt, ntiles = (total + rpt - 1) >> lrpt;
   const uint32_t ring_a = smem_addr(step_smem + kRingOff);
@@ -816,22 +824,30 @@ static __device__ __forceinline__ uint32_t router_stage(uint32_t tile, const flo
 #pragma unroll 1
     for (int r = warp; r < nr; r += 8) {
       float acc = 0.0f;
-#pragma unroll 4
-      for (int i = 0; i < n; ++i) {
-        const int k0 = (i * 32 + lane) * 8;
-        const uint4 wv = lds128(tb + (uint32_t)r * (uint32_t)(H * 2) + (uint32_t)k0 * 2u);
-        const float4 a0 = *reinterpret_cast<const float4 *>(hn + k0), a1 = *reinterpret_cast<const float4 *>(hn + k0 + 4);
-        acc = fmaf(u2f(wv.x << 16), a0.x, acc);
-        acc = fmaf(u2f(wv.x & 0xFFFF0000u), a0.y, acc);
-        acc = fmaf(u2f(wv.y << 16), a0.z, acc);
-        acc = fmaf(u2f(wv.y & 0xFFFF0000u), a0.w, acc);
-        acc = fmaf(u2f(wv.z << 16), a1.x, acc);
-        acc = fmaf(u2f(wv.z & 0xFFFF0000u), a1.y, acc);
-        acc = fmaf(u2f(wv.w << 16), a1.z, acc);
-        acc = fmaf(u2f(wv.w & 0xFFFF0000u), a1.w, acc);
+      const uint32_t wb = tb + (uint32_t)r * (uint32_t)(H * 2) + (uint32_t)lane * 16u;
+      const float *hb = hn + lane * 8;
+      uint4 wv = lds128(wb);
+      float4 a0 = *reinterpret_cast<const float4 *>(hb), a1 = *reinterpret_cast<const float4 *>(hb + 4);
+#pragma unroll 1
+      for (int i = 1; i <= n; ++i) {   // the next piece is on its way while this one is added
+        const uint4 w = wv;
+        const float4 x0 = a0, x1 = a1;
+        if (i < n) {
+          wv = lds128(wb + (uint32_t)i * 512u);
+          a0 = *reinterpret_cast<const float4 *>(hb + i * 256);
+          a1 = *reinterpret_cast<const float4 *>(hb + i * 256 + 4);
+        }
+        acc = fmaf(u2f(w.x << 16), x0.x, acc);
+        acc = fmaf(u2f(w.x & 0xFFFF0000u), x0.y, acc);
+        acc = fmaf(u2f(w.y << 16), x0.z, acc);
+        acc = fmaf(u2f(w.y & 0xFFFF0000u), x0.w, acc);
+        acc = fmaf(u2f(w.z << 16), x1.x, acc);
+        acc = fmaf(u2f(w.z & 0xFFFF0000u), x1.y, acc);
+        acc = fmaf(u2f(w.w << 16), x1.z, acc);
+        acc = fmaf(u2f(w.w & 0xFFFF0000u), x1.w, acc);
       }
       acc = warp_tree_sum(acc);
-      if (lane == 0) PL.RLogits[lo + j * rpt + r] = acc;
+      if (lane == 0) put(out + lo + j * rpt + r, acc, flag);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive_a(smem_addr(&SH->empty[slot]));
@@ -845,73 +861,75 @@ static __device__ __forceinline__ uint32_t router_stage(uint32_t tile, const flo
 // probability + 1 (it is >= 0, so the bits order like integers), then the lower index. The
 // nsel-th largest of the sixteen warps' largest keys bounds the nsel-th largest of all from below,
 // so the entries at or above it (about 17 of 512 for a top 10) hold the whole selection: they are
-// gathered, and each one's rank is the number of candidates ahead of it (k + 1 rounds of extraction in
-// two levels, and the records fetched after them: 4.5 + 0.8 us a layer; so 2.9). slots <= 12, so nsel <=
-// 13 of the sixteen maxima.
-static __device__ __forceinline__ void router_select_cons(unsigned epoch, const ExpertW *experts, int E, int k, bool has_shared) {
+// gathered, and each one's rank is the number of candidates ahead of it. slots <= 12, so nsel <=
+// 13 of the sixteen maxima. The exponentials are padded to whole runs of 512 entries with zeros.
+static __device__ __forceinline__ void router_select_cons(unsigned target, const unsigned long long *logits, unsigned flag, const ExpertW *experts,
+                                                          int E, int k, bool has_shared) {
   float *lg = reinterpret_cast<float *>(step_smem + kFbufOff), *sp = lg + 2048, *pr = lg + 4096;
   unsigned long long *cand = reinterpret_cast<unsigned long long *>(step_smem + kTOff);   // up to E candidates
   StepShared *sh = SH;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  grid_wait(epoch);
-#pragma unroll
-  for (int u = 0; u < 3; ++u) {
-    const int e = tid + kCons * u;
-    if (e < E || (has_shared && e == E)) lg[e] = __ldcg(PL.RLogits + e);
-  }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, runs = (E + kCons - 1) / kCons;
+  await(target);
+  gather(lg, logits, E + (has_shared ? 1 : 0), flag);
   if (tid == 0) sh->ncand = 0;
   csync();
+  stamp(1);
   // maximum and sum keep the one-warp partition (lane l takes entries l, l+32, ... in ascending
   // order, then the xor butterfly); every warp evaluates them for itself, which gives every warp
   // the same bits and saves two block barriers and two one-warp sections
   float m = -INFINITY;
-#pragma unroll 8
+#pragma unroll 4
   for (int e = lane; e < E; e += 32) m = fmaxf(m, lg[e]);
-  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(m));
-  float ex[2] = {0.0f, 0.0f};
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
+  m = warp_largest(m);
+#pragma unroll 1
+  for (int u = 0; u < runs; ++u) {
     const int e = tid + kCons * u;
-    if (e < E) {
-      ex[u] = det_expf(lg[e] - m);
-      sp[e] = ex[u];
-    }
+    sp[e] = e < E ? det_expf(lg[e] - m) : 0.0f;
   }
   csync();
   float sum = 0.0f;
-#pragma unroll 8
-  for (int e = lane; e < E; e += 32) sum = sum + sp[e];
-  sum = warp_tree_sum(sum);
-  unsigned key[2];
+#pragma unroll 1
+  for (int e = lane; e < runs * kCons; e += 256) {
+    float v[8];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) key[u] = tid + kCons * u < E ? __float_as_uint(ex[u] / sum) + 1u : 0u;
-  const unsigned wk = __reduce_max_sync(kFull, key[0] > key[1] ? key[0] : key[1]);
+    for (int i = 0; i < 8; ++i) v[i] = sp[e + 32 * i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sum = sum + v[i];
+  }
+  sum = warp_tree_sum(sum);
+  unsigned *keys = reinterpret_cast<unsigned *>(lg);   // over the logits, which every warp has read (lg[E] stays)
+  unsigned wk = 0u;
+#pragma unroll 1
+  for (int e = tid; e < E; e += kCons) {
+    const unsigned key = __float_as_uint(sp[e] / sum) + 1u;
+    keys[e] = key;   // read by the same thread
+    wk = key > wk ? key : wk;
+  }
+  wk = __reduce_max_sync(kFull, wk);
   if (lane == 0) sh->kmax[warp] = wk;
   csync();
   const int nsel = k < E ? k + 1 : k;
-  unsigned bound;
-  {
-    const unsigned mine = lane < 16 ? sh->kmax[lane] : 0u;
-    int ahead = 0;
+  const unsigned mine = lane < 16 ? sh->kmax[lane] : 0u;
+  int ahead = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const unsigned o = sh->kmax[i];
-      ahead += o > mine || (o == mine && i < lane);
-    }
-    bound = __reduce_min_sync(kFull, lane < 16 && ahead < nsel ? mine : 0xFFFFFFFFu);
-    if (bound == 0u) bound = 1u;   // fewer warps than nsel hold entries: all of them are candidates
+  for (int i = 0; i < 16; ++i) {
+    const unsigned o = sh->kmax[i];
+    ahead += o > mine || (o == mine && i < lane);
   }
-#pragma unroll
-  for (int u = 0; u < 2; ++u)
-    if (key[u] >= bound)
-      cand[atomicAdd(&sh->ncand, 1)] = ((unsigned long long)key[u] << 32) | (0xFFFFFFFFu - (unsigned)(tid + kCons * u));
+  unsigned bound = __reduce_min_sync(kFull, lane < 16 && ahead < nsel ? mine : 0xFFFFFFFFu);
+  if (bound == 0u) bound = 1u;   // fewer warps than nsel hold entries: all of them are candidates
+#pragma unroll 1
+  for (int e = tid; e < E; e += kCons)
+    if (keys[e] >= bound) cand[atomicAdd(&sh->ncand, 1)] = ((unsigned long long)keys[e] << 32) | (0xFFFFFFFFu - (unsigned)e);
   csync();
   const int nc = sh->ncand;
+#pragma unroll 1
   for (int i = warp; i < nc; i += 16) {
     const unsigned long long c = cand[i];
     int rank = 0;
+#pragma unroll 1
     for (int j0 = 0; j0 < nc; j0 += 32) rank += __popc(__ballot_sync(kFull, j0 + lane < nc && cand[j0 + lane] > c));
-    if (rank > k || rank >= E) continue;
+    if (rank > k) continue;
     const int e = (int)(0xFFFFFFFFu - (unsigned)c);
     if (rank < k && lane < 3)
       reinterpret_cast<uint4 *>(sh->sew + rank)[lane] = __ldg(reinterpret_cast<const uint4 *>(experts + e) + lane);
@@ -925,14 +943,16 @@ static __device__ __forceinline__ void router_select_cons(unsigned epoch, const 
       reinterpret_cast<uint4 *>(sh->sew + k)[lane] = __ldg(reinterpret_cast<const uint4 *>(experts + E) + lane);
     if (lane == 0) {
       sh->sel_idx[k] = E;
-      sh->sel_w[k] = has_shared ? 1.0f / (1.0f + det_expf(-lg[E])) : 0.0f;
+      sh->sel_w[k] = has_shared ? over_exp(1.0f, -lg[E]) : 0.0f;
     }
   }
   csync();
   if (tid == 0) mbar_arrive(&sh->sel_bar);  // the producer may now stream the experts
+  stamp(5);
   // the weights are needed by the down projection only
   if (warp == 1) {
     float s = 0.0f;
+#pragma unroll 1
     for (int j = 0; j < k && j < E; ++j) s = s + pr[j];
     if (lane < k) sh->sel_w[lane] = (lane < E ? pr[lane] : 0.0f) / s;
     if (lane == 0) {
@@ -943,76 +963,77 @@ static __device__ __forceinline__ void router_select_cons(unsigned epoch, const 
 }
 
 // ------------------------------------------------------------ gated delta rule ---
-// One (head, column slice) item per block, 256 threads, state in registers; the arithmetic is
-// DeltaNetStep's (deltanet_core.cuh). The state of the block's first item is loaded before the
-// grid barrier is waited for: it was last written one token ago by this same block.
-static __device__ __forceinline__ void deltanet_stage(unsigned epoch, const StepLayer &ly) {
+// One (head, column slice) item per block; the arithmetic is DeltaNetStep's (deltanet_core.cuh). The
+// slice of the state, 128 rows of 32 columns, comes to shared memory by asynchronous copies while the words are
+// waited for: it was last written one token ago by this same block. Warp w < 8 owns segment w of the rows.
+static __device__ __noinline__ void deltanet_stage(unsigned target, const StepLayer &ly, const unsigned long long *Mx,
+                                                   const unsigned long long *Bt, const unsigned long long *Gt, unsigned long long *O,
+                                                   unsigned flag) {
   const StepPlan &P = PL;
   constexpr int D = 128, SEG = kDnSeg;
-  DeltaNetStepArgs a{P.O, P.Mx, ly.S, P.Bt, P.Gt, P.nK, P.nV};
-  const int nitems = P.nV * kDnSlices;
-  const bool worker = threadIdx.x < 256;
-  float s[SEG];
-  if (worker && (int)blockIdx.x < nitems) deltanet_load_state(a, (int)blockIdx.x, s);
-  grid_wait(epoch);
-  if (!worker) return;
-  float *qs = reinterpret_cast<float *>(step_smem + kFbufOff), *ks = qs + D;
-  float(*part)[32] = reinterpret_cast<float(*)[32]>(ks + D);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nitems = P.nV * kDnSlices, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, per_k = P.nV / P.nK;
+  // q | k | value slice | beta | decay of the item, then the segments' partial sums
+  float *raw = reinterpret_cast<float *>(step_smem + kTOff), *st = reinterpret_cast<float *>(step_smem + kFbufOff);
+  float *part = raw + 512;
+  csync();   // the first projections' terms and operands are read
 #pragma unroll 1
   for (int item = (int)blockIdx.x; item < nitems; item += (int)gridDim.x) {
-    const int h = item / kDnSlices, slice = item % kDnSlices;
-    const int kh = h / (a.nV / a.nK);
-    const int col = slice * 32 + lane;
-    float *Sh = a.S + (size_t)h * D * D;
-    if (item != (int)blockIdx.x) deltanet_load_state(a, item, s);
-    if (warp < 2) {
-      const float *src = a.Mx + (warp == 0 ? (size_t)kh * D : (size_t)a.nK * D + (size_t)kh * D);
-      float x[4];
-      float ss = 0.0f;
+    const int h = item / kDnSlices, slice = item % kDnSlices, kh = h / per_k;
+    float *S0 = ly.S + (size_t)h * D * D + slice * 32;
+#pragma unroll 1
+    for (int i = tid; i < D * 8; i += kCons) cp_async16(st + i * 4, S0 + (i >> 3) * D + (i & 7) * 4);
+    if (item == (int)blockIdx.x) await(target);
+    if (tid < 290) {
+      const unsigned long long *w = tid < 128 ? Mx + kh * D + tid
+                                    : tid < 256 ? Mx + (P.nK + kh) * D + tid - 128
+                                    : tid < 288 ? Mx + (2 * P.nK + h) * D + slice * 32 + tid - 256
+                                    : tid == 288 ? Bt + h : Gt + h;
+      raw[tid] = take(w, flag);
+    }
+    cp_async_wait();
+    csync();
+    stamp(1);
+    if (tid < 256) {
+      float sq = 0.0f, sk = 0.0f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        x[i] = __ldcg(src + lane + 32 * i);
-        ss = fmaf(x[i], x[i], ss);
+        const float q = raw[lane + 32 * i], k = raw[D + lane + 32 * i];
+        sq = fmaf(q, q, sq);
+        sk = fmaf(k, k, sk);
       }
-      ss = warp_tree_sum(ss);
-      const float inv = 1.0f / sqrtf(ss + 1e-6f);
-      const float f = inv * (warp == 0 ? 0.0883883476483184405f : 1.0f);
-      float *dst = warp == 0 ? qs : ks;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dst[lane + 32 * i] = x[i] * f;
+      for (int off = 16; off > 0; off >>= 1) {
+        sq = sq + __shfl_xor_sync(kFull, sq, off);
+        sk = sk + __shfl_xor_sync(kFull, sk, off);
+      }
+      const float fq = inv_sqrt(sq + 1e-6f) * 0.0883883476483184405f, fk = inv_sqrt(sk + 1e-6f);
+      const float val = raw[256 + lane], beta = raw[288], gt = det_expf(raw[289]);
+      const float *kr = raw + D + warp * SEG, *qr = raw + warp * SEG, *sr = st + warp * SEG * 32 + lane;
+      float acc = 0.0f;
+#pragma unroll 4
+      for (int r = 0; r < SEG; ++r) acc = fmaf(sr[r * 32] * gt, kr[r] * fk, acc);
+      part[tid] = acc;
+      hsync();
+      const float *p = part + lane;
+      const float kv = ((p[0] + p[32]) + (p[64] + p[96])) + ((p[128] + p[160]) + (p[192] + p[224]));
+      const float dl = (val - kv) * beta;
+      float *Sh = S0 + (size_t)warp * SEG * D + lane;
+      acc = 0.0f;
+#pragma unroll 4
+      for (int r = 0; r < SEG; ++r) {
+        const float s = fmaf(kr[r] * fk, dl, sr[r * 32] * gt);
+        acc = fmaf(s, qr[r] * fq, acc);
+        Sh[r * D] = s;
+      }
+      part[256 + tid] = acc;
+      hsync();
+      if (warp == 0) {
+        p += 256;
+        const float o = ((p[0] + p[32]) + (p[64] + p[96])) + ((p[128] + p[160]) + (p[192] + p[224]));
+        put(O + item * 32 + lane, o, flag);
+      }
     }
-    const float val = __ldcg(a.Mx + (size_t)2 * a.nK * D + (size_t)h * D + col);
-    const float beta = __ldcg(a.Bt + h);
-    const float gt = det_expf(__ldcg(a.Gt + h));
-    hsync();
-    float acc = 0.0f;
-#pragma unroll
-    for (int r = 0; r < SEG; ++r) {
-      s[r] = s[r] * gt;
-      acc = fmaf(s[r], ks[warp * SEG + r], acc);
-    }
-    part[warp][lane] = acc;
-    hsync();
-    const float kv = ((part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane])) +
-                     ((part[4][lane] + part[5][lane]) + (part[6][lane] + part[7][lane]));
-    const float dl = (val - kv) * beta;
-    hsync();
-    acc = 0.0f;
-#pragma unroll
-    for (int r = 0; r < SEG; ++r) {
-      s[r] = fmaf(ks[warp * SEG + r], dl, s[r]);
-      acc = fmaf(s[r], qs[warp * SEG + r], acc);
-      Sh[(size_t)(warp * SEG + r) * D + col] = s[r];
-    }
-    part[warp][lane] = acc;
-    hsync();
-    if (warp == 0) {
-      const float o = ((part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane])) +
-                      ((part[4][lane] + part[5][lane]) + (part[6][lane] + part[7][lane]));
-      a.Out[(size_t)h * D + col] = o;
-    }
-    hsync();
+    if (item + (int)gridDim.x < nitems) csync();   // the item's memory is rewritten
   }
 }
 
@@ -1020,77 +1041,59 @@ static __device__ __forceinline__ void deltanet_stage(unsigned epoch, const Step
 // One 64-token chunk of one KV head per item: head norm + RoPE of the group's query heads
 // (and, in the chunk that holds the new position, of the new key; INT8 append of key and
 // value), scores, chunk softmax, weighted values. Arithmetic of AttnPrep + AttnSplit
-// (attention_core.cuh). K/V rows of earlier tokens are fetched before the grid barrier is
-// waited for (they were written by earlier steps).
+// (attention_core.cuh). K/V rows of earlier tokens are on their way while the words are waited
+// for (they were written by earlier steps). Sixteen warps: in the score pass eight of every eighth token for
+// each half of the heads, whose queries they hold in registers; an INT8 value becomes a float by a byte permute
+// and an addition (in the mantissa of 2^23, less 2^23 + 128: exact) instead of the quarter-rate conversion.
+static __device__ __forceinline__ float byte_f32(uint32_t biased, int i) {
+  return __uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7540 + i)) - 8388736.0f;
+}
 template <int GQ>
-static __device__ __noinline__ void attn_stage_t(unsigned epoch, const StepLayer &ly, int pos, int T) {
+static __device__ __noinline__ void attn_stage_t(unsigned target, const StepLayer &ly, const unsigned long long *Q, const unsigned long long *K,
+                                                 const unsigned long long *V, unsigned flag, int pos, int T) {
   const StepPlan &P = PL;
   constexpr int D = kHeadDim, C = kAttnChunk;
-  constexpr int GH = (GQ + 1) / 2;  // query heads per half of the block in the value pass
+  constexpr int GH = (GQ + 1) / 2;  // query heads per half of the warps
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nKV = P.nKV;
   const int nch = (T + C - 1) / C, nitems = nch * nKV;
   unsigned char *kvs = step_smem + kFbufOff;  // K rows [C][D], then V rows [C][D]
   float *qs = reinterpret_cast<float *>(step_smem + kTOff);  // [GQ][D]
-  float *sc = qs + GQ * D;                                // [C][GQ]: per token the heads' scores, then weights
-  uint16_t *kss = reinterpret_cast<uint16_t *>(sc + GQ * C), *vss = kss + C;
-  StepShared *sh = SH;
+  float *sc = qs + 2048;   // [C][GQ] scores, then exponentials
+  float *pw = sc + 512;    // [C][GQ] weights x value scales
+  uint16_t *kss = reinterpret_cast<uint16_t *>(pw + 512), *vss = kss + C;
   const int p = pos < P.max_ctx ? pos : P.max_ctx - 1;  // clamp, kernels.cpp:456
   const float scale = 1.0f / sqrtf((float)D);
-
-  uint4 kvr[4];
-  uint16_t scr = 0;
-  auto load_chunk = [&](int item) {
-    const int ch = item / nKV, kv = item % nKV, t0 = ch * C;
-    const int nt = (T < t0 + C ? T : t0 + C) - t0;
-    const size_t rs = (size_t)nKV * (D / 16);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = tid + kCons * u, which = i >> 10, row = (i & 1023) >> 4, pc = i & 15;
-      kvr[u] = make_uint4(0, 0, 0, 0);
-      if (row < nt && t0 + row != p) {
-        const int8_t *base = which ? ly.Vc : ly.Kc;
-        kvr[u] = __ldcg(reinterpret_cast<const uint4 *>(base + ((size_t)t0 * nKV + kv) * D) + row * rs + pc);
-      }
-    }
-    if (tid < 2 * C) {
-      const int row = tid & (C - 1);
-      scr = 0;
-      if (row < nt && t0 + row != p) scr = __ldcg((tid < C ? ly.Ks : ly.Vs) + (size_t)(t0 + row) * nKV + kv);
-    }
-  };
-  if ((int)blockIdx.x < nitems) load_chunk((int)blockIdx.x);
-  grid_wait(epoch);
 #pragma unroll 1
   for (int item = (int)blockIdx.x; item < nitems; item += (int)gridDim.x) {
     const int ch = item / nKV, kv = item % nKV, t0 = ch * C;
     const int nt = (T < t0 + C ? T : t0 + C) - t0;
-    if (item != (int)blockIdx.x) load_chunk(item);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) reinterpret_cast<uint4 *>(kvs)[tid + kCons * u] = kvr[u];
-    if (tid < C) kss[tid] = scr;
-    else if (tid < 2 * C) vss[tid - C] = scr;
-    csync();
-    stamp(20);
+    csync();   // the stage before, or the item before, is done with this memory
+    {
+      const size_t first = ((size_t)t0 * nKV + kv) * D, rs = (size_t)nKV * D;
+#pragma unroll 1
+      for (int i = tid; i < 2 * C * (D / 16); i += kCons) {
+        const int which = i >> 10, row = (i & 1023) >> 4, pc = i & 15;
+        if (row < nt && t0 + row != p) cp_async16(kvs + (size_t)i * 16, (which ? ly.Vc : ly.Kc) + first + row * rs + pc * 16);
+      }
+      if (tid < 2 * C) {
+        const int row = tid & (C - 1);
+        if (row < nt && t0 + row != p) (tid < C ? kss : vss)[row] = __ldcg((tid < C ? ly.Ks : ly.Vs) + (size_t)(t0 + row) * nKV + kv);
+      }
+    }
+    if (item == (int)blockIdx.x) await(target);
     // query heads of the group: warp g. New key row: warp GQ, new value row: warp GQ+1.
     if (warp < GQ || ((warp == GQ || warp == GQ + 1) && p >= t0 && p < t0 + nt)) {
+      const unsigned long long *src = warp < GQ ? Q + (size_t)(kv * GQ + warp) * 2 * D : (warp == GQ ? K : V) + (size_t)kv * D;
       float x[8];
-      if (warp == GQ + 1) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = __ldcg(P.V16 + (size_t)kv * D + lane + 32 * i);
-      } else {
-        const bool isq = warp < GQ;
-        const float *src = isq ? P.Q16 + (size_t)(kv * GQ + warp) * 2 * D : P.K16 + (size_t)kv * D;
-        const float *w = isq ? ly.q_norm : ly.k_norm;
+      take8(x, src + lane, flag);
+      if (warp <= GQ) {
+        const float *w = warp < GQ ? ly.q_norm : ly.k_norm;
         double ss = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          x[i] = __ldcg(src + lane + 32 * i);
-          const double dv = (double)x[i];
-          ss = ss + dv * dv;
-        }
+        for (int i = 0; i < 8; ++i) ss = fma((double)x[i], (double)x[i], ss);
         ss = warp_tree_sum(ss);
-        const float inv = 1.0f / sqrtf((float)(ss / (double)D) + P.eps);
+        const float inv = inv_sqrt((float)(ss * (1.0 / D)) + P.eps);
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = (x[i] * inv) * (1.0f + __ldg(w + lane + 32 * i));
         if (P.rot / 2 == 32) {
@@ -1115,173 +1118,197 @@ static __device__ __noinline__ void attn_stage_t(unsigned epoch, const StepLayer
         if (lane == 0) ((isk ? ly.Ks : ly.Vs))[(size_t)p * nKV + kv] = *ssc;
       }
     }
+    cp_async_wait();
     csync();
-    stamp(21);
-    // scores: warp w takes tokens w, w+16, ...
-#pragma unroll 1
-    for (int tt = warp; tt < nt; tt += 16) {
-      const uint2 kw = reinterpret_cast<const uint2 *>(kvs)[tt * (D / 8) + lane];
-      const float ksf = f16_to_f32(kss[tt]);
-      float kf[8];
+    stamp(20);
+    const int g0 = (warp >> 3) * GH;   // this half's first head
+    if (g0 < GQ) {
+      float q[GH][8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        kf[j] = (float)(int)(int8_t)((kw.x >> (8 * j)) & 0xFF);
-        kf[4 + j] = (float)(int)(int8_t)((kw.y >> (8 * j)) & 0xFF);
+      for (int g = 0; g < GH; ++g) {
+        const float4 a = *reinterpret_cast<const float4 *>(qs + (g0 + g) * D + lane * 8), b = *reinterpret_cast<const float4 *>(qs + (g0 + g) * D + lane * 8 + 4);
+        q[g][0] = a.x; q[g][1] = a.y; q[g][2] = a.z; q[g][3] = a.w;
+        q[g][4] = b.x; q[g][5] = b.y; q[g][6] = b.z; q[g][7] = b.w;
       }
-      float part[GQ];
+#pragma unroll 2
+      for (int tt = warp & 7; tt < nt; tt += 8) {
+        const uint2 kw = reinterpret_cast<const uint2 *>(kvs)[tt * (D / 8) + lane];
+        const uint32_t b0 = kw.x ^ 0x80808080u, b1 = kw.y ^ 0x80808080u;
+        float kf[8], part[GH];
 #pragma unroll
-      for (int g = 0; g < GQ; ++g) {
-        const float4 q0 = *reinterpret_cast<const float4 *>(qs + g * D + lane * 8),
-                     q1 = *reinterpret_cast<const float4 *>(qs + g * D + lane * 8 + 4);
-        float acc = 0.0f;
-        acc = fmaf(q0.x, kf[0], acc);
-        acc = fmaf(q0.y, kf[1], acc);
-        acc = fmaf(q0.z, kf[2], acc);
-        acc = fmaf(q0.w, kf[3], acc);
-        acc = fmaf(q1.x, kf[4], acc);
-        acc = fmaf(q1.y, kf[5], acc);
-        acc = fmaf(q1.z, kf[6], acc);
-        acc = fmaf(q1.w, kf[7], acc);
-        part[g] = acc;
+        for (int j = 0; j < 4; ++j) {
+          kf[j] = byte_f32(b0, j);
+          kf[4 + j] = byte_f32(b1, j);
+        }
+#pragma unroll
+        for (int g = 0; g < GH; ++g) {
+          float acc = 0.0f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc = fmaf(q[g][j], kf[j], acc);
+          part[g] = acc;
+        }
+        attn_store_scores<GH>(part, lane, sc + tt * GQ + g0, f16_to_f32(kss[tt]), scale);
       }
-      attn_store_scores<GQ>(part, lane, sc + tt * GQ, ksf, scale);   // one butterfly for all heads
     }
     csync();
     stamp(22);
-    if (tid < GQ) {
-      float mx = -INFINITY;
-      for (int tt = 0; tt < nt; ++tt) mx = fmaxf(mx, sc[tt * GQ + tid]);
-      sh->hmax[tid] = mx;
+    if (warp < GQ) {   // chunk softmax of a head
+      const float s0 = lane < nt ? sc[lane * GQ + warp] : -INFINITY, s1 = lane + 32 < nt ? sc[(lane + 32) * GQ + warp] : -INFINITY;
+      const float mx = warp_largest(fmaxf(s0, s1));
+#pragma unroll 1
+      for (int u = 0; u < 2; ++u) {
+        const int tt = lane + 32 * u;
+        if (tt < nt) {
+          const float e = det_expf((u ? s1 : s0) - mx);
+          sc[tt * GQ + warp] = e;
+          pw[tt * GQ + warp] = e * f16_to_f32(vss[tt]);
+        }
+      }
+      if (lane == 0) P.Pm[(size_t)(kv * GQ + warp) * P.max_chunks + ch] = mx;
     }
-    csync();
-    for (int i = tid; i < GQ * nt; i += kCons) sc[i] = det_expf(sc[i] - sh->hmax[i % GQ]);
-    csync();
-    if (tid < GQ) {
-      float se = 0.0f;
-      for (int tt = 0; tt < nt; ++tt) se = se + sc[tt * GQ + tid];
-      sh->hse[tid] = se;
-    }
-    csync();
-    for (int i = tid; i < GQ * nt; i += kCons) sc[i] = sc[i] * f16_to_f32(vss[i / GQ]);
     csync();
     stamp(23);
-    // weighted values: thread (dim, half) accumulates its dim for the heads of its half
-    {
-      const int dim = tid & 255, g0 = (tid >> 8) * GH;
-      float acc[GH];
-#pragma unroll
-      for (int g = 0; g < GH; ++g) acc[g] = 0.0f;
-      const int8_t *vs = reinterpret_cast<const int8_t *>(kvs + C * D) + dim;
-      if constexpr (GQ == 8) {   // four heads per half: one 16-byte read gives a token's four weights
+    if (warp == 15 && lane < GQ) {   // the sum of exponentials, in token order
+      float se = 0.0f;
 #pragma unroll 8
-        for (int tt = 0; tt < nt; ++tt) {
-          const float v = (float)(int)vs[tt * D];
-          const float4 pw = *reinterpret_cast<const float4 *>(sc + tt * GQ + g0);
-          acc[0] = fmaf(pw.x, v, acc[0]);
-          acc[1] = fmaf(pw.y, v, acc[1]);
-          acc[2] = fmaf(pw.z, v, acc[2]);
-          acc[3] = fmaf(pw.w, v, acc[3]);
-        }
+      for (int tt = 0; tt < nt; ++tt) se = se + sc[tt * GQ + lane];
+      P.Pse[(size_t)(kv * GQ + lane) * P.max_chunks + ch] = se;
+    }
+    // weighted values: thread (dim, half) accumulates its dim for the heads of its half
+    const int dim = tid & 255;
+    float acc[GH];
+#pragma unroll
+    for (int g = 0; g < GH; ++g) acc[g] = 0.0f;
+    const uint8_t *vs = reinterpret_cast<const uint8_t *>(kvs + C * D) + dim;
+#pragma unroll 4
+    for (int tt = 0; tt < nt; ++tt) {
+      const float v = __uint_as_float(0x4B000000u | ((uint32_t)vs[tt * D] ^ 0x80u)) - 8388736.0f;
+      if constexpr (GQ == 8) {   // four heads per half: one 16-byte read gives a token's four weights
+        const float4 w = *reinterpret_cast<const float4 *>(pw + tt * GQ + g0);
+        acc[0] = fmaf(w.x, v, acc[0]);
+        acc[1] = fmaf(w.y, v, acc[1]);
+        acc[2] = fmaf(w.z, v, acc[2]);
+        acc[3] = fmaf(w.w, v, acc[3]);
       } else {
-#pragma unroll 2
-        for (int tt = 0; tt < nt; ++tt) {
-          const float v = (float)(int)vs[tt * D];
 #pragma unroll
-          for (int g = 0; g < GH; ++g)
-            if (g0 + g < GQ) acc[g] = fmaf(sc[tt * GQ + g0 + g], v, acc[g]);
-        }
-      }
-#pragma unroll
-      for (int g = 0; g < GH; ++g) {
-        if (g0 + g < GQ) {
-          const size_t slot = (size_t)(kv * GQ + g0 + g) * P.max_chunks + ch;
-          P.Pacc[slot * D + dim] = acc[g];
-          if (dim == 0) {
-            P.Pm[slot] = sh->hmax[g0 + g];
-            P.Pse[slot] = sh->hse[g0 + g];
-          }
-        }
+        for (int g = 0; g < GH; ++g)
+          if (g0 + g < GQ) acc[g] = fmaf(pw[tt * GQ + g0 + g], v, acc[g]);
       }
     }
+#pragma unroll
+    for (int g = 0; g < GH; ++g)
+      if (g0 + g < GQ) P.Pacc[((size_t)(kv * GQ + g0 + g) * P.max_chunks + ch) * D + dim] = acc[g];
     stamp(24);
-    csync();
   }
 }
-static __device__ __noinline__ void attn_stage(unsigned epoch, const StepLayer &ly, int pos, int T) {
+static __device__ __forceinline__ void attn_stage(unsigned target, const StepLayer &ly, const unsigned long long *Q, const unsigned long long *K,
+                                                  const unsigned long long *V, unsigned flag, int pos, int T) {
   switch (PL.nQ / PL.nKV) {
-    case 1: attn_stage_t<1>(epoch, ly, pos, T); break;
-    case 2: attn_stage_t<2>(epoch, ly, pos, T); break;
-    case 4: attn_stage_t<4>(epoch, ly, pos, T); break;
-    case 6: attn_stage_t<6>(epoch, ly, pos, T); break;
-    case 8: attn_stage_t<8>(epoch, ly, pos, T); break;
-    default: grid_wait(epoch); break;  // rejected on the host
+    case 1: attn_stage_t<1>(target, ly, Q, K, V, flag, pos, T); break;
+    case 2: attn_stage_t<2>(target, ly, Q, K, V, flag, pos, T); break;
+    case 4: attn_stage_t<4>(target, ly, Q, K, V, flag, pos, T); break;
+    case 6: attn_stage_t<6>(target, ly, Q, K, V, flag, pos, T); break;
+    case 8: attn_stage_t<8>(target, ly, Q, K, V, flag, pos, T); break;
+    default: break;  // rejected on the host
   }
 }
 
-// Ordered merge of the chunk partials of one query head per block (256 threads), sigmoid
-// gate, quantiser: AttnCombine's arithmetic (attention_core.cuh).
-static __device__ __noinline__ void attn_combine_stage(int T) {
+// Ordered merge of the chunk partials, sigmoid gate, quantiser: AttnCombine's arithmetic
+// (attention_core.cuh). An item is half a query head, the 128 dims of a quantiser group: thread d < 128 adds
+// its dim over the chunks in ascending order, from 64 chunks at a time in shared memory. Its
+// words: 32 of four INT8 values, and the scale.
+static __device__ __noinline__ void attn_merge(unsigned target, const unsigned long long *Q, unsigned long long *q8, unsigned flag, int T) {
   const StepPlan &P = PL;
   constexpr int D = kHeadDim, C = kAttnChunk;
-  if (threadIdx.x >= 256) return;
-  float *s_pm = reinterpret_cast<float *>(step_smem + kFbufOff), *s_pf = s_pm + 2048;
-  float *wmax = SH->wmax;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nch = (T + C - 1) / C;
+  float *pa = reinterpret_cast<float *>(step_smem + kFbufOff);   // [64][128] partials
+  float *fs = reinterpret_cast<float *>(step_smem + kTOff), *es = fs + 64;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nch = (T + C - 1) / C;
 #pragma unroll 1
-  for (int h = (int)blockIdx.x; h < P.nQ; h += (int)gridDim.x) {
-    const float *pm = P.Pm + (size_t)h * P.max_chunks;
-    const float *pse = P.Pse + (size_t)h * P.max_chunks;
-    const float *pacc = P.Pacc + (size_t)h * P.max_chunks * D;
-    const float gate = __ldcg(P.Q16 + (size_t)h * 2 * D + D + tid);
+  for (int it = (int)blockIdx.x; it < 2 * P.nQ; it += (int)gridDim.x) {
+    const int h = it >> 1, d0 = (it & 1) * 128;
+    const float *pm = P.Pm + (size_t)h * P.max_chunks, *pse = P.Pse + (size_t)h * P.max_chunks;
+    const float *pacc = P.Pacc + (size_t)h * P.max_chunks * D + d0;
+    const float gate = tid < 128 ? take(Q + (size_t)h * 2 * D + D + d0 + tid, flag) : 0.0f;
     float M = -INFINITY, se = 0.0f, acc = 0.0f;
-    if (nch <= 2048) {
-      hsync();
-      for (int ch = tid; ch < nch; ch += 256) {
-        s_pm[ch] = __ldcg(pm + ch);
-        s_pf[ch] = __ldcg(pse + ch);
+    const auto fetch = [&](int c0, int nb) {
+#pragma unroll 1
+      for (int i = tid; i < nb * 32; i += kCons) cp_async16(pa + i * 4, pacc + (size_t)(c0 + (i >> 5)) * D + (i & 31) * 4);
+    };
+    if (it != (int)blockIdx.x) csync();   // the memory's last readers are done
+    fetch(0, nch < 64 ? nch : 64);
+#pragma unroll 1
+    for (int ch = lane; ch < nch; ch += 32) M = fmaxf(M, __ldcg(pm + ch));
+    M = warp_largest(M);
+#pragma unroll 1
+    for (int c0 = 0; c0 < nch; c0 += 64) {
+      const int nb = nch - c0 < 64 ? nch - c0 : 64;
+      if (c0) {
+        csync();
+        fetch(c0, nb);
       }
-      hsync();
-      for (int ch = 0; ch < nch; ++ch) M = fmaxf(M, s_pm[ch]);
-      hsync();
-      for (int ch = tid; ch < nch; ch += 256) s_pm[ch] = det_expf(s_pm[ch] - M);
-      hsync();
-      for (int ch = 0; ch < nch; ++ch) se = fmaf(s_pf[ch], s_pm[ch], se);
-#pragma unroll 16
-      for (int ch = 0; ch < nch; ++ch) acc = fmaf(__ldcg(pacc + (size_t)ch * D + tid), s_pm[ch], acc);
-    } else {
-      for (int ch = 0; ch < nch; ++ch) M = fmaxf(M, __ldcg(pm + ch));
-      for (int ch = 0; ch < nch; ++ch) {
-        const float f = det_expf(__ldcg(pm + ch) - M);
-        se = fmaf(__ldcg(pse + ch), f, se);
-        acc = fmaf(__ldcg(pacc + (size_t)ch * D + tid), f, acc);
+      if (tid < nb) {
+        fs[tid] = det_expf(__ldcg(pm + c0 + tid) - M);
+        es[tid] = __ldcg(pse + c0 + tid);
+      }
+      cp_async_wait();
+      csync();
+      if (tid < 128) {
+#pragma unroll 8
+        for (int c = 0; c < nb; ++c) acc = fmaf(pa[c * 128 + tid], fs[c], acc);
+      } else if (tid == 128) {
+#pragma unroll 8
+        for (int c = 0; c < nb; ++c) se = fmaf(es[c], fs[c], se);
       }
     }
-    const float o = acc / se;
-    const float y = o / (1.0f + det_expf(-gate));
-    float m = warp_max(fabsf(y));
-    if (lane == 0) wmax[warp] = m;
-    hsync();
-    const int g0 = (warp >> 2) * 4;
-    m = fmaxf(fmaxf(wmax[g0], wmax[g0 + 1]), fmaxf(wmax[g0 + 2], wmax[g0 + 3]));
-    float s = m / 127.0f;
-    if (s == 0.0f) s = 1.0f;
-    if ((tid & 127) == 0) P.SQ[(size_t)h * 2 + (tid >> 7)] = s;
-    P.Q8[(size_t)h * D + tid] = (int8_t)quant_round(y, s);
-    hsync();
+    if (tid == 128) SH->wmax[8] = se;
+    csync();
+    float y = 0.0f;
+    if (tid < 128) {
+      y = over_exp(acc / SH->wmax[8], -gate);
+      const float m = warp_absmax(y);
+      if (lane == 0) SH->wmax[warp] = m;
+    }
+    csync();
+    if (tid < 128) {
+      const float m = fmaxf(fmaxf(SH->wmax[0], SH->wmax[1]), fmaxf(SH->wmax[2], SH->wmax[3]));
+      float s = m / 127.0f;
+      if (s == 0.0f) s = 1.0f;
+      uint32_t w = (uint32_t)(quant_round(y, s) & 0xFF);
+      w |= __shfl_down_sync(kFull, w, 1) << 8;
+      w |= __shfl_down_sync(kFull, w, 2) << 16;
+      if ((tid & 3) == 0) put(q8 + it * 32 + (tid >> 2), __uint_as_float(w), flag);
+      if (tid == 0) put(q8 + P.nQ * 64 + it, s, flag);
+    }
   }
+  // the merged vector into the staged form
+  const int K = P.nQ * D, G = K >> 7;
+  unsigned char *act = step_smem + kActOff;
+  uint32_t *xw = reinterpret_cast<uint32_t *>(act);
+  arrive<false>();
+  await(target);
+  gather(pa, q8, P.nQ * 66, flag);
+  csync();
+  stamp(1);
+#pragma unroll 1
+  for (int pc = tid; pc < K / 8; pc += kCons) {
+    const uint2 v = reinterpret_cast<const uint2 *>(pa)[pc];
+    const int g = pc >> 4, i = pc & 15;
+    uint32_t *dst = xw + ((((i >> 1) * G + g) << 2) + ((i & 1) << 1));
+    dst[0] = __byte_perm(v.x, v.y, 0x6420);
+    dst[1] = __byte_perm(v.x, v.y, 0x7531);
+  }
+  if (tid < G) reinterpret_cast<float *>(act + K)[tid] = pa[P.nQ * 64 + tid];
+  csync();
 }
 
 // ------------------------------------------------------------------- MoE stages ---
-static __device__ __forceinline__ uint32_t gateup_stage(uint32_t tile) {
+static __device__ __forceinline__ uint32_t gateup_stage(uint32_t tile, unsigned long long *out, unsigned flag) {
   const StepPlan &P = PL;
   const int H = P.H, lgI = __ffs(P.I) - 1, lg = 31 - __clz(H >> 7);
   const int lo = SH->rng[kRngGateUp].x, hi = SH->rng[kRngGateUp].y, np = hi - lo;
-  if (np <= 0) return tile;
-  float *T = reinterpret_cast<float *>(step_smem + kTOff);
-  unsigned char *act = step_smem + kActOff;
-  tile = dot_tiles<false>(tile, lg, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + H), T, 2 * np, 0);
-  csync();
+  const float *T = reinterpret_cast<const float *>(step_smem + kTOff);
+  csync();   // the candidates of the selection lie where the terms go
+  tile = dot_tiles(tile, lg, H, 2 * np, 0.0f);
   // the producer streams, slot by slot, the slot's gate rows and then its up rows: the pair row
   // lo + r of slot s (rows a .. a + n - 1 of the share belong to it) has its gate term at
   // 2 (a - lo) + i and its up term n rows later
@@ -1291,59 +1318,69 @@ static __device__ __forceinline__ uint32_t gateup_stage(uint32_t tile) {
     const int a = lo > s * P.I ? lo : s * P.I, b = hi < (s + 1) * P.I ? hi : (s + 1) * P.I;
     const int n = b - a, i = lo + r - a, fg = 2 * (a - lo) + i;
     const float g = row_terms(T, fg, lg), u = row_terms(T, fg + n, lg);
-    P.Act[lo + r] = (g / (1.0f + det_expf(-g))) * u;
+    put(out + lo + r, over_exp(g, -g) * u, flag);
   }
   return tile;
 }
 
 // Output row n: residual + sum over the slots in rank order of weight x product. One thread a (slot,
 // row) adds the row's group terms, then one a row adds the slots.
-static __device__ __forceinline__ uint32_t down_stage(unsigned epoch, uint32_t tile, int L) {
+static __device__ __forceinline__ uint32_t down_stage(unsigned target, uint32_t tile, const unsigned long long *in, unsigned long long *out, unsigned flag,
+                                                      float res, int L) {
   const StepPlan &P = PL;
-  const int H = P.H, I = P.I, lg = 31 - __clz(I >> 7);
-  const int lo = SH->rng[kRngDown].x, nr = SH->rng[kRngDown].y - lo;
-  // residual input of this block's rows: complete since the router's barrier
-  float res0 = 0.0f;
-  if ((int)threadIdx.x < nr) res0 = __ldcg(P.Tmp + lo + threadIdx.x);
-  grid_wait(epoch);
-  quant_rows(P.Act, lg, P.slots);
-  stamp(2);
-  if (nr <= 0) return tile;
-  float *T = reinterpret_cast<float *>(step_smem + kTOff), *ts = reinterpret_cast<float *>(step_smem + kFbufOff);
+  const int H = P.H, I = P.I, lg = 31 - __clz(I >> 7), warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int lo = SH->rng[kRngDown].x, nr = SH->rng[kRngDown].y - lo, n = P.slots * nr;
+  float *xs = reinterpret_cast<float *>(step_smem + kFbufOff), *ts = xs + 4096;
+  const float *T = reinterpret_cast<const float *>(step_smem + kTOff);
   unsigned char *act = step_smem + kActOff;
-  const int n = P.slots * nr;
-  tile = dot_tiles<true>(tile, lg, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + (size_t)P.slots * I), T,
-                         n, nr);
+  await(target);
+  gather(xs, in, P.slots * I, flag);
   csync();
+  stamp(1);
+  if ((int)blockIdx.x == 0 && tid <= P.topk) {
+    const StepShared *sh = SH;
+    P.SelIdx[tid] = sh->sel_idx[tid];
+    P.SelW[tid] = sh->sel_w[tid];
+    if (tid == 0) *P.NearGap = sh->gap;
+    if (P.routed) {
+      P.routed[(size_t)L * (P.topk + 1) + tid] = sh->sel_idx[tid];
+      if (tid == 0) P.near_gap[L] = sh->gap;
+    }
+  }
 #pragma unroll 1
-  for (int f = threadIdx.x; f < n; f += kCons) ts[f] = SH->sel_w[f / nr] * row_terms(T, f, lg);
+  for (int gi = warp; gi < P.slots << lg; gi += 16)
+    stage_group(reinterpret_cast<uint32_t *>(act), reinterpret_cast<float *>(act + P.slots * I), 1 << lg, gi >> lg, gi & ((1 << lg) - 1),
+                quant_group(*reinterpret_cast<const float4 *>(xs + gi * 128 + lane * 4)));
   csync();
+  stamp(2);
+  tile = dot_tiles(tile, lg, P.slots * I, n, SH->down_recip);
 #pragma unroll 1
-  for (int r = threadIdx.x; r < nr; r += kCons) {
-    const float res = r < kCons ? res0 : __ldcg(P.Tmp + lo + r);
+  for (int f = tid; f < n; f += kCons) ts[f] = SH->sel_w[(int)(((float)f + 0.5f) * SH->down_recip)] * row_terms(T, f, lg);
+  csync();
+  if (tid < nr) {
     float acc = 0.0f;
 #pragma unroll 4
-    for (int s = 0; s < P.slots; ++s) acc = acc + ts[s * nr + r];
+    for (int s = 0; s < P.slots; ++s) acc = acc + ts[s * nr + tid];
     const float x = res + acc;
-    P.X[lo + r] = x;
-    if (P.layer_out) P.layer_out[(size_t)L * H + lo + r] = x;
+    put(out + lo + tid, x, flag);
+    if (L + 1 == P.layers) P.X[lo + tid] = x;
+    if (P.layer_out) P.layer_out[(size_t)L * H + lo + tid] = x;
   }
+  stamp(3);
   return tile;
 }
 
 // LM head in sub-blocks of 16 tiles (t[][] holds 256 rows of K = 2048), running argmax per thread.
-static __device__ __forceinline__ uint32_t lm_head_stage(uint32_t tile, float &bv, int &bi) {
+static __device__ __noinline__ uint32_t lm_head_stage(uint32_t tile, float &bv, int &bi) {
   const StepPlan &P = PL;
   const int K = P.H, lg = 31 - __clz(K >> 7);
   const int lo = SH->rng[kRngHead].x, hi = SH->rng[kRngHead].y;
-  float *T = reinterpret_cast<float *>(step_smem + kTOff);
-  unsigned char *act = step_smem + kActOff;
+  const float *T = reinterpret_cast<const float *>(step_smem + kTOff);
   const int sub = kTCap >> lg;  // rows whose terms fit t[][]: a whole, even number of tiles
 #pragma unroll 1
   for (int base = 0; base < hi - lo; base += sub) {
     const int nrows = (hi - lo) - base < sub ? (hi - lo) - base : sub;
-    tile = dot_tiles<false>(tile, lg, reinterpret_cast<const uint4 *>(act), reinterpret_cast<const float *>(act + K), T, nrows, 0);
-    csync();
+    tile = dot_tiles(tile, lg, K, nrows, 0.0f);
 #pragma unroll 1
     for (int r = threadIdx.x; r < nrows; r += kCons) {
       const float v = row_terms(T, r, lg);
@@ -1359,7 +1396,7 @@ static __device__ __forceinline__ uint32_t lm_head_stage(uint32_t tile, float &b
 // Block-wide first-max-wins argmax over the consumer threads; result valid in thread 0.
 static __device__ __noinline__ void cons_argmax(float &bv, int &bi) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
+#pragma unroll 1
   for (int off = 16; off > 0; off >>= 1)
     argmax_merge(bv, bi, __shfl_xor_sync(kFull, bv, off), __shfl_xor_sync(kFull, bi, off));
   if (lane == 0) {
@@ -1370,7 +1407,7 @@ static __device__ __noinline__ void cons_argmax(float &bv, int &bi) {
   if (warp == 0) {
     bv = lane < 16 ? SH->av[lane] : -INFINITY;
     bi = lane < 16 ? SH->ai[lane] : 0x7FFFFFFF;
-#pragma unroll
+#pragma unroll 1
     for (int off = 16; off > 0; off >>= 1)
       argmax_merge(bv, bi, __shfl_xor_sync(kFull, bv, off), __shfl_xor_sync(kFull, bi, off));
   }
@@ -1381,131 +1418,117 @@ static __device__ __forceinline__ void consumer_main(int mode) {
   StepShared *sh = SH;
   const int H = P.H, tid = threadIdx.x;
   uint32_t tile = 0;   // running index of the next ring tile to consume
-  unsigned epoch = 0;  // grid barriers this block has arrived at
+  const unsigned seq = __ldcg(P.sync + STEP_LAUNCHES), bar0 = __ldcg(P.sync + STEP_BAR_BASE);
+  unsigned bar = bar0;   // the count of arrivals when all blocks have ended the last stage
   const int token = __ldcg(P.ctrl + CTRL_TOKEN), pos = __ldcg(P.ctrl + CTRL_POS);
   int T = __ldcg(P.ctrl + CTRL_LEN);
   if (T > P.max_ctx) T = P.max_ctx;
   const int tok = token < 0 ? 0 : (token >= P.vocab ? P.vocab - 1 : token);
-  float *hn = reinterpret_cast<float *>(step_smem + kFbufOff) + 4096;
+  unsigned flag = seq * (unsigned)P.layers;
+  float res;
 
+#pragma unroll 1
   for (int L = 0; L < P.layers; ++L) {
     // the layer's record into shared memory (the previous layer's is no longer read: every
     // consumer has passed a block barrier behind its last use)
-    {
-      const uint4 *src = reinterpret_cast<const uint4 *>(P.L + L);
-      if (tid < (int)(sizeof(StepLayer) / 16)) reinterpret_cast<uint4 *>(&sh->ly)[tid] = __ldg(src + tid);
-      csync();
-    }
+    if (tid < (int)(sizeof(StepLayer) / 16))
+      reinterpret_cast<uint4 *>(&sh->ly)[tid] = __ldg(reinterpret_cast<const uint4 *>(P.L + L) + tid);
+    csync();
     const StepLayer &ly = sh->ly;
     const bool lin = ly.type == 0;
-    // the layer's table of experts into L2, a line a thread over the grid's first blocks
+    // words of this layer; the input's are the layer before's
+    unsigned long long *W = P.words + (L & 1 ? P.words_set : 0), *Wx = P.words + (L & 1 ? 0 : P.words_set);
+    // the layer's table of experts into L2, two lines a block
     {
       const int line = (int)blockIdx.x * 2 + tid;
       if (tid < 2 && line * 128 < (P.E + 1) * (int)sizeof(ExpertW))
         prefetch_l2(reinterpret_cast<const unsigned char *>(ly.experts) + line * 128);
     }
     // ---- stage 1: input norm + quantiser, first projections ----
-    norm_quant(epoch, P.X, L == 0 ? P.emb + (size_t)tok * H : nullptr, ly.in_norm, H, nullptr,
-               (L == 0 && (int)blockIdx.x == 0) ? P.X : nullptr);
-    stamp(2);
-    tile = gemv_stage_run(tile, &ly.m[0], lin ? 4 : 3, H, kRngIn + ly.type);
-    stamp(3);
-    grid_arrive();
-    ++epoch;
+    res = norm_quant(bar, Wx + P.wX, flag, L == 0 ? P.emb + (size_t)tok * H : nullptr, ly.in_norm, H, sh->rng[kRngOut + ly.type]);
+    ++flag;
+    tile = gemv_stage_run(tile, &ly.m[0], lin ? 4 : 3, H, sh->rng[kRngIn + ly.type], flag, 0.0f);
+    bar += gridDim.x;
+    arrive<false>();
     if (lin) {
-      // ---- stage 2: gated delta rule ----
-      deltanet_stage(epoch, ly);  // waits for the barrier inside, after its state loads
-      grid_arrive();
-      ++epoch;
-      // ---- stage 3: gated norm, out_proj + residual ----
-      gated_norm_quant(epoch, P.O, P.Z, ly.lin_norm, P.nV);
+      // ---- stage 2: gated delta rule; stage 3: gated norm, out_proj + residual ----
+      deltanet_stage(bar, ly, W + P.wM, W + P.wB, W + P.wG, W + P.wO, flag);
+      bar += gridDim.x;
+      arrive<false>();
+      gated_norm_quant(bar, W + P.wO, W + P.wZ, flag, ly.lin_norm, P.nV);
     } else {
-      attn_stage(epoch, ly, pos, T);  // waits for the barrier inside, after its KV loads
-      grid_arrive();
-      ++epoch;
-      grid_wait(epoch);
-      attn_combine_stage(T);
-      grid_arrive();
-      ++epoch;
-      grid_wait(epoch);
-      stage_q8(P.Q8, P.SQ, P.nQ * 256);
+      attn_stage(bar, ly, W + P.wQ, W + P.wK, W + P.wV, flag, pos, T);
+      bar += gridDim.x;
+      arrive<true>();   // the chunk partials are plain stores
+      await(bar);
+      stamp(1);
+      bar += gridDim.x;
+      attn_merge(bar, W + P.wQ, W + P.w8, flag, T);
     }
     stamp(2);
-    tile = gemv_stage_run(tile, &ly.m[4], 1, lin ? P.nV * 128 : P.nQ * 256, kRngOut + ly.type);
-    stamp(3);
-    grid_arrive();
-    ++epoch;
+    tile = gemv_stage_run(tile, &ly.m[4], 1, lin ? P.nV * 128 : P.nQ * 256, sh->rng[kRngOut + ly.type], flag, res);
+    bar += gridDim.x;
+    arrive<false>();
     // ---- stage 4: post norm + quantiser (kept staged for the experts), router logits ----
-    norm_quant(epoch, P.Tmp, nullptr, ly.post_norm, H, hn, nullptr);
-    stamp(2);
-    tile = router_stage(tile, hn, H);
+    res = norm_quant(bar, W + P.wT, flag, nullptr, ly.post_norm, H, sh->rng[kRngDown]);
+    tile = router_stage(tile, W + P.wR, flag, H);
     stamp(3);
-    grid_arrive();
-    ++epoch;
+    bar += gridDim.x;
+    arrive<false>();
     // ---- stage 5: selection, expert gate/up ----
-    router_select_cons(epoch, ly.experts, P.E, P.topk, ly.shared_gate != nullptr);
-    stamp(5);
-    tile = gateup_stage(tile);
+    router_select_cons(bar, W + P.wR, flag, ly.experts, P.E, P.topk, ly.shared_gate != nullptr);
+    tile = gateup_stage(tile, W + P.wA, flag);
     stamp(3);
-    grid_arrive();
-    ++epoch;
-    if ((int)blockIdx.x == 0 && tid <= P.topk) {
-      P.SelIdx[tid] = sh->sel_idx[tid];
-      P.SelW[tid] = sh->sel_w[tid];
-      if (tid == 0) *P.NearGap = sh->gap;
-      if (P.routed) {
-        P.routed[(size_t)L * (P.topk + 1) + tid] = sh->sel_idx[tid];
-        if (tid == 0) P.near_gap[L] = sh->gap;
-      }
-    }
+    bar += gridDim.x;
+    arrive<false>();
     // ---- stage 6: expert down, combine, residual ----
-    tile = down_stage(epoch, tile, L);
-    stamp(3);
-    grid_arrive();
-    ++epoch;
+    tile = down_stage(bar, tile, W + P.wA, W + P.wX, flag, res, L);
+    bar += gridDim.x;
+    arrive<false>();
   }
 
-  if (mode == 0) {
-    // prompt step: no logits; move on to the next prompt id
-    if ((int)blockIdx.x == 0 && tid == 0) {
-      const int np = pos + 1;
-      P.ctrl[CTRL_POS] = np;
-      P.ctrl[CTRL_LEN] = P.ctrl[CTRL_LEN] + 1;
-      if (np < P.max_ctx) P.ctrl[CTRL_TOKEN] = P.ids[np];
-      P.ctrl[CTRL_SELECTED] = -1;
-    }
-    return;
-  }
-  // ---- tail: final norm, LM head, first-max-wins argmax, control update ----
-  norm_quant(epoch, P.X, nullptr, P.final_norm, H, nullptr, nullptr);
-  float bv = -INFINITY;
-  int bi = 0x7FFFFFFF;
-  tile = lm_head_stage(tile, bv, bi);
-  cons_argmax(bv, bi);
-  if (tid == 0) {
-    P.PV[(int)blockIdx.x] = bv;
-    P.PI[(int)blockIdx.x] = bi;
-  }
-  grid_arrive();
-  ++epoch;
-  if ((int)blockIdx.x == 0) {
-    grid_wait(epoch);
-    bv = -INFINITY;
-    bi = 0x7FFFFFFF;
-    for (int i = tid; i < (int)gridDim.x; i += kCons) argmax_merge(bv, bi, __ldcg(P.PV + i), __ldcg(P.PI + i));
-    csync();
+  const bool lead = (int)blockIdx.x == 0;
+  if (mode != 0) {
+    // ---- tail: final norm, LM head, first-max-wins argmax ----
+    norm_quant(bar, P.words + (P.layers & 1 ? 0 : P.words_set) + P.wX, flag, nullptr, P.final_norm, H, make_int2(0, 0));
+    float bv = -INFINITY;
+    int bi = 0x7FFFFFFF;
+    tile = lm_head_stage(tile, bv, bi);
     cons_argmax(bv, bi);
     if (tid == 0) {
-      P.out_tok[0] = bi;
-      if (P.history && P.history_cap > 0) P.history[pos % P.history_cap] = bi;
-      P.ctrl[CTRL_SELECTED] = bi;
-      P.ctrl[CTRL_TOKEN] = bi;
-      P.ctrl[CTRL_POS] = pos + 1;
-      P.ctrl[CTRL_LEN] = P.ctrl[CTRL_LEN] + 1;
+      P.PV[(int)blockIdx.x] = bv;
+      P.PI[(int)blockIdx.x] = bi;
     }
+    bar += gridDim.x;
+    arrive<true>();
+    if (lead) {
+      await(bar);
+      bv = -INFINITY;
+      bi = 0x7FFFFFFF;
+      for (int i = tid; i < (int)gridDim.x; i += kCons) argmax_merge(bv, bi, __ldcg(P.PV + i), __ldcg(P.PI + i));
+      csync();
+      cons_argmax(bv, bi);
+      if (tid == 0) {
+        P.out_tok[0] = bi;
+        if (P.history && P.history_cap > 0) P.history[pos % P.history_cap] = bi;
+        P.ctrl[CTRL_SELECTED] = bi;
+        P.ctrl[CTRL_TOKEN] = bi;
+      }
+    }
+  } else if (lead && tid == 0) {
+    // prompt step: no logits; move on to the next prompt id
+    if (pos + 1 < P.max_ctx) P.ctrl[CTRL_TOKEN] = P.ids[pos + 1];
+    P.ctrl[CTRL_SELECTED] = -1;
+  }
+  // The control block and the launch's numbers for the next launch. Every block has read them: block 0 is
+  // here behind words that depend on every block's rows of the last layer.
+  if (lead && tid == 0) {
+    P.ctrl[CTRL_POS] = pos + 1;
+    P.ctrl[CTRL_LEN] = P.ctrl[CTRL_LEN] + 1;
+    P.sync[STEP_BAR_BASE] = bar;
+    P.sync[STEP_LAUNCHES] = seq + 1u;
   }
 }
-
 };
 
 template <bool kClock>
@@ -1521,7 +1544,6 @@ __device__ __forceinline__ void decode_step(const DecodeStepArgs &args) {
     sh->fail = 0;
     sh->nstamp[0] = 0;
     sh->nstamp[1] = 0;
-    sh->nseg = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x < sizeof(StepPlan) / 16)

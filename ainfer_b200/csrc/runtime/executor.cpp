@@ -311,20 +311,39 @@ int build_step(Session *s) {
   const int H = c.hidden, D = c.head_dim, nQ = c.q_heads, nKV = c.kv_heads, nV = c.lin_v_heads;
   const int C = c.conv_dim(), VD = c.value_dim(), E = c.experts;
   int status = 0;
+  StepPlan P;
+  std::memset(&P, 0, sizeof P);
+  {   // the words between the stages
+    const int slots = c.top_k + (c.shared_experts ? 1 : 0);
+    int at = 0;
+    auto part = [&](int32_t &off, int n) {
+      off = at;
+      at += (n + 1) & ~1;
+    };
+    part(P.wX, H); part(P.wT, H);
+    part(P.wM, C); part(P.wZ, VD); part(P.wB, nV); part(P.wG, nV); part(P.wO, VD);
+    part(P.wQ, nQ * 2 * D); part(P.wK, nKV * D); part(P.wV, nKV * D); part(P.w8, nQ * 66);
+    part(P.wR, E + 1); part(P.wA, slots * c.expert_inter);
+    P.words_set = at;
+    if (salloc(s, (size_t)2 * at, &s->step_words) || salloc(s, (size_t)STEP_SYNC_WORDS, &s->step_sync)) return 1;
+    P.words = s->step_words;
+    P.sync = s->step_sync;
+  }
   std::vector<StepLayer> layers((size_t)c.layers);
   for (int L = 0; L < c.layers && !status; ++L) {
     StepLayer &ly = layers[(size_t)L];
     std::memset(&ly, 0, sizeof ly);
     const std::string p = layer_prefix(L);
     const int slot = m->slot[L];
+    auto words = [&](int32_t off) { return reinterpret_cast<float *>(P.words + (L & 1 ? P.words_set : 0) + off); };
     ly.in_norm = m->in_norm + (size_t)L * H;
     ly.post_norm = m->post_norm + (size_t)L * H;
     if (c.layer_types[L] == 'A') {
       ly.type = 1;
-      ly.m[0] = make_mat(s, status, p + "self_attn.q_proj.weight", H, s->Q16, EPI_STORE, nullptr, nullptr, nullptr);
-      ly.m[1] = make_mat(s, status, p + "self_attn.k_proj.weight", H, s->K16, EPI_STORE, nullptr, nullptr, nullptr);
-      ly.m[2] = make_mat(s, status, p + "self_attn.v_proj.weight", H, s->V16, EPI_STORE, nullptr, nullptr, nullptr);
-      ly.m[4] = make_mat(s, status, p + "self_attn.o_proj.weight", nQ * D, s->Tmp, EPI_RESADD, s->X, nullptr, nullptr);
+      ly.m[0] = make_mat(s, status, p + "self_attn.q_proj.weight", H, words(P.wQ), EPI_STORE, nullptr, nullptr, nullptr);
+      ly.m[1] = make_mat(s, status, p + "self_attn.k_proj.weight", H, words(P.wK), EPI_STORE, nullptr, nullptr, nullptr);
+      ly.m[2] = make_mat(s, status, p + "self_attn.v_proj.weight", H, words(P.wV), EPI_STORE, nullptr, nullptr, nullptr);
+      ly.m[4] = make_mat(s, status, p + "self_attn.o_proj.weight", nQ * D, words(P.wT), EPI_RESADD, nullptr, nullptr, nullptr);
       ly.q_norm = m->q_norm + (size_t)slot * D;
       ly.k_norm = m->k_norm + (size_t)slot * D;
       size_t kv_off = (size_t)slot * s->max_ctx * nKV;
@@ -332,13 +351,13 @@ int build_step(Session *s) {
       ly.Ks = s->Ks + kv_off; ly.Vs = s->Vs + kv_off;
     } else {
       ly.type = 0;
-      ly.m[0] = make_mat(s, status, p + "linear_attn.in_proj_qkv.weight", H, s->Mx, EPI_CONV_SILU,
+      ly.m[0] = make_mat(s, status, p + "linear_attn.in_proj_qkv.weight", H, words(P.wM), EPI_CONV_SILU,
                          m->conv_w + (size_t)slot * C * 4, s->conv + (size_t)slot * C * 3, nullptr);
-      ly.m[1] = make_mat(s, status, p + "linear_attn.in_proj_z.weight", H, s->Z, EPI_SILU, nullptr, nullptr, nullptr);
-      ly.m[2] = make_mat(s, status, p + "linear_attn.in_proj_b.weight", H, s->Bt, EPI_BETA, nullptr, nullptr, nullptr);
-      ly.m[3] = make_mat(s, status, p + "linear_attn.in_proj_a.weight", H, s->Gt, EPI_GDECAY,
+      ly.m[1] = make_mat(s, status, p + "linear_attn.in_proj_z.weight", H, words(P.wZ), EPI_SILU, nullptr, nullptr, nullptr);
+      ly.m[2] = make_mat(s, status, p + "linear_attn.in_proj_b.weight", H, words(P.wB), EPI_BETA, nullptr, nullptr, nullptr);
+      ly.m[3] = make_mat(s, status, p + "linear_attn.in_proj_a.weight", H, words(P.wG), EPI_GDECAY,
                          m->a_log + (size_t)slot * nV, nullptr, m->dt_bias + (size_t)slot * nV);
-      ly.m[4] = make_mat(s, status, p + "linear_attn.out_proj.weight", VD, s->Tmp, EPI_RESADD, s->X, nullptr, nullptr);
+      ly.m[4] = make_mat(s, status, p + "linear_attn.out_proj.weight", VD, words(P.wT), EPI_RESADD, nullptr, nullptr, nullptr);
       ly.S = s->S + (size_t)slot * nV * 128 * 128;
       ly.lin_norm = m->lin_norm + (size_t)slot * c.lin_head_dim;
     }
@@ -349,8 +368,6 @@ int build_step(Session *s) {
     ly.experts = (const ExpertW *)m->expert_tables + (size_t)L * (E + 1);
   }
   if (status) return status;
-  StepPlan P;
-  std::memset(&P, 0, sizeof P);
   P.H = H; P.layers = c.layers; P.vocab = c.vocab;
   P.nQ = nQ; P.nKV = nKV; P.rot = c.rotary_dim; P.nK = c.lin_k_heads; P.nV = nV;
   P.E = E; P.topk = c.top_k; P.slots = c.top_k + (c.shared_experts ? 1 : 0); P.I = c.expert_inter;
@@ -364,20 +381,18 @@ int build_step(Session *s) {
   P.lm_head = make_mat(s, status, "lm_head.weight", H, s->Logits, EPI_STORE, nullptr, nullptr, nullptr);
   if (status) return status;
   P.Cos = m->rope_cos; P.Sin = m->rope_sin;
-  P.X = s->X; P.Tmp = s->Tmp; P.Mx = s->Mx; P.Z = s->Z; P.Bt = s->Bt; P.Gt = s->Gt; P.O = s->O;
-  P.Q16 = s->Q16; P.K16 = s->K16; P.V16 = s->V16; P.Qn = s->Qn; P.Pm = s->Pm; P.Pse = s->Pse; P.Pacc = s->Pacc;
-  P.RLogits = s->RLogits; P.Act = s->Act; P.Logits = s->Logits; P.PV = s->PV; P.PI = s->PI;
-  P.Q8 = s->Q8; P.SQ = s->SQ; P.SelIdx = s->SelIdx; P.SelW = s->SelW; P.NearGap = s->NearGap;
+  P.X = s->X; P.Pm = s->Pm; P.Pse = s->Pse; P.Pacc = s->Pacc; P.Logits = s->Logits; P.PV = s->PV; P.PI = s->PI;
+  P.SelIdx = s->SelIdx; P.SelW = s->SelW; P.NearGap = s->NearGap;
   P.ctrl = s->ctrl; P.history = s->history; P.out_tok = s->out_tok; P.ids = s->ids;
   P.layer_out = s->layer_out; P.routed = s->routed; P.near_gap = s->near_gap;
-  if (salloc(s, 1, &s->bar_count) || salloc(s, 1, &s->step_error)) return 1;
+  if (salloc(s, 1, &s->step_error)) return 1;
   if (s->flags & SESSION_STAGE_CLOCK) {
     s->stage_stamp_cap = 2 * (c.layers * 64 + 64);  // first half: barrier clock, second half: fine clock
     if (salloc(s, (size_t)s->stage_stamp_cap, &s->stage_stamps)) return 1;
     P.stage_stamps = s->stage_stamps;
     P.stage_stamp_cap = s->stage_stamp_cap;
   }
-  P.bar_count = s->bar_count; P.error = s->step_error;
+  P.error = s->step_error;
   P.in_rows[0] = C + VD + 2 * nV;
   P.in_rows[1] = nQ * 2 * D + 2 * nKV * D;
   StepLayer *dl = nullptr;
@@ -406,6 +421,12 @@ int build_step(Session *s) {
     return 1;
   }
   groups = std::min<uint32_t>(groups, (uint32_t)s->sm_count);
+  // every block owns rows of every layer's first stage: the words' two sets rely on it (k_step.cu)
+  for (int t = 0; t < 2; ++t)
+    if (t == 0 ? c.n_lin() > 0 : c.n_attn() > 0) {
+      const int unit = H >= 1024 ? 1 : 1024 / H;
+      groups = std::min<uint32_t>(groups, (uint32_t)((P.in_rows[t] + unit - 1) / unit));
+    }
   if ((int)groups > s->argmax_parts) { s->err = "internal: argmax partial buffers too small"; return 3; }
   {
     // what one block must hold per stage: (rows x K/128) group terms <= 4096, staged activations
@@ -420,7 +441,8 @@ int build_step(Session *s) {
     ok = ok && 2 * share((long)slots * P.I, unit(H)) * (H / 128) <= 4096;
     ok = ok && slots * share(H, unit(P.I)) * (P.I / 128) <= 4096;
     ok = ok && (long)slots * P.I <= 8192 && std::max(VD, nQ * D) <= 4096 && H <= 4096 && slots <= 12 && E + 1 <= 8192;
-    ok = ok && (c.n_attn() == 0 || nQ / nKV <= 8);
+    ok = ok && (c.n_attn() == 0 || nQ / nKV <= 8) && share(H, 8) <= 512;
+    ok = ok && share(std::max(in_rows, qkv_rows), unit(H)) <= 512;
     if (!ok) {
       s->err = "usage: this model's shapes do not fit the persistent decode kernel on " + std::to_string(groups) +
                " blocks; use the recorded list";
@@ -432,8 +454,7 @@ int build_step(Session *s) {
     if (ainfer_list_create(s->dev, l) != AINFER_OK) { s->err = "list create failed"; return 1; }
     mode = md;
     ainfer_kernel_set_arg(k, 1, sizeof mode, &mode);
-    if (ainfer_list_append_fill(*l, s->bar_count, 0, 4) != AINFER_OK ||
-        ainfer_list_append_launch(*l, k, groups) != AINFER_OK || ainfer_list_close(*l) != AINFER_OK) {
+    if (ainfer_list_append_launch(*l, k, groups) != AINFER_OK || ainfer_list_close(*l) != AINFER_OK) {
       s->err = std::string("recording the persistent step failed: ") + ainfer_last_error(s->dev);
       return 1;
     }

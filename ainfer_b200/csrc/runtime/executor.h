@@ -84,7 +84,8 @@ struct Session {
   ainfer_list_t embed_list = nullptr, tail_list = nullptr, advance_list = nullptr;
   // persistent-kernel path: device plan, barrier counter, sticky error word
   void *step_plan = nullptr, *step_layers = nullptr;
-  uint32_t *bar_count = nullptr;
+  uint32_t *step_sync = nullptr;        // STEP_SYNC_WORDS numbers of the persistent step
+  unsigned long long *step_words = nullptr;
   int32_t *step_error = nullptr;
   bool persistent = false;
   unsigned long long *stage_stamps = nullptr;  // [stage_stamp_cap] of the last launch
