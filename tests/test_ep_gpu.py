@@ -78,6 +78,20 @@ def test_counts_by_rows_of_an_expert(batch):
     ep.close(); model.close(); dev.close()
 
 
+# mean rows of an expert 8 and just above, 20 and just above, and 24: problems of 16, 32 and 64 rows
+@pytest.mark.parametrize("batch", [128, 129, 320, 321, 384])
+def test_problems_of_every_cut(batch):
+    from ainfer_b200 import cuda_abi, runtime
+    dev = cuda_abi.Device(0)
+    model = runtime.Model(dev, "synth:tiny:seed=2")
+    ep = runtime.EpMoe(model, batch)
+    res = _batch(model.config["hidden"], batch, seed=batch)
+    got = ep.layer(1, res)
+    want, _ = _oracle_rows("tiny", 2, 1, res)
+    assert np.array_equal(got, want)
+    ep.close(); model.close(); dev.close()
+
+
 @pytest.mark.parametrize("world,n,cut", [(2, 20, 16), (4, 3, 64), (2, 40, 64), (1, 9, 5)])
 def test_kernels_of_several_ranks_one_after_the_other(world, n, cut):
     """Plan, pack, group, gather, both grouped products, scatter and combine of every rank, one rank after the other on one
