@@ -198,7 +198,7 @@ struct EpTcGroup {           // = TcGroup of the grouped tensor-core GEMM
 static_assert(sizeof(EpTcGroup) == 32, "layout of the grouped GEMM's problem record");
 // Counts of a grouping: items in total; gate/up and down problems of experts with at most eight rows; the same of experts
 // with more; gate/up and down problems in the lists.
-constexpr int kEpFewRows = 8, kEpCountGateUp = 5, kEpCountDown = 6;
+constexpr int kEpFewRows = 8;
 __device__ __forceinline__ void ep_store_counts(int32_t *c, int items, int few, int all) {
   reinterpret_cast<int4 *>(c)[0] = make_int4(items, 2 * few, few, 2 * (all - few));
   reinterpret_cast<int4 *>(c)[1] = make_int4(all - few, 2 * all, all, 0);
@@ -325,9 +325,13 @@ struct EpGroupLocalArgs {
   int32_t *Counts;            // [8], see ep_store_counts
   int32_t n, k, E, I;
   int32_t shared_row0, shared_rows, max_rows;
-  int32_t *Lists;             // optional (null: Counts counts by max_rows): [2] lengths of the lists, and Counts counts by 64 rows
 };
-__global__ void __launch_bounds__(1024) EpGroupLocal(const EpGroupLocalArgs a) {
+struct EpGroupLocalCutArgs {
+  EpGroupLocalArgs g;
+  int32_t *Lists;             // [2] lengths of the lists; Counts counts by 64 rows whatever max_rows is
+};
+// Lists: null: Counts counts by max_rows.
+__device__ __forceinline__ void ep_group_local(const EpGroupLocalArgs &a, int32_t *Lists) {
   __shared__ int hist[1024], start[1024], wsum[2][33];
   pdl_launch_dependents();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, items = a.n * a.k;
@@ -379,15 +383,15 @@ __global__ void __launch_bounds__(1024) EpGroupLocal(const EpGroupLocalArgs a) {
   if (c > 0) ep_problems(a.GroupsGateUp, a.GroupsDown, a.Experts[tid], first, c, a.max_rows, a.I, g0);
   const int few = __syncthreads_count(c > 0 && c <= kEpFewRows);
   int counted = total, by = a.max_rows;
-  if (a.Lists) {   // the documented counts are by 64 rows, whatever the lists' cut
+  if (Lists) {   // the documented counts are by 64 rows, whatever the lists' cut
     by = 64;
     counted = 0;
 #pragma unroll 1
     for (int j = 0; j * 64 < a.n; ++j) counted += __syncthreads_count(c > j * 64);   // an expert has an item of a row at most once
     if (tid == 0) {
       const int lists = total + (a.shared_rows + a.max_rows - 1) / a.max_rows;
-      a.Lists[0] = 2 * lists;
-      a.Lists[1] = lists;
+      Lists[0] = 2 * lists;
+      Lists[1] = lists;
     }
   }
   if (tid == 1023) {
@@ -395,6 +399,8 @@ __global__ void __launch_bounds__(1024) EpGroupLocal(const EpGroupLocalArgs a) {
     ep_store_counts(a.Counts, items, few + (a.shared_rows > 0 && a.shared_rows <= kEpFewRows), counted + (a.shared_rows + by - 1) / by);
   }
 }
+__global__ void __launch_bounds__(1024) EpGroupLocal(const EpGroupLocalArgs a) { ep_group_local(a, nullptr); }
+__global__ void __launch_bounds__(1024) EpGroupLocalCut(const EpGroupLocalCutArgs a) { ep_group_local(a.g, a.Lists); }
 struct EpGatherLocalArgs {
   const int8_t *Q8;        // [n][H]
   const float *SQ;         // [n][H/128]
@@ -528,7 +534,11 @@ AINFER_REGISTER(EpGather, EpGatherArgs, 128, 1, 0, nullptr, F(Recv), F(Sorted), 
 #undef F
 #define F(f) AINFER_ARG(EpGroupLocalArgs, f)
 AINFER_REGISTER(EpGroupLocal, EpGroupLocalArgs, 1024, 0, 0, nullptr, F(SelIdx), F(Experts), F(Sorted), F(ItemRow), F(GroupsGateUp), F(GroupsDown),
-                F(Counts), F(n), F(k), F(E), F(I), F(shared_row0), F(shared_rows), F(max_rows), F(Lists));
+                F(Counts), F(n), F(k), F(E), F(I), F(shared_row0), F(shared_rows), F(max_rows));
+#undef F
+#define F(f) AINFER_ARG(EpGroupLocalCutArgs, f)
+AINFER_REGISTER(EpGroupLocalCut, EpGroupLocalCutArgs, 1024, 0, 0, nullptr, F(g.SelIdx), F(g.Experts), F(g.Sorted), F(g.ItemRow), F(g.GroupsGateUp),
+                F(g.GroupsDown), F(g.Counts), F(g.n), F(g.k), F(g.E), F(g.I), F(g.shared_row0), F(g.shared_rows), F(g.max_rows), F(Lists));
 #undef F
 #define F(f) AINFER_ARG(EpGatherLocalArgs, f)
 AINFER_REGISTER(EpGatherLocal, EpGatherLocalArgs, 128, 1, 0, nullptr, F(Q8), F(SQ), F(Sorted), F(XQ), F(XS), F(H), F(k));
@@ -546,6 +556,7 @@ AINFER_REGISTER(EpCombine, EpCombineArgs, 256, 0, 0, nullptr, F(Res), F(Back), F
 AINFER_EARLY_LAUNCH(RouterLogitsRows);
 AINFER_EARLY_LAUNCH(RouterSelectRows);
 AINFER_EARLY_LAUNCH(EpGroupLocal);
+AINFER_EARLY_LAUNCH(EpGroupLocalCut);
 AINFER_EARLY_LAUNCH(EpGatherLocal);
 AINFER_EARLY_LAUNCH(SiluQuantRows);
 AINFER_EARLY_LAUNCH(EpCombine);

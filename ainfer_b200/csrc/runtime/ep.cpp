@@ -244,7 +244,7 @@ int emit_local(EpMoe *e, Rec &r, int L, int rows) {
   if (emit_route(e, r, L, rows)) return 1;
   const ExpertW *tab = (const ExpertW *)e->m->expert_tables + (size_t)L * (e->E + 1);
   const int items = rows * e->k, shared_rows = e->shared ? rows : 0, cut = std::min(rows, problem_rows(items, e->E));
-  r.launch("EpGroupLocal", 1u, (const int32_t *)e->SelIdx, tab, e->Sorted, e->ItemDest, e->GroupsGU, e->GroupsD, e->Counts, (int32_t)rows,
+  r.launch("EpGroupLocalCut", 1u, (const int32_t *)e->SelIdx, tab, e->Sorted, e->ItemDest, e->GroupsGU, e->GroupsD, e->Counts, (int32_t)rows,
            (int32_t)e->k, (int32_t)e->E, (int32_t)e->I, (int32_t)e->cap, (int32_t)shared_rows, (int32_t)cut, e->Lists);
   r.launch("EpGatherLocal", (uint32_t)items, (const int8_t *)e->Q8, (const float *)e->SQ, (const int32_t *)e->Sorted, e->XQs, e->SQs, (int32_t)e->H,
            (int32_t)e->k);
