@@ -100,10 +100,12 @@ extern __shared__ __align__(16) float chunk_smem[];
 // One block per (head, 32-column slice); grid = nV * 4. Per row the arithmetic of deltanet_step_body:
 // S *= exp(g); kv = tree8 of 16-row fma chains; d = (v - kv) * beta; S += k d; o = tree8 of fma chains
 // with q. A warp holds eight columns, a lane two of a column's eight segments of 16 rows (two chains side by
-// side), so that the tree is one addition and two exchanges inside the warp and the rows of a chunk need no
-// barrier; a row's output is summed beside the next row's kv. Eight more warps normalise the next chunk's
+// side, one packed instruction for both), so that the tree is one addition and two exchanges inside the warp and the rows of a
+// chunk need no barrier; a row's output is summed beside the next row's kv. Eight more warps normalise the next chunk's
 // q and k meanwhile and fetch its values. Bound by the chain of a row. (Segments in different warps, two
-// block barriers a row: 130 us for 192 rows of 32 heads; this form 58.)
+// block barriers a row: 130 us for 192 rows of 32 heads; this form 58. 701 rows: 199 us with scalar, 193 with packed instructions;
+// output and next row's kv in one pass over the state 215, and with one segment of two columns a lane 226: what a pass more costs in
+// reads of shared memory or in exchanges is more than the chain it shortens.)
 __global__ void __launch_bounds__(kChunkThreads) ChunkDeltaNet(const ChunkDeltaNetArgs a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(kChunkThreads) ChunkDeltaNet(const ChunkDeltaN
         float *dst = (which == 0 ? qs : ks) + mm * kChunkRow;
         if (mm < rows) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) dst[36 * i + lane] = x[u][i] * f;
+          for (int i = 0; i < 4; ++i) dst[36 * i + 2 * (lane & 15) + (lane >> 4)] = x[u][i] * f;   // the two segments of a quarter take turns
         }
       }
     }
@@ -160,13 +162,14 @@ __global__ void __launch_bounds__(kChunkThreads) ChunkDeltaNet(const ChunkDeltaN
   const bool helper = warp >= kChunkWarps;
   const int quarter = lane & 3, wcol = warp * 8 + (lane >> 2), col = slice * 32 + wcol;   // a lane's segments: 2 quarter, 2 quarter + 1
   float *Sh = a.S + (size_t)h * D * D + (size_t)quarter * (2 * SEG) * D + col;
-  float s[2 * SEG], po = 0.0f;
+  uint64_t s[SEG];   // row r of the lane's two segments
+  float po = 0.0f;
   float *out = a.Out + (size_t)h * D + col;   // of the last row begun
   if (helper) {
     if (chunks > 0) stage(0);
   } else {
 #pragma unroll
-    for (int r = 0; r < 2 * SEG; ++r) s[r] = Sh[(size_t)r * D];
+    for (int r = 0; r < SEG; ++r) s[r] = pair2(Sh[(size_t)r * D], Sh[(size_t)(SEG + r) * D]);
   }
   __syncthreads();
   for (int ch = 0; ch < chunks; ++ch) {
@@ -180,45 +183,47 @@ __global__ void __launch_bounds__(kChunkThreads) ChunkDeltaNet(const ChunkDeltaN
 #pragma unroll 1
       for (int m = 0; m < rows; ++m) {
         const float gt = s_gt[ch & 1][m], beta = s_beta[ch & 1][m], val = vs[m * 32];
-        float k[2 * SEG], q[2 * SEG];
+        uint64_t k[SEG], q[SEG];
 #pragma unroll
-        for (int i = 0; i < 2 * SEG / 4; ++i) {
-          const float4 k4 = *reinterpret_cast<const float4 *>(ks + m * kChunkRow + 4 * i);
-          k[4 * i] = k4.x; k[4 * i + 1] = k4.y; k[4 * i + 2] = k4.z; k[4 * i + 3] = k4.w;
+        for (int i = 0; i < SEG / 2; ++i) {
+          const ulonglong2 k2 = *reinterpret_cast<const ulonglong2 *>(ks + m * kChunkRow + 4 * i);
+          k[2 * i] = k2.x; k[2 * i + 1] = k2.y;
         }
 #pragma unroll
-        for (int i = 0; i < 2 * SEG / 4; ++i) {
-          const float4 q4 = *reinterpret_cast<const float4 *>(qs + m * kChunkRow + 4 * i);
-          q[4 * i] = q4.x; q[4 * i + 1] = q4.y; q[4 * i + 2] = q4.z; q[4 * i + 3] = q4.w;
+        for (int i = 0; i < SEG / 2; ++i) {
+          const ulonglong2 q2 = *reinterpret_cast<const ulonglong2 *>(qs + m * kChunkRow + 4 * i);
+          q[2 * i] = q2.x; q[2 * i + 1] = q2.y;
         }
-        float c0 = 0.0f, c1 = 0.0f;
+        const uint64_t gt2 = pair2(gt, gt);
+        uint64_t c = 0;   // two zeros
 #pragma unroll
         for (int r = 0; r < SEG; ++r) {
-          s[r] = s[r] * gt;
-          s[SEG + r] = s[SEG + r] * gt;
-          c0 = fmaf(s[r], k[r], c0);
-          c1 = fmaf(s[SEG + r], k[SEG + r], c1);
+          s[r] = mul2(s[r], gt2);
+          c = fma2(s[r], k[r], c);
         }
-        float kv = c0 + c1, o = po;   // the tree's first level; then this row's kv beside the last row's output
+        float kv = sum2(c), o = po;   // the tree's first level; then this row's kv beside the last row's output
         kv = kv + __shfl_xor_sync(kFull, kv, 1);
         o = o + __shfl_xor_sync(kFull, o, 1);
         kv = kv + __shfl_xor_sync(kFull, kv, 2);
         o = o + __shfl_xor_sync(kFull, o, 2);
         if (quarter == 0 && m0 + m > 0) out[(size_t)(m0 + m - 1) * a.nV * D] = o;
         const float dl = (val - kv) * beta;
-        c0 = c1 = 0.0f;
+        const uint64_t dl2 = pair2(dl, dl);
+        c = 0;
 #pragma unroll
         for (int r = 0; r < SEG; ++r) {
-          s[r] = fmaf(k[r], dl, s[r]);
-          s[SEG + r] = fmaf(k[SEG + r], dl, s[SEG + r]);
-          c0 = fmaf(s[r], q[r], c0);
-          c1 = fmaf(s[SEG + r], q[SEG + r], c1);
+          s[r] = fma2(k[r], dl2, s[r]);
+          c = fma2(s[r], q[r], c);
         }
-        po = c0 + c1;
+        po = sum2(c);
         if (a.Snap) {
           float *sn = a.Snap + (size_t)(m0 + m) * a.snap_stride + (size_t)h * D * D + (size_t)quarter * (2 * SEG) * D + col;
 #pragma unroll
-          for (int r = 0; r < 2 * SEG; ++r) sn[(size_t)r * D] = s[r];
+          for (int r = 0; r < SEG; ++r) {
+            const float2 v = unpair2(s[r]);
+            sn[(size_t)r * D] = v.x;
+            sn[(size_t)(SEG + r) * D] = v.y;
+          }
         }
       }
     }
@@ -229,7 +234,11 @@ __global__ void __launch_bounds__(kChunkThreads) ChunkDeltaNet(const ChunkDeltaN
     o = o + __shfl_xor_sync(kFull, o, 2);
     if (quarter == 0 && a.M > 0) out[(size_t)(a.M - 1) * a.nV * D] = o;
 #pragma unroll
-    for (int r = 0; r < 2 * SEG; ++r) Sh[(size_t)r * D] = s[r];
+    for (int r = 0; r < SEG; ++r) {
+      const float2 v = unpair2(s[r]);
+      Sh[(size_t)r * D] = v.x;
+      Sh[(size_t)(SEG + r) * D] = v.y;
+    }
   }
 }
 

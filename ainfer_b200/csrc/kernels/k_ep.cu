@@ -38,12 +38,13 @@ struct RouterLogitsRowsArgs {
 // chunk for 32 16-byte reads of activations at 16 tokens, which the shared memory serves in the time of the
 // multiply-adds. Activations are staged 1024 columns at a time, a lane's two quarters of its eight values
 // apart (side by side they meet the same banks). (One router row per warp and four tokens: bound by those
-// reads, 74 us for 192 tokens of 513 x 2048; this form 25.)
+// reads, 74 us for 192 tokens of 513 x 2048; this form 25.) Tokens go in pairs, one packed multiply-add for both, so
+// they lie in turns in shared memory: 701 tokens 76 us with scalar instructions, 64 packed.
 constexpr int kRlRows = 32, kRlCols = 1024, kRlChunks = kRlCols / 256;
 __host__ __device__ inline int rl_tokens(int tokens_per_block) { return tokens_per_block >= 16 ? 16 : 8; }
 template <int TT>
 __device__ __forceinline__ void router_logits_rows_unit(const RouterLogitsRowsArgs &a, int unit) {
-  extern __shared__ __align__(16) float rl_smem[];   // [TT][kRlChunks][2][32 lanes][4]
+  extern __shared__ __align__(16) float rl_smem[];   // [TT / 2][kRlChunks][4][32 lanes][2 columns][2 tokens]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nrows = a.E + (a.Wsg ? 1 : 0), n = a.H / 256;
   const int nrb = (a.E + 1 + kRlRows - 1) / kRlRows, e0 = (unit % nrb) * kRlRows + warp * 4, t0 = (unit / nrb) * TT;
@@ -53,18 +54,22 @@ __device__ __forceinline__ void router_logits_rows_unit(const RouterLogitsRowsAr
     const int e = min(e0 + j, nrows - 1);
     w[j] = reinterpret_cast<const uint4 *>(e < a.E ? a.Wr + (size_t)e * a.H : a.Wsg) + lane;
   }
-  float acc[TT][4];
+  uint64_t acc[TT / 2][4];   // two tokens' sums
 #pragma unroll
-  for (int u = 0; u < TT; ++u)
+  for (int u = 0; u < TT / 2; ++u)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[u][j] = 0.0f;
+    for (int j = 0; j < 4; ++j) acc[u][j] = 0;
   for (int i0 = 0; i0 < n; i0 += kRlChunks) {
     const int nc = min(kRlChunks, n - i0);
     __syncthreads();   // the last columns' readers are done
-    for (int i = threadIdx.x; i < TT * nc * 64; i += 256) {
-      const int u = i / (nc * 64), f = i % (nc * 64), c = f >> 6, q = f & 63;   // token (past the end: the last one, not stored), chunk, quarter
-      const float4 v = __ldcg(reinterpret_cast<const float4 *>(a.Hn + (size_t)min(t0 + u, a.rows - 1) * a.H + (size_t)(i0 + c) * 256) + q);
-      reinterpret_cast<float4 *>(rl_smem)[((u * kRlChunks + c) * 2 + (q & 1)) * 32 + (q >> 1)] = v;
+    for (int i = threadIdx.x; i < TT / 2 * nc * 64; i += 256) {
+      const int u = i / (nc * 64), f = i % (nc * 64), c = f >> 6, q = f & 63;   // pair of tokens (past the end: the last one, not stored), chunk, quarter
+      const float *h = a.Hn + (size_t)(i0 + c) * 256 + q * 4;
+      const float4 v0 = __ldcg(reinterpret_cast<const float4 *>(h + (size_t)min(t0 + 2 * u, a.rows - 1) * a.H)),
+                   v1 = __ldcg(reinterpret_cast<const float4 *>(h + (size_t)min(t0 + 2 * u + 1, a.rows - 1) * a.H));
+      float4 *d = reinterpret_cast<float4 *>(rl_smem) + ((u * kRlChunks + c) * 4 + 2 * (q & 1)) * 32 + (q >> 1);
+      d[0] = make_float4(v0.x, v1.x, v0.y, v1.y);
+      d[32] = make_float4(v0.z, v1.z, v0.w, v1.w);
     }
     __syncthreads();
     uint4 wv[4];
@@ -72,38 +77,38 @@ __device__ __forceinline__ void router_logits_rows_unit(const RouterLogitsRowsAr
     for (int j = 0; j < 4; ++j) wv[j] = __ldg(w[j] + (size_t)i0 * 32);
 #pragma unroll 1
     for (int c = 0; c < nc; ++c) {
-      float f[4][8];
+      uint4 wn[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        f[j][0] = u2f(wv[j].x << 16); f[j][1] = u2f(wv[j].x & 0xFFFF0000u); f[j][2] = u2f(wv[j].y << 16); f[j][3] = u2f(wv[j].y & 0xFFFF0000u);
-        f[j][4] = u2f(wv[j].z << 16); f[j][5] = u2f(wv[j].z & 0xFFFF0000u); f[j][6] = u2f(wv[j].w << 16); f[j][7] = u2f(wv[j].w & 0xFFFF0000u);
-      }
+      for (int j = 0; j < 4; ++j) wn[j] = __ldg(w[j] + (size_t)min(i0 + c + 1, n - 1) * 32);
+      const ulonglong2 *x = reinterpret_cast<const ulonglong2 *>(rl_smem) + c * 128 + lane;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) wv[j] = __ldg(w[j] + (size_t)min(i0 + c + 1, n - 1) * 32);
-      const float4 *x = reinterpret_cast<const float4 *>(rl_smem) + c * 64 + lane;
-#pragma unroll
-      for (int u = 0; u < TT; ++u) {
-        const float4 x0 = x[u * (kRlChunks * 64)], x1 = x[u * (kRlChunks * 64) + 32];
+      for (int p = 0; p < 4; ++p) {   // columns 2 p and 2 p + 1 of the lane's eight
+        uint64_t f0[4], f1[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          float s = acc[u][j];
-          s = fmaf(f[j][0], x0.x, s);
-          s = fmaf(f[j][1], x0.y, s);
-          s = fmaf(f[j][2], x0.z, s);
-          s = fmaf(f[j][3], x0.w, s);
-          s = fmaf(f[j][4], x1.x, s);
-          s = fmaf(f[j][5], x1.y, s);
-          s = fmaf(f[j][6], x1.z, s);
-          s = fmaf(f[j][7], x1.w, s);
-          acc[u][j] = s;
+          const uint32_t v = p == 0 ? wv[j].x : p == 1 ? wv[j].y : p == 2 ? wv[j].z : wv[j].w;
+          const float lo = u2f(v << 16), hi = u2f(v & 0xFFFF0000u);
+          f0[j] = pair2(lo, lo);
+          f1[j] = pair2(hi, hi);
+        }
+#pragma unroll
+        for (int u = 0; u < TT / 2; ++u) {
+          const ulonglong2 xv = x[(u * kRlChunks * 4 + p) * 32];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[u][j] = fma2(f0[j], xv.x, acc[u][j]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[u][j] = fma2(f1[j], xv.y, acc[u][j]);
         }
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) wv[j] = wn[j];
     }
   }
   const int own = warp_tree_owner<8>(lane);   // of eight sums (two tokens x four rows), the one this lane ends with
 #pragma unroll
   for (int u = 0; u < TT; u += 2) {
-    const float v[8] = {acc[u][0], acc[u][1], acc[u][2], acc[u][3], acc[u + 1][0], acc[u + 1][1], acc[u + 1][2], acc[u + 1][3]};
+    const float2 s0 = unpair2(acc[u / 2][0]), s1 = unpair2(acc[u / 2][1]), s2 = unpair2(acc[u / 2][2]), s3 = unpair2(acc[u / 2][3]);
+    const float v[8] = {s0.x, s1.x, s2.x, s3.x, s0.y, s1.y, s2.y, s3.y};
     const float sum = warp_tree_sum_multi<8>(v, lane);
     const int t = t0 + u + (own >> 2), e = e0 + (own & 3);
     if ((lane & 3) == 0 && t < a.rows && e < nrows)
