@@ -31,6 +31,10 @@
 //   2048 x 4096, 64                    61.8 -> 13.3                 151936 x 2048, 64  286 -> 98
 //   experts of 512, gate and up, 1.25 / 3.75 / 13.7 rows on average   136 -> 107, 277 -> 148, 793 -> 174
 //   the same, down                                                     85 -> 72, 173 -> 101, 430 -> 113
+// Rescaling two entries in one packed instruction, and the first product of a group starting from the constant itself: experts of
+// a 701-row pass 145 -> 138 us a launch on average. Several matrices over the same rows in one launch (Int4GemmA8TcMany: a hybrid
+// layer's 8192 + 4096 + 32 + 32 outputs of 2048, where a matrix of 32 rows alone is 8..11 us): 701 rows 140 -> 99 us,
+// 64 rows 36 -> 18. Three blocks per SM of three stages each for lists of few rows: 73 us a launch against 69.
 #include "block_dot.cuh"
 
 namespace ainfer {
@@ -42,6 +46,17 @@ struct Int4GemmA8TcArgs {
   const float *SQ;     // [M][K/128] activation group scales
   float *Y;            // [M][ldy]
   int32_t N, K, M, ldy;
+  int32_t ahead;       // LaunchAhead
+};
+// One to four matrices of the same K over the same rows; an output's row stride is its matrix's N.
+struct Int4GemmA8TcManyArgs {
+  const int8_t *XQ;
+  const float *SQ;
+  int32_t K, M, count;
+  const uint8_t *P0; const uint16_t *S0; float *Y0; int32_t N0;
+  const uint8_t *P1; const uint16_t *S1; float *Y1; int32_t N1;
+  const uint8_t *P2; const uint16_t *S2; float *Y2; int32_t N2;
+  const uint8_t *P3; const uint16_t *S3; float *Y3; int32_t N3;
   int32_t ahead;       // LaunchAhead
 };
 
@@ -75,6 +90,12 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint
       : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The first product of a chain: d = a b + start in all four.
+__device__ __forceinline__ void mma_s8_from(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int start) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(start));
+}
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
@@ -89,8 +110,7 @@ __host__ __device__ constexpr int tc_stages(int nt) { return nt == 16 ? 5 : nt =
 __host__ __device__ constexpr uint32_t tc_stage_bytes(int nt) { return kTcWBytes + (uint32_t)nt * kTcXPitch + (uint32_t)nt * 8u + kTcRows * 4u; }
 // Entries per unit of one problem: what finishes first over whole rounds of units on the SMs. A stage costs
 // the products of its entries, and the widening and copying whatever their number.
-__host__ __device__ inline int tc_entries(int N, int M) {
-  const int tiles = (N + kTcRows - 1) / kTcRows;
+__host__ __device__ inline int tc_entries(int tiles, int M) {
   int best = 16;
   long cost = -1;
   for (int nt = 16; nt <= 64; nt *= 2) {
@@ -102,36 +122,48 @@ __host__ __device__ inline int tc_entries(int N, int M) {
 }
 __host__ __device__ inline int tc_entries_grouped(int max_m) { return max_m <= 16 ? 16 : max_m <= 32 ? 32 : 64; }
 
+struct TcMat {
+  const uint8_t *P;
+  const uint16_t *S;
+  float *Y;
+  int32_t N, ldy;
+};
 struct TcShape {
-  const TcGroup *groups;   // null: the one problem `single`
+  const TcGroup *groups;   // null: the matrices `mats` over rows 0..M
   const int32_t *ngroups;
-  TcGroup single;
+  TcMat mats[4];
+  int32_t ends[4];         // row tiles of mats[0..i]
+  int32_t M;
   const int8_t *XQ;
   const float *SQ;
   float *Y;
-  int32_t N, K, ldy;
-  bool ahead;              // the one problem's weights may travel before the dependency wait
+  int32_t N, K, ldy;       // of the groups
+  bool ahead;              // the matrices' weights may travel before the dependency wait
 };
 struct TcUnit {
   const uint8_t *P;        // of the problem's row 0
   const uint16_t *S;
-  int32_t x0, M, y_col, row0;
+  float *Y;                // of its first column and entry 0
+  int32_t x0, M, row0, N, ldy, pad;
 };
 
 // One block of eight entries: the four products of a group, then rescale and add.
-struct TcScales { float r0, r1; };   // a sixteenth of the weight scales of a lane's rows
 __device__ __forceinline__ void tc_products(int (&d)[4], const uint32_t (&a)[4][4], const uint4 &x0, const uint4 &x1) {
-  d[0] = d[1] = d[2] = d[3] = 0x4B400000;   // 1.5 x 2^23 as a float
-  mma_s8(d, a[0], x0.x, x0.y);
+  mma_s8_from(d, a[0], x0.x, x0.y, 0x4B400000);   // 1.5 x 2^23 as a float
   mma_s8(d, a[1], x0.z, x0.w);
   mma_s8(d, a[2], x1.x, x1.y);
   mma_s8(d, a[3], x1.z, x1.w);
 }
-__device__ __forceinline__ void tc_finish(float (&acc)[4], const int (&d)[4], TcScales c, float2 q) {
-  acc[0] = acc[0] + ((__int_as_float(d[0]) - 12582912.0f) * c.r0) * q.x;
-  acc[1] = acc[1] + ((__int_as_float(d[1]) - 12582912.0f) * c.r0) * q.y;
-  acc[2] = acc[2] + ((__int_as_float(d[2]) - 12582912.0f) * c.r1) * q.x;
-  acc[3] = acc[3] + ((__int_as_float(d[3]) - 12582912.0f) * c.r1) * q.y;
+// Both entries of a row in one packed instruction each, but for the last addition: a packed product and a packed sum
+// are fused by the assembler (found by the bits of a row), which rounds once where the sum's order asks for two.
+__device__ __forceinline__ void tc_finish(float (&acc)[4], const int (&d)[4], const uint64_t (&r)[2], float2 q) {
+  const uint64_t bias = pair2(-12582912.0f, -12582912.0f), q2 = pair2(q.x, q.y);
+  const float2 t0 = unpair2(mul2(mul2(add2(pair2(__int_as_float(d[0]), __int_as_float(d[1])), bias), r[0]), q2)),
+               t1 = unpair2(mul2(mul2(add2(pair2(__int_as_float(d[2]), __int_as_float(d[3])), bias), r[1]), q2));
+  acc[0] = acc[0] + t0.x;
+  acc[1] = acc[1] + t0.y;
+  acc[2] = acc[2] + t1.x;
+  acc[3] = acc[3] + t1.y;
 }
 
 template <int NT>
@@ -144,11 +176,11 @@ __device__ __forceinline__ void tc_body(const TcShape &c) {
   const int K = c.K, G = K >> 7;
   const size_t row_bytes = (size_t)(K >> 1);
   const int tpg = (c.N + kTcRows - 1) / kTcRows;      // row tiles per problem
-  const int nrb = (c.single.M + NT - 1) / NT;         // blocks of entries of the one problem
+  const int nrb = (c.M + NT - 1) / NT;                // blocks of entries of the matrices
   const int stride = (int)gridDim.x;
   const uint32_t base = smem_addr(tc_smem);
   if (!c.ahead) pdl_wait();
-  const int units = c.groups ? __ldcg(c.ngroups) * tpg : tpg * nrb;
+  const int units = c.groups ? __ldcg(c.ngroups) * tpg : c.ends[3] * nrb;
   // ---- copies: this thread's sources of the next stage; rows and entries that do not exist keep what is there (never stored) ----
   const bool pair_scales = (G & 1) == 0;
   const int wr = warp * 16 + (lane >> 3), wpc = lane & 7;   // weights: eight neighbours copy a row's line, four rows apart
@@ -172,14 +204,18 @@ __device__ __forceinline__ void tc_body(const TcShape &c) {
     if (c.groups) {
       union { uint4 q[2]; TcGroup g; } r;
       r.q[0] = rec[0]; r.q[1] = rec[1];
-      n.P = r.g.P; n.S = r.g.S; n.x0 = r.g.x_row0; n.M = min(r.g.M, NT); n.y_col = r.g.y_col; n.row0 = (lu % tpg) * kTcRows;
+      n.P = r.g.P; n.S = r.g.S; n.x0 = r.g.x_row0; n.M = min(r.g.M, NT); n.row0 = (lu % tpg) * kTcRows;
+      n.Y = c.Y + r.g.y_col; n.N = c.N; n.ldy = c.ldy;
     } else {
-      const int rb = lu % nrb;
-      n.P = c.single.P; n.S = c.single.S; n.x0 = rb * NT; n.M = min(NT, c.single.M - n.x0); n.y_col = 0; n.row0 = (lu / nrb) * kTcRows;
+      const int rb = lu % nrb, tile = lu / nrb, i = (tile >= c.ends[0]) + (tile >= c.ends[1]) + (tile >= c.ends[2]);
+      const TcMat m = i == 0 ? c.mats[0] : i == 1 ? c.mats[1] : i == 2 ? c.mats[2] : c.mats[3];
+      const int before = i == 0 ? 0 : i == 1 ? c.ends[0] : i == 2 ? c.ends[1] : c.ends[2];
+      n.P = m.P; n.S = m.S; n.x0 = rb * NT; n.M = min(NT, c.M - n.x0); n.row0 = (tile - before) * kTcRows;
+      n.Y = m.Y; n.N = m.N; n.ldy = m.ldy;
     }
     if (tid == 0) ring[lk & 7] = n;
     ++lk;
-    const int rows = c.N - n.row0;
+    const int rows = n.N - n.row0;
     wp = n.P + (size_t)(n.row0 + wr) * row_bytes + wpc * 16;
     xp = c.XQ + (size_t)(n.x0 + xm) * K + xpc * 16;
     wmask = xmask = 0;
@@ -277,7 +313,7 @@ __device__ __forceinline__ void tc_body(const TcShape &c) {
         s0 = *reinterpret_cast<const uint32_t *>(sp + CO + r0 * 4);
         s1 = *reinterpret_cast<const uint32_t *>(sp + CO + (r0 + 8) * 4);
       } else {
-        const uint16_t *w0 = n.S + (size_t)min(n.row0 + r0, c.N - 1) * G + g0, *w1 = n.S + (size_t)min(n.row0 + r0 + 8, c.N - 1) * G + g0;
+        const uint16_t *w0 = n.S + (size_t)min(n.row0 + r0, n.N - 1) * G + g0, *w1 = n.S + (size_t)min(n.row0 + r0 + 8, n.N - 1) * G + g0;
         s0 = __ldg(w0) | (uint32_t)__ldg(w0 + ng - 1) << 16;
         s1 = __ldg(w1) | (uint32_t)__ldg(w1 + ng - 1) << 16;
       }
@@ -296,9 +332,9 @@ __device__ __forceinline__ void tc_body(const TcShape &c) {
             a[s][2 + h] = __byte_perm(lo, hi, 0x7362);
           }
         }
-        TcScales sc;
-        sc.r0 = __uint_as_float(gl ? s0 & 0xFFFF0000u : s0 << 16) * 0.0625f;
-        sc.r1 = __uint_as_float(gl ? s1 & 0xFFFF0000u : s1 << 16) * 0.0625f;
+        // a sixteenth of the weight scales of the lane's rows
+        const float f0 = __uint_as_float(gl ? s0 & 0xFFFF0000u : s0 << 16) * 0.0625f, f1 = __uint_as_float(gl ? s1 & 0xFFFF0000u : s1 << 16) * 0.0625f;
+        const uint64_t sc[2] = {pair2(f0, f0), pair2(f1, f1)};
         const uint32_t xb = sb + XO + (uint32_t)g * kTcXPitch + (uint32_t)(gl * 128 + t * 32);
         const float *sq = reinterpret_cast<const float *>(sp + QO) + gl * NT + 2 * t;
 #pragma unroll
@@ -325,15 +361,15 @@ __device__ __forceinline__ void tc_body(const TcShape &c) {
       cs = cs == ST - 1 ? 0 : cs + 1;
     }
     const TcUnit &n = ring[ck & 7];
-    float *y = c.Y + (size_t)n.x0 * c.ldy + n.y_col + n.row0 + r0;
-    const bool in0 = n.row0 + r0 < c.N, in1 = n.row0 + r0 + 8 < c.N;
-    const int M = n.M;
+    float *y = n.Y + (size_t)n.x0 * n.ldy + n.row0 + r0;
+    const bool in0 = n.row0 + r0 < n.N, in1 = n.row0 + r0 + 8 < n.N;
+    const int M = n.M, ldy = n.ldy;
 #pragma unroll
     for (int j = 0; j < NT / 8; ++j) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int m = 8 * j + 2 * t + (q & 1);
-        if (m < M && (q < 2 ? in0 : in1)) y[(size_t)m * c.ldy + (q < 2 ? 0 : 8)] = acc[j][q];
+        if (m < M && (q < 2 ? in0 : in1)) y[(size_t)m * ldy + (q < 2 ? 0 : 8)] = acc[j][q];
         acc[j][q] = 0.0f;
       }
     }
@@ -346,37 +382,71 @@ __device__ __forceinline__ void tc_dispatch(const TcShape &c, int nt) {
   else if (nt == 32) tc_body<32>(c);
   else tc_body<64>(c);
 }
+__host__ __device__ inline int tc_tiles(int N) { return (N + kTcRows - 1) / kTcRows; }
+__host__ __device__ inline int tc_tiles(const Int4GemmA8TcManyArgs &a) {
+  return tc_tiles(a.N0) + (a.count > 1 ? tc_tiles(a.N1) : 0) + (a.count > 2 ? tc_tiles(a.N2) : 0) + (a.count > 3 ? tc_tiles(a.N3) : 0);
+}
+__global__ void __launch_bounds__(kTcThreads, 2) Int4GemmA8TcMany(const Int4GemmA8TcManyArgs a) {
+  TcShape c;
+  c.groups = nullptr;
+  c.ngroups = nullptr;
+  c.mats[0] = TcMat{a.P0, a.S0, a.Y0, a.N0, a.N0};
+  c.mats[1] = TcMat{a.P1, a.S1, a.Y1, a.N1, a.N1};
+  c.mats[2] = TcMat{a.P2, a.S2, a.Y2, a.N2, a.N2};
+  c.mats[3] = TcMat{a.P3, a.S3, a.Y3, a.N3, a.N3};
+  c.ends[0] = tc_tiles(a.N0);
+  c.ends[1] = c.ends[0] + (a.count > 1 ? tc_tiles(a.N1) : 0);
+  c.ends[2] = c.ends[1] + (a.count > 2 ? tc_tiles(a.N2) : 0);
+  c.ends[3] = c.ends[2] + (a.count > 3 ? tc_tiles(a.N3) : 0);
+  c.M = a.M;
+  c.XQ = a.XQ; c.SQ = a.SQ; c.Y = nullptr;
+  c.N = 0; c.K = a.K; c.ldy = 0;
+  c.ahead = (a.ahead & AHEAD_WEIGHTS) != 0;
+  tc_dispatch(c, tc_entries(c.ends[3], a.M));
+}
 __global__ void __launch_bounds__(kTcThreads, 2) Int4GemmA8Tc(const Int4GemmA8TcArgs a) {
   TcShape c;
   c.groups = nullptr;
   c.ngroups = nullptr;
-  c.single.P = a.P; c.single.S = a.S; c.single.x_row0 = 0; c.single.M = a.M; c.single.y_col = 0; c.single.pad = 0;
-  c.XQ = a.XQ; c.SQ = a.SQ; c.Y = a.Y;
-  c.N = a.N; c.K = a.K; c.ldy = a.ldy;
+  c.mats[0] = c.mats[1] = c.mats[2] = c.mats[3] = TcMat{a.P, a.S, a.Y, a.N, a.ldy};
+  c.ends[0] = c.ends[1] = c.ends[2] = c.ends[3] = tc_tiles(a.N);
+  c.M = a.M;
+  c.XQ = a.XQ; c.SQ = a.SQ; c.Y = nullptr;
+  c.N = 0; c.K = a.K; c.ldy = 0;
   c.ahead = (a.ahead & AHEAD_WEIGHTS) != 0;
-  tc_dispatch(c, tc_entries(a.N, a.M));
+  tc_dispatch(c, tc_entries(c.ends[3], a.M));
 }
 
-__global__ void __launch_bounds__(kTcThreads, 2) Int4GemmA8TcGrouped(const Int4GemmA8TcGroupedArgs a) {
+__device__ __forceinline__ TcShape tc_groups(const Int4GemmA8TcGroupedArgs &a) {
   TcShape c;
   c.groups = a.Groups;
   c.ngroups = a.NGroups;
-  c.single = TcGroup{nullptr, nullptr, 0, 0, 0, 0};
+  c.ends[3] = c.M = 0;
   c.XQ = a.XQ; c.SQ = a.SQ; c.Y = a.Y;
   c.N = a.N; c.K = a.K; c.ldy = a.ldy;
   c.ahead = false;
-  tc_dispatch(c, tc_entries_grouped(a.max_m));
+  return c;
 }
-
+__global__ void __launch_bounds__(kTcThreads, 2) Int4GemmA8TcGrouped(const Int4GemmA8TcGroupedArgs a) {
+  tc_dispatch(tc_groups(a), tc_entries_grouped(a.max_m));
+}
 static uint32_t tc_smem_bytes(int nt) { return (uint32_t)tc_stages(nt) * tc_stage_bytes(nt); }
 static uint32_t tc_smem_fn(const void *args) {
   const Int4GemmA8TcArgs *a = (const Int4GemmA8TcArgs *)args;
-  return tc_smem_bytes(tc_entries(a->N, a->M));
+  return tc_smem_bytes(tc_entries(tc_tiles(a->N), a->M));
+}
+static uint32_t tc_many_smem_fn(const void *args) {
+  const Int4GemmA8TcManyArgs *a = (const Int4GemmA8TcManyArgs *)args;
+  return tc_smem_bytes(tc_entries(tc_tiles(*a), a->M));
 }
 static uint32_t tc_grouped_smem_fn(const void *args) { return tc_smem_bytes(tc_entries_grouped(((const Int4GemmA8TcGroupedArgs *)args)->max_m)); }
 
 #define F(f) AINFER_ARG(Int4GemmA8TcArgs, f)
 AINFER_REGISTER(Int4GemmA8Tc, Int4GemmA8TcArgs, kTcThreads, 0, 0, tc_smem_fn, F(P), F(S), F(XQ), F(SQ), F(Y), F(N), F(K), F(M), F(ldy));
+#undef F
+#define F(f) AINFER_ARG(Int4GemmA8TcManyArgs, f)
+AINFER_REGISTER(Int4GemmA8TcMany, Int4GemmA8TcManyArgs, kTcThreads, 0, 0, tc_many_smem_fn, F(XQ), F(SQ), F(K), F(M), F(count), F(P0), F(S0), F(Y0),
+                F(N0), F(P1), F(S1), F(Y1), F(N1), F(P2), F(S2), F(Y2), F(N2), F(P3), F(S3), F(Y3), F(N3));
 #undef F
 #define F(f) AINFER_ARG(Int4GemmA8TcGroupedArgs, f)
 AINFER_REGISTER(Int4GemmA8TcGrouped, Int4GemmA8TcGroupedArgs, kTcThreads, 0, 0, tc_grouped_smem_fn, F(Groups), F(NGroups), F(XQ), F(SQ),
@@ -384,6 +454,7 @@ AINFER_REGISTER(Int4GemmA8TcGrouped, Int4GemmA8TcGroupedArgs, kTcThreads, 0, 0, 
 #undef F
 
 AINFER_EARLY_LAUNCH_AHEAD(Int4GemmA8Tc, Int4GemmA8TcArgs);
+AINFER_EARLY_LAUNCH_AHEAD(Int4GemmA8TcMany, Int4GemmA8TcManyArgs);
 AINFER_EARLY_LAUNCH(Int4GemmA8TcGrouped);
 
 }  // namespace ainfer

@@ -13,6 +13,7 @@
 #include <cstring>
 
 #include "batch.h"
+#include "row_products.h"
 
 namespace ainfer {
 
@@ -20,25 +21,8 @@ namespace {
 struct Rec : KernelCalls {   // appends launches to a list; arguments by index in member order
   BatchDecode *b;
   Rec(BatchDecode *bd, ainfer_list_t l) : KernelCalls(bd->dev, &bd->kernels, &bd->err, l), b(bd) {}
-  void gemm(const DeviceTensor &t, const int8_t *XQ, const float *SQ, float *Y, int K, int rows) {
-    if (status) return;
-    if (!t.entry || (int)t.entry->shape[1] != K || t.entry->storage != DT_INT4_SYM_G128) {
-      b->err = "batch: missing tensor or unexpected shape/storage" + (t.entry ? " of " + t.entry->name : std::string());
-      status = 2;
-      return;
-    }
-    const int N = (int)t.entry->shape[0];
-    const int G = K / 128;
-    if (rows <= 8 && G <= 256 && 256 % G == 0) {
-      // few rows: the dp4a kernel streams the weights once and has a fraction of the tensor-core kernel's latency
-      const uint32_t tiles = (uint32_t)((N + 256 / G - 1) / (256 / G));
-      launch("Int4GemvA8Multi", std::min<uint32_t>(tiles, 2u * (uint32_t)b->sm_count), (const uint8_t *)t.data, (const uint16_t *)t.scales, XQ, SQ,
-             Y, (int32_t)N, (int32_t)K, (int32_t)rows, (int32_t)N);
-      return;
-    }
-    const long units = (long)((N + 127) / 128) * ((rows + 15) / 16);
-    launch("Int4GemmA8Tc", (uint32_t)std::min<long>(units, 2L * b->sm_count), (const uint8_t *)t.data, (const uint16_t *)t.scales, XQ, SQ, Y, (int32_t)N,
-           (int32_t)K, (int32_t)rows, (int32_t)N);
+  void products(std::initializer_list<RowProduct> of, const int8_t *XQ, const float *SQ, int K, int rows) {
+    row_products(*this, "batch", b->sm_count, of, XQ, SQ, K, rows);
   }
 };
 }  // namespace
@@ -165,9 +149,8 @@ int BatchDecode::record() {
     r.launch("RmsNormQuant", (uint32_t)n, (const float *)X, (const float *)nullptr, (float *)nullptr,
              (const float *)(m->in_norm + (size_t)L * H), (float *)nullptr, Q8, SQ, (int32_t)H, eps);
     if (c.layer_types[L] == 'A') {
-      r.gemm(m->tensor(pf + "self_attn.q_proj.weight"), Q8, SQ, Q16, H, n);
-      r.gemm(m->tensor(pf + "self_attn.k_proj.weight"), Q8, SQ, K16, H, n);
-      r.gemm(m->tensor(pf + "self_attn.v_proj.weight"), Q8, SQ, V16, H, n);
+      r.products({{m->tensor(pf + "self_attn.q_proj.weight"), Q16}, {m->tensor(pf + "self_attn.k_proj.weight"), K16},
+                  {m->tensor(pf + "self_attn.v_proj.weight"), V16}}, Q8, SQ, H, n);
       const size_t off = (size_t)slot * max_ctx * nKV;   // this layer's rows inside a sequence's cache
       auto attn = [&](const char *name, int groups) {
         r.launch(name, (uint32_t)(n * groups), (const float *)Q16, (const float *)K16, (const float *)V16,
@@ -179,12 +162,10 @@ int BatchDecode::record() {
       attn("BatchAttnPrep", (nQ + 2 * nKV + 7) / 8);
       attn("BatchAttnSplit", std::max(1, std::min(max_chunks * nKV, (sm_count * 8 + n - 1) / n)));
       attn("BatchAttnCombine", nQ);
-      r.gemm(m->tensor(pf + "self_attn.o_proj.weight"), Q8, SQ, ep.Add, AK, n);
+      r.products({{m->tensor(pf + "self_attn.o_proj.weight"), ep.Add}}, Q8, SQ, AK, n);
     } else {
-      r.gemm(m->tensor(pf + "linear_attn.in_proj_qkv.weight"), Q8, SQ, Pq, H, n);
-      r.gemm(m->tensor(pf + "linear_attn.in_proj_z.weight"), Q8, SQ, Z, H, n);
-      r.gemm(m->tensor(pf + "linear_attn.in_proj_b.weight"), Q8, SQ, Br, H, n);
-      r.gemm(m->tensor(pf + "linear_attn.in_proj_a.weight"), Q8, SQ, Ar, H, n);
+      r.products({{m->tensor(pf + "linear_attn.in_proj_qkv.weight"), Pq}, {m->tensor(pf + "linear_attn.in_proj_z.weight"), Z},
+                  {m->tensor(pf + "linear_attn.in_proj_b.weight"), Br}, {m->tensor(pf + "linear_attn.in_proj_a.weight"), Ar}}, Q8, SQ, H, n);
       r.launch("BatchConvSilu", (uint32_t)(((size_t)n * C + 255) / 256), Mx, (const float *)Pq, conv + (size_t)slot * C * 3,
                (const float *)(m->conv_w + (size_t)slot * C * 4), (int32_t)C, (int32_t)n, (int64_t)conv_stride);
       r.launch("ChunkBetaDecay", (uint32_t)((n * nV + 255) / 256), (const float *)Br, (const float *)Ar,
@@ -194,7 +175,7 @@ int BatchDecode::record() {
                (const float *)Gt, (int32_t)nK, (int32_t)nV, (int32_t)n, (int64_t)s_stride);
       r.launch("GatedNormQuant", (uint32_t)((n * nV + 3) / 4), (const float *)O, (const float *)Z,
                (const float *)(m->lin_norm + (size_t)slot * c.lin_head_dim), Q8, SQ, (float *)nullptr, (int32_t)(n * nV), eps);
-      r.gemm(m->tensor(pf + "linear_attn.out_proj.weight"), Q8, SQ, ep.Add, VD, n);
+      r.products({{m->tensor(pf + "linear_attn.out_proj.weight"), ep.Add}}, Q8, SQ, VD, n);
     }
     if (int e = close(r)) return e;
   }
@@ -204,7 +185,7 @@ int BatchDecode::record() {
     Rec r(this, l);
     r.launch("RmsNormQuant", (uint32_t)n, (const float *)X, (const float *)nullptr, (float *)nullptr, (const float *)m->final_norm,
              (float *)nullptr, Q8, SQ, (int32_t)H, eps);
-    r.gemm(m->tensor("lm_head.weight"), Q8, SQ, Logits, H, n);
+    r.products({{m->tensor("lm_head.weight"), Logits}}, Q8, SQ, H, n);
     r.launch("BatchArgmax", (uint32_t)n, (const float *)Logits, OutT, Ctrl, (int32_t)c.vocab, (int32_t)1);
     if (int e = close(r)) return e;
   }

@@ -25,6 +25,7 @@
 #include "arch.h"
 #include "ep.h"
 #include "executor.h"
+#include "row_products.h"
 
 namespace ainfer {
 
@@ -85,27 +86,8 @@ struct Launcher : KernelCalls {   // immediate launches, or appended to recorded
     }
     if (open_next && (ainfer_list_create(s->dev, &list) != AINFER_OK || ainfer_list_one_step(list) != AINFER_OK)) { s->err = ainfer_last_error(s->dev); status = 1; }
   }
-  // Y[rows][N] = X[rows][K] . W^T on the tensor cores
-  void gemm(const DeviceTensor &t, const int8_t *XQ, const float *SQ, float *Y, int K, int rows) {
-    if (status) return;
-    Session *s = p->s;
-    if (!t.entry || (int)t.entry->shape[1] != K || t.entry->storage != DT_INT4_SYM_G128) {
-      s->err = "prefill: missing tensor or unexpected shape/storage" + (t.entry ? " of " + t.entry->name : std::string());
-      status = 2;
-      return;
-    }
-    const int N = (int)t.entry->shape[0];
-    const int G = K / 128;
-    if (rows <= 8 && G <= 256 && 256 % G == 0) {
-      // few rows: the dp4a kernel streams the weights once and has a fraction of the tensor-core kernel's latency
-      const uint32_t tiles = (uint32_t)((N + 256 / G - 1) / (256 / G));
-      launch("Int4GemvA8Multi", std::min<uint32_t>(tiles, 2u * (uint32_t)s->sm_count), (const uint8_t *)t.data, (const uint16_t *)t.scales, XQ, SQ,
-             Y, (int32_t)N, (int32_t)K, (int32_t)rows, (int32_t)N);
-      return;
-    }
-    const long units = (long)((N + 127) / 128) * ((rows + 15) / 16);
-    launch("Int4GemmA8Tc", (uint32_t)std::min<long>(units, 2L * s->sm_count), (const uint8_t *)t.data, (const uint16_t *)t.scales, XQ, SQ, Y, (int32_t)N,
-           (int32_t)K, (int32_t)rows, (int32_t)N);
+  void products(std::initializer_list<RowProduct> of, const int8_t *XQ, const float *SQ, int K, int rows) {
+    row_products(*this, "prefill", p->s->sm_count, of, XQ, SQ, K, rows);
   }
 };
 
@@ -244,9 +226,8 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
       l.launch("RmsNormQuant", (uint32_t)rows, (const float *)X, (const float *)nullptr, (float *)nullptr,
                (const float *)(m->in_norm + (size_t)L * H), (float *)nullptr, p->Q8, p->SQ, (int32_t)H, eps);
       if (c.layer_types[L] == 'A') {
-        l.gemm(m->tensor(pf + "self_attn.q_proj.weight"), p->Q8, p->SQ, p->Q16, H, rows);
-        l.gemm(m->tensor(pf + "self_attn.k_proj.weight"), p->Q8, p->SQ, p->K16, H, rows);
-        l.gemm(m->tensor(pf + "self_attn.v_proj.weight"), p->Q8, p->SQ, p->V16, H, rows);
+        l.products({{m->tensor(pf + "self_attn.q_proj.weight"), p->Q16}, {m->tensor(pf + "self_attn.k_proj.weight"), p->K16},
+                    {m->tensor(pf + "self_attn.v_proj.weight"), p->V16}}, p->Q8, p->SQ, H, rows);
         const size_t kv_off = (size_t)slot * s->max_ctx * nKV;
         int8_t *Kc = s->Kc + kv_off * D, *Vc = s->Vc + kv_off * D;
         uint16_t *Ks = s->Ks + kv_off, *Vs = s->Vs + kv_off;
@@ -267,12 +248,10 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
           attn("BatchAttnSplit", r0, some, std::max(1, std::min(s->max_chunks * nKV, (s->sm_count * 8 + some - 1) / some)));
           attn("BatchAttnCombine", r0, some, nQ);
         }
-        l.gemm(m->tensor(pf + "self_attn.o_proj.weight"), p->Q8, p->SQ, ep.Add, AK, rows);
+        l.products({{m->tensor(pf + "self_attn.o_proj.weight"), ep.Add}}, p->Q8, p->SQ, AK, rows);
       } else {
-        l.gemm(m->tensor(pf + "linear_attn.in_proj_qkv.weight"), p->Q8, p->SQ, p->Pq, H, rows);
-        l.gemm(m->tensor(pf + "linear_attn.in_proj_z.weight"), p->Q8, p->SQ, p->Z, H, rows);
-        l.gemm(m->tensor(pf + "linear_attn.in_proj_b.weight"), p->Q8, p->SQ, p->Br, H, rows);
-        l.gemm(m->tensor(pf + "linear_attn.in_proj_a.weight"), p->Q8, p->SQ, p->Ar, H, rows);
+        l.products({{m->tensor(pf + "linear_attn.in_proj_qkv.weight"), p->Pq}, {m->tensor(pf + "linear_attn.in_proj_z.weight"), p->Z},
+                    {m->tensor(pf + "linear_attn.in_proj_b.weight"), p->Br}, {m->tensor(pf + "linear_attn.in_proj_a.weight"), p->Ar}}, p->Q8, p->SQ, H, rows);
         l.launch("ChunkConvSilu", (uint32_t)((C + 255) / 256 * ((rows + 15) / 16)), p->Mx, (const float *)p->Pq, s->conv + (size_t)slot * C * 3,
                  (const float *)(m->conv_w + (size_t)slot * C * 4), (int32_t)C, (int32_t)rows,
                  (float *)(verify ? p->SnapC + (size_t)slot * C * 3 : nullptr), (int64_t)p->snap_c_stride);
@@ -284,7 +263,7 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
                  (float *)(verify ? p->SnapS + (size_t)slot * nV * 128 * 128 : nullptr), (int64_t)p->snap_s_stride);
         l.launch("GatedNormQuant", (uint32_t)((rows * nV + 3) / 4), (const float *)p->O, (const float *)p->Z,
                  (const float *)(m->lin_norm + (size_t)slot * c.lin_head_dim), p->Q8, p->SQ, (float *)nullptr, (int32_t)(rows * nV), eps);
-        l.gemm(m->tensor(pf + "linear_attn.out_proj.weight"), p->Q8, p->SQ, ep.Add, VD, rows);
+        l.products({{m->tensor(pf + "linear_attn.out_proj.weight"), ep.Add}}, p->Q8, p->SQ, VD, rows);
       }
       if (l.status) break;
       if (l.recording) {
@@ -300,7 +279,7 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
       // every row's greedy prediction: final norm, LM head over the rows, argmax per row (no control advance)
       l.launch("RmsNormQuant", (uint32_t)rows, (const float *)ep.Res, (const float *)nullptr, (float *)nullptr,
                (const float *)m->final_norm, (float *)nullptr, p->Q8, p->SQ, (int32_t)H, eps);
-      l.gemm(m->tensor("lm_head.weight"), p->Q8, p->SQ, p->Logits, H, rows);
+      l.products({{m->tensor("lm_head.weight"), p->Logits}}, p->Q8, p->SQ, H, rows);
       l.launch("BatchArgmax", (uint32_t)rows, (const float *)p->Logits, p->OutT, p->Ctrl, (int32_t)c.vocab, (int32_t)0);
     }
     if (l.recording) l.cut(false);

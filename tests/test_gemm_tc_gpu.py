@@ -98,3 +98,22 @@ def test_grouped_gemm_a8_tc_bit_exact(dev, N, K, blocks):
     k(blocks, dTab, dN, dev.upload(xq), dev.upload(sq), dY, N, K, 64, ldy)
     dev.sync()
     assert np.all(dev.download(dY, rows * ldy, np.float32) == 3.0)
+
+
+# matrices that end inside a tile, below one and above one; rows around the blocks of entries; odd and even group counts
+@pytest.mark.parametrize("K,rows,sizes", [(256, 9, (130, 32)), (384, 64, (32, 257, 128)), (2048, 65, (512, 256, 32, 32)), (128, 17, (8, 8, 8, 8)),
+                                          (1024, 130, (129,)), (2048, 1, (136, 40, 264))])
+def test_many_matrices_in_one_launch(dev, K, rows, sizes):
+    rng = np.random.default_rng(K + rows)
+    x = rng.standard_normal((rows, K)).astype(np.float32) * 2
+    q = [O.aquant(v) for v in x]
+    xq, sq = np.stack([a for a, _ in q]), np.stack([b for _, b in q])
+    mats = [O.quantize_int4((rng.standard_normal((n, K)) * 0.02).astype(np.float32)) for n in sizes]
+    outs = [dev.zeros(rows * n * 4) for n in sizes]
+    args = []
+    for i in range(4):
+        args += [dev.upload(mats[i][0]), dev.upload(mats[i][1]), outs[i], sizes[i]] if i < len(sizes) else [0, 0, 0, 0]
+    dev.kernel("Int4GemmA8TcMany")(8, dev.upload(xq), dev.upload(sq), K, rows, len(sizes), *args)
+    dev.sync()
+    for (P, S), n, y in zip(mats, sizes, outs):
+        assert np.array_equal(dev.download(y, rows * n, np.float32).reshape(rows, n), run_tc(dev, P, S, xq, sq, n, K, rows)), n
