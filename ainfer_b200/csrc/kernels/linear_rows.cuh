@@ -23,7 +23,7 @@ struct LinearRowsShared {
 
 template <int BM, int BN>
 struct LinearRowsTile {
-  static constexpr int TM = BM == 64 ? 8 : 4, TN = 8, TX = BN / TN;
+  static constexpr int TM = BM == 64 ? 8 : 4, TN = BM == 64 ? BN / 8 : 8, TX = BN / TN;
   static_assert(BM / TM * TX == kLrThreads && TM % 4 == 0, "64 threads own the tile");
   static constexpr int XP = BM * kLrK / kLrThreads, XR = kLrThreads / BM;   // values of a thread, threads of a row
   static constexpr int WN = BN / kLrThreads;                                // weight rows of a thread
@@ -33,9 +33,9 @@ struct LinearRowsTile {
   float xr[XP];
   uint4 wr[WN][2];
 
-  // Rows and columns of the thread's sums: quads, half a tile apart.
+  // Rows and columns of the thread's sums: quads, spread evenly over the tile.
   __device__ static int row(int i) { return (i >> 2) * (BM / (TM / 4)) + (int)threadIdx.x / TX * 4 + (i & 3); }
-  __device__ static int col(int j) { return (j >> 2) * (BN / 2) + (int)threadIdx.x % TX * 4 + (j & 3); }
+  __device__ static int col(int j) { return (j >> 2) * (BN / (TN / 4)) + (int)threadIdx.x % TX * 4 + (j & 3); }
 
   // Columns [k0, k0 + 16) of `rows` rows of X and `cols` rows of W: zeros beyond K; rows and columns past the last repeat
   // it (their sums are not stored).
@@ -109,7 +109,7 @@ struct LinearRowsTile {
 #pragma unroll
         for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4 *>(xv + i) = *reinterpret_cast<const float4 *>(&sh.x[b][k][i / 4 * (BM / (TM / 4)) + ty]);
 #pragma unroll
-        for (int j = 0; j < TN; j += 4) wv[j / 4] = *reinterpret_cast<const ulonglong2 *>(&sh.w[b][k][j / 4 * (BN / 2) + tx]);
+        for (int j = 0; j < TN; j += 4) wv[j / 4] = *reinterpret_cast<const ulonglong2 *>(&sh.w[b][k][j / 4 * (BN / (TN / 4)) + tx]);
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
           const uint64_t x2 = pair2(xv[i], xv[i]);

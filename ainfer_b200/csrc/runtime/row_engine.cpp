@@ -148,15 +148,28 @@ int RowEngineBase::alloc_bytes(size_t bytes, void **out) {
 void RowEngineBase::linear(KernelCalls &k, const RowMatrix &mt, const char *Xp, int ldx, int rows, void *Yp, int ldy, int act, bool out16, float cap) {
   if (k.status) return;
   if (f32) {
-    // Tiles of 64 x 64, or 16 x 128 for up to 16 rows. A block of 64 threads multiplies alone on a quarter of an SM's
+    // Tiles of 64 x 64 or 64 x 128, or 16 x 128 for up to 16 rows. A block of 64 threads multiplies alone on a quarter of an SM's
     // schedulers, so K is split over a cluster until there are four blocks an SM, down to 128 columns a block.
     const bool few = rows <= 16;
-    const int tiles = few ? (mt.N + 127) / 128 : ((mt.N + 63) / 64) * ((rows + 63) / 64);
-    int cl = 0;
-    while (cl < 3 && (tiles << cl) < 4 * sm_count && mt.K >= (256 << cl)) ++cl;
-    static const char *const names[2][4] = {{"LinearRows", "LinearRowsSplit2", "LinearRowsSplit4", "LinearRowsSplit8"},
-                                            {"LinearRowsFew", "LinearRowsFewSplit2", "LinearRowsFewSplit4", "LinearRowsFewSplit8"}};
-    k.launch(names[few][cl], (uint32_t)(tiles << cl), (const float *)Xp, mt.w, mt.bias, (float *)Yp, (int32_t)rows, (int32_t)mt.N, (int32_t)mt.K,
+    auto columns = [&](int cl) { return mt.K >= (128 << cl); };
+    int tiles = few ? (mt.N + 127) / 128 : ((mt.N + 63) / 64) * ((rows + 63) / 64), cl = 0, kind = few ? 1 : 0;
+    while (cl < 3 && (tiles << cl) < 4 * sm_count && columns(cl + 1)) ++cl;
+    if (!few) {
+      // 64 x 128 tiles read shared memory for 6 of every 8 cycles that they multiply, 64 x 64 ones for 8: they are the faster ones
+      // where they come to four blocks an SM with K in four parts at most, or to 2.75 in the most parts; us of both: 777 rows x
+      // 4096 x 1024 192 / 163, x 1280 x 1024 74 / 63, x 1024 x 4096 192 / 187, 100 x 4096 x 1024 41 / 36, 2048 x 2048 x 2048 497 / 394;
+      // below, 33 x 2048 x 2048 27 / 34, 100 x 1024 x 4096 45 / 59. A wide tile takes about 1.65 times as long, so the last columns' half
+      // tile must not cost more than that (N = 64, 192).
+      const int wide = ((mt.N + 127) / 128) * ((rows + 63) / 64);
+      int w = 0;
+      while (w < 2 && (wide << w) < 4 * sm_count && columns(w + 1)) ++w;
+      if (w == 2 && 4 * (wide << w) < 11 * sm_count && columns(3)) w = 3;
+      if (4 * (wide << w) >= 11 * sm_count && 5 * wide <= 3 * tiles) { tiles = wide; cl = w; kind = 2; }
+    }
+    static const char *const names[3][4] = {{"LinearRows", "LinearRowsSplit2", "LinearRowsSplit4", "LinearRowsSplit8"},
+                                            {"LinearRowsFew", "LinearRowsFewSplit2", "LinearRowsFewSplit4", "LinearRowsFewSplit8"},
+                                            {"LinearRowsWide", "LinearRowsWideSplit2", "LinearRowsWideSplit4", "LinearRowsWideSplit8"}};
+    k.launch(names[kind][cl], (uint32_t)(tiles << cl), (const float *)Xp, mt.w, mt.bias, (float *)Yp, (int32_t)rows, (int32_t)mt.N, (int32_t)mt.K,
              (int32_t)ldx, (int32_t)mt.ldw, (int32_t)ldy, (int32_t)act, cap);
     return;
   }

@@ -327,6 +327,29 @@ def test_linear_rows_32bit_tiles(dev, R, N, K, act, pad, splits, few):
     assert not got[:, N:].any()
 
 
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("R,N,K,act,pad", [(1, 5, 7, 1, 0), (63, 127, 16, 0, 4), (64, 128, 128, 2, 4), (65, 129, 1000, 0, 0), (17, 260, 530, 1, 2), (130, 200, 4096, 0, 4)])
+def test_linear_rows_32bit_wide_tiles(dev, R, N, K, act, pad, splits):
+    """64 x 128 tiles: their edges, K in parts (empty ones too), rows of 16-byte alignment and others. With K in as many parts the
+    64 x 64 tiles add up in the same order."""
+    g = torch.Generator().manual_seed(R)
+    x, w, b = torch.randn(R, K, generator=g), bf16(torch.randn(N, K, generator=g)), torch.randn(N, generator=g)
+    ldw, ldx, ldy = -(-K // 8) * 8, K + pad, N + pad
+    wp, xp = torch.full((N, ldw), 3.0), torch.full((R, ldx), float("nan"))   # what lies beyond K is not read as a value
+    wp[:, :K], xp[:, :K] = w.float(), x
+    dx, dw, db = dev.upload(f32(xp)), dev.upload(bits(wp)), dev.upload(f32(b))
+    got = []
+    for wide, bn in (("Wide", 128), ("", 64)):
+        y = dev.zeros(R * ldy * 4)
+        dev.kernel("LinearRows" + wide + (f"Split{splits}" if splits > 1 else ""))(
+            -(-N // bn) * -(-R // 64) * splits, dx, dw, db, y, R, N, K, ldx, ldw, ldy, act, 3.0)
+        dev.sync()
+        got.append(dev.download(y, (R, ldy), np.float32))
+    close(got[0][:, :N], ACTS[act](x.double() @ w.double().T + b.double(), 3.0), 1e-5)
+    assert not got[0][:, N:].any()
+    assert np.array_equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("R,N,K,nt,splits,act,out16", [
     (1, 5, 40, 16, 1, 0, 0), (17, 130, 200, 32, 1, 2, 0), (64, 256, 1024, 64, 4, 0, 0), (300, 384, 136, 128, 1, 1, 1), (520, 640, 512, 256, 1, 0, 0),
     (30, 100, 4096, 16, 8, 1, 1), (1000, 1536, 320, 256, 1, 1, 1), (129, 128, 64, 128, 1, 0, 0), (5, 300, 520, 16, 2, 0, 0), (100, 260, 2048, 128, 8, 2, 0),
