@@ -231,13 +231,19 @@ AINFER_REGISTER(ChunkAttnRowsB16, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_rows_
 // and 4 x DP / 16 sums. Bound by the fused multiply-adds: scores read eight 16-byte pieces of shared memory for
 // 64 of them, sums twelve for 128, where the form above read two words for each (and one key per lane). Rows are
 // padded by four floats, so eight lanes' pieces fall into different banks. Scores add up in the order of the
-// dimensions, sums in the order of the keys, as above. 777 rows, 8 heads of 128, one chunk: 762 us above, 159 here.
+// dimensions, sums in the order of the keys, as above. 777 rows, 8 heads of 128, one chunk: 762 us above, 159 with a block
+// for all keys of its rows: 200 blocks on 148 SMs, the last ones with 13 tiles after one another and 10 us for each, since four
+// warps hide little of the latency of a tile. So the blocks of a cluster of CL share the rows' keys, tile by tile in
+// turn, and add up through shared memory in the order of their ranks; the blocks with the most keys come first, and sums take two
+// dimensions an instruction. Same rows: 139 us with CL = 1, 86 with 2, 76 with 4, 109 with 8. (64 rows a block read shared memory
+// a third less often, but only two blocks are resident: 195, 115, 88, 118.)
 constexpr int kCtRows = 32, kCtKeys = 64, kCtPP = kCtKeys + 4;
-template <int DP>
+template <int DP, int CL>
 __device__ __forceinline__ void chunk_attn_tile_body(const ChunkAttnRowsArgs &a) {
   extern __shared__ __align__(16) float ca_smem[];   // q [32][DP + 4], k [64][DP + 4], weights [32][68]
   constexpr int P = DP + 4, NC = DP / 64;
-  const int D = a.D, h = blockIdx.x % a.H, r0 = blockIdx.x / a.H * kCtRows, g = h / (a.H / a.G);
+  const int block = (int)gridDim.x / CL - 1 - (int)blockIdx.x / CL, rank = CL > 1 ? blockIdx.x % CL : 0;
+  const int D = a.D, h = block % a.H, r0 = block / a.H * kCtRows, g = h / (a.H / a.G);
   float *qs = ca_smem, *ks = qs + kCtRows * P, *ws = ks + kCtKeys * P;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int nr = min(kCtRows, a.rows - r0), KW = a.G * D;
@@ -256,15 +262,16 @@ __device__ __forceinline__ void chunk_attn_tile_body(const ChunkAttnRowsArgs &a)
   const int pos0 = a.Ctrl[4 * r0 + CTRL_POS];
   const float mul = a.scale, temp = a.Temp[h];
   const float *lb = a.LB + (size_t)h * a.lb_len;
-  float m[4], l[4], acc[4][4 * NC];
+  float m[4], l[4];
+  uint64_t acc[4][2 * NC];   // neighbouring dimensions in pairs
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     m[i] = -INFINITY; l[i] = 0.0f;
 #pragma unroll
-    for (int x = 0; x < 4 * NC; ++x) acc[i][x] = 0.0f;
+    for (int x = 0; x < 2 * NC; ++x) acc[i][x] = 0;
   }
   const int lo = pos0 - pos0 % a.chunk, hi = pos0 + nr - 1;
-  for (int k0 = lo; k0 <= hi; k0 += kCtKeys) {
+  for (int k0 = lo + rank * kCtKeys; k0 <= hi; k0 += CL * kCtKeys) {
     __syncthreads();
 #pragma unroll 8
     for (int i = tid; i < kCtKeys * (DP / 4); i += 128) {
@@ -311,8 +318,9 @@ __device__ __forceinline__ void chunk_attn_tile_body(const ChunkAttnRowsArgs &a)
       for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
       m[i] = mx;
       l[i] = fmaf(l[i], corr, sum);
+      const uint64_t corr2 = pair2(corr, corr);
 #pragma unroll
-      for (int x = 0; x < 4 * NC; ++x) acc[i][x] *= corr;
+      for (int x = 0; x < 2 * NC; ++x) acc[i][x] = mul2(acc[i][x], corr2);
     }
     __syncwarp();   // a row's weights are written and read by 16 lanes of one warp
 #pragma unroll 2
@@ -321,36 +329,93 @@ __device__ __forceinline__ void chunk_attn_tile_body(const ChunkAttnRowsArgs &a)
 #pragma unroll
       for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4 *>(ws + (ty * 4 + i) * kCtPP + j);
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj)
+      for (int jj = 0; jj < 4; ++jj) {
+        uint64_t w2[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float wi = jj == 0 ? w[i].x : jj == 1 ? w[i].y : jj == 2 ? w[i].z : w[i].w;
+          w2[i] = pair2(wi, wi);
+        }
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          const float4 v = *reinterpret_cast<const float4 *>(ks + (j + jj) * P + 64 * c + tx * 4);
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(ks + (j + jj) * P + 64 * c + tx * 4);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const float wi = jj == 0 ? w[i].x : jj == 1 ? w[i].y : jj == 2 ? w[i].z : w[i].w;
-            acc[i][4 * c] = fmaf(wi, v.x, acc[i][4 * c]);
-            acc[i][4 * c + 1] = fmaf(wi, v.y, acc[i][4 * c + 1]);
-            acc[i][4 * c + 2] = fmaf(wi, v.z, acc[i][4 * c + 2]);
-            acc[i][4 * c + 3] = fmaf(wi, v.w, acc[i][4 * c + 3]);
+            acc[i][2 * c] = fma2(w2[i], v.x, acc[i][2 * c]);
+            acc[i][2 * c + 1] = fma2(w2[i], v.y, acc[i][2 * c + 1]);
           }
         }
+      }
     }
     __syncwarp();
   }
   float *O = reinterpret_cast<float *>(a.O) + (size_t)r0 * a.ldo + (size_t)h * D;
+  if constexpr (CL == 1) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int rr = ty * 4 + i;
-    if (rr >= nr) continue;
+    for (int i = 0; i < 4; ++i) {
+      const int rr = ty * 4 + i;
+      if (rr >= nr) continue;
 #pragma unroll
-    for (int x = 0; x < 4 * NC; ++x) {
-      const int d = x / 4 * 64 + tx * 4 + x % 4;
-      if (d < D) O[(size_t)rr * a.ldo + d] = acc[i][x] / l[i];
+      for (int x = 0; x < 4 * NC; ++x) {
+        const int d = x / 4 * 64 + tx * 4 + x % 4;
+        const float2 v = unpair2(acc[i][x / 2]);
+        if (d < D) O[(size_t)rr * a.ldo + d] = (x & 1 ? v.y : v.x) / l[i];
+      }
     }
+  } else {
+    // every block's sums in the keys' place, maximum and sum of weights of a row in the weights'; then each block ends
+    // its share of the rows, over the blocks in rank order
+    __syncthreads();   // the last tile's readers are done
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int rr = ty * 4 + i;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) *reinterpret_cast<ulonglong2 *>(ks + rr * P + 64 * c + tx * 4) = make_ulonglong2(acc[i][2 * c], acc[i][2 * c + 1]);
+      if (tx == 0) *reinterpret_cast<float2 *>(ws + rr * 2) = make_float2(m[i], l[i]);
+    }
+    cluster_sync_all();
+    constexpr int RB = kCtRows / CL;
+    for (int i = tid; i < RB * (DP / 4); i += 128) {
+      const int rr = rank * RB + i / (DP / 4), d = i % (DP / 4) * 4;
+      if (rr >= nr || d >= D) continue;
+      float pm[CL], pl[CL], pv[CL][4], M = -INFINITY, L = 0.0f, v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int c = 0; c < CL; ++c) {
+        uint32_t at, ml;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(ks + rr * P + d)), "r"(c));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ml) : "r"((uint32_t)__cvta_generic_to_shared(ws + rr * 2)), "r"(c));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(pv[c][0]), "=f"(pv[c][1]), "=f"(pv[c][2]), "=f"(pv[c][3]) : "r"(at) : "memory");
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(pm[c]), "=f"(pl[c]) : "r"(ml) : "memory");
+      }
+#pragma unroll
+      for (int c = 0; c < CL; ++c) M = fmaxf(M, pm[c]);
+#pragma unroll
+      for (int c = 0; c < CL; ++c) {
+        const float f = expf(pm[c] - M);   // a row sees its own key: M is finite
+        L = fmaf(pl[c], f, L);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = fmaf(pv[c][e], f, v[e]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (d + e < D) O[(size_t)rr * a.ldo + d + e] = v[e] / L;
+    }
+    cluster_sync_all();   // a block's sums stay until every reader is done
   }
 }
-__global__ void __launch_bounds__(128) ChunkAttnTile64(const ChunkAttnRowsArgs a) { chunk_attn_tile_body<64>(a); }
-__global__ void __launch_bounds__(128) ChunkAttnTile128(const ChunkAttnRowsArgs a) { chunk_attn_tile_body<128>(a); }
+__global__ void __launch_bounds__(128) ChunkAttnTile64(const ChunkAttnRowsArgs a) { chunk_attn_tile_body<64, 1>(a); }
+__global__ void __launch_bounds__(128) ChunkAttnTile128(const ChunkAttnRowsArgs a) { chunk_attn_tile_body<128, 1>(a); }
+// The keys of a block's rows over a cluster of CL blocks.
+#define CT_SPLIT(DP, CL)                                                                                                      \
+  __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(128) ChunkAttnTile##DP##Split##CL(const ChunkAttnRowsArgs a) { \
+    chunk_attn_tile_body<DP, CL>(a);                                                                                          \
+  }
+CT_SPLIT(64, 2)
+CT_SPLIT(64, 4)
+CT_SPLIT(64, 8)
+CT_SPLIT(128, 2)
+CT_SPLIT(128, 4)
+CT_SPLIT(128, 8)
 template <int DP>
 static uint32_t chunk_attn_tile_smem(const void *) {
   return 4u * (uint32_t)((kCtRows + kCtKeys) * (DP + 4) + kCtRows * kCtPP);
@@ -358,6 +423,12 @@ static uint32_t chunk_attn_tile_smem(const void *) {
 #define F(f) AINFER_ARG(ChunkAttnRowsArgs, f)
 AINFER_REGISTER(ChunkAttnTile64, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<64>, CAR_FIELDS);
 AINFER_REGISTER(ChunkAttnTile128, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<128>, CAR_FIELDS);
+AINFER_REGISTER(ChunkAttnTile64Split2, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<64>, CAR_FIELDS);
+AINFER_REGISTER(ChunkAttnTile64Split4, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<64>, CAR_FIELDS);
+AINFER_REGISTER(ChunkAttnTile64Split8, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<64>, CAR_FIELDS);
+AINFER_REGISTER(ChunkAttnTile128Split2, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<128>, CAR_FIELDS);
+AINFER_REGISTER(ChunkAttnTile128Split4, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<128>, CAR_FIELDS);
+AINFER_REGISTER(ChunkAttnTile128Split8, ChunkAttnRowsArgs, 128, 0, 0, chunk_attn_tile_smem<128>, CAR_FIELDS);
 #undef F
 AINFER_EARLY_LAUNCH(ShortConvRowsF32);
 AINFER_EARLY_LAUNCH(ShortConvRowsB16);

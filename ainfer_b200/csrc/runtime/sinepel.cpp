@@ -347,8 +347,17 @@ struct Engine : RowEngineBase {
                    (int32_t)s.chunk, (int32_t)lw.lb_len, (int32_t)ldo, (float)r.scale);
         else {
           const bool tile = f32 && r.dim <= 128;   // the registers of larger heads' sums would spill
-          k.launch(tile ? r.dim <= 64 ? "ChunkAttnTile64" : "ChunkAttnTile128" : f32 ? "ChunkAttnRowsF32" : "ChunkAttnRowsB16",
-                   (uint32_t)(tile ? (R + 31) / 32 * r.heads : (R + 15) / 16 * r.heads), (const void *)Q, (const void *)s.k, lw.lb,
+          // The keys of 32 rows over a cluster until there are three blocks an SM, all that are resident, a tile of 64 keys each at
+          // least (rows late in a chunk have the most; the pass does not know its position). us with 1, 2, 4 and 8 blocks: 777 rows, 8
+          // heads, chunk 1024 139, 86, 76, 109; 800 rows, 16 heads, chunk 2048 162, 117, 141, 206; 130 rows at position 800 156, 87, 57,
+          // 41, at 0 33, 23, 21, 24; 777 rows, chunk 64 23, 27, 44, 80.
+          const int blocks = (R + 31) / 32 * r.heads, keys = std::min(s.chunk, max_ctx);
+          int cl = 0;
+          while (cl < 3 && (blocks << cl) < 3 * sm_count && keys >= (128 << cl)) ++cl;
+          static const char *const tiles[2][4] = {{"ChunkAttnTile64", "ChunkAttnTile64Split2", "ChunkAttnTile64Split4", "ChunkAttnTile64Split8"},
+                                                  {"ChunkAttnTile128", "ChunkAttnTile128Split2", "ChunkAttnTile128Split4", "ChunkAttnTile128Split8"}};
+          k.launch(tile ? tiles[r.dim > 64][cl] : f32 ? "ChunkAttnRowsF32" : "ChunkAttnRowsB16",
+                   (uint32_t)(tile ? blocks << cl : (R + 15) / 16 * r.heads), (const void *)Q, (const void *)s.k, lw.lb,
                    lw.temp, sp.ctrl, (void *)Att, (int32_t)R, (int32_t)r.heads, (int32_t)r.kv_heads, (int32_t)r.dim, (int32_t)s.cap,
                    (int32_t)s.chunk, (int32_t)lw.lb_len, (int32_t)ldo, (float)r.scale);
         }

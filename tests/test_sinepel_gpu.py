@@ -245,6 +245,30 @@ def test_chunk_attention_in_tiles_32bit(dev, T, H, G, D, chunk, cap, first):
     assert not got[:, H * D:].any()
 
 
+@pytest.mark.parametrize("splits", [2, 4, 8])
+@pytest.mark.parametrize("T,H,G,D,chunk,cap,first", [(1, 2, 1, 128, 10, 64, 9), (33, 3, 3, 5, 1, 64, 7), (31, 4, 1, 64, 600, 640, 569), (40, 2, 2, 128, 64, 130, 44),
+                                                     (150, 8, 2, 96, 61, 212, 400), (129, 2, 2, 65, 1000, 1129, 871)])
+def test_chunk_attention_in_tiles_32bit_split(dev, T, H, G, D, chunk, cap, first, splits):
+    """The keys of a block over a cluster: blocks without keys, rows that begin a chunk within the block, blocks with fewer rows."""
+    lo, n = first - first % chunk, min(chunk, 512)
+    total = first + T - lo
+    assert total <= cap
+    q, k, r1, r2, temp = _attn_case(total, H, G, D, chunk, T)
+    want = P.shared_kv_attention(q.double(), k.double(), 0.25, temp.double(), r1.double(), r2.double(), chunk).reshape(total, H * D)[first - lo:]
+    ring = torch.full((cap, G * D), 7.0)
+    for i in range(total):
+        ring[(lo + i) % cap] = k[i].reshape(G * D)
+    ldo = H * D + 3
+    o = dev.zeros(T * ldo * 4)
+    dev.kernel(f"ChunkAttnTile{64 if D <= 64 else 128}Split{splits}")(
+        -(-T // 32) * H * splits, dev.upload(f32(q[first - lo:].reshape(T, H * D))), dev.upload(f32(ring)), _table(dev, r1, r2, max(n, total)),
+        dev.upload(f32(temp)), dev.upload(ctrl(range(first, first + T))), o, T, H, G, D, cap, chunk, max(n, total), ldo, 0.25)
+    dev.sync()
+    got = dev.download(o, (T, ldo), np.float32)
+    close(got[:, :H * D], want, 1e-5)
+    assert not got[:, H * D:].any()
+
+
 @pytest.mark.parametrize("kind", ["f32", "b16", "mma"])
 @pytest.mark.parametrize("H,G,D,chunk,taps,splits", [(16, 1, 96, 190, 3, 4), (4, 2, 192, 130, 4, 3), (4, 2, 256, 64, 2, 2), (4, 2, 16, 24, 3, 1), (6, 2, 20, 100, 1, 5), (8, 1, 64, 150, 4, 2), (3, 3, 33, 1, 2, 3),
                                                      (4, 4, 128, 90, 4, 8), (12, 2, 40, 200, 5, 16)])
