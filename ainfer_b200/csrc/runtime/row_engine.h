@@ -68,7 +68,7 @@ struct RowEngineBase : RowEngine {
   // one fp32 row; the same for kernels that prepare the row themselves: rows per block and blocks
   int gemv_rows(int N) const { return (N + 2 * sm_count - 1) / (2 * sm_count); }
   uint32_t gemv_blocks(int N) const { return (uint32_t)((N + gemv_rows(N) - 1) / gemv_rows(N)); }
-  void gemv(KernelCalls &k, const RowMatrix &mt, const float *x, float *y, int act);
+  void gemv(KernelCalls &k, const RowMatrix &mt, const float *x, float *y, int act, float cap = 0.0f);
   // name of the instance of a kernel family whose padded head size holds `dim`
   static std::string sized(const char *base, int dim) {
     for (int d : {32, 64, 96, 128, 192})
