@@ -185,7 +185,7 @@ struct ChunkAttnStepMmaArgs {
   float scale;
   int32_t ahead;           // LaunchAhead
 };
-constexpr int kSmStages = 3, kSmMaxSplits = 16;   // at most 16 splits
+constexpr int kSmStages = 3;
 // Bound by a chain of latencies, so in a list of one step all that does not come from the step's own projections is done
 // before the dependency wait, while the block would only stand by: positions, the first tiles of keys (of earlier steps; the row of
 // this step is put in later), the convolution over the history, and the first tile's penalties. What is left is
@@ -194,8 +194,6 @@ constexpr int kSmStages = 3, kSmMaxSplits = 16;   // at most 16 splits
 template <int DP>
 __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &a) {
   extern __shared__ __align__(128) unsigned char sm_raw[];
-  __shared__ float wm[4][16], wl[4][16];
-  __shared__ int s_last;
   constexpr int LD = DP + 8;
   uint16_t *Qs = reinterpret_cast<uint16_t *>(sm_raw);                // [16][LD]
   uint16_t *kn = Qs + 16 * LD;                                        // the new key [DP]
@@ -332,82 +330,21 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
     values<DP, 16>(o, s, kt, lane);
   }
   cpa_wait<0>();
-  // ---- the four warps' shares of this block ----
-  float *os = reinterpret_cast<float *>(Ks);   // [4][16][DP], in the key tiles' place
-  __syncthreads();
+  __syncthreads();   // the tiles' place is free
+  auto end = [&](int hh, int d, const float4 &v, float L, float, int) {
+    const size_t at = (size_t)seq * a.ldo + (size_t)(g * HG + hh) * D + d;
+    const float r[4] = {v.x / L, v.y / L, v.z / L, v.w / L};
 #pragma unroll
-  for (int x = 0; x < 2; ++x) {
-    const int r = (lane >> 2) + 8 * x;
-    l[x] = quad_sum(l[x]);
-    if ((lane & 3) == 0) { wm[warp][r] = m[x]; wl[warp][r] = l[x]; }
-    if (r < HG)
-#pragma unroll
-      for (int d = 0; d < DP / 8; ++d) *reinterpret_cast<float2 *>(os + (warp * 16 + r) * DP + d * 8 + (lane & 3) * 2) = make_float2(o[d][2 * x], o[d][2 * x + 1]);
-  }
-  __syncthreads();
-  auto put = [&](int h, int d, float v) {
-    const size_t at = (size_t)seq * a.ldo + (size_t)h * D + d;
-    if (a.out16) reinterpret_cast<uint16_t *>(a.O)[at] = f32_to_bf16(v);
-    else reinterpret_cast<float *>(a.O)[at] = v;
+    for (int e = 0; e < 4; ++e) {
+      if (a.out16) reinterpret_cast<uint16_t *>(a.O)[at + e] = f32_to_bf16(r[e]);
+      else reinterpret_cast<float *>(a.O)[at + e] = r[e];
+    }
   };
-  // partials of a (sequence, key head): sums [splits][HG][D], then (maximum, sum) [splits][HG][2]
-  float *base_p = a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (D + 4);   // D + 4 keeps 16-byte alignment
-  float *base_m = base_p + (size_t)a.splits * HG * D;
-#pragma unroll 1
-  for (int i = tid; i < HG * D; i += 128) {
-    const int hh = i / D, d = i - hh * D;
-    const float M = fmaxf(fmaxf(wm[0][hh], wm[1][hh]), fmaxf(wm[2][hh], wm[3][hh]));
-    float v = 0.0f, L = 0.0f;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float f = fast_exp2(wm[w][hh] - M);
-      v = fmaf(os[(w * 16 + hh) * DP + d], f, v);
-      L = fmaf(wl[w][hh], f, L);
-    }
-    if (active == 1) {
-      put(g * HG + hh, d, v / L);
-    } else {
-      __stcg(base_p + (size_t)split * HG * D + i, v);
-      if (d == 0) __stcg(reinterpret_cast<float2 *>(base_m) + split * HG + hh, make_float2(M, L));
-    }
-  }
-  if (active == 1) return;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    const uint32_t n = atomicAdd(a.Count + (size_t)seq * a.G + g, 1u);
-    s_last = n + 1 == (uint32_t)active;
-    if (s_last) a.Count[(size_t)seq * a.G + g] = 0;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  // every split's factor exp2(m_s - M) / L, then the sums with the loads of all splits in flight
-  float *fac = os;   // [HG][kSmMaxSplits]
-#pragma unroll 1
-  for (int hh = warp; hh < HG; hh += 4) {
-    const float2 ml = lane < active ? __ldcg(reinterpret_cast<const float2 *>(base_m) + lane * HG + hh) : make_float2(-INFINITY, 0.0f);
-    const float M = warp_max(ml.x), f = fast_exp2(ml.x - M), L = warp_tree_sum(ml.y * f);
-    if (lane < kSmMaxSplits) fac[hh * kSmMaxSplits + lane] = lane < active ? f / L : 0.0f;
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int i = tid * 4; i < HG * D; i += 512) {
-    const int hh = i / D;
-    const float *p = base_p + i, *f = fac + hh * kSmMaxSplits;
-    float4 x[kSmMaxSplits], v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-    for (int s = 0; s < kSmMaxSplits; ++s) x[s] = __ldcg(reinterpret_cast<const float4 *>(p + (size_t)min(s, active - 1) * HG * D));
-#pragma unroll
-    for (int s = 0; s < kSmMaxSplits; ++s) {
-      const float w = f[s];
-      v.x = fmaf(x[s].x, w, v.x); v.y = fmaf(x[s].y, w, v.y); v.z = fmaf(x[s].z, w, v.z); v.w = fmaf(x[s].w, w, v.w);
-    }
-    put(g * HG + hh, i % D, v.x); put(g * HG + hh, i % D + 1, v.y); put(g * HG + hh, i % D + 2, v.z); put(g * HG + hh, i % D + 3, v.w);
-  }
+  step_merge<DP>(reinterpret_cast<float *>(Ks), o, m, l, HG, D, a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (D + 4),   // D + 4 keeps 16-byte alignment
+                 a.Count + (size_t)seq * a.G + g, split, a.splits, active, [](int, int) { return 0; }, end);
 }
 #define CHUNK_STEP(DP)                                                                                                  \
-  __global__ void __launch_bounds__(128) ChunkAttnStepMma##DP(const __grid_constant__ ChunkAttnStepMmaArgs a) {         \
+  __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) ChunkAttnStepMma##DP(const __grid_constant__ ChunkAttnStepMmaArgs a) { \
     pdl_launch_dependents();                                                                                            \
     chunk_step_mma_body<DP>(a);                                                                                         \
   }                                                                                                                     \
@@ -415,7 +352,7 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
     const ChunkAttnStepMmaArgs *a = (const ChunkAttnStepMmaArgs *)args;                                                 \
     return (16 + 1 + kSmStages * kCmKeys) * (DP + 8) * 2 + (a->H / a->G + 1) * a->D * 4;                                \
   }                                                                                                                     \
-  static_assert(kSmStages * kCmKeys * (DP + 8) * 2 >= 4 * 16 * DP * 4 && 16 * kSmMaxSplits <= 4 * 16 * DP, "merge buffers lie in the key tiles' place");
+  static_assert(kSmStages * kCmKeys * (DP + 8) * 2 >= 4 * 16 * (DP + 8) * 4, "the merge lies in the key tiles' place");
 CHUNK_STEP(32)
 CHUNK_STEP(64)
 CHUNK_STEP(96)

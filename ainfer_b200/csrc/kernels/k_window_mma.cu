@@ -223,7 +223,7 @@ struct WindowAttnStepMmaArgs {
   float scale, softcap, eps;
   int32_t ahead;           // LaunchAhead
 };
-constexpr int kWsStages = 2, kWsMaxSplits = 16;
+constexpr int kWsStages = 2;
 // As the chunk form, a list of one step fetches positions and the first tile (rows of earlier steps) before the dependency wait. Where
 // another layer of the same step appends the rows (koff < 0), the tile that ends in the step's own row waits.
 // Loops stay rolled: a step runs the kernel once, and a third of its stalls were on code not yet fetched (90 KB of it; with
@@ -231,8 +231,6 @@ constexpr int kWsStages = 2, kWsMaxSplits = 16;
 template <int DP>
 __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs &a) {
   extern __shared__ __align__(128) unsigned char sm_raw[];
-  __shared__ float wm[4][16], wl[4][16];
-  __shared__ int s_last;
   constexpr int LD = DP + 8;
   uint16_t *Qs = reinterpret_cast<uint16_t *>(sm_raw);                // [16][LD]
   uint16_t *kn = Qs + 16 * LD, *vn = kn + LD;                         // the new key and value [DP]
@@ -366,90 +364,36 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
     values<DP, 16>(o, s, va + off, lane);
   }
   cpa_wait<0>();
-  // ---- the four warps' shares of this block ----
-  float *os = reinterpret_cast<float *>(Ks);   // [4][16][DP], in the tiles' place
-  __syncthreads();
-#pragma unroll
-  for (int x = 0; x < 2; ++x) {
-    const int r = (lane >> 2) + 8 * x;
-    l[x] = quad_sum(l[x]);
-    if ((lane & 3) == 0) { wm[warp][r] = m[x]; wl[warp][r] = l[x]; }
-    if (r < HG)
-#pragma unroll
-      for (int d = 0; d < DP / 8; ++d) *reinterpret_cast<float2 *>(os + (warp * 16 + r) * DP + d * 8 + (lane & 3) * 2) = make_float2(o[d][2 * x], o[d][2 * x + 1]);
-  }
-  __syncthreads();
-  auto put = [&](int hh, int d, float v) {
-    const int c = (g * HG + hh) * E + d;
-    if (a.goff >= 0) v *= fast_logistic(u[a.goff + c]);
-    const size_t at = (size_t)seq * a.ldo + c;
-    if (a.out16) reinterpret_cast<uint16_t *>(a.O)[at] = f32_to_bf16(v);
-    else reinterpret_cast<float *>(a.O)[at] = v;
+  __syncthreads();   // the tiles' place is free
+  auto gates = [&](int hh, int d) {   // of the output
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (a.goff >= 0) {
+      const float *p = u + a.goff + (g * HG + hh) * E + d;
+      v = make_float4(p[0], p[1], p[2], p[3]);
+    }
+    return v;
   };
-  auto sink = [&](int hh, float M) { return a.Sink ? fast_exp2(a.Sink[g * HG + hh] * kLog2e - M) : 0.0f; };
-  // partials of a (sequence, key head): sums [splits][HG][E], then (maximum, sum) [splits][HG][2]
-  float *base_p = a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (E + 4);   // E + 4 keeps 16-byte alignment
-  float *base_m = base_p + (size_t)a.splits * HG * E;
-#pragma unroll 1
-  for (int i = tid; i < HG * E; i += 128) {
-    const int hh = i / E, d = i - hh * E;
-    const float M = fmaxf(fmaxf(wm[0][hh], wm[1][hh]), fmaxf(wm[2][hh], wm[3][hh]));
-    float v = 0.0f, L = 0.0f;
+  auto end = [&](int hh, int d, const float4 &v, float L, float M, const float4 &gate) {
+    if (a.Sink) L += fast_exp2(a.Sink[g * HG + hh] * kLog2e - M);
+    const size_t at = (size_t)seq * a.ldo + (g * HG + hh) * E + d;
+    const float r[4] = {v.x / L, v.y / L, v.z / L, v.w / L}, z[4] = {gate.x, gate.y, gate.z, gate.w};
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float f = fast_exp2(wm[w][hh] - M);
-      v = fmaf(os[(w * 16 + hh) * DP + d], f, v);
-      L = fmaf(wl[w][hh], f, L);
+    for (int e = 0; e < 4; ++e) {
+      const float w = a.goff >= 0 ? r[e] * fast_logistic(z[e]) : r[e];
+      if (a.out16) reinterpret_cast<uint16_t *>(a.O)[at + e] = f32_to_bf16(w);
+      else reinterpret_cast<float *>(a.O)[at + e] = w;
     }
-    if (active == 1) {
-      put(hh, d, v / (L + sink(hh, M)));
-    } else {
-      __stcg(base_p + (size_t)split * HG * E + i, v);
-      if (d == 0) __stcg(reinterpret_cast<float2 *>(base_m) + split * HG + hh, make_float2(M, L));
-    }
-  }
-  if (active == 1) return;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    const uint32_t c = atomicAdd(a.Count + (size_t)seq * a.G + g, 1u);
-    s_last = c + 1 == (uint32_t)active;
-    if (s_last) a.Count[(size_t)seq * a.G + g] = 0;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  // every split's factor exp2(m_s - M) / L, then the sums with the loads of all splits in flight
-  float *fac = os;   // [HG][kWsMaxSplits]
-#pragma unroll 1
-  for (int hh = warp; hh < HG; hh += 4) {
-    const float2 ml = lane < active ? __ldcg(reinterpret_cast<const float2 *>(base_m) + lane * HG + hh) : make_float2(-INFINITY, 0.0f);
-    const float M = warp_max(ml.x), f = fast_exp2(ml.x - M), L = warp_tree_sum(ml.y * f) + sink(hh, M);
-    if (lane < kWsMaxSplits) fac[hh * kWsMaxSplits + lane] = lane < active ? f / L : 0.0f;
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int i = tid * 4; i < HG * E; i += 512) {
-    const int hh = i / E;
-    const float *p = base_p + i, *f = fac + hh * kWsMaxSplits;
-    float4 x[kWsMaxSplits], v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-    for (int s = 0; s < kWsMaxSplits; ++s) x[s] = __ldcg(reinterpret_cast<const float4 *>(p + (size_t)min(s, active - 1) * HG * E));
-#pragma unroll
-    for (int s = 0; s < kWsMaxSplits; ++s) {
-      const float w = f[s];
-      v.x = fmaf(x[s].x, w, v.x); v.y = fmaf(x[s].y, w, v.y); v.z = fmaf(x[s].z, w, v.z); v.w = fmaf(x[s].w, w, v.w);
-    }
-    put(hh, i % E, v.x); put(hh, i % E + 1, v.y); put(hh, i % E + 2, v.z); put(hh, i % E + 3, v.w);
-  }
+  };
+  step_merge<DP>(reinterpret_cast<float *>(Ks), o, m, l, HG, E, a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (E + 4),   // E + 4 keeps 16-byte alignment
+                 a.Count + (size_t)seq * a.G + g, split, a.splits, active, gates, end);
 }
 #define WINDOW_STEP(DP)                                                                                              \
-  __global__ void __launch_bounds__(128) WindowAttnStepMma##DP(const __grid_constant__ WindowAttnStepMmaArgs a) {    \
+  __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) WindowAttnStepMma##DP(const __grid_constant__ WindowAttnStepMmaArgs a) { \
     pdl_launch_dependents();                                                                                         \
     window_step_mma_body<DP>(a);                                                                                     \
   }                                                                                                                  \
   static uint32_t window_step_smem##DP(const void *) { return (16 + 2 + 2 * kWsStages * kCmKeys) * (DP + 8) * 2; }   \
-  static_assert(2 * kWsStages * kCmKeys * (DP + 8) * 2 >= 4 * 16 * DP * 4 && 16 * kWsMaxSplits <= 4 * 16 * DP, "merge buffers lie in the tiles' place");
+  static_assert(2 * kWsStages * kCmKeys * (DP + 8) * 2 >= 4 * 16 * (DP + 8) * 4, "the merge lies in the tiles' place");
 WINDOW_STEP(32)
 WINDOW_STEP(64)
 WINDOW_STEP(96)

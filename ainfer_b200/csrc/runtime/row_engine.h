@@ -87,9 +87,13 @@ struct RowEngineBase : RowEngine {
   // the order of the sums, so it depends on the sequences and heads alone and not on the context that was asked for:
   // the same tokens give the same logits in a session or batch of any length. (A cut by whole rounds of blocks over the
   // keys of the longest context took 257 us against 280 for 16 sequences of Sinepel at 600, with other last bits.)
-  int step_splits(int max_kv_heads) const {
+  // Sequences side by side: one round of blocks, three an SM in the tensor-core form (its tiles and registers); what comes in a second
+  // round starts where the first one's merges end. us of a layer with 3 / 4 / 8 blocks an SM: 16 sequences of Sinepel, 2048 wide, at 600
+  // 7.8 / 7.9 / 14.1, 64 of Robopel, 2048 wide, at 700 27 / 34 / 41. The other forms multiply on the CUDA cores and keep eight.
+  int step_splits(int max_kv_heads, bool mma) const {
     if (nseq == 1) return std::max(1, std::min(16, 2 * sm_count / max_kv_heads));
-    return std::max(1, std::min(16, 8 * sm_count / (std::min(nseq, 8 * sm_count) * max_kv_heads)));
+    const int blocks = (mma ? 3 : 8) * sm_count;
+    return std::max(1, std::min(16, blocks / (std::min(nseq, blocks) * max_kv_heads)));
   }
 };
 
