@@ -51,7 +51,7 @@ struct Prefill {
   float *Qn = nullptr, *Pm = nullptr, *Pse = nullptr, *Pacc = nullptr;   // per-row attention scratch
   std::map<std::string, ainfer_kernel_t> kernels;
   // architectures with a row engine: the rows' sequence (0), its first row (0), and the rows whose logits are wanted
-  int32_t *Seq = nullptr, *First = nullptr, *Want = nullptr;
+  int32_t *Seq = nullptr, *First = nullptr;
   int logits_cap = 0;                            // rows Logits holds
 };
 
@@ -101,7 +101,7 @@ int prefill_create(Session *s, int rows_cap, bool verify, Prefill **out, int ep_
   if (s->rows) {
     p->rows_cap = std::min(rows_cap, s->rows->rows_cap);
     const size_t n = (size_t)p->rows_cap;
-    if (palloc(p, n * 4, &p->Ctrl) || palloc(p, n, &p->Seq) || palloc(p, n, &p->First) || palloc(p, n, &p->Want)) {
+    if (palloc(p, n * 5, &p->Ctrl) || palloc(p, n, &p->Seq) || palloc(p, n, &p->First)) {   // control blocks, then wanted rows
       prefill_destroy(p);
       return 1;
     }
@@ -162,35 +162,36 @@ static int row_passes(Prefill *p, const int *tokens, int n, int start_pos, const
     if (rc != AINFER_OK) s->err = ainfer_last_error(s->dev);
     return rc != AINFER_OK;
   };
-  std::vector<int32_t> ctrl((size_t)p->rows_cap * 4), rel;
+  std::vector<int32_t> ctrl;
   int w = 0;
   for (int t0 = 0; t0 < n; t0 += p->rows_cap) {
     const int rows = std::min(p->rows_cap, n - t0);
+    ctrl.resize((size_t)rows * 4);
     for (int i = 0; i < rows; ++i) {
       ctrl[4 * i] = tokens[t0 + i];
       ctrl[4 * i + 1] = start_pos + t0 + i;
       ctrl[4 * i + 2] = start_pos + t0 + i + 1;
       ctrl[4 * i + 3] = -1;
     }
-    if (failed(ainfer_memcpy_h2d(s->dev, p->Ctrl, ctrl.data(), (size_t)rows * 16))) return 1;
+    const int w0 = w;
+    while (w < n_want && want[w] < t0 + rows) ctrl.push_back(want[w++] - t0);
+    // One copy, and no wait for it: it is ordered on the queue, and pageable memory is read before the call returns. A wait for the
+    // pass before left the GPU idle until this one's first kernels were there.
+    if (failed(ainfer_memcpy_h2d_async(s->dev, p->Ctrl, ctrl.data(), ctrl.size() * 4))) return 1;
     RowSpan span;
     span.ctrl = p->Ctrl; span.seq = p->Seq; span.first = p->First;
     span.rows = rows;
-    rel.clear();
-    const int w0 = w;
-    while (w < n_want && want[w] < t0 + rows) rel.push_back(want[w++] - t0);
-    if (!rel.empty()) {
-      if (failed(ainfer_memcpy_h2d(s->dev, p->Want, rel.data(), rel.size() * 4))) return 1;
-      if (p->logits_cap < (int)rel.size()) {   // grows by whole steps: few reallocations over a session
-        p->logits_cap = std::min(p->rows_cap, ((int)rel.size() + 63) / 64 * 64);
+    if (w > w0) {
+      if (p->logits_cap < w - w0) {   // grows by whole steps: few reallocations over a session
+        p->logits_cap = std::min(p->rows_cap, (w - w0 + 63) / 64 * 64);
         if (palloc(p, (size_t)p->logits_cap * V, &p->Logits)) return 1;
       }
-      span.want = p->Want; span.n_want = (int)rel.size(); span.logits = p->Logits;
+      span.want = p->Ctrl + (size_t)rows * 4; span.n_want = w - w0; span.logits = p->Logits;
     }
     Launcher l(p);
     s->rows->emit(l, span);
     if (l.status) return l.status;
-    if (!rel.empty() && failed(ainfer_memcpy_d2h(s->dev, out + (size_t)w0 * V, p->Logits, rel.size() * V * 4))) return 1;
+    if (w > w0 && failed(ainfer_memcpy_d2h(s->dev, out + (size_t)w0 * V, p->Logits, (size_t)(w - w0) * V * 4))) return 1;
   }
   return failed(ainfer_sync(s->dev, UINT64_MAX)) ? 1 : 0;
 }
@@ -309,7 +310,7 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
       ctrl[4 * i + 2] = start_pos + t0 + i + 1;
       ctrl[4 * i + 3] = -1;
     }
-    if (ainfer_memcpy_h2d(s->dev, p->Ctrl, ctrl.data(), (size_t)rows * 16) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
+    if (ainfer_memcpy_h2d_async(s->dev, p->Ctrl, ctrl.data(), (size_t)rows * 16) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
     if (use_lists) {
       for (int L = 0; L < c.layers; ++L) {
         if (ainfer_list_execute(p->vlists[L]) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
