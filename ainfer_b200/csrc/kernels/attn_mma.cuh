@@ -123,9 +123,10 @@ __device__ __forceinline__ float quad_sum(float v) {
 // the quad). Blocks leave their share in part, sums [splits][heads][E], then (maximum, sum of weights) [splits][heads]; the last of
 // `active` to come ends the heads. A chain of latencies, so: four dimensions a thread; rows of os padded, the quads of a warp
 // store to different banks; one release and acquire, by the thread that counts, between two barriers, and the shares are read past L1
-// (two fences of all threads took 2300 cycles each, now 900 and none); maxima, sums and what before(head, dimension) loads are
-// one round of loads. In a step of 16 heads over 4 key heads at position 1500 from the last tile to the end: 8800 cycles, now
-// 6900; 16 sequences of Sinepel at 600 17.1 us a layer, 14.1 (7.8 with the blocks in one round). end(head, dimension, four values, their weights' sum and maximum, what before gave).
+// (fences of all threads took 1600 cycles with the counting and 2300 after it); maxima, sums and what before(head, dimension)
+// loads are one round of loads. In a step of 16 heads over 4 key heads at position 1500 from the last tile to the end: 8800
+// cycles, now 6900; 16 sequences of Sinepel at 600 17.1 us a layer, now 14.1 (7.8 with the blocks in one round).
+// end(head, dimension, four values, the weights' sum, the maximum, what before gave).
 constexpr int kStepMaxSplits = 16;
 __device__ __forceinline__ uint32_t count_up(uint32_t *p) {   // release and acquire on the GPU
   uint32_t n;
