@@ -121,21 +121,22 @@ __device__ __forceinline__ float quad_sum(float v) {
 // ---- the end of a decode step's attention: a block's warps, then the blocks of a (sequence, key head) ----
 // Four warps hold sums o of up to 16 heads (a thread's heads lane / 4 and 8 more) with maxima m and sums of weights l (not yet over
 // the quad). Blocks leave their share in part, sums [splits][heads][E], then (maximum, sum of weights) [splits][heads]; the last of
-// `active` to come ends the heads. A chain of latencies, so: four dimensions a thread; rows of os padded, the quads of a warp
-// store to different banks; one release and acquire, by the thread that counts, between two barriers, and the shares are read past L1
-// (fences of all threads took 1600 cycles with the counting and 2300 after it); maxima, sums and what before(head, dimension)
-// loads are one round of loads. In a step of 16 heads over 4 key heads at position 1500 from the last tile to the end: 8800
-// cycles, now 6900; 16 sequences of Sinepel at 600 17.1 us a layer, now 14.1 (7.8 with the blocks in one round).
-// end(head, dimension, four values, the weights' sum, the maximum, what before gave).
+// `active` to come ends the heads: a share's factor exp2(m_s - M) / L first, then the shares times their factors, in their order
+// (outputs travel through the layers that follow in 16 bits, so the order is part of the result). A chain of latencies, so: four
+// dimensions a thread; rows of os padded, the quads of a warp store to different banks; one release and acquire, by the
+// thread that counts, between two barriers, and the shares are read past L1 (fences of all threads took 1600 cycles with the
+// counting and 2300 after it); the shares and what before(head, dimension) loads are under way while the factors are made. us of a step: 16
+// sequences of Sinepel, four layers of 2048, at 600 280 -> 272, 64 of Robopel at 700 441 -> 434, one of Sinepel at 1500 238 -> 231.
+// sink(head, the maximum): more weight in the sum. end(head, dimension, four values, what before gave).
 constexpr int kStepMaxSplits = 16;
 __device__ __forceinline__ uint32_t count_up(uint32_t *p) {   // release and acquire on the GPU
   uint32_t n;
   asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(n) : "l"(p) : "memory");
   return n;
 }
-template <int DP, typename Before, typename End>
+template <int DP, typename Sink, typename Before, typename End>
 __device__ __forceinline__ void step_merge(float *os, const float (&o)[DP / 8][4], const float (&m)[2], float (&l)[2], int heads, int E, float *part,
-                                           uint32_t *count, int split, int splits, int active, const Before &before, const End &end) {
+                                           uint32_t *count, int split, int splits, int active, const Sink &sink, const Before &before, const End &end) {
   constexpr int LO = DP + 8;   // os: [4][16][LO]
   __shared__ float wm[4][16], wl[4][16];
   __shared__ int s_last;
@@ -165,7 +166,9 @@ __device__ __forceinline__ void step_merge(float *os, const float (&o)[DP / 8][4
       L = fmaf(wl[w][hh], f, L);
     }
     if (active == 1) {
-      end(hh, d, v, L, M, before(hh, d));
+      const auto with = before(hh, d);
+      L += sink(hh, M);
+      end(hh, d, make_float4(v.x / L, v.y / L, v.z / L, v.w / L), with);
     } else {
       __stcg(reinterpret_cast<float4 *>(part + ((size_t)split * heads + hh) * E + d), v);
       if (d == 0) __stcg(part_m + split * heads + hh, make_float2(M, L));
@@ -179,28 +182,32 @@ __device__ __forceinline__ void step_merge(float *os, const float (&o)[DP / 8][4
   }
   __syncthreads();
   if (!s_last) return;
+  static_assert(16 * kStepMaxSplits <= 4 * 16 * LO, "the factors lie in the sums' place");
+  float *fac = os;   // [16][kStepMaxSplits]
+  const int n = heads * quads;
 #pragma unroll 1
-  for (int i = tid; i < heads * quads; i += 128) {
-    const int hh = i / quads, d = (i - hh * quads) * 4;
+  for (int i0 = 0; i0 < n; i0 += 128) {
+    const int i = min(i0 + tid, n - 1), hh = i / quads, d = (i - hh * quads) * 4;
     const auto with = before(hh, d);
     float4 x[kStepMaxSplits], v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float2 ml[kStepMaxSplits];
-    float M = -INFINITY, L = 0.0f;
 #pragma unroll
-    for (int s = 0; s < kStepMaxSplits; ++s) {
-      const int at = min(s, active - 1);
-      ml[s] = __ldcg(part_m + at * heads + hh);
-      x[s] = __ldcg(reinterpret_cast<const float4 *>(part + ((size_t)at * heads + hh) * E + d));
+    for (int s = 0; s < kStepMaxSplits; ++s) x[s] = __ldcg(reinterpret_cast<const float4 *>(part + ((size_t)min(s, active - 1) * heads + hh) * E + d));
+    if (i0 == 0) {   // a lane a share, a warp a head
+#pragma unroll 1
+      for (int r = warp; r < heads; r += 4) {
+        const float2 ml = lane < active ? __ldcg(part_m + lane * heads + r) : make_float2(-INFINITY, 0.0f);
+        const float M = warp_max(ml.x), f = fast_exp2(ml.x - M), L = warp_tree_sum(ml.y * f) + sink(r, M);
+        if (lane < kStepMaxSplits) fac[r * kStepMaxSplits + lane] = lane < active ? f / L : 0.0f;
+      }
+      __syncthreads();
     }
-#pragma unroll
-    for (int s = 0; s < kStepMaxSplits; ++s) M = fmaxf(M, ml[s].x);
+    const float *f = fac + hh * kStepMaxSplits;
 #pragma unroll
     for (int s = 0; s < kStepMaxSplits; ++s) {
-      const float w = s < active ? fast_exp2(ml[s].x - M) : 0.0f;
-      L = fmaf(ml[s].y, w, L);
+      const float w = f[s];
       v.x = fmaf(x[s].x, w, v.x); v.y = fmaf(x[s].y, w, v.y); v.z = fmaf(x[s].z, w, v.z); v.w = fmaf(x[s].w, w, v.w);
     }
-    end(hh, d, v, L, M, with);
+    if (i0 + tid < n) end(hh, d, v, with);
   }
 }
 

@@ -331,9 +331,9 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
   }
   cpa_wait<0>();
   __syncthreads();   // the tiles' place is free
-  auto end = [&](int hh, int d, const float4 &v, float L, float, int) {
+  auto end = [&](int hh, int d, const float4 &v, int) {
     const size_t at = (size_t)seq * a.ldo + (size_t)(g * HG + hh) * D + d;
-    const float r[4] = {v.x / L, v.y / L, v.z / L, v.w / L};
+    const float r[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       if (a.out16) reinterpret_cast<uint16_t *>(a.O)[at + e] = f32_to_bf16(r[e]);
@@ -341,10 +341,10 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
     }
   };
   step_merge<DP>(reinterpret_cast<float *>(Ks), o, m, l, HG, D, a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (D + 4),   // D + 4 keeps 16-byte alignment
-                 a.Count + (size_t)seq * a.G + g, split, a.splits, active, [](int, int) { return 0; }, end);
+                 a.Count + (size_t)seq * a.G + g, split, a.splits, active, [](int, float) { return 0.0f; }, [](int, int) { return 0; }, end);
 }
 #define CHUNK_STEP(DP)                                                                                                  \
-  __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) ChunkAttnStepMma##DP(const __grid_constant__ ChunkAttnStepMmaArgs a) { \
+  __global__ void __launch_bounds__(128) ChunkAttnStepMma##DP(const __grid_constant__ ChunkAttnStepMmaArgs a) {         \
     pdl_launch_dependents();                                                                                            \
     chunk_step_mma_body<DP>(a);                                                                                         \
   }                                                                                                                     \

@@ -373,10 +373,10 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
     }
     return v;
   };
-  auto end = [&](int hh, int d, const float4 &v, float L, float M, const float4 &gate) {
-    if (a.Sink) L += fast_exp2(a.Sink[g * HG + hh] * kLog2e - M);
+  auto sink = [&](int hh, float M) { return a.Sink ? fast_exp2(a.Sink[g * HG + hh] * kLog2e - M) : 0.0f; };
+  auto end = [&](int hh, int d, const float4 &v, const float4 &gate) {
     const size_t at = (size_t)seq * a.ldo + (g * HG + hh) * E + d;
-    const float r[4] = {v.x / L, v.y / L, v.z / L, v.w / L}, z[4] = {gate.x, gate.y, gate.z, gate.w};
+    const float r[4] = {v.x, v.y, v.z, v.w}, z[4] = {gate.x, gate.y, gate.z, gate.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float w = a.goff >= 0 ? r[e] * fast_logistic(z[e]) : r[e];
@@ -385,10 +385,10 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
     }
   };
   step_merge<DP>(reinterpret_cast<float *>(Ks), o, m, l, HG, E, a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (E + 4),   // E + 4 keeps 16-byte alignment
-                 a.Count + (size_t)seq * a.G + g, split, a.splits, active, gates, end);
+                 a.Count + (size_t)seq * a.G + g, split, a.splits, active, sink, gates, end);
 }
 #define WINDOW_STEP(DP)                                                                                              \
-  __global__ void __launch_bounds__(128, DP <= 128 ? 3 : 1) WindowAttnStepMma##DP(const __grid_constant__ WindowAttnStepMmaArgs a) { \
+  __global__ void __launch_bounds__(128) WindowAttnStepMma##DP(const __grid_constant__ WindowAttnStepMmaArgs a) {    \
     pdl_launch_dependents();                                                                                         \
     window_step_mma_body<DP>(a);                                                                                     \
   }                                                                                                                  \

@@ -399,7 +399,6 @@ struct Engine : RowEngineBase {
     // ---- buffers of a pass ----
     size_t maxU = 1, maxQ = 1, maxA = 1, maxF = 1, maxKe = 0, maxEI = 1, maxS = 1, maxK = 1, maxHE = 1, maxHp = 0, y_rows = R, tiles = 1;
     int maxG = 1;
-    bool mma = true;
     for (const RowLayerConfig &r : c.row_layers) {
       maxA = std::max(maxA, (size_t)inner(r));
       if (r.mixer == RowLayerConfig::MINGRU) {
@@ -410,7 +409,6 @@ struct Engine : RowEngineBase {
         maxQ = std::max(maxQ, (size_t)r.heads * r.dim);
         maxHE = std::max(maxHE, (size_t)r.heads * (r.vdim + 4));
         maxG = std::max(maxG, r.kv_heads);
-        mma = mma && mma_step(r);
       }
       if (r.experts) {
         const size_t slots = R * r.top;
@@ -427,7 +425,7 @@ struct Engine : RowEngineBase {
     ldw = round_up((int)W, 8);
     ldq = round_up((int)maxA, 8);
     ldf = round_up((int)maxF, 8);
-    att_splits = step_splits(maxG, mma);
+    att_splits = step_splits(maxG);
     for (int i = 0; i < 2; ++i) e |= alloc(R * W, &X[i]);
     e |= alloc(R * ldw * esz(), &H); e |= alloc(R * maxU, &U); e |= alloc(R * maxQ * esz(), &Q);
     e |= alloc(R * ldq * 4, &Att); e |= alloc(y_rows * W, &Y); e |= alloc(R * ldf * 4, &Z);
@@ -607,14 +605,14 @@ struct Engine : RowEngineBase {
 
   // sizes the tensor-core attention takes (bf16)
   bool mma_dims(const RowLayerConfig &r) const { return !f32 && r.dim % 8 == 0 && r.vdim % 8 == 0 && std::max(r.dim, r.vdim) <= 256; }
-  bool mma_step(const RowLayerConfig &r) const { return mma_dims(r) && r.heads / r.kv_heads <= 16; }
   void attention_step(KernelCalls &k, const RowLayerConfig &r, const LayerWeights &lw, const LayerState &s, const int32_t *ctrl, int n, int ldo, bool out16) {
     const int Hd = r.heads * r.dim, Gd = r.kv_heads * r.dim, Ge = r.kv_heads * r.vdim;
     const bool own = r.kv_from < 0;
     const int koff = own ? Hd : -1, voff = Hd + Gd, goff = own ? voff + Ge : Hd;
     const Means *mn = s.means >= 0 ? &means[(size_t)s.means] : nullptr;
     const int64_t blocks = mn ? mn->blocks : 0;
-    const std::string name = mma_step(r) ? sized("WindowAttnStepMma", std::max(r.dim, r.vdim)) : std::string(f32 ? "WindowAttnStepF32" : "WindowAttnStepB16");
+    const std::string name = mma_dims(r) && r.heads / r.kv_heads <= 16 ? sized("WindowAttnStepMma", std::max(r.dim, r.vdim))
+                                                                       : std::string(f32 ? "WindowAttnStepF32" : "WindowAttnStepB16");
     k.launch(name.c_str(), (uint32_t)(n * r.kv_heads * (att_splits + 1)), (const float *)U, lw.q_norm, lw.k_norm, s.rot, ctrl, (void *)s.ring.k,
              (void *)s.ring.v, (void *)(mn ? mn->k : nullptr), (void *)(mn ? mn->v : nullptr), (int64_t)s.ring.cap * Gd, (int64_t)s.ring.cap * Ge,
              blocks * Gd, blocks * Ge, lw.sink, AttPart, AttCount, (void *)Att, (int32_t)n, (int32_t)r.heads, (int32_t)r.kv_heads, (int32_t)r.dim,

@@ -83,16 +83,14 @@ struct RowEngineBase : RowEngine {
   // lose (1500 rows, 8192 x 2048 48.1 / 49.4; 2048 x 8192 44.3 / 46.2). 32 experts of 375 rows 1024 x 2048 61.4 / 56.9,
   // 2048 x 1024 60.5 / 61.5; of 100 rows 33.8 / 34.9.
   static bool pairs_pay(int nt, long rounds, int K) { return nt >= 208 && K >= 1536 && rounds * K >= 6144; }
-  // Blocks of a step's attention per (sequence, key head). The cut decides the order of the sums, so it depends on the sequences and
-  // heads alone and not on the context that was asked for: the same tokens give the same logits in a session or batch of
-  // any length. Sequences side by side get one round of blocks, three an SM in the tensor-core form (its tiles and registers): what
-  // comes in a second round starts where the first one's merges end. us of a layer with 3 / 4 / 8 blocks an SM: 16 sequences of Sinepel,
-  // 2048 wide, at 600 7.8 / 7.9 / 14.1, 64 of Robopel, 2048 wide, at 700 27 / 34 / 41. The other forms multiply on the CUDA cores and
-  // keep eight.
-  int step_splits(int max_kv_heads, bool mma) const {
+  // Blocks of a step's attention per (sequence, key head): few tiles each when there are many sequences. The cut decides
+  // the order of the sums, so it depends on the sequences and heads alone and not on the context that was asked for:
+  // the same tokens give the same logits in a session or batch of any length. (Fewer blocks for batches, three an SM, all of them
+  // resident, took 254 us against 277 for a step of 16 sequences of Sinepel at 600 and 422 against 433 for 64 of Robopel at 700; but a
+  // batch's logits moved by 0.5 % and 1.6 %, about their distance from 64 bits, and came no nearer to it.)
+  int step_splits(int max_kv_heads) const {
     if (nseq == 1) return std::max(1, std::min(16, 2 * sm_count / max_kv_heads));
-    const int blocks = (mma ? 3 : 8) * sm_count;
-    return std::max(1, std::min(16, blocks / (std::min(nseq, blocks) * max_kv_heads)));
+    return std::max(1, std::min(16, 8 * sm_count / (std::min(nseq, 8 * sm_count) * max_kv_heads)));
   }
 };
 

@@ -277,7 +277,7 @@ struct Engine : RowEngineBase {
       ts.push_back({s.pend_shift, s.shift, nullptr, nullptr, C, 1});   // steps keep their convolution ring themselves
     }
     ldw = round_up((int)W, 8); ldq = round_up(maxQ, 8); ldf = round_up(maxF, 8);
-    att_splits = step_splits(maxG, std::all_of(c.row_layers.begin(), c.row_layers.end(), [&](const RowLayerConfig &r) { return mma_step(r); }));
+    att_splits = step_splits(maxG);
     for (int i = 0; i < 2; ++i) e |= alloc(R * S * W, &X[i]);
     e |= alloc(R * ldw * esz(), &H); e |= alloc(R * maxC, &U); e |= alloc(R * ldq * esz(), &Q);
     e |= alloc(R * ldq * 4, &Att); e |= alloc(R * W, &Y); e |= alloc(R * ldf * 4, &Act);
@@ -385,10 +385,10 @@ struct Engine : RowEngineBase {
 
   // head sizes the tensor-core attention takes (bf16)
   bool mma_dim(const RowLayerConfig &r) const { return !f32 && r.dim % 8 == 0 && r.dim <= 256; }
-  bool mma_step(const RowLayerConfig &r) const { return mma_dim(r) && r.heads / r.kv_heads <= 16; }
   void attn_step(KernelCalls &k, const RowLayerConfig &r, const RowLayerWeights &lw, const LayerState &s, const int32_t *ctrl, int n, int C, int ldo,
                  bool out16) {
-    const std::string name = mma_step(r) ? sized("ChunkAttnStepMma", r.dim) : std::string(f32 ? "ChunkAttnStepF32" : "ChunkAttnStepB16");
+    const std::string name = mma_dim(r) && r.heads / r.kv_heads <= 16 ? sized("ChunkAttnStepMma", r.dim)
+                                                                      : std::string(f32 ? "ChunkAttnStepF32" : "ChunkAttnStepB16");
     k.launch(name.c_str(), (uint32_t)(n * r.kv_heads * att_splits), (const float *)U, lw.conv, s.conv, ctrl,
              (void *)s.k, (int64_t)s.cap * r.kv_heads * r.dim, lw.lb, lw.temp, AttPart, AttCount, (void *)Att, (int32_t)n, (int32_t)r.heads,
              (int32_t)r.kv_heads, (int32_t)r.dim, (int32_t)r.taps, (int32_t)s.cap, (int32_t)s.chunk, (int32_t)lw.lb_len, (int32_t)att_splits,
