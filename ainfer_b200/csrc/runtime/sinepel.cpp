@@ -348,12 +348,13 @@ struct Engine : RowEngineBase {
         else {
           const bool tile = f32 && r.dim <= 128;   // the registers of larger heads' sums would spill
           // The keys of 32 rows over a cluster until there are three blocks an SM, all that are resident, a tile of 64 keys each at
-          // least (rows late in a chunk have the most; the pass does not know its position). us with 1, 2, 4 and 8 blocks: 777 rows, 8
-          // heads, chunk 1024 139, 86, 76, 109; 800 rows, 16 heads, chunk 2048 162, 117, 141, 206; 130 rows at position 800 156, 87, 57,
-          // 41, at 0 33, 23, 21, 24; 777 rows, chunk 64 23, 27, 44, 80.
-          const int blocks = (R + 31) / 32 * r.heads, keys = std::min(s.chunk, max_ctx);
+          // least (rows late in a chunk have the most; the pass does not know its position). By the rows, the heads and the chunk alone: the
+          // cut decides the order of the sums, and the same tokens give the same logits in a session of any length. us with 1, 2, 4
+          // and 8 blocks: 777 rows, 8 heads, chunk 1024 139, 86, 76, 109; 800 rows, 16 heads, chunk 2048 162, 117, 141, 206; 130 rows at
+          // position 800 156, 87, 57, 41, at 0 33, 23, 21, 24; 777 rows, chunk 64 23, 27, 44, 80.
+          const int blocks = (R + 31) / 32 * r.heads;
           int cl = 0;
-          while (cl < 3 && (blocks << cl) < 3 * sm_count && keys >= (128 << cl)) ++cl;
+          while (cl < 3 && (blocks << cl) < 3 * sm_count && s.chunk >= (128 << cl)) ++cl;
           static const char *const tiles[2][4] = {{"ChunkAttnTile64", "ChunkAttnTile64Split2", "ChunkAttnTile64Split4", "ChunkAttnTile64Split8"},
                                                   {"ChunkAttnTile128", "ChunkAttnTile128Split2", "ChunkAttnTile128Split4", "ChunkAttnTile128Split8"}};
           k.launch(tile ? tiles[r.dim > 64][cl] : f32 ? "ChunkAttnRowsF32" : "ChunkAttnRowsB16",

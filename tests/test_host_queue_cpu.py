@@ -1,0 +1,83 @@
+"""What the runtime queues for the device, over a device boundary on host memory (fake_device.cpp) that reads every host buffer as
+late as its interface allows. Each case is a process of its own: the boundary is chosen when the libraries are loaded."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    from ainfer_b200 import _build, cuda_abi
+    _build.build_all()
+    folder = tmp_path_factory.mktemp("fake")
+    source = open(os.path.join(ROOT, "tests", "fake_device.cpp")).read()
+    rest = "".join(f'extern "C" int {n}() {{ return 1; }}\n' for n in cuda_abi.SIGNATURES if f" {n}(" not in source and f"*{n}(" not in source)
+    (folder / "rest.cpp").write_text(rest)
+    out = str(folder / "libfake.so")
+    subprocess.run([_build._cxx(), "-shared", "-fPIC", "-O1", "-std=c++17", "-I", os.path.join(ROOT, "include"), "-o", out,
+                    os.path.join(ROOT, "tests", "fake_device.cpp"), str(folder / "rest.cpp")], check=True)
+    return out
+
+
+def run(fake, script, **env):
+    prelude = f"""
+    import ctypes, os, sys, tempfile
+    sys.path[:0] = [{ROOT!r}, {os.path.join(ROOT, "tests")!r}]
+    import numpy as np
+    from ainfer_b200 import cuda_abi
+    cuda_abi.CUDA_LIB = {fake!r}
+    from ainfer_b200 import runtime
+    L = cuda_abi.load()
+    L.fake_log.restype = ctypes.c_char_p
+    dev = cuda_abi.Device(0)
+    def log():
+        text = L.fake_log().decode()
+        L.fake_clear()
+        return [line.split() for line in text.splitlines()]
+    def open_model(arch, c=None):
+        if arch == "hybrid":
+            return runtime.Model(dev, "synth:tiny:seed=0")
+        import robopel_models, robopel_plain, sinepel_plain
+        P = sinepel_plain if arch == "sinepel" else robopel_plain
+        c = c or (P.make_config(layers=[P.make_layer()]) if arch == "sinepel" else robopel_models.MODELS["shared"])
+        with tempfile.TemporaryDirectory() as d:
+            P.write_model(d, c, P.make_weights(c, 1))
+            return runtime.Model(dev, d)
+    """
+    r = subprocess.run([sys.executable, "-c", textwrap.dedent(prelude) + textwrap.dedent(script)], capture_output=True, text=True, timeout=300,
+                       env={**os.environ, **env})
+    assert r.returncode == 0, r.stderr[-3000:]
+    return r.stdout
+
+
+@pytest.mark.parametrize("flags", ["0", "runtime.Session.F32"])
+@pytest.mark.parametrize("arch", ["sinepel", "robopel"])
+def test_launches_do_not_depend_on_the_context_asked_for(fake, arch, flags):
+    """The cut of a sum is in the kernel and its blocks: prompts and steps launch the same ones in a session that just holds
+    the tokens and in a longer one."""
+    out = run(fake, f"""
+    import robopel_plain, sinepel_plain
+    if {arch!r} == "sinepel":
+        c = sinepel_plain.make_config(max_positions=4096, layers=[sinepel_plain.make_layer(heads=8, dim=32, chunk=n) for n in (600, 100, 3000)])
+    else:
+        c = robopel_plain.make_config(layers=[robopel_plain.attention(size=600), robopel_plain.mingru(56), robopel_plain.attention(size=90, kv_from=0)])
+    model = open_model({arch!r}, c)
+    got = []
+    for ctx in (204, 256, 1000, 4096):
+        s = runtime.Session(model, ctx, {flags})
+        log()
+        for n in (1, 7, 40, 130, 200):
+            s.reset()
+            s.prefill_logits(np.arange(n) % 50, [n - 1])
+            s.step(3, n)
+        got.append([line[:2] for line in log()])
+        s.close()
+    assert all(len(g) > 50 and g == got[0] for g in got)
+    print("PASSED")
+    """)
+    assert "PASSED" in out

@@ -819,6 +819,21 @@ def test_logits_do_not_depend_on_the_context_asked_for(dev, rt, tmp_path, seqs):
     assert np.array_equal(got[0], got[1])
 
 
+def test_32_bit_prompt_does_not_depend_on_the_context_asked_for(dev, rt, tmp_path):
+    """130 rows of a chunk of 600: bit for bit the same logits in a session that just holds them and in one of more than a chunk."""
+    c = P.make_config(width=64, vocab=64, streams=2, max_positions=4096, layers=[L(heads=8, kv_heads=2, dim=32, conv=4, chunk=600, ff=64)] * 2)
+    P.write_model(str(tmp_path), c, P.make_weights(c, 4))
+    model = rt.Model(dev, str(tmp_path))
+    toks = np.random.default_rng(3).integers(0, 64, 130).astype(np.int32)
+    got = []
+    for ctx in (130, 1000):
+        s = rt.Session(model, ctx, rt.Session.F32)
+        got.append(s.prefill_logits(toks, range(130)))
+        s.close()
+    model.close()
+    assert np.array_equal(got[0], got[1])
+
+
 def test_limits_are_refused(dev, rt, tmp_path):
     c = P.make_config(max_positions=20, layers=[L()])
     P.write_model(str(tmp_path), c, P.make_weights(c, 0))
