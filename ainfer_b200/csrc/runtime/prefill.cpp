@@ -151,6 +151,24 @@ void prefill_destroy(Prefill *p) {
   delete p;
 }
 
+// The control blocks (and wanted rows) of all passes of a call, each pass's in words of its own. They are sent without a
+// wait (a wait for the pass before left the GPU idle until the next one's first kernels were there), and such a copy may read its
+// source at any time until the queue has been waited for: words are not written again, and live until then, however the call ends.
+struct PassWords {
+  ainfer_device_t dev;
+  std::vector<int32_t> words;
+  bool waited = false;
+  PassWords(ainfer_device_t d, size_t most) : dev(d) { words.reserve(most); }
+  ~PassWords() {
+    if (!waited) ainfer_sync(dev, UINT64_MAX);
+  }
+  void control(int token, int pos) {
+    for (int32_t v : {token, pos, pos + 1, -1}) words.push_back(v);
+  }
+  // Sends what was added since word `from`.
+  int send(int32_t *to, size_t from) { return ainfer_memcpy_h2d_async(dev, to, words.data() + from, (words.size() - from) * 4); }
+};
+
 // Advances the session over tokens[0..n) at positions start_pos... predictions (optional, needs a
 // verification object and n <= its rows): every row's greedy next token; the state after every
 // row is then also kept for prefill_rollback.
@@ -162,22 +180,15 @@ static int row_passes(Prefill *p, const int *tokens, int n, int start_pos, const
     if (rc != AINFER_OK) s->err = ainfer_last_error(s->dev);
     return rc != AINFER_OK;
   };
-  std::vector<int32_t> ctrl;
+  PassWords blocks(s->dev, (size_t)n * 4 + n_want);
   int w = 0;
   for (int t0 = 0; t0 < n; t0 += p->rows_cap) {
     const int rows = std::min(p->rows_cap, n - t0);
-    ctrl.resize((size_t)rows * 4);
-    for (int i = 0; i < rows; ++i) {
-      ctrl[4 * i] = tokens[t0 + i];
-      ctrl[4 * i + 1] = start_pos + t0 + i;
-      ctrl[4 * i + 2] = start_pos + t0 + i + 1;
-      ctrl[4 * i + 3] = -1;
-    }
+    const size_t from = blocks.words.size();
+    for (int i = t0; i < t0 + rows; ++i) blocks.control(tokens[i], start_pos + i);
     const int w0 = w;
-    while (w < n_want && want[w] < t0 + rows) ctrl.push_back(want[w++] - t0);
-    // One copy, and no wait for it: it is ordered on the queue, and pageable memory is read before the call returns. A wait for the
-    // pass before left the GPU idle until this one's first kernels were there.
-    if (failed(ainfer_memcpy_h2d_async(s->dev, p->Ctrl, ctrl.data(), ctrl.size() * 4))) return 1;
+    while (w < n_want && want[w] < t0 + rows) blocks.words.push_back(want[w++] - t0);
+    if (failed(blocks.send(p->Ctrl, from))) return 1;
     RowSpan span;
     span.ctrl = p->Ctrl; span.seq = p->Seq; span.first = p->First;
     span.rows = rows;
@@ -193,6 +204,7 @@ static int row_passes(Prefill *p, const int *tokens, int n, int start_pos, const
     if (l.status) return l.status;
     if (w > w0 && failed(ainfer_memcpy_d2h(s->dev, out + (size_t)w0 * V, p->Logits, (size_t)(w - w0) * V * 4))) return 1;
   }
+  blocks.waited = true;   // by what follows
   return failed(ainfer_sync(s->dev, UINT64_MAX)) ? 1 : 0;
 }
 
@@ -286,7 +298,6 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
     if (l.recording) l.cut(false);
     return l.status;
   };
-  std::vector<int32_t> ctrl((size_t)p->rows_cap * 4);
   const bool use_lists = verify && n == p->rows_cap;
   if (use_lists && p->vlists.empty()) {
     Launcher rec(p);
@@ -302,15 +313,12 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
   }
   // passes of equal size, as few as the buffers allow (several ranks: whole buffers, the ranks' calls must agree)
   const int passes = std::max(1, (n + p->rows_cap - 1) / p->rows_cap), per = ep.world > 1 ? p->rows_cap : std::max(1, (n + passes - 1) / passes);
+  PassWords blocks(s->dev, (size_t)n * 4);
   for (int t0 = 0; t0 < n; t0 += per) {
     const int rows = std::min(per, n - t0);
-    for (int i = 0; i < rows; ++i) {
-      ctrl[4 * i] = tokens[t0 + i];
-      ctrl[4 * i + 1] = start_pos + t0 + i;
-      ctrl[4 * i + 2] = start_pos + t0 + i + 1;
-      ctrl[4 * i + 3] = -1;
-    }
-    if (ainfer_memcpy_h2d_async(s->dev, p->Ctrl, ctrl.data(), (size_t)rows * 16) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
+    const size_t from = blocks.words.size();
+    for (int i = t0; i < t0 + rows; ++i) blocks.control(tokens[i], start_pos + i);
+    if (blocks.send(p->Ctrl, from) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
     if (use_lists) {
       for (int L = 0; L < c.layers; ++L) {
         if (ainfer_list_execute(p->vlists[L]) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
@@ -324,6 +332,7 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
       if (e) return e;
     }
   }
+  blocks.waited = true;   // by what follows
   if (verify) {
     if (ainfer_memcpy_d2h(s->dev, predictions, p->OutT, (size_t)n * 4) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
   } else if (ainfer_sync(s->dev, UINT64_MAX) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }

@@ -81,3 +81,45 @@ def test_launches_do_not_depend_on_the_context_asked_for(fake, arch, flags):
     print("PASSED")
     """)
     assert "PASSED" in out
+
+
+@pytest.mark.parametrize("arch", ["hybrid", "sinepel", "robopel"])
+def test_every_pass_reads_its_own_rows(fake, arch):
+    """Passes of five rows inside one call: each meets its own tokens and positions, whenever its control blocks are read."""
+    out = run(fake, f"""
+    s = runtime.Session(open_model({arch!r}), 64)
+    s.prefill_rows(5)
+    ids = np.arange(10, 33, dtype=np.int32)
+    log()
+    s.prefill(ids, start_pos=3)
+    got = [r for line in log() if line[0].startswith("Embed") for r in line[2:]]
+    assert got == [f"{{t}}@{{3 + i}}" for i, t in enumerate(ids)], got
+    if {arch!r} != "hybrid":
+        s.prefill_logits(ids, [0, 7, 8, 22])
+        got = [r for line in log() if line[0].startswith("Embed") for r in line[2:]]
+        assert got == [f"{{t}}@{{i}}" for i, t in enumerate(ids)], got
+    print("PASSED")
+    """)
+    assert "PASSED" in out
+
+
+@pytest.mark.parametrize("arch,kernel", [("hybrid", "EmbedRow"), ("sinepel", "EmbedPosRows"), ("robopel", "EmbedPosRows")])
+def test_nothing_is_queued_after_a_refused_launch(fake, arch, kernel):
+    """The third pass of a call fails: what the passes before it queued has been carried out when the call returns, so no copy reads
+    memory that the call owned."""
+    out = run(fake, f"""
+    s = runtime.Session(open_model({arch!r}), 64)
+    s.prefill_rows(5)
+    ids = np.arange(10, 33, dtype=np.int32)
+    log()
+    try:
+        s.prefill(ids)
+        print("NOT REFUSED")
+    except runtime.RuntimeError_ as e:
+        assert "refused by the test" in str(e)
+    assert L.fake_queued() == 0
+    got = [r for line in log() if line[0].startswith("Embed") for r in line[2:]]
+    assert got == [f"{{t}}@{{i}}" for i, t in enumerate(ids[:10])], got
+    print("PASSED")
+    """, FAKE_FAIL=kernel + ":3")
+    assert "PASSED" in out and "NOT" not in out
