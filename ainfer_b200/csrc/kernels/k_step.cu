@@ -1571,11 +1571,29 @@ __device__ __forceinline__ void decode_step(const DecodeStepArgs &args) {
 __global__ void __launch_bounds__(kStepThreads, 1) DecodeStep(const DecodeStepArgs args) { decode_step<false>(args); }
 __global__ void __launch_bounds__(kStepThreads, 1) DecodeStepClock(const DecodeStepArgs args) { decode_step<true>(args); }
 
+// quant_group() alone, a warp a group: its bound is checked with this.
+struct StepQuantGroupsArgs {
+  const float *X;   // [groups][128]
+  int8_t *Q;
+  float *S;
+  int32_t groups;
+};
+__global__ void __launch_bounds__(128) StepQuantGroups(const StepQuantGroupsArgs a) {
+  const int g = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (g >= a.groups) return;
+  const uint2 q = Step<false>::quant_group(reinterpret_cast<const float4 *>(a.X + (size_t)g * 128)[lane]);
+  reinterpret_cast<uint32_t *>(a.Q + (size_t)g * 128)[lane] = q.x;
+  if (lane == 0) a.S[g] = __uint_as_float(q.y);
+}
+
 static uint32_t step_smem_fn(const void *) { return (uint32_t)kStepSmemBytes; }
 
 #define F(f) AINFER_ARG(DecodeStepArgs, f)
 AINFER_REGISTER_COOP(DecodeStep, DecodeStepArgs, kStepThreads, 0, 0, step_smem_fn, F(plan), F(mode));
 AINFER_REGISTER_COOP(DecodeStepClock, DecodeStepArgs, kStepThreads, 0, 0, step_smem_fn, F(plan), F(mode));
+#undef F
+#define F(f) AINFER_ARG(StepQuantGroupsArgs, f)
+AINFER_REGISTER(StepQuantGroups, StepQuantGroupsArgs, 128, 4, 0, nullptr, F(X), F(Q), F(S), F(groups));
 #undef F
 
 }  // namespace ainfer

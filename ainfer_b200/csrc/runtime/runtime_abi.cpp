@@ -6,6 +6,7 @@
 #include "arch.h"
 #include "batch.h"
 #include "ep.h"
+#include "../common/step_plan.h"
 #include "executor.h"
 #include "host_sampler.h"
 #include "model.h"
@@ -158,6 +159,7 @@ int ainfer_session_buffer(ainfer_session_t h, const char *which, void **dptr, ui
   else if (w == "layer_out") { *dptr = s->layer_out; *bytes = s->layer_out ? (uint64_t)c.layers * c.hidden * 4 : 0; }
   else if (w == "routed") { *dptr = s->routed; *bytes = s->routed ? (uint64_t)c.layers * (c.top_k + 1) * 4 : 0; }
   else if (w == "stage_stamps") { *dptr = s->stage_stamps; *bytes = (uint64_t)s->stage_stamp_cap * 8; }
+  else if (w == "step_sync") { *dptr = s->step_sync; *bytes = s->step_sync ? (uint64_t)STEP_SYNC_WORDS * 4 : 0; }
   else if (w == "near_gap") { *dptr = s->near_gap; *bytes = s->near_gap ? (uint64_t)c.layers * 4 : 0; }
   else return set_err(2, "unknown session buffer: " + w);
   return 0;

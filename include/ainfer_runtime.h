@@ -94,7 +94,7 @@ int ainfer_session_reset(ainfer_session_t s);
  * Robopel "gru", "Kc" (rings of keys and values), "means"; and the common "logits", "ctrl", "history",
  * "layer_out"):
  * "conv", "S", "Kc", "Vc", "Ks", "Vs", "logits", "x", "ctrl", "layer_out",
- * "routed", "near_gap", "history", "stage_stamps". */
+ * "routed", "near_gap", "history", "stage_stamps", "step_sync" (persistent step: its counts). */
 int ainfer_session_buffer(ainfer_session_t s, const char *which, void **dptr, uint64_t *bytes);
 /* One token at a position; returns the greedy token (4-byte readback). */
 int ainfer_session_step(ainfer_session_t s, int token, int pos, int *out_token);

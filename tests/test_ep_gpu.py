@@ -92,6 +92,41 @@ def test_problems_of_every_cut(batch):
     ep.close(); model.close(); dev.close()
 
 
+# the cut at, above and below the rows of an expert, and counts by 64 rows beside lists cut by fewer
+@pytest.mark.parametrize("n,k,E,cut,shared", [(1, 3, 32, 1, 1), (9, 3, 40, 5, 9), (100, 11, 32, 16, 0), (130, 4, 1024, 32, 130), (744, 11, 64, 64, 744), (2048, 4, 96, 64, 7)])
+@pytest.mark.parametrize("name", ["EpGroupLocal", "EpGroupLocalCut"])
+def test_grouping_of_one_rank(name, n, k, E, cut, shared):
+    """Items by expert, their places, and the problem lists; EpGroupLocal counts the problems by its own cut, EpGroupLocalCut by 64 rows."""
+    from ainfer_b200 import cuda_abi
+    dev = cuda_abi.Device(0)
+    rng = np.random.default_rng(n)
+    p = 1.0 / (1 + np.arange(E)); p /= p.sum()
+    sel = np.stack([np.append(rng.choice(E, k, replace=False, p=p), E) for _ in range(n)]).astype(np.int32)
+    tab = (np.arange((E + 1) * 6, dtype=np.uint64) + 1) * 256           # weights' addresses: not followed here
+    items, rows = n * k, np.bincount(sel[:, :k].ravel(), minlength=E)
+    start, I, row0 = np.cumsum(rows) - rows, 128, n * k
+    want = [(e, int(start[e]) + j, min(cut, int(rows[e]) - j)) for e in range(E) for j in range(0, int(rows[e]), cut)]
+    want += [(E, row0 + j, min(cut, shared - j)) for j in range(0, shared, cut)]
+    by = cut if name == "EpGroupLocal" else 64
+    every, few = sum(-(-int(c) // by) for c in (*rows, shared)), int(((rows > 0) & (rows <= 8)).sum()) + (0 < shared <= 8)
+    dsorted, dplace, gu, gd, counts, lists = (dev.zeros(b) for b in (items * 4, items * 4, 64 * len(want), 32 * len(want), 32, 16))
+    dev.kernel(name)(1, dev.upload(sel), dev.upload(tab), dsorted, dplace, gu, gd, counts, n, k, E, I, row0, shared, cut,
+                     *([lists] if name == "EpGroupLocalCut" else []))
+    dev.sync()
+    got, place = dev.download(dsorted, items, np.int32), dev.download(dplace, items, np.int32)
+    flat = sel[:, :k].ravel()
+    assert np.array_equal(np.sort(got), np.arange(items)) and np.array_equal(got[place], np.arange(items)) and (np.diff(flat[got]) >= 0).all()
+    assert dev.download(counts, 8, np.int32).tolist() == [items, 2 * few, few, 2 * (every - few), every - few, 2 * every, every, 0]
+    if name == "EpGroupLocalCut":
+        assert dev.download(lists, 2, np.int32).tolist() == [2 * len(want), len(want)]
+    kind = np.dtype([("P", "<u8"), ("S", "<u8"), ("row0", "<i4"), ("M", "<i4"), ("col", "<i4"), ("pad", "<i4")])
+    t = tab.reshape(E + 1, 6)
+    down, gate_up = dev.download(gd, 32 * len(want), np.uint8).view(kind), dev.download(gu, 64 * len(want), np.uint8).view(kind)
+    assert [tuple(x)[:5] for x in down.tolist()] == [(int(t[e, 4]), int(t[e, 5]), r, m, 0) for e, r, m in want]
+    assert [tuple(x)[:5] for x in gate_up.tolist()] == [(int(t[e, 2 * u]), int(t[e, 2 * u + 1]), r, m, u * I) for e, r, m in want for u in (0, 1)]
+    dev.close()
+
+
 @pytest.mark.parametrize("world,n,cut", [(2, 20, 16), (4, 3, 64), (2, 40, 64), (1, 9, 5)])
 def test_kernels_of_several_ranks_one_after_the_other(world, n, cut):
     """Plan, pack, group, gather, both grouped products, scatter and combine of every rank, one rank after the other on one

@@ -315,6 +315,33 @@ def test_decode_attention_with_convolution(dev, H, G, D, chunk, taps, splits, ki
         close(got[s], want[s], 2e-5 if kind == "f32" else 2e-2)
 
 
+@pytest.mark.parametrize("H,G,D,splits", [(8, 2, 128, 16), (8, 2, 128, 12), (16, 1, 64, 16), (2, 2, 32, 5)])
+def test_decode_attention_in_many_shares(dev, H, G, D, splits):
+    """Late in a chunk: one tile of keys, as many as there are shares, and several a share; heads that fill the merge's threads and fewer."""
+    pos, chunk = [63, 64 * splits - 1, 1023, 2047, 0], 2048
+    n, C = len(pos), (H + G) * D
+    g = torch.Generator().manual_seed(splits)
+    u, cw = torch.randn(n, C, generator=g), 0.7 + 0.1 * torch.randn(C, generator=g)
+    r1, r2, temp = torch.rand(H, generator=g), torch.rand(H, generator=g) * 3, 0.5 + torch.rand(H, generator=g)
+    keys = bf16(torch.randn(n, chunk, G, D, generator=g))
+    kc = dev.upload(bits(keys))
+    part, cnt, o = dev.zeros(n * splits * H * (D + 4) * 4), dev.zeros(n * G * 4), dev.zeros(n * H * D * 4)
+    for _ in range(2):      # the counts end at zero
+        dev.kernel(_mma("ChunkAttnStepMma", D))(n * G * splits, dev.upload(f32(u)), dev.upload(f32(cw)), dev.zeros(n * C * 4), dev.upload(ctrl(pos)), kc,
+                                                chunk * G * D, _table(dev, r1, r2, chunk), dev.upload(f32(temp)), part, cnt, o, n, H, G, D, 1, chunk, chunk, chunk,
+                                                splits, C, H * D, 0, 0.3)
+    dev.sync()
+    got = dev.download(o, (n, H, D), np.float32)
+    for s, p in enumerate(pos):
+        y = (u[s] * cw).double()
+        q, k = bf16(y[:H * D]).double().reshape(H, D), keys[s, :p + 1].double()
+        k[p] = bf16(y[H * D:]).double().reshape(G, D)
+        far = (p - torch.arange(p + 1)).double()
+        for h in range(H):
+            w = torch.softmax((k[:, h // (H // G)] @ q[h]) * 0.3 * temp[h].double() - r1[h].double() * torch.log1p(r2[h].double() * far), 0)
+            close(got[s, h], w @ k[:, h // (H // G)], 2e-2)
+
+
 ACTS = {0: lambda v, cap: v, 1: lambda v, cap: torch.relu(v) ** 2, 2: lambda v, cap: P.softcap(v, cap)}
 
 
