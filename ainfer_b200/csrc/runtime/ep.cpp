@@ -143,10 +143,17 @@ struct Rec {   // appends launches to a list (none: launches at once); arguments
   }
 };
 // Rows of a problem of the experts' products when `items` (row, expert) pairs go to E experts: a unit of 16, 32 or 64
-// rows has five, four or three stages of weights in flight, and most experts should be one unit. Full preset, us of a
-// whole batch step of 64 rows (1.25 rows an expert) in problems of 64 / 32 / 16: 17430 / 16610 / 15270; of a prompt of 701
-// (13.7): 45230 / 44680 / 44890.
-int problem_rows(int items, int E) { return items <= 8 * E ? 16 : items <= 20 * E ? 32 : 64; }
+// rows has five, four or three stages of weights in flight, and most experts should be one unit. us of a layer's grouping, products and
+// quantiser in problems of 16 / 32 / 64 rows. 512 experts of 512 x 2048, ten a row, by mean rows of an expert: 2 178 / 204 / 232, 8
+// 230 / 251 / 283, 12 265 / 275 / 302, 13.7 293 / 287 / 315, 16 338 / 301 / 326. 128 experts, eight a row: 12 81 / 87 / 98, 16 96 / 91 /
+// 100, 20 118 / 96 / 106, 24 133 / 103 / 113, 30 153 / 128 / 121, 60 273 / 221 / 195; with rows that favour experts by rank^-0.7 12
+// 86 / 86 / 101, 16 99 / 104 / 102, 24 126 / 117 / 114, 30 152 / 136 / 131. Where a problem of every expert is one round of units on the
+// SMs, a second problem of some is a second round: 64 experts of 256 x 1024, four a row: 8 19.0 / 20.8 / 24.3, 10 22.6 / 21.3 / 24.6,
+// 12 23.6 / 21.6 / 25.1, 16 27.4 / 22.8 / 26.0, 20 30.2 / 28.8 / 27.1, 24 34.1 / 30.3 / 28.5.
+int problem_rows(int items, int E, int I, int sm_count) {
+  const bool one_round = 2L * E * (I / 128) <= 2L * sm_count;
+  return items <= (one_round ? 8 : 12) * E ? 16 : items <= (one_round ? 20 : 24) * E ? 32 : 64;
+}
 }  // namespace
 
 int EpMoe::create(DeviceModel *model, const void *id128, int rank_, int world_, int batch_, int flags_) {
@@ -243,7 +250,7 @@ void emit_experts(EpMoe *e, Rec &r, int front, int shared_rows, int max_rows, co
 int emit_local(EpMoe *e, Rec &r, int L, int rows) {
   if (emit_route(e, r, L, rows)) return 1;
   const ExpertW *tab = (const ExpertW *)e->m->expert_tables + (size_t)L * (e->E + 1);
-  const int items = rows * e->k, shared_rows = e->shared ? rows : 0, cut = std::min(rows, problem_rows(items, e->E));
+  const int items = rows * e->k, shared_rows = e->shared ? rows : 0, cut = std::min(rows, problem_rows(items, e->E, e->I, e->sm_count));
   r.launch("EpGroupLocalCut", 1u, (const int32_t *)e->SelIdx, tab, e->Sorted, e->ItemDest, e->GroupsGU, e->GroupsD, e->Counts, (int32_t)rows,
            (int32_t)e->k, (int32_t)e->E, (int32_t)e->I, (int32_t)e->cap, (int32_t)shared_rows, (int32_t)cut, e->Lists);
   r.launch("EpGatherLocal", (uint32_t)items, (const int8_t *)e->Q8, (const float *)e->SQ, (const int32_t *)e->Sorted, e->XQs, e->SQs, (int32_t)e->H,

@@ -68,6 +68,24 @@ def test_passes_inside_a_call_hand_the_state_on(dev, preset, n, rows):
     a.close(); b.close(); model.close()
 
 
+# 160 experts, eight a row: 12 and 24 mean rows of an expert and just above, problems of 16, 32 and 64 rows
+@pytest.mark.parametrize("n", [240, 241, 480, 481])
+def test_problems_of_more_experts_than_a_round_of_blocks(dev, tmp_path, n):
+    import json
+    from ainfer_b200 import runtime
+    f = tmp_path / "model.json"
+    f.write_text(json.dumps({**json.loads(runtime.preset_config_json("tiny")), "experts": 160, "top_k": 8, "mtp_layers": 0}))
+    model = runtime.Model(dev, f"synth:config:{f}:seed=4")
+    ids = np.random.default_rng(n).integers(0, model.config["vocab"], n).astype(np.int32)
+    a, b = runtime.Session(model, n + 8), runtime.Session(model, n + 8)
+    for i in range(n):
+        a.step(int(ids[i]), i)
+    b.prefill(ids)
+    for name, dt in STATE:
+        assert np.array_equal(a.read(name, dt), b.read(name, dt)), name
+    a.close(); b.close(); model.close()
+
+
 def test_a_long_prompt_after_a_short_one(dev):
     """Two rows, then three hundred on the same session: nothing of the smaller pass (row counts, problem lists) is met again."""
     from ainfer_b200 import runtime
