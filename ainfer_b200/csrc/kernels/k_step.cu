@@ -99,8 +99,8 @@ struct StepShared {
   unsigned long long sel_bar;   // consumers -> producer: this layer's routing is in sew[]
   int32_t sel_idx[12];
   float sel_w[12];
-  float gap, s_inv, s_m, s_sum;
-  float hmax[8], hse[8], wmax[16];
+  float gap;
+  float wmax[16];
   float av[16];
   int32_t ai[16];
   unsigned kmax[16];            // selection: each warp's largest key
@@ -242,7 +242,10 @@ static __device__ __noinline__ long long poll_late(unsigned n, long long t0) {
   return SH->fail ? -1 : t0;
 }
 // Until the count has reached `target`. One thread polls: the words themselves, polled by every thread
-// of every block, keep their own writers out (a router's 513 words took 5.5 us to arrive, against 1.1).
+// of every block, keep their own writers out (a router's 513 words took 5.5 us to arrive, against 1.1). A block that has
+// no item of the recurrence or of the attention counts itself in for that stage without waiting for the one before, so there the
+// count may be met early and the words are polled by all threads after all; a barrier (arrive<true>) is still one, as no
+// block can count more often than it has ended stages.
 static __device__ __noinline__ void await(unsigned target) {
   if (threadIdx.x == 0) {
     long long t0 = 0;
@@ -427,8 +430,8 @@ static __device__ __forceinline__ void take8(float (&x)[8], const unsigned long 
     if (ok || ((++n & 63u) == 0u && (t0 = poll_late(n, t0)) < 0)) break;
   }
 }
-// n consecutive words (16-byte aligned) into shared memory, by the whole consumer group: up to four
-// pairs a thread in flight. The caller synchronises.
+// n consecutive words (16-byte aligned) into shared memory, by the whole consumer group: two pairs
+// (four words) a thread in flight. The caller synchronises.
 static __device__ __noinline__ void gather(float *dst, const unsigned long long *src, int n, unsigned flag) {
   unsigned tries = 0;
   long long t0 = 0;
