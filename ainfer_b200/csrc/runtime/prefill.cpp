@@ -21,6 +21,7 @@
 // rolls back to the last accepted row (the INT8 cache needs no rollback: rows beyond the accepted
 // ones are overwritten before any later position reads them).
 #include <cstring>
+#include <memory>
 
 #include "arch.h"
 #include "ep.h"
@@ -156,17 +157,25 @@ void prefill_destroy(Prefill *p) {
 // source at any time until the queue has been waited for: words are not written again, and live until then, however the call ends.
 struct PassWords {
   ainfer_device_t dev;
-  std::vector<int32_t> words;
+  std::unique_ptr<int32_t[]> words;
+  size_t used = 0;
   bool waited = false;
-  PassWords(ainfer_device_t d, size_t most) : dev(d) { words.reserve(most); }
+  PassWords(ainfer_device_t d, size_t most) : dev(d), words(new int32_t[most]) {}
   ~PassWords() {
     if (!waited) ainfer_sync(dev, UINT64_MAX);
   }
-  void control(int token, int pos) {
-    for (int32_t v : {token, pos, pos + 1, -1}) words.push_back(v);
+  void controls(const int *tokens, int pos, int rows) {
+    int32_t *w = words.get() + used;
+    for (int i = 0; i < rows; ++i, w += 4) {
+      w[0] = tokens[i];
+      w[1] = pos + i;
+      w[2] = pos + i + 1;
+      w[3] = -1;
+    }
+    used += (size_t)rows * 4;
   }
   // Sends what was added since word `from`.
-  int send(int32_t *to, size_t from) { return ainfer_memcpy_h2d_async(dev, to, words.data() + from, (words.size() - from) * 4); }
+  int send(int32_t *to, size_t from) { return ainfer_memcpy_h2d_async(dev, to, words.get() + from, (used - from) * 4); }
 };
 
 // Advances the session over tokens[0..n) at positions start_pos... predictions (optional, needs a
@@ -184,10 +193,10 @@ static int row_passes(Prefill *p, const int *tokens, int n, int start_pos, const
   int w = 0;
   for (int t0 = 0; t0 < n; t0 += p->rows_cap) {
     const int rows = std::min(p->rows_cap, n - t0);
-    const size_t from = blocks.words.size();
-    for (int i = t0; i < t0 + rows; ++i) blocks.control(tokens[i], start_pos + i);
+    const size_t from = blocks.used;
+    blocks.controls(tokens + t0, start_pos + t0, rows);
     const int w0 = w;
-    while (w < n_want && want[w] < t0 + rows) blocks.words.push_back(want[w++] - t0);
+    while (w < n_want && want[w] < t0 + rows) blocks.words[blocks.used++] = want[w++] - t0;
     if (failed(blocks.send(p->Ctrl, from))) return 1;
     RowSpan span;
     span.ctrl = p->Ctrl; span.seq = p->Seq; span.first = p->First;
@@ -316,8 +325,8 @@ int prefill_run(Prefill *p, const int *tokens, int n, int start_pos, int *predic
   PassWords blocks(s->dev, (size_t)n * 4);
   for (int t0 = 0; t0 < n; t0 += per) {
     const int rows = std::min(per, n - t0);
-    const size_t from = blocks.words.size();
-    for (int i = t0; i < t0 + rows; ++i) blocks.control(tokens[i], start_pos + i);
+    const size_t from = blocks.used;
+    blocks.controls(tokens + t0, start_pos + t0, rows);
     if (blocks.send(p->Ctrl, from) != AINFER_OK) { s->err = ainfer_last_error(s->dev); return 1; }
     if (use_lists) {
       for (int L = 0; L < c.layers; ++L) {
