@@ -127,7 +127,7 @@ __device__ __forceinline__ float quad_sum(float v) {
 // thread that counts, between two barriers, and the shares are read past L1 (fences of all threads took 1600 cycles with the
 // counting and 2300 after it); the shares and what before(head, dimension) loads are under way while the factors are made. us of a step: 16
 // sequences of Sinepel, four layers of 2048, at 600 280 -> 272, 64 of Robopel at 700 441 -> 434, one of Sinepel at 1500 238 -> 231.
-// sink(head): more weight in the sum, as its base-2 logarithm. end(head, dimension, four values, what before gave).
+// sink(head, the maximum): more weight in the sum. end(head, dimension, four values, what before gave).
 constexpr int kStepMaxSplits = 16;
 __device__ __forceinline__ uint32_t count_up(uint32_t *p) {   // release and acquire on the GPU
   uint32_t n;
@@ -167,7 +167,7 @@ __device__ __forceinline__ void step_merge(float *os, const float (&o)[DP / 8][4
     }
     if (active == 1) {
       const auto with = before(hh, d);
-      L += fast_exp2(sink(hh) - M);
+      L += sink(hh, M);
       end(hh, d, make_float4(v.x / L, v.y / L, v.z / L, v.w / L), with);
     } else {
       __stcg(reinterpret_cast<float4 *>(part + ((size_t)split * heads + hh) * E + d), v);
@@ -194,18 +194,17 @@ __device__ __forceinline__ void step_merge(float *os, const float (&o)[DP / 8][4
     for (int s = 0; s < kStepMaxSplits; ++s) x[s] = __ldcg(reinterpret_cast<const float4 *>(part + ((size_t)min(s, active - 1) * heads + hh) * E + d));
     if (i0 == 0) {   // a lane a share, a warp every fourth head
       float2 ml[4];
-      float more[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int r = min(warp + 4 * u, heads - 1);
-        ml[u] = lane < active ? __ldcg(part_m + lane * heads + r) : make_float2(-INFINITY, 0.0f);
-        more[u] = sink(r);
+        const int r = warp + 4 * u;
+        ml[u] = r < heads && lane < active ? __ldcg(part_m + lane * heads + r) : make_float2(-INFINITY, 0.0f);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int r = warp + 4 * u;
-        const float M = warp_max(ml[u].x), f = fast_exp2(ml[u].x - M), L = warp_tree_sum(ml[u].y * f) + fast_exp2(more[u] - M);
-        if (r < heads && lane < kStepMaxSplits) fac[r * kStepMaxSplits + lane] = lane < active ? f / L : 0.0f;
+        if (r >= heads) break;
+        const float M = warp_max(ml[u].x), f = fast_exp2(ml[u].x - M), L = warp_tree_sum(ml[u].y * f) + sink(r, M);
+        if (lane < kStepMaxSplits) fac[r * kStepMaxSplits + lane] = lane < active ? f / L : 0.0f;
       }
       __syncthreads();
     }

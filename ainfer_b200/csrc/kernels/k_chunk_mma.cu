@@ -341,7 +341,7 @@ __device__ __forceinline__ void chunk_step_mma_body(const ChunkAttnStepMmaArgs &
     }
   };
   step_merge<DP>(reinterpret_cast<float *>(Ks), o, m, l, HG, D, a.Part + ((size_t)seq * a.G + g) * a.splits * HG * (D + 4),   // D + 4 keeps 16-byte alignment
-                 a.Count + (size_t)seq * a.G + g, split, a.splits, active, [](int) { return -INFINITY; }, [](int, int) { return 0; }, end);
+                 a.Count + (size_t)seq * a.G + g, split, a.splits, active, [](int, float) { return 0.0f; }, [](int, int) { return 0; }, end);
 }
 #define CHUNK_STEP(DP)                                                                                                  \
   __global__ void __launch_bounds__(128) ChunkAttnStepMma##DP(const __grid_constant__ ChunkAttnStepMmaArgs a) {         \

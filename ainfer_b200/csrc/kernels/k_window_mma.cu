@@ -373,7 +373,7 @@ __device__ __forceinline__ void window_step_mma_body(const WindowAttnStepMmaArgs
     }
     return v;
   };
-  auto sink = [&](int hh) { return a.Sink ? a.Sink[g * HG + hh] * kLog2e : -INFINITY; };
+  auto sink = [&](int hh, float M) { return a.Sink ? fast_exp2(a.Sink[g * HG + hh] * kLog2e - M) : 0.0f; };
   auto end = [&](int hh, int d, const float4 &v, const float4 &gate) {
     const size_t at = (size_t)seq * a.ldo + (g * HG + hh) * E + d;
     const float r[4] = {v.x, v.y, v.z, v.w}, z[4] = {gate.x, gate.y, gate.z, gate.w};
